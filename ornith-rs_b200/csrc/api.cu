@@ -111,12 +111,8 @@ int32_t orn_ctx_destroy(orn_ctx* ctx) {
   if (ctx->t0) cudaEventDestroy(ctx->t0);
   if (ctx->t1) cudaEventDestroy(ctx->t1);
   cudaFree(ctx->dev_err);
-  cudaFree(ctx->split_partial_side);
-  cudaFree(ctx->split_arrivals_side);
-  cudaFree(ctx->split_partial);
   cudaFree(ctx->attn_partial);
   cudaFree(ctx->attn_arrivals);
-  cudaFree(ctx->split_arrivals);
   if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
@@ -430,7 +426,7 @@ int32_t orn_gather_gemv(orn_ctx* ctx, const orn_linear* lin, const uint16_t* dev
 
 int32_t orn_gemm(orn_ctx* ctx, const orn_linear* lin, const uint16_t* dev_x, int32_t M, void* dev_y, int32_t out_f32) {
   if (!ctx || !lin || !dev_x || !dev_y || M < 1) return ORN_ERR_ARG;
-  return f_qgemm(ctx, ctx->stream, lin, dev_x, M, dev_y, lin->O, nullptr, nullptr, out_f32);
+  return f_qgemm(ctx, ctx->stream, lin, dev_x, M, dev_y, lin->O, nullptr, out_f32);
 }
 
 int32_t orn_gemm_multi(orn_ctx* ctx, const orn_linear* const* lins, int32_t n, const uint16_t* x, int32_t M,
@@ -441,7 +437,7 @@ int32_t orn_gemm_multi(orn_ctx* ctx, const orn_linear* const* lins, int32_t n, c
     if (!lins[j] || !ys[j]) return ORN_ERR_ARG;
     ld[j] = lins[j]->O;
   }
-  return f_qgemm_multi(ctx, ctx->stream, lins, ys, ld, n, x, M, nullptr, nullptr, out_f32, 0);
+  return f_qgemm_multi(ctx, ctx->stream, lins, ys, ld, n, x, M, nullptr, out_f32);
 }
 
 int32_t orn_gather_gemm(orn_ctx* ctx, const orn_linear* lin, const uint16_t* dev_x, const uint32_t* dev_lhs,
@@ -452,16 +448,15 @@ int32_t orn_gather_gemm(orn_ctx* ctx, const orn_linear* lin, const uint16_t* dev
   const size_t seg_b = ((size_t)(2 * lin->E + 2) * sizeof(int) + 255) & ~(size_t)255;
   const size_t perm_b = ((size_t)rows * sizeof(uint32_t) + 255) & ~(size_t)255;
   const size_t xs_b = ((size_t)rows * lin->K * sizeof(bf16_t) + 255) & ~(size_t)255;
-  const size_t sc_b = qgemm_scratch_bytes(rows, lin->E, lin->O);
   uint8_t* buf = nullptr;
-  CK(orn_alloc(ctx, seg_b + perm_b + xs_b + sc_b, (void**)&buf));
+  CK(orn_alloc(ctx, seg_b + perm_b + xs_b, (void**)&buf));
   int* seg = reinterpret_cast<int*>(buf);
   uint32_t* perm = reinterpret_cast<uint32_t*>(buf + seg_b);
   bf16_t* xs = reinterpret_cast<bf16_t*>(buf + seg_b + perm_b);
   int rc = f_route_sort(ctx, s, dev_rhs, rows, lin->E, seg, seg + lin->E + 1, perm);
   if (rc == ORN_OK) rc = f_gather_rows(ctx, s, dev_x, dev_lhs, perm, rows, lin->K, xs);
   QGemmGroup g{seg, perm, 0};
-  if (rc == ORN_OK) rc = f_qgemm(ctx, s, lin, xs, rows, dev_y, lin->O, &g, buf + seg_b + perm_b + xs_b, out_f32);
+  if (rc == ORN_OK) rc = f_qgemm(ctx, s, lin, xs, rows, dev_y, lin->O, &g, out_f32);
   if (rc == ORN_OK) rc = orn_sync(ctx);
   else cudaStreamSynchronize(s);
   cudaFree(buf);

@@ -13,28 +13,33 @@
 // the B operand, D[feature, token] = sum_k W[feature, k] x[token, k]: the tensor core's M is always
 // a full 128 features, its N is the token-tile width BN (16..256), so a launch with few tokens per
 // expert (a routed prompt chunk, a batched decode step) wastes no tensor-core work on padding.
-//   - a CTA owns (feature tile of 128, up to NT token tiles) and keeps NT accumulators of
-//     128 x BN float32 in tensor memory (NT * BN <= 512 columns);
-//   - per block of 64 weights along K: one warp's elected lane brings the NT token tiles
-//     [BN, 64] bf16 and the raw bytes of the 128 x 64 weight tile with TMA (cp.async.bulk.tensor.2d,
-//     this GPU's memory, no multicast); eight (or four) warps dequantise the tile (one thread per
-//     feature row: Q4_K / Q6_K / affine-8 / affine-4 -> bf16) and store it with tcgen05.st into TENSOR
-//     MEMORY, where the MMA takes its A operand from (row = lane, two bf16 per column): a 16 KB tile
-//     per K block neither crosses shared memory twice nor needs a proxy fence (bf16 weights land in
-//     shared memory swizzled and are read from there); another elected lane issues 4 * NT tcgen05.mma
-//     (128 x BN x 16, kind::f16, bf16 inputs, f32 accumulate) and commits the stage back to the
-//     producers;
-//   - the eight dequantising warps then read the accumulators (tcgen05.ld, one TMEM lane = one
-//     feature per thread), round to bfloat16 and store y[token, feature].
-// Stages are a ring guarded by mbarriers; every wait is bounded and reports through the context's
-// device error flag, and the CTA frees its tensor memory on every path.
+// One persistent CTA per SM walks work items (feature tile of 128, up to BN tokens, a range of K);
+// its warps have fixed roles and meet only at mbarriers:
+//   warp 0        TMA of the raw weight bytes, one super-block (256 weights along K) of the 128 rows
+//                 per slot: the scales of a super-block are fetched once, rows arrive as 128-byte
+//                 swizzled boxes that the dequantising threads read without bank conflicts
+//   warp 2        TMA of the token tiles [BN, 64] (and of bf16 weights)
+//   warps 8..15   dequantise: two groups of four warps, a group owns every second unit of two K blocks
+//                 (128 weights a thread: one feature row), stores them with tcgen05.st into TENSOR MEMORY,
+//                 where the MMA takes its A operand from, and hands the unit over with one arrival per
+//                 warp.  Fewer, longer steps won over sixteen warps of one K block each (154 -> 118 us for
+//                 1024 routed Q4_K rows): a hand-over costs a warp several hundred cycles of waiting
+//                 whatever it carries, and with 128 registers the conversions of a step interleave
+//   warp 1        issues 4 tcgen05.mma (128 x BN x 16, bf16 in, f32 accumulate) per K block and one
+//                 commit per unit: a commit occupies the issuing thread for about 160 cycles, twice
+//                 what the four MMAs of a block take
+//   warps 4..7    epilogue: accumulators (two buffers where they fit) to registers, round, store
+// bf16 weights need no dequantisation: their box lands swizzled in shared memory and the MMA reads it
+// there (8 warps).  Every wait is bounded and reports through the context's device error flag, and
+// the CTA frees its tensor memory on every path.
 //
 // The grouped form serves rows sorted by expert (counting_sort + switch_glu_rows,
-// src/ops/moe.rs:283-314,463-508): a small plan kernel turns the experts' row ranges into work
-// items (expert, first row, rows, feature tile) and persistent CTAs walk that list.
+// src/ops/moe.rs:283-314,463-508): every CTA derives the work items (expert, rows, feature tile) from
+// the experts' row ranges at its start.
 #include <cuda.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -50,44 +55,50 @@ namespace {
 
 constexpr int BM = 128;            // features per tile: the tensor core's M
 constexpr int BK = 64;             // weights per K block: one 128-byte swizzle row of bf16
-// warp 0: TMA, warp 1: MMA, then DQW warps that dequantise and run the epilogue: 8 (two threads per
-// feature row of a tile) for launches with one or two CTAs per SM, 4 (one thread per row) for
-// launches of narrow items, where up to four small CTAs share an SM
-constexpr int gemm_threads(int dqw) { return 64 + 32 * dqw; }
-constexpr uint32_t kAccColsMax = 384;   // accumulator columns of an item: the rest of tensor memory holds weight tiles
+constexpr int kDqGroups = 2, kDqWarps = 8;
+constexpr int kSB = 4;          // K blocks of a super-block (256 weights), the step of the raw ring
+constexpr int U = 2;            // K blocks of a unit, the step of the ring the MMA reads
+constexpr int gemm_threads(bool direct) { return direct ? 256 : 256 + 32 * kDqWarps; }
 constexpr uint32_t kWCols = BK / 2;     // tensor-memory columns of one dequantised 128 x 64 tile (two bf16 per column)
-constexpr int kSplitMaxRows = 512;                      // dense products up to this many rows may split K
-constexpr size_t kSplitPartialBytes = (size_t)64 << 20;  // f32 partials of one launch
-constexpr size_t kSplitTiles = 4096;                     // arrival counters
+constexpr int kSplitMaxRows = 512;      // dense products up to this many rows may split K
+constexpr int kMaxSplit = 8;            // = the portable cluster size: the splits of a tile are one cluster
 constexpr uint32_t kWTileBytes = BM * BK * 2;
-constexpr int kMaxIn = 12;  // IN ring slots (raw weight boxes + token tiles)
-constexpr int kMaxW = 4;    // W ring slots (dequantised weight tile)
+constexpr int kMaxRaw = 8;  // raw ring slots (super-blocks)
+constexpr int kMaxUnits = 8; // units of the ring the MMA reads (token tiles + dequantised weight tiles)
+constexpr int kMaxE = 1024;     // experts of the grouped form
+constexpr int kItemCache = 256; // work items a CTA lays out at its start (later ones are derived one by one)
+constexpr int kStageLd = BM + 8;  // elements between the rows of the epilogue's staging tile
+constexpr uint32_t kGemmSmem = 209 * 1024;     // dynamic shared memory a CTA may take
 constexpr uint32_t kGemmWaitLimit = 1u << 16;  // try_wait rounds (each may sleep kGemmHintNs)
 constexpr uint32_t kGemmHintNs = 20000;
 
-constexpr int kMaxJobs = 4;  // matrices of one dense launch (projections that share their input rows)
+constexpr int kMaxJobs = 4;  // matrices of one launch (projections that share their input rows)
 struct GemmJob {
   int O, tile0;        // output features; first feature tile of this matrix in the launch's tile space
   int ldy;             // elements between output rows
   bf16_t* y;
   float* y_f32;        // non-null: float32 output instead of bfloat16
+  int vec8;            // y may be stored eight bfloat16 at a time
 };
 struct GemmParams {
   int njobs;
   GemmJob job[kMaxJobs];
-  const int4* items;   // grouped: {expert, first row, rows, feature tile}; null = dense
-  const int* n_items;  // grouped: device count
-  int dense_items;     // dense: feature tiles x token groups
+  const int* seg;      // grouped: expert e owns sorted rows seg[e] .. seg[e+1]-1; null = dense
+  int E;
+  int dense_tiles;     // dense: feature tiles x token groups
   int rows;            // rows of x (dense) / of the sorted row space (grouped)
   int K;
   const uint32_t* row_map;   // nullable: output row of sorted row p
-  int BN, NT, stages /*IN ring*/, w_stages /*W ring*/, f_tiles;
-  uint32_t stage_bytes;
-  uint32_t tmem_cols;  // power of two >= acc_cols + the W ring's columns (and >= 32): what the CTA takes of tensor memory
-  uint32_t acc_cols;   // NT * BN rounded up to 32: the accumulators; the dequantised weight tiles follow
-  int splits;          // dense products over few rows: an item is one of `splits` ranges of the K blocks of a tile
-  float* partial;      // [tile][split][token][128 features] f32 partial sums of the split items
-  int* arrivals;       // [tile] how many splits of the tile have stored their partial (the last one reduces)
+  int BN, f_tiles;
+  int raw_slots, units;      // slots of the raw ring, units of the MMA's ring
+  uint32_t raw_bytes;        // bytes of one raw slot
+  int nacc;                  // sets of accumulators (2 where they fit beside the weight ring)
+  uint32_t acc_cols;         // columns of one accumulator
+  uint32_t tmem_cols;        // power of two: what the CTA takes of tensor memory
+  // dense products over few rows sum their K blocks in `splits` ranges of `per` blocks, each range in an
+  // accumulator of its own, the ranges then in order: `seq` of them one after the other in a CTA, the
+  // CTAs of a cluster of splits / seq side by side
+  int splits, seq, per;
   int* err;
 };
 
@@ -114,6 +125,19 @@ ORN_D bool mbar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+ORN_D bool mbar_test(uint32_t bar, uint32_t parity) {  // does not suspend
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // bounded wait: false (and the error flag set) when the phase never completes
 ORN_D bool mbar_wait(uint32_t bar, uint32_t parity, int* err) {
   for (uint32_t it = 0; it < kGemmWaitLimit; ++it)
@@ -130,18 +154,53 @@ ORN_D void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint3
 ORN_D void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 ORN_D void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 ORN_D void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// The MMA warp runs its loop with all 32 lanes and one elected lane issues: operands stay in uniform
+// registers (a lane-0 branch costs about 100 cycles per instruction in register moves).
 ORN_D void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// D[tmem] (+)= A[smem] * B[smem]^T, 128 x N x 16, bf16 in, f32 out
-ORN_D void tc_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(bar)
+      : "memory");
+}
+// one K block: D[tmem] (+)= A[smem] * B[smem]^T, four times 128 x N x 16, bf16 in, f32 out; `add` = 0
+// starts a new sum
+ORN_D void tc_mma_block(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t add) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e, p;\n"
+      ".reg .b64 a1, a2, a3, b1, b2, b3;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "add.u64 a1, %1, 2;\nadd.u64 a2, %1, 4;\nadd.u64 a3, %1, 6;\n"
+      "add.u64 b1, %2, 2;\nadd.u64 b2, %2, 4;\nadd.u64 b3, %2, 6;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n"
       "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(add)
+      : "memory");
+}
+// the same with A in tensor memory: 128 lanes x 8 columns (16 bf16 of K per row) per step
+ORN_D void tc_mma_block_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t add) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e, p;\n"
+      ".reg .b32 a1, a2, a3;\n"
+      ".reg .b64 b1, b2, b3;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "add.u32 a1, %1, 8;\nadd.u32 a2, %1, 16;\nadd.u32 a3, %1, 24;\n"
+      "add.u64 b1, %2, 2;\nadd.u64 b2, %2, 4;\nadd.u64 b3, %2, 6;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, 1;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, 1;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, 1;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(add)
       : "memory");
 }
 // shared-memory operand descriptor: K-major, 128-byte swizzle, rows of 128 bytes, groups of 8 rows
@@ -166,21 +225,14 @@ ORN_D void tmem_st16(uint32_t taddr, const uint32_t* v) {
       : "memory");
 }
 ORN_D void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// D[tmem] (+)= A[tmem] * B[smem]^T: A is 128 lanes x 8 columns (16 bf16 of K per row)
-ORN_D void tc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 ORN_D uint4 lds128(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+ORN_D uint2 lds64(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
   return v;
 }
 ORN_D uint32_t lds32(uint32_t addr) {
@@ -193,27 +245,24 @@ ORN_D uint32_t lds16(uint32_t addr) {
   asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(addr));
   return v;
 }
-// Four code bytes of a word -> two words of two bfloat16 each, w = a * q + b per byte q, in two
-// packed fused multiply-adds on the code word itself: a code byte dropped into a float's bit
-// pattern IS a float that is linear in the code.
-//   * codes below 128 go into the third byte of 0x3F000000, already shifted left by s bits so that
-//     they fill the byte's top (s = 3 for 4-bit codes, 1 for 6-bit ones): the float is
-//     0.5 + (q << s) / 256, hence w = (a 2^(8-s)) * F + (b - a 2^(7-s)); both constants are exact
-//     up to one float32 rounding of b - a 2^(7-s), which is of the size of w itself;
-//   * 8-bit codes go into the second byte of 0x47000000: the float is 32768 + q and
-//     w = a * F + (b - 32768 a), whose constant carries an error of a / 512 at most (far below the
-//     bfloat16 rounding of an affine weight, which is of the size of 64 a).
-// This path agrees with the mat-vec to rounding, not bit for bit.
-template <int I>  // top-aligned code bytes I and I + 1 of w as a packed pair of floats
-ORN_D uint64_t code_pair_hi(uint32_t w) {
-  // selector nibbles, result byte 3..0: magic byte 3 (0x3F), code byte, magic bytes 1 and 0 (0)
-  return pk2(__uint_as_float(__byte_perm(w, 0x3F000000u, 0x7054 + 256 * I)),
-             __uint_as_float(__byte_perm(w, 0x3F000000u, 0x7054 + 256 * (I + 1))));
+// Codes to floats.  The integer (ALU) pipe is what bounds the dequantising warps: it takes a warp
+// instruction every two cycles, the FMA pipe one per cycle.  So a code is never widened on the ALU:
+// one logic op (or byte permute) drops TWO codes into the mantissas of a pair of halves, and the mixed
+// add f32 = f16 + f32 (one FMA-pipe instruction) turns each into the exact float the product wants.
+//   0x6400 | q           is the half 1024 + q   (q in bits 0..3 or a whole byte)
+//   0x5400 | (q << 4)    is the half   64 + q   (q in bits 4..7)
+// The scale then needs one packed fma per two weights and one conversion packs the bfloat16 pair: 1.1
+// ALU instructions per 4-bit weight instead of 2, 1.0 instead of 1.5 per 8-bit weight (the grouped
+// Q4_K product of 1024 routed rows: 140 -> 112 us).
+ORN_D float add_lo(uint32_t h2, float c) {  // low half of h2 + c
+  float d;
+  asm("{\n.reg .b16 l, h;\nmov.b32 {l, h}, %1;\nadd.rn.f32.f16 %0, l, %2;\n}\n" : "=f"(d) : "r"(h2), "f"(c));
+  return d;
 }
-template <int I>  // 8-bit code bytes I and I + 1 of w as the packed pair (32768 + q_I, 32768 + q_I+1)
-ORN_D uint64_t code_pair_8(uint32_t w) {
-  return pk2(__uint_as_float(__byte_perm(w, 0x47000000u, 0x7604 + 16 * I)),
-             __uint_as_float(__byte_perm(w, 0x47000000u, 0x7604 + 16 * (I + 1))));
+ORN_D float add_hi(uint32_t h2, float c) {
+  float d;
+  asm("{\n.reg .b16 l, h;\nmov.b32 {l, h}, %1;\nadd.rn.f32.f16 %0, h, %2;\n}\n" : "=f"(d) : "r"(h2), "f"(c));
+  return d;
 }
 ORN_D uint32_t bf2_of(uint64_t p) {  // packed pair of floats -> two bfloat16, the first in the low half
   uint32_t r;
@@ -226,83 +275,125 @@ ORN_D uint32_t bf2_of(uint64_t p) {  // packed pair of floats -> two bfloat16, t
       : "l"(p));
   return r;
 }
-template <bool kEightBit>
-ORN_D void codes4_bf(uint32_t w, uint64_t a2, uint64_t b2, uint32_t& o0, uint32_t& o1) {
-  o0 = bf2_of(ffma2(a2, kEightBit ? code_pair_8<0>(w) : code_pair_hi<0>(w), b2));
-  o1 = bf2_of(ffma2(a2, kEightBit ? code_pair_8<2>(w) : code_pair_hi<2>(w), b2));
+ORN_D uint64_t fmul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
-// (w >> sh) << up for every byte's field, as one rotation (the bits that wrap land outside the mask)
-ORN_D uint32_t field_up(uint32_t w, int sh, int up) { return __funnelshift_r(w, w, (sh - up) & 31); }
+ORN_D uint32_t mask_or(uint32_t w, uint32_t mask, uint32_t magic) { return (w & mask) | magic; }  // one LOP3
 
-// The raw bytes of a K block arrive by TMA as boxes of [128 rows x 16 / 32 / 64 bytes] cut out of
-// the row records (no swizzle: row r of a box is at r * box bytes).  A thread dequantises HALF of
-// one feature row's K block: 32 weights -> 16 words of two bfloat16 each, in K order (word w of the
-// half = weights 2w, 2w + 1), which become 16 tensor-memory columns of the row's lane.
+// The raw bytes of a super-block (4 K blocks, 256 weights along K) of 128 rows arrive by TMA as boxes
+// cut out of the row records.  Code boxes are 128 (or 64) bytes wide and swizzled, so that the 8 rows
+// that a quarter of a warp reads with one 16-byte load each lie in different banks; scale boxes of 16
+// bytes per row need no swizzle.  Bytes past the end of a record (the last, partial super-block) hold
+// the next field or the fill value and are never converted.
 //
-// Raw tile layout per format (byte offsets inside the stage's raw area) and the record offsets
-// (x coordinates, multiples of 16) the boxes are cut at, for K block kb (b = kb / 4):
-//   Q4_K  [0, 4096)      codes, box 32:   x = b*128 + (kb&3)*32
-//         [4096, 6144)   header, box 16:  x = b0 + b*16
-//   Q6_K  [0, 8192)      ql, box 64:      x = b*192 + 64*half128          (half128 = (kb>>1)&1)
-//         [8192, 12288)  qh, box 32:      x = b*192 + 128 + 32*half128
-//         [12288, 14336) scales, box 16:  x = b0 + b*16
-//         [14336, 16384) d, box 16:       x = b0 + b1 + ((2b) & ~15)
-//   A8    [0, 8192)      codes, box 64:   x = kb*64
-//         [8192, 10240)  {scale,bias}, box 16: x = b0 + ((4kb) & ~15)
-//   A4    [0, 4096)      codes, box 32:   x = kb*32
-//         [4096, 6144)   {scale,bias}, box 16: x = b0 + ((8kb) & ~15)
+// Slot layout per format and the record offsets (x coordinates, multiples of 16) the boxes are cut at,
+// for super-block sb:
+//   Q4_K  [0, 16384)      codes, box 128 swizzled:   x = sb*128
+//         [16384, 18432)  header, box 16:            x = b0 + sb*16
+//   Q6_K  [0, 16384)      ql, box 128 swizzled:      x = sb*192
+//         [16384, 24576)  qh, box 64 swizzled:       x = sb*192 + 128
+//         [24576, 26624)  scales, box 16:            x = b0 + sb*16
+//         [26624, 28672)  d, box 16:                 x = b0 + b1 + ((2 sb) & ~15)
+//   A8    [0, 32768)      codes, 2 boxes 128 sw.:    x = sb*256, sb*256 + 128
+//         [32768, 34816)  {scale,bias}, box 16:      x = b0 + sb*16
+//   A4    [0, 16384)      codes, box 128 swizzled:   x = sb*128
+//         [16384, 20480)  {scale,bias}, box 32:      x = b0 + sb*32
 //   BF16  none: the [128 x 64] bf16 box lands in the MMA tile itself (128-byte swizzle)
+//
+// A thread holds the raw bytes of one row and of a pair of K blocks (g = 0: the super-block's first two,
+// 1: its last two) in registers: load() reads them, convert() turns them into 64 words of two bfloat16
+// each, in K order, 16 words (= 16 tensor-memory columns of the row's lane) at a time through st(h, words).
+struct WeightMaps {
+  CUtensorMap wide;   // row records as bytes [E*O, rec], box [128 rows, 128 bytes], 128-byte swizzle (bf16: [E*O, K] bf16, box [128, 64])
+  CUtensorMap mid;    // Q6_K: box [128, 64], 64-byte swizzle
+  CUtensorMap scale;  // box [128, 16] (A4: 32)
+};
+ORN_D uint4 lds_sw128(uint32_t base, int r, int c) { return lds128(base + r * 128 + (((uint32_t)c ^ ((uint32_t)r & 7u)) << 4)); }
+ORN_D uint4 lds_sw64(uint32_t base, int r, int c) { return lds128(base + r * 64 + (((uint32_t)c ^ (((uint32_t)r >> 1) & 3u)) << 4)); }
+
 template <int KIND> struct Fmt;
 
 template <> struct Fmt<ORN_BF16> {
-  static constexpr uint32_t kRawBytes = 0;
-  ORN_D static void issue(const CUtensorMap*, const CUtensorMap*, const CUtensorMap*, const CUtensorMap* wsw, const RecGeom&,
-                          int kb, int row, uint32_t raw, uint32_t wtile, uint32_t bar) {
-    tma_load_2d(raw, wsw, kb * BK, row, bar);
+  static constexpr uint32_t kRawBytes = kWTileBytes;
+  struct Raw {};
+  ORN_D static void issue(const WeightMaps& m, const RecGeom&, int kb, int row, uint32_t raw, uint32_t bar) {
+    tma_load_2d(raw, &m.wide, kb * BK, row, bar);
   }
-  static constexpr uint32_t kTxBytes = kWTileBytes;
-  ORN_D static void convert(uint32_t, int, int, int, uint32_t*, const RecGeom&) {}
+  ORN_D static void load(Raw&, uint32_t, int, int, int) {}
+  template <class St> ORN_D static void convert(const Raw&, int, St) {}
 };
 
 // affine 8-bit, group 64: w = scale * q + bias (one fma, as the embedding lookup computes it)
 template <> struct Fmt<ORN_A8> {
-  static constexpr uint32_t kRawBytes = 10240, kTxBytes = 8192 + 2048;
-  ORN_D static void issue(const CUtensorMap* m64, const CUtensorMap*, const CUtensorMap* m16, const CUtensorMap*, const RecGeom& g,
-                          int kb, int row, uint32_t raw, uint32_t, uint32_t bar) {
-    tma_load_2d(raw, m64, kb * 64, row, bar);
-    tma_load_2d(raw + 8192, m16, (int)g.b0 + ((4 * kb) & ~15), row, bar);
+  static constexpr uint32_t kRawBytes = 32768 + 2048;
+  struct Raw { uint4 c[8]; uint2 sb; };
+  ORN_D static void issue(const WeightMaps& m, const RecGeom& g, int sb, int row, uint32_t raw, uint32_t bar) {
+    tma_load_2d(raw, &m.wide, sb * 256, row, bar);
+    tma_load_2d(raw + 16384, &m.wide, sb * 256 + 128, row, bar);
+    tma_load_2d(raw + 32768, &m.scale, (int)g.b0 + sb * 16, row, bar);
   }
-  ORN_D static void convert(uint32_t raw, int r, int kb, int half, uint32_t* out, const RecGeom&) {
-    const uint4 q0 = lds128(raw + r * 64 + half * 32), q1 = lds128(raw + r * 64 + half * 32 + 16);
-    const uint32_t sb = lds32(raw + 8192 + r * 16 + ((4 * kb) & 15));
-    const float sc = bf_lo(sb), bi = fmaf(-32768.0f, sc, bf_hi(sb));
-    const uint64_t a2 = pk2(sc, sc), b2 = pk2(bi, bi);
-    const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+  ORN_D static void load(Raw& R, uint32_t raw, int r, int g, int) {
+    R.sb = lds64(raw + 32768 + r * 16 + 8 * g);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) codes4_bf<true>(w[i], a2, b2, out[2 * i], out[2 * i + 1]);
+    for (int i = 0; i < 8; ++i) R.c[i] = lds_sw128(raw + 16384 * g, r, i);
+  }
+  template <class St> ORN_D static void convert(const Raw& R, int, St st) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      // w = sc * (32768 + q) + (bias - 32768 sc)
+      const uint32_t sb = h < 2 ? R.sb.x : R.sb.y;
+      const float sc = bf_lo(sb), bi = fmaf(-32768.0f, sc, bf_hi(sb));
+      const uint64_t a2 = pk2(sc, sc), b2 = pk2(bi, bi);
+      const uint4 q0 = R.c[2 * h], q1 = R.c[2 * h + 1];
+      const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+      uint32_t out[16];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t h01 = __byte_perm(w[i], 0x64646464u, 0x4140), h23 = __byte_perm(w[i], 0x64646464u, 0x4342);
+        out[2 * i] = bf2_of(ffma2(a2, pk2(add_lo(h01, 31744.0f), add_hi(h01, 31744.0f)), b2));
+        out[2 * i + 1] = bf2_of(ffma2(a2, pk2(add_lo(h23, 31744.0f), add_hi(h23, 31744.0f)), b2));
+      }
+      st(h, out);
+    }
   }
 };
 
 // affine 4-bit, group 32: half a K block is one group; byte b holds weights 2b (low nibble), 2b+1 (high)
 template <> struct Fmt<ORN_A4> {
-  static constexpr uint32_t kRawBytes = 6144, kTxBytes = 4096 + 2048;
-  ORN_D static void issue(const CUtensorMap*, const CUtensorMap* m32, const CUtensorMap* m16, const CUtensorMap*, const RecGeom& g,
-                          int kb, int row, uint32_t raw, uint32_t, uint32_t bar) {
-    tma_load_2d(raw, m32, kb * 32, row, bar);
-    tma_load_2d(raw + 4096, m16, (int)g.b0 + ((8 * kb) & ~15), row, bar);
+  static constexpr uint32_t kRawBytes = 16384 + 4096;
+  struct Raw { uint4 c[4], sb; };
+  ORN_D static void issue(const WeightMaps& m, const RecGeom& g, int sb, int row, uint32_t raw, uint32_t bar) {
+    tma_load_2d(raw, &m.wide, sb * 128, row, bar);
+    tma_load_2d(raw + 16384, &m.scale, (int)g.b0 + sb * 32, row, bar);
   }
-  ORN_D static void convert(uint32_t raw, int r, int kb, int half, uint32_t* out, const RecGeom&) {
-    const uint4 q = lds128(raw + r * 32 + half * 16);
-    const uint32_t sb = lds32(raw + 4096 + r * 16 + ((8 * kb) & 15) + 4 * half);
-    const float sc = bf_lo(sb), a32 = 32.0f * sc, bi = fmaf(-16.0f, sc, bf_hi(sb));
-    const uint64_t a2 = pk2(a32, a32), b2 = pk2(bi, bi);
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+  ORN_D static void load(Raw& R, uint32_t raw, int r, int g, int) {
+    R.sb = lds128(raw + 16384 + r * 32 + 16 * g);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {  // one word = 8 weights = 4 words of bfloat16 pairs (low nibble first)
-      const uint32_t l4 = field_up(w[c], 0, 3) & 0x78787878u, h4 = field_up(w[c], 4, 3) & 0x78787878u;
-      // weights 2b, 2b + 1 = (low, high) nibble of byte b: interleave the two nibble words bytewise
-      codes4_bf<false>(__byte_perm(l4, h4, 0x5140), a2, b2, out[4 * c], out[4 * c + 1]);
-      codes4_bf<false>(__byte_perm(l4, h4, 0x7362), a2, b2, out[4 * c + 2], out[4 * c + 3]);
+    for (int i = 0; i < 4; ++i) R.c[i] = lds_sw128(raw, r, 4 * g + i);
+  }
+  template <class St> ORN_D static void convert(const Raw& R, int, St st) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      // w = sc * (16 + q) + (bias - 16 sc)
+      const uint32_t sb = h == 0 ? R.sb.x : h == 1 ? R.sb.y : h == 2 ? R.sb.z : R.sb.w;
+      const float sc = bf_lo(sb), bi = fmaf(-16.0f, sc, bf_hi(sb));
+      const uint64_t a2 = pk2(sc, sc), b2 = pk2(bi, bi);
+      const uint4 q = R.c[h];
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+      uint32_t out[16];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {  // one word = 8 weights = 4 words of bfloat16 pairs (low nibble first)
+        const uint32_t w8 = w[c] >> 8;
+        const uint32_t l02 = mask_or(w[c], 0x000F000Fu, 0x64006400u), h02 = mask_or(w[c], 0x00F000F0u, 0x54005400u);
+        const uint32_t l13 = mask_or(w8, 0x000F000Fu, 0x64006400u), h13 = mask_or(w8, 0x00F000F0u, 0x54005400u);
+        out[4 * c] = bf2_of(ffma2(a2, pk2(add_lo(l02, -1008.0f), add_lo(h02, -48.0f)), b2));
+        out[4 * c + 1] = bf2_of(ffma2(a2, pk2(add_lo(l13, -1008.0f), add_lo(h13, -48.0f)), b2));
+        out[4 * c + 2] = bf2_of(ffma2(a2, pk2(add_hi(l02, -1008.0f), add_hi(h02, -48.0f)), b2));
+        out[4 * c + 3] = bf2_of(ffma2(a2, pk2(add_hi(l13, -1008.0f), add_hi(h13, -48.0f)), b2));
+      }
+      st(h, out);
     }
   }
 };
@@ -311,358 +402,514 @@ template <> struct Fmt<ORN_A4> {
 // half of the K block), high nibbles sub-block 2i+1 (the second half); w = (d * sc) * q - dmin * m,
 // evaluated as one fma per weight (this path agrees with the mat-vec to rounding, not bit for bit)
 template <> struct Fmt<ORN_Q4K> {
-  static constexpr uint32_t kRawBytes = 6144, kTxBytes = 4096 + 2048;
-  ORN_D static void issue(const CUtensorMap*, const CUtensorMap* m32, const CUtensorMap* m16, const CUtensorMap*, const RecGeom& g,
-                          int kb, int row, uint32_t raw, uint32_t, uint32_t bar) {
-    tma_load_2d(raw, m32, (kb >> 2) * 128 + (kb & 3) * 32, row, bar);
-    tma_load_2d(raw + 4096, m16, (int)g.b0 + (kb >> 2) * 16, row, bar);
+  static constexpr uint32_t kRawBytes = 16384 + 2048;
+  struct Raw { uint4 c[4], hdr; };
+  ORN_D static void issue(const WeightMaps& m, const RecGeom& g, int sb, int row, uint32_t raw, uint32_t bar) {
+    tma_load_2d(raw, &m.wide, sb * 128, row, bar);
+    tma_load_2d(raw + 16384, &m.scale, (int)g.b0 + sb * 16, row, bar);
   }
-  ORN_D static void convert(uint32_t raw, int r, int kb, int half, uint32_t* out, const RecGeom&) {
-    const uint4 qa = lds128(raw + r * 32), qb = lds128(raw + r * 32 + 16), hdr = lds128(raw + 4096 + r * 16);
-    const float d = h2f((uint16_t)(hdr.x & 0xffff)), dmin = h2f((uint16_t)(hdr.x >> 16));
-    float sc, m;
-    q4k_scale_min(2 * (kb & 3) + half, hdr.y, hdr.z, hdr.w, &sc, &m);
-    const float a = d * sc, a32 = 32.0f * a, nb = fmaf(-16.0f, a, -(dmin * m));
-    const uint64_t a2 = pk2(a32, a32), b2 = pk2(nb, nb);
-    const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-    const int sh = 4 * half;
+  ORN_D static void load(Raw& R, uint32_t raw, int r, int g, int) {
+    R.hdr = lds128(raw + 16384 + r * 16);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) codes4_bf<false>(field_up(w[i], sh, 3) & 0x78787878u, a2, b2, out[2 * i], out[2 * i + 1]);
+    for (int i = 0; i < 4; ++i) R.c[i] = lds_sw128(raw, r, 4 * g + i);
   }
-};
-
-// Q6_K (kernels/q6k.metal:47-77): per 128 weights, byte l of ql / qh gives q1 (weight l), q2 (l + 32),
-// q3 (l + 64), q4 (l + 96); a K block of 64 is (q1, q2) or (q3, q4) of one half-block, this thread's
-// half of it one of the two code sets; w = (d * sc) * (q - 32)
-template <> struct Fmt<ORN_Q6K> {
-  static constexpr uint32_t kRawBytes = 16384, kTxBytes = 8192 + 4096 + 2048 + 2048;
-  ORN_D static void issue(const CUtensorMap* m64, const CUtensorMap* m32, const CUtensorMap* m16, const CUtensorMap*,
-                          const RecGeom& g, int kb, int row, uint32_t raw, uint32_t, uint32_t bar) {
-    const int b = kb >> 2, half128 = (kb >> 1) & 1;
-    tma_load_2d(raw, m64, b * 192 + 64 * half128, row, bar);
-    tma_load_2d(raw + 8192, m32, b * 192 + 128 + 32 * half128, row, bar);
-    tma_load_2d(raw + 12288, m16, (int)g.b0 + b * 16, row, bar);
-    tma_load_2d(raw + 14336, m16, (int)(g.b0 + g.b1) + ((2 * b) & ~15), row, bar);
-  }
-  ORN_D static void convert(uint32_t raw, int r, int kb, int set, uint32_t* out, const RecGeom&) {
-    const int b = kb >> 2, half128 = (kb >> 1) & 1, hi = kb & 1;
-    const uint4 l0 = lds128(raw + r * 64 + 32 * set), l1 = lds128(raw + r * 64 + 32 * set + 16);
-    const uint4 h0 = lds128(raw + 8192 + r * 32), h1 = lds128(raw + 8192 + r * 32 + 16);
-    const uint32_t sc2 = lds16(raw + 12288 + r * 16 + 8 * half128 + 4 * hi + 2 * set);
-    const float d = h2f((uint16_t)lds16(raw + 14336 + r * 16 + ((2 * b) & 15)));
-    const float s0 = d * (float)(int8_t)(sc2 & 0xff), s1 = d * (float)(int8_t)(sc2 >> 8);
-    // w = s (q - 32) = 128 s (0.5 + q / 128) - 96 s
-    const uint64_t a20 = pk2(128.0f * s0, 128.0f * s0), a21 = pk2(128.0f * s1, 128.0f * s1);
-    const uint64_t b20 = pk2(-96.0f * s0, -96.0f * s0), b21 = pk2(-96.0f * s1, -96.0f * s1);
-    const uint32_t lw[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-    const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-    const int hs = 2 * set + 4 * hi;  // bit position of this code set's two high bits in qh
-    const int ls = 4 * hi;
+  template <class St> ORN_D static void convert(const Raw& R, int g, St st) {
+    const float d = h2f((uint16_t)(R.hdr.x & 0xffff)), dmin = h2f((uint16_t)(R.hdr.x >> 16));
+    // 6-bit scales and minima of sub-blocks 4 g .. 4 g + 3, a byte each (g is the same for the whole warp)
+    uint32_t sc4, mn4;
+    if (g == 0) { sc4 = R.hdr.y & 0x3F3F3F3Fu; mn4 = R.hdr.z & 0x3F3F3F3Fu; }
+    else {
+      sc4 = (R.hdr.w & 0x0F0F0F0Fu) | ((R.hdr.y >> 2) & 0x30303030u);
+      mn4 = ((R.hdr.w >> 4) & 0x0F0F0F0Fu) | ((R.hdr.z >> 2) & 0x30303030u);
+    }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const uint32_t q = (field_up(lw[i], ls, 1) & 0x1E1E1E1Eu) | (field_up(hw[i], hs, 5) & 0x60606060u);  // code << 1
-      codes4_bf<false>(q, i < 4 ? a20 : a21, i < 4 ? b20 : b21, out[2 * i], out[2 * i + 1]);
+    for (int h = 0; h < 4; ++h) {
+      // w = (d sc) * (16 + q) + (-16 d sc - dmin m)
+      const float a = d * (float)((sc4 >> (8 * h)) & 0xffu), nb = fmaf(-16.0f, a, -(dmin * (float)((mn4 >> (8 * h)) & 0xffu)));
+      const uint64_t a2 = pk2(a, a), b2 = pk2(nb, nb);
+      const uint32_t mask = h & 1 ? 0x00F000F0u : 0x000F000Fu, magic = h & 1 ? 0x54005400u : 0x64006400u;
+      const float c = h & 1 ? -48.0f : -1008.0f;
+      const uint4 q0 = R.c[h & 2], q1 = R.c[(h & 2) + 1];
+      const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+      uint32_t out[16];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t h02 = mask_or(w[i], mask, magic), h13 = mask_or(w[i] >> 8, mask, magic);
+        out[2 * i] = bf2_of(ffma2(a2, pk2(add_lo(h02, c), add_lo(h13, c)), b2));
+        out[2 * i + 1] = bf2_of(ffma2(a2, pk2(add_hi(h02, c), add_hi(h13, c)), b2));
+      }
+      st(h, out);
     }
   }
 };
 
-struct Item {
-  int e, tok0, ntok, ft;
-  int kb0, kb1;  // K blocks of this item
-  int tile, split;
-  int job;       // which matrix of the launch (ft counts inside it)
-};
-ORN_D bool get_item(const GemmParams& P, int w, int n_items, Item& it) {
-  if (w >= n_items) return false;
-  if (P.items != nullptr) {
-    const int4 v = P.items[w];
-    it.e = v.x; it.tok0 = v.y; it.ntok = v.z; it.ft = v.w;
-    it.kb0 = 0; it.kb1 = P.K / BK; it.tile = w; it.split = 0; it.job = 0;
-    while (it.job + 1 < P.njobs && it.ft >= P.job[it.job + 1].tile0) ++it.job;
-    it.ft -= P.job[it.job].tile0;
-  } else {
-    const int tile = w / P.splits;
-    const int g = tile / P.f_tiles;
-    it.e = 0;
-    it.ft = tile - g * P.f_tiles;
-    it.job = 0;
-    while (it.job + 1 < P.njobs && it.ft >= P.job[it.job + 1].tile0) ++it.job;
-    it.ft -= P.job[it.job].tile0;
-    it.tok0 = g * P.NT * P.BN;
-    it.ntok = min(P.NT * P.BN, P.rows - it.tok0);
-    const int KB = P.K / BK, per = (KB + P.splits - 1) / P.splits;
-    it.tile = tile; it.split = w - tile * P.splits;
-    it.kb0 = it.split * per; it.kb1 = min(KB, it.kb0 + per);
+// Q6_K (kernels/q6k.metal:47-77): per 128 weights, byte l of ql / qh gives q1 (weight l), q2 (l + 32),
+// q3 (l + 64), q4 (l + 96); the pair of K blocks is one such half-block: the first takes the low nibbles
+// of ql (q1, q2), the second the high ones (q3, q4); w = (d * sc) * (q - 32)
+template <> struct Fmt<ORN_Q6K> {
+  static constexpr uint32_t kRawBytes = 16384 + 8192 + 2048 + 2048;
+  struct Raw { uint4 l[4], h[2]; uint2 sc; uint32_t d; };
+  ORN_D static void issue(const WeightMaps& m, const RecGeom& g, int sb, int row, uint32_t raw, uint32_t bar) {
+    tma_load_2d(raw, &m.wide, sb * 192, row, bar);
+    tma_load_2d(raw + 16384, &m.mid, sb * 192 + 128, row, bar);
+    tma_load_2d(raw + 24576, &m.scale, (int)g.b0 + sb * 16, row, bar);
+    tma_load_2d(raw + 26624, &m.scale, (int)(g.b0 + g.b1) + ((2 * sb) & ~15), row, bar);
   }
-  return true;
+  ORN_D static void load(Raw& R, uint32_t raw, int r, int g, int sb) {
+    R.d = lds16(raw + 26624 + r * 16 + ((2 * sb) & 15));
+    R.sc = lds64(raw + 24576 + r * 16 + 8 * g);   // the half-block's eight sub-block scales
+#pragma unroll
+    for (int i = 0; i < 4; ++i) R.l[i] = lds_sw128(raw, r, 4 * g + i);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) R.h[i] = lds_sw64(raw + 16384, r, 2 * g + i);
+  }
+  template <class St> ORN_D static void convert(const Raw& R, int, St st) {
+    const float d = h2f((uint16_t)R.d);
+    const uint32_t hw[8] = {R.h[0].x, R.h[0].y, R.h[0].z, R.h[0].w, R.h[1].x, R.h[1].y, R.h[1].z, R.h[1].w};
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {  // code set h: nibble h >> 1 of ql bytes 32 (h & 1) .., bits 2 h of qh
+      const uint32_t s2 = (h < 2 ? R.sc.x : R.sc.y) >> (16 * (h & 1));
+      const float s0 = d * (float)(int8_t)(s2 & 0xff), s1 = d * (float)(int8_t)((s2 >> 8) & 0xff);
+      // w = s * (q - 32), exact in float32 (18 + 6 bits)
+      const uint64_t a20 = pk2(s0, s0), a21 = pk2(s1, s1);
+      const uint4 l0 = R.l[2 * (h & 1)], l1 = R.l[2 * (h & 1) + 1];
+      const uint32_t lw[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+      uint32_t out[16];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t hb = h == 0 ? hw[i] << 4 : h == 1 ? hw[i] << 2 : h == 2 ? hw[i] : hw[i] >> 2;
+        const uint32_t q = ((h >= 2 ? lw[i] >> 4 : lw[i]) & 0x0F0F0F0Fu) | (hb & 0x30303030u);
+        const uint32_t h01 = __byte_perm(q, 0x64646464u, 0x4140), h23 = __byte_perm(q, 0x64646464u, 0x4342);
+        const uint64_t a2 = i < 4 ? a20 : a21;
+        out[2 * i] = bf2_of(fmul2(a2, pk2(add_lo(h01, -1056.0f), add_hi(h01, -1056.0f))));
+        out[2 * i + 1] = bf2_of(fmul2(a2, pk2(add_lo(h23, -1056.0f), add_hi(h23, -1056.0f))));
+      }
+      st(h, out);
+    }
+  }
+};
+
+// One work item: 128 feature rows starting at weight row `wrow`, ntok tokens from tok0, K blocks kb0..kb1-1
+struct Item {
+  int wrow, tok0, ntok, job, ft, kb0, kb1;
+};
+ORN_D int4 pack_item(const Item& it) {
+  return make_int4(it.wrow, it.tok0, it.ntok | (it.job << 12) | (it.ft << 16), it.kb0 | (it.kb1 << 16));
+}
+ORN_D Item unpack_item(const int4& v) {
+  return Item{v.x, v.y, v.z & 0xfff, (v.z >> 12) & 3, (int)((uint32_t)v.z >> 16), v.w & 0xffff, (int)((uint32_t)v.w >> 16)};
+}
+// item w of the launch (off: the experts' first items, grouped form only)
+ORN_D Item derive_item(const GemmParams& P, int w, int split /*rank in the cluster*/, const int* off) {
+  Item it;
+  int e = 0, ft;
+  const int KB = P.K / BK;
+  if (off != nullptr) {
+    int lo = 0, hi = P.E;  // off[lo] <= w < off[hi]
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (off[mid] <= w) lo = mid; else hi = mid;
+    }
+    e = lo;
+    const int in = w - off[e], g = in / P.f_tiles;
+    ft = in - g * P.f_tiles;
+    it.tok0 = P.seg[e] + g * P.BN;
+    it.ntok = min(P.BN, P.seg[e + 1] - it.tok0);
+    it.kb0 = 0; it.kb1 = KB;
+  } else {
+    const int g = w / P.f_tiles;
+    ft = w - g * P.f_tiles;
+    it.tok0 = g * P.BN;
+    it.ntok = min(P.BN, P.rows - it.tok0);
+    it.kb0 = split * P.seq * P.per; it.kb1 = min(KB, it.kb0 + P.seq * P.per);
+  }
+  it.job = 0;
+  while (it.job + 1 < P.njobs && ft >= P.job[it.job + 1].tile0) ++it.job;
+  it.ft = ft - P.job[it.job].tile0;
+  it.wrow = e * P.job[it.job].O + it.ft * BM;
+  return it;
 }
 
-struct WeightMaps {
-  CUtensorMap w64;  // row records as bytes [E*O, rec], boxes [128, 64] / [128, 32] / [128, 16], no swizzle
-  CUtensorMap w32;
-  CUtensorMap w16;
-  CUtensorMap wsw;  // bf16 weights only: [E*O, K] bf16, box [128, 64], 128-byte swizzle
-};
+ORN_D uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+ORN_D void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+ORN_D void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+ORN_D uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// 16 bytes into another CTA's shared memory; its barrier counts them as they land
+ORN_D void push_f4(uint32_t dst, const uint32_t* v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "r"(v[0]), "r"(v[1]),
+               "r"(v[2]), "r"(v[3]), "r"(bar)
+               : "memory");
+}
+
 struct GemmMaps {
   CUtensorMap x;    // tokens [rows, K] bf16, box [BN, 64], 128-byte swizzle
   WeightMaps w[kMaxJobs];
 };
 
-// Two rings per CTA.  The IN ring in shared memory (deep: TMA latency is a few thousand cycles) holds
-// what TMA brings per K block: the raw weight boxes and the token tiles.  The W ring in tensor memory
-// (two or three slots of 32 columns behind the accumulators) holds the dequantised weight tile the
-// MMAs read as their A operand.  bf16 weights need no dequantisation: their box lands swizzled in the
-// IN ring and the MMAs read it there (A from shared memory).
-//   landed[i]   TMA boxes of IN slot i arrived            (producer's expect_tx)
-//   full[w]     W slot w dequantised                       (one arrival per dequantising warp)
-//   in_free[i]  the MMAs that read IN slot i are done      (tcgen05.commit)
-//   w_free[w]   the MMAs that read W slot w are done       (tcgen05.commit)
-template <int KIND, int DQW>
-__global__ void __launch_bounds__(gemm_threads(DQW), DQW == 4 ? 4 : 1) k_qgemm(const __grid_constant__ GemmMaps maps, GemmParams P) {
+// Barriers (every ring position is counted from the CTA's first K block on):
+//   raw_full[i]  the boxes of raw slot i arrived            (producer's expect_tx)
+//   raw_free[i]  every dequantising warp has read slot i    (one arrival per warp)
+//   full[u]      the unit's token tiles landed and its weight tiles are in tensor memory (expect_tx + one arrival per
+//                warp of the group that owns the unit)
+//   free[u]      the MMAs that read unit slot u are done (tcgen05.commit)
+//   acc_full[b]  accumulator b is complete (commit);  acc_free[b]  the epilogue has read it
+//   part_full    split-K: the partial sums of this CTA's share of the tokens have arrived from the whole cluster
+template <int KIND>
+__global__ void __launch_bounds__(gemm_threads(KIND == ORN_BF16), 1) k_qgemm(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmParams P) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t s_bar[2 * kMaxIn + 2 * kMaxW + 2];
+  __shared__ __align__(8) uint64_t s_bar[2 * kMaxRaw + 2 * kMaxUnits + 5];
+  __shared__ int4 s_items[kItemCache];
+  __shared__ int s_off[kMaxE + 1];
+  __shared__ __align__(16) bf16_t s_stage[2][16][kStageLd];
   __shared__ uint32_t s_tmem;
-  __shared__ int s_last;  // split-K: this CTA stored the last partial of its tile and reduces it
   using F = Fmt<KIND>;
   constexpr bool kDirect = KIND == ORN_BF16;  // the MMA reads the weight box where TMA put it
-  constexpr uint32_t kInRaw = kDirect ? kWTileBytes : F::kRawBytes;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t smem0 = (smem_addr(smem_raw) + 1023u) & ~1023u;  // swizzled tiles want 1024-byte alignment
-  const int SI = P.stages, SW = P.w_stages;
-  const uint32_t in0 = smem0;
-  const uint32_t bar_landed = smem_addr(&s_bar[0]), bar_in_free = smem_addr(&s_bar[kMaxIn]);
-  const uint32_t bar_full = smem_addr(&s_bar[2 * kMaxIn]), bar_w_free = smem_addr(&s_bar[2 * kMaxIn + kMaxW]);
-  const uint32_t bar_acc_full = smem_addr(&s_bar[2 * kMaxIn + 2 * kMaxW]), bar_acc_empty = bar_acc_full + 8;
+  const int RS = P.raw_slots;
+  const int NU = P.units;
+  const uint32_t x_bytes = (uint32_t)P.BN * 128u;
+  const uint32_t raw0 = smem0, x0 = raw0 + (uint32_t)RS * P.raw_bytes;
+  const uint32_t part0 = x0 + (uint32_t)(U * NU) * x_bytes;  // split-K: where the cluster's partial sums arrive
+  const uint32_t b0 = smem_addr(s_bar);
+  const uint32_t raw_full = b0, raw_free = b0 + 8 * kMaxRaw, full = b0 + 16 * kMaxRaw, free_ = full + 8 * kMaxUnits;
+  const uint32_t acc_full = free_ + 8 * kMaxUnits, acc_free = acc_full + 16, part_full = acc_free + 16;
+  const bool grouped = P.seg != nullptr;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < SI; ++i) {
-      mbar_init(bar_landed + 8 * i, 1);
-      mbar_init(bar_in_free + 8 * i, 1);
+    for (int i = 0; i < (kDirect ? 0 : RS); ++i) {
+      mbar_init(raw_full + 8 * i, 1);
+      mbar_init(raw_free + 8 * i, kDqWarps);
     }
-    for (int i = 0; i < SW; ++i) {
-      mbar_init(bar_full + 8 * i, DQW);
-      mbar_init(bar_w_free + 8 * i, 1);
+    for (int i = 0; i < NU; ++i) {
+      mbar_init(full + 8 * i, kDirect ? 1 : 1 + kDqWarps / kDqGroups);
+      mbar_init(free_ + 8 * i, 1);
     }
-    mbar_init(bar_acc_full, 1);
-    mbar_init(bar_acc_empty, DQW);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(acc_full + 8 * i, 1);
+      mbar_init(acc_free + 8 * i, 4);
+    }
+    mbar_init(part_full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
   }
   __syncwarp();
-  if (warp == 0) {  // tensor memory: the columns of one item's accumulators (two CTAs of a narrow launch share an SM)
+  if (warp == 3) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)), "r"(P.tmem_cols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  // ---- the CTA's work items
+  int n_items;
+  if (grouped) {
+    // items before expert e: its predecessors' started groups of BN rows times the feature tiles
+    for (int e = threadIdx.x; e < P.E; e += blockDim.x) s_off[e + 1] = (P.seg[e + 1] - P.seg[e] + P.BN - 1) / P.BN * P.f_tiles;
+    __syncthreads();
+    if (warp == 0) {
+      int carry = 0;
+      for (int e0 = 0; e0 < P.E; e0 += 32) {
+        int v = e0 + lane < P.E ? s_off[e0 + lane + 1] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane >= o) v += u;
+        }
+        if (e0 + lane < P.E) s_off[e0 + lane + 1] = carry + v;
+        carry += __shfl_sync(0xffffffffu, v, 31);
+      }
+      if (lane == 0) s_off[0] = 0;
+    }
+    __syncthreads();
+    n_items = s_off[P.E];
+  } else {
+    n_items = P.dense_tiles;
+  }
+  const int C = P.splits / P.seq;  // CTAs of a cluster
+  const int split = C > 1 ? (int)cluster_rank() : 0;
+  const int first = C > 1 ? (int)blockIdx.x / C : (int)blockIdx.x;
+  const int stride = C > 1 ? (int)gridDim.x / C : (int)gridDim.x;
+  const int* off = grouped ? s_off : nullptr;
+  const int mine = n_items > first ? (n_items - first + stride - 1) / stride : 0;
+  // (the items of a grouped launch are searched once, here; those of a dense one are derived where they are needed)
+  for (int i = threadIdx.x; grouped && i < min(mine, kItemCache); i += blockDim.x) s_items[i] = pack_item(derive_item(P, first + i * stride, split, off));
+  auto item = [&](int i) { return grouped && i < kItemCache ? unpack_item(s_items[i]) : derive_item(P, first + i * stride, split, off); };
   tc_fence_before();
   __syncthreads();
+  if (C > 1) cluster_arrive();  // this CTA's barriers exist
   tc_fence_after();
-  const uint32_t tmem = s_tmem;
-  const int n_items = P.items != nullptr ? *P.n_items : P.dense_items;
-  const uint32_t x_tile_bytes = (uint32_t)P.BN * 128u;
+  const uint32_t tmem = s_tmem, tmem_w = tmem + P.acc_cols * P.nacc * P.seq;
   const RecGeom geo = rec_geom(KIND, P.K);
 
-  if (warp == 0) {
-    // ---- TMA producer: the raw weight boxes and the token tiles of every K block
+  if (warp == 0 && !kDirect) {
+    // ---- raw weight boxes, a super-block at a time
     if (lane == 0) {
-      // ring positions are counted, not divided: an integer division is a hundred cycles of this one thread
-      int si = 0;
-      uint32_t si_ph = 0;
-      Item w;
+      int rs = 0;
+      uint32_t ph = 0;
       bool ok = true;
-      for (int wi = blockIdx.x; ok && get_item(P, wi, n_items, w); wi += gridDim.x) {
-        const int nt = (w.ntok + P.BN - 1) / P.BN;
-        const int wrow = w.e * P.job[w.job].O + w.ft * BM;
+      for (int i = 0; ok && i < mine; ++i) {
+        const Item w = item(i);
         const WeightMaps& wm = maps.w[w.job];
-        for (int kb = w.kb0; kb < w.kb1; ++kb, si = (si + 1 == SI ? 0 : si + 1), si_ph ^= (si == 0 ? 1u : 0u)) {
-          ok = mbar_wait(bar_in_free + 8 * si, si_ph ^ 1u, P.err);
+        for (int sb = w.kb0 / kSB; sb <= (w.kb1 - 1) / kSB; ++sb) {
+          ok = mbar_wait(raw_free + 8 * rs, ph ^ 1u, P.err);
           if (!ok) break;
-          const uint32_t bar = bar_landed + 8 * si, base = in0 + si * P.stage_bytes;
-          mbar_expect_tx(bar, (uint32_t)nt * x_tile_bytes + F::kTxBytes);
-          F::issue(&wm.w64, &wm.w32, &wm.w16, &wm.wsw, geo, kb, wrow, base, base, bar);
-          for (int t = 0; t < nt; ++t) tma_load_2d(base + kInRaw + t * x_tile_bytes, &maps.x, kb * BK, w.tok0 + t * P.BN, bar);
+          mbar_expect_tx(raw_full + 8 * rs, F::kRawBytes);
+          F::issue(wm, geo, sb, w.wrow, raw0 + (uint32_t)rs * P.raw_bytes, raw_full + 8 * rs);
+          if (++rs == RS) { rs = 0; ph ^= 1u; }
+        }
+      }
+    }
+  } else if (warp == 2) {
+    // ---- token tiles, a unit at a time (and the weight boxes of a bf16 matrix)
+    if (lane == 0) {
+      int us = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int i = 0; ok && i < mine; ++i) {
+        const Item w = item(i);
+        const int k1 = ((w.kb1 - 1) / kSB + 1) * kSB;
+        for (int k0 = w.kb0 / kSB * kSB; k0 < k1; k0 += U) {  // every unit of the super-blocks the item touches
+          ok = mbar_wait(free_ + 8 * us, ph ^ 1u, P.err);
+          if (!ok) break;
+          const int lo = max(w.kb0, k0), hi = min(w.kb1, k0 + U);
+          mbar_expect_tx(full + 8 * us, (uint32_t)max(0, hi - lo) * (x_bytes + (kDirect ? kWTileBytes : 0u)));
+          for (int kb = lo; kb < hi; ++kb) {
+            const uint32_t slot = (uint32_t)(us * U + kb % U);
+            if (kDirect) F::issue(maps.w[w.job], geo, kb, w.wrow, raw0 + slot * kWTileBytes, full + 8 * us);
+            tma_load_2d(x0 + slot * x_bytes, &maps.x, kb * BK, w.tok0, full + 8 * us);
+          }
+          if (++us == NU) { us = 0; ph ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
-    // ---- MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(P.BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-      uint32_t acc_ph = 0, sw_ph = 0;
-      int si = 0, sw = 0;
-      Item w;
-      bool ok = true;
-      for (int wi = blockIdx.x; ok && get_item(P, wi, n_items, w); wi += gridDim.x) {
-        const int nt = (w.ntok + P.BN - 1) / P.BN;
-        ok = mbar_wait(bar_acc_empty, acc_ph ^ 1u, P.err);  // the previous item's accumulators were read
+    // ---- MMA issuer (all lanes run the loop, see tc_commit)
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(P.BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    const uint64_t xd0 = smem_desc(x0), wd0 = smem_desc(raw0);
+    int us = 0;
+    uint32_t ph = 0, ab = 0, aph = 0;
+    bool ok = true, ready = false;
+    // everything the loop branches on goes through a warp reduction or vote: the compiler then knows it to be
+    // uniform and keeps descriptors and addresses in uniform registers
+    const int n_mine = __reduce_max_sync(0xffffffffu, mine);
+    for (int i = 0; ok && i < n_mine; ++i) {
+      const Item w = item(i);
+      const int kb0 = __reduce_max_sync(0xffffffffu, w.kb0), kb1 = __reduce_max_sync(0xffffffffu, w.kb1);
+      ok = __all_sync(0xffffffffu, mbar_wait(acc_free + 8 * ab, aph ^ 1u, P.err));  // this buffer's last accumulators were read
+      uint32_t acc = tmem + ab * (P.acc_cols * P.seq), add = 0;
+      int left = P.per;  // K blocks until the next range and its accumulator
+      const int k1 = ((kb1 - 1) / kSB + 1) * kSB;
+      for (int k0 = kb0 / kSB * kSB; ok && k0 < k1; k0 += U) {
+        if (!ready) ok = __all_sync(0xffffffffu, mbar_wait(full + 8 * us, ph, P.err));
+        if (!ok) break;
         tc_fence_after();
-        for (int kb = w.kb0; kb < w.kb1 && ok;
-             ++kb, si = (si + 1 == SI ? 0 : si + 1), sw = (sw + 1 == SW ? 0 : sw + 1), sw_ph ^= (sw == 0 ? 1u : 0u)) {
-          ok = mbar_wait(bar_full + 8 * sw, sw_ph, P.err);  // implies landed[si]: the dequantisers waited for it
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t inb = in0 + si * P.stage_bytes;
-          const uint32_t xa = inb + kInRaw;
-          const uint32_t wt = tmem + P.acc_cols + (uint32_t)sw * kWCols;  // this K block's weight tile in tensor memory
-          for (int t = 0; t < nt; ++t)
+        const int cur = us;
+        if (++us == NU) { us = 0; ph ^= 1u; }
+        ready = __all_sync(0xffffffffu, mbar_test(full + 8 * us, ph));  // the next unit's barrier, looked at while this one's instructions go out
 #pragma unroll
-            for (int j = 0; j < BK / 16; ++j) {
-              const uint64_t xb = smem_desc(xa + t * x_tile_bytes + j * 32);
-              if (kDirect) tc_mma(tmem + (uint32_t)(t * P.BN), smem_desc(inb + j * 32), xb, idesc, (kb > w.kb0 || j > 0) ? 1u : 0u);
-              else tc_mma_ts(tmem + (uint32_t)(t * P.BN), wt + j * 8, xb, idesc, (kb > w.kb0 || j > 0) ? 1u : 0u);
-            }
-          tc_commit(bar_in_free + 8 * si);  // both slots are free once these MMAs have read them
-          tc_commit(bar_w_free + 8 * sw);
+        for (int b = 0; b < U; ++b) {
+          if (k0 + b < kb0 || k0 + b >= kb1) continue;
+          if (left == 0) { left = P.per; acc += P.acc_cols; add = 0; }
+          --left;
+          const uint64_t xd = xd0 + (uint32_t)(cur * U + b) * (x_bytes >> 4);
+          if (kDirect) tc_mma_block(acc, wd0 + (uint32_t)(cur * U + b) * (kWTileBytes >> 4), xd, idesc, add);
+          else tc_mma_block_ts(acc, tmem_w + (uint32_t)(cur * U + b) * kWCols, xd, idesc, add);
+          add = 1;
         }
-        if (!ok) break;
-        tc_commit(bar_acc_full);
-        acc_ph ^= 1u;
-      }
-    }
-  } else {
-    // ---- dequantising warps, then the epilogue of the item
-    const int dq = threadIdx.x - 64;   // 0 .. 32 * DQW - 1
-    const int q = warp & 3;            // tensor-memory lane quadrant this warp may touch
-    const int r = 32 * q + lane;       // feature row of the tile this thread dequantises = its tensor-memory lane
-    const int colhalf = (warp - 2) >> 2;  // DQW == 8: the two warps of a quadrant split a K block's weights and the
-                                          // epilogue's 16-column groups (DQW == 4: one warp does both halves)
-    uint32_t acc_ph = 0, si_ph = 0, sw_ph = 0;
-    int si = 0, sw = 0;
-    Item w;
-    bool ok = true;
-    for (int wi = blockIdx.x; ok && get_item(P, wi, n_items, w); wi += gridDim.x) {
-      for (int kb = w.kb0; kb < w.kb1; ++kb, si = (si + 1 == SI ? 0 : si + 1), si_ph ^= (si == 0 ? 1u : 0u),
-               sw = (sw + 1 == SW ? 0 : sw + 1), sw_ph ^= (sw == 0 ? 1u : 0u)) {
-        ok = mbar_wait(bar_w_free + 8 * sw, sw_ph ^ 1u, P.err) && mbar_wait(bar_landed + 8 * si, si_ph, P.err);
-        if (!ok) break;
-        if (!kDirect) {
-          tc_fence_after();  // the MMAs that read this slot's last tile are done (w_free)
-          const uint32_t wt = tmem + ((uint32_t)(q * 32) << 16) + P.acc_cols + (uint32_t)sw * kWCols;
-          uint32_t o[16];
-          if (DQW == 8) {
-            F::convert(in0 + si * P.stage_bytes, r, kb, colhalf, o, geo);
-            tmem_st16(wt + 16 * colhalf, o);
-          } else {
-            F::convert(in0 + si * P.stage_bytes, r, kb, 0, o, geo);
-            tmem_st16(wt, o);
-            F::convert(in0 + si * P.stage_bytes, r, kb, 1, o, geo);
-            tmem_st16(wt + 16, o);
-          }
-          tmem_st_wait();
-          tc_fence_before();  // ordered before the MMA thread's reads through the barrier below
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_full + 8 * sw);
-      }
-      if (ok) ok = mbar_wait(bar_acc_full, acc_ph, P.err);
-      if (P.splits > 1) {
-        // the warps of a split item meet at named barriers below: they leave together or not at all
-        // (a warp whose bounded wait ran out still comes here, and its verdict is everybody's)
-        uint32_t all;
-        asm volatile(
-            "{\n"
-            ".reg .pred p, q;\n"
-            "setp.ne.u32 q, %1, 0;\n"
-            "barrier.red.and.pred p, 1, %2, q;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n"
-            : "=r"(all)
-            : "r"(ok ? 1u : 0u), "n"(DQW * 32)
-            : "memory");
-        ok = all != 0;
+        tc_commit(free_ + 8 * cur);
       }
       if (!ok) break;
-      acc_ph ^= 1u;
+      tc_commit(acc_full + 8 * ab);
+      if (++ab == (uint32_t)P.nacc) { ab = 0; aph ^= 1u; }
+    }
+  } else if (warp >= 8) {
+    // ---- dequantising warps
+    const int g = (warp - 8) >> 2, q = warp & 3, r = 32 * q + lane;
+    const uint32_t wcol = tmem_w + ((uint32_t)(q * 32) << 16);
+    int us = g, rs = 0, i = 0, sb = 0, sb1 = -1;  // the group owns every second unit of the ring (NU is even)
+    uint32_t uph = 1, rph = 0;
+    bool ok = true;
+    typename F::Raw R;
+    // moves on to the next unit of the CTA's items and reads this thread's part of it into R; false when none is left.
+    // Every unit is converted whole: blocks outside the item's K range are never multiplied.
+    auto next = [&]() {
+      if (sb > sb1) {
+        if (i >= mine) return false;
+        const Item w = item(i++);
+        sb = w.kb0 / kSB; sb1 = (w.kb1 - 1) / kSB;
+      }
+      ok = mbar_wait(raw_full + 8 * rs, rph, P.err);
+      if (!ok) return false;
+      F::load(R, raw0 + (uint32_t)rs * P.raw_bytes, r, g, sb++);
+      return true;
+    };
+    bool more = next();
+    while (more) {
+      ok = mbar_wait(free_ + 8 * us, uph, P.err);  // the MMAs that read this unit's last tiles are done
+      if (!ok) break;
       tc_fence_after();
+      const uint32_t dst = wcol + (uint32_t)us * (U * kWCols), done = full + 8 * us, rfree = raw_free + 8 * rs;
+      F::convert(R, g, [&](int h, const uint32_t* v) { tmem_st16(dst + 16 * h, v); });
+      if ((us += kDqGroups) >= NU) { us = g; uph ^= 1u; }
+      if (++rs == RS) { rs = 0; rph ^= 1u; }
+      tmem_st_wait();
+      tc_fence_before();  // ordered before the MMA warp's reads through the barrier below
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(done);
+        mbar_arrive(rfree);
+      }
+      more = next();
+    }
+  } else if (warp >= 4) {
+    // ---- epilogue: tensor-memory lane = feature of the tile
+    const int q = warp & 3;
+    uint32_t ab = 0, aph = 0;
+    int sbuf = 0;
+    bool ok = true;
+    for (int i = 0; ok && i < mine; ++i) {
+      const Item w = item(i);
       const GemmJob& J = P.job[w.job];
-      const int fo = w.ft * BM + q * 32 + lane;  // TMEM lane = feature
-      const int nt = (w.ntok + P.BN - 1) / P.BN;
-      // split-K items store f32 partials [token][128 features] instead of results
-      float* part = P.splits > 1 ? P.partial + (size_t)(w.tile * P.splits + w.split) * (size_t)(P.NT * P.BN) * BM : nullptr;
-      for (int t = 0; t < nt; ++t) {
-        for (int c0 = 16 * colhalf; c0 < P.BN; c0 += (DQW == 8 ? 32 : 16)) {
-          if (t * P.BN + c0 >= w.ntok) break;  // warp-uniform
-          uint32_t v[16];
-          tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(t * P.BN + c0), v);
+      const int fo = w.ft * BM + q * 32 + lane;
+      ok = mbar_wait(acc_full + 8 * ab, aph, P.err);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t acc = tmem + ab * (P.acc_cols * P.seq) + ((uint32_t)(q * 32) << 16);
+      // results of up to 16 tokens (v: this lane's feature of each; tok(r): which token row r is, >= ntok: none).
+      // They go through shared memory, so that a token's 128 features leave in 16-byte pieces (a lane holds one
+      // feature: stored from there, every token costs each warp a store of 64 bytes).
+      auto emit = [&](const float* v, auto tok) {
+        if (J.vec8) {
+          const int row = (int)(threadIdx.x & 127) >> 3, piece = threadIdx.x & 7, t = tok(row);
+          size_t orow = 0;
+          if (t < w.ntok) orow = P.row_map != nullptr ? P.row_map[w.tok0 + t] : (size_t)(w.tok0 + t);
+          bf16_t* st = &s_stage[sbuf][0][q * 32 + lane];
+#pragma unroll
+          for (int r = 0; r < 16; ++r) st[r * kStageLd] = f2bf(v[r]);
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          if (t < w.ntok) {
+            const uint4 a0 = *reinterpret_cast<const uint4*>(&s_stage[sbuf][row][8 * piece]);
+            const uint4 a1 = *reinterpret_cast<const uint4*>(&s_stage[sbuf][row][64 + 8 * piece]);
+            bf16_t* y = J.y + orow * J.ldy + w.ft * BM + 8 * piece;
+            if (w.ft * BM + 8 * piece < J.O) *reinterpret_cast<uint4*>(y) = a0;
+            if (w.ft * BM + 64 + 8 * piece < J.O) *reinterpret_cast<uint4*>(y + 64) = a1;
+          }
+          sbuf ^= 1;
+          return;
+        }
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+          const int t = tok(r);
+          if (t < w.ntok && fo < J.O) {
+            const size_t orow = P.row_map != nullptr ? P.row_map[w.tok0 + t] : (size_t)(w.tok0 + t);
+            const size_t at = orow * J.ldy + fo;
+            if (J.y_f32 != nullptr) J.y_f32[at] = v[r];
+            else J.y[at] = f2bf(v[r]);
+          }
+        }
+      };
+      if (C == 1) {
+        for (int c0 = 0; c0 < w.ntok; c0 += 16) {  // warp-uniform
+          uint32_t u[16];
+          float v[16];
+          tmem_ld16(acc + c0, u);
           tmem_ld_wait();
-          if (part != nullptr) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int tok = t * P.BN + c0 + j;
-              if (tok < w.ntok) part[(size_t)tok * BM + q * 32 + lane] = __uint_as_float(v[j]);
-            }
-          } else if (fo < J.O) {
+          for (int t = 0; t < 16; ++t) v[t] = __uint_as_float(u[t]);
+          if (P.seq > 1) {  // the ranges of K in order
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int tok = t * P.BN + c0 + j;
-              if (tok < w.ntok) {
-                const size_t orow = P.row_map != nullptr ? P.row_map[w.tok0 + tok] : (size_t)(w.tok0 + tok);
-                if (J.y_f32 != nullptr) J.y_f32[orow * J.ldy + fo] = __uint_as_float(v[j]);
-                else J.y[orow * J.ldy + fo] = f2bf(__uint_as_float(v[j]));
-              }
+            for (int t = 0; t < 16; ++t) v[t] = 0.f + v[t];
+            for (int d = 1; d < P.seq; ++d) {
+              tmem_ld16(acc + d * P.acc_cols + c0, u);
+              tmem_ld_wait();
+#pragma unroll
+              for (int t = 0; t < 16; ++t) v[t] += __uint_as_float(u[t]);
             }
           }
+          emit(v, [&](int r) { return c0 + r; });
+        }
+      } else {
+        // Four tokens of a feature at a time go to the CTA of the cluster that owns them (group g of four to
+        // rank g mod C), which adds the ranges in order: a fixed order, so the result depends neither on timing
+        // nor on the rows beside it.  The sums are pushed, not fetched: the receiver waits on a barrier of its
+        // own (reading them from the other CTAs' memory behind remote arrivals took 6700 cycles for 24
+        // tokens instead of 2000), and a CTA may leave once its share has arrived.
+        const int groups = (w.ntok + 3) / 4, own = groups > split ? (groups - split + C - 1) / C : 0;
+        if (threadIdx.x == 128) mbar_expect_tx(part_full, (uint32_t)(own * P.splits) * (BM * 16));
+        cluster_wait();  // every CTA's barriers exist
+        const uint32_t mine16 = (uint32_t)(q * 32 + lane) * 16;
+        int owner = 0, slot = 0;
+        for (int c0 = 0; c0 < w.ntok; c0 += 16) {
+          const int owner0 = owner, slot0 = slot;
+          for (int d = 0; d < P.seq; ++d) {
+            uint32_t v[16];
+            tmem_ld16(acc + d * P.acc_cols + c0, v);
+            tmem_ld_wait();
+            owner = owner0; slot = slot0;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              if (c0 + 4 * t < w.ntok)
+                push_f4(map_to_rank(part0 + (uint32_t)((slot * P.splits + split * P.seq + d) * BM) * 16 + mine16, owner), v + 4 * t,
+                        map_to_rank(part_full, owner));
+              if (++owner == C) { owner = 0; ++slot; }
+            }
+          }
+        }
+        ok = mbar_wait(part_full, 0, P.err);
+        if (P.splits > 1) {
+          // the warps meet at a named barrier below: they leave together or not at all
+          uint32_t all;
+          asm volatile(
+              "{\n"
+              ".reg .pred p, q;\n"
+              "setp.ne.u32 q, %1, 0;\n"
+              "barrier.red.and.pred p, 1, 128, q;\n"
+              "selp.u32 %0, 1, 0, p;\n"
+              "}\n"
+              : "=r"(all)
+              : "r"(ok ? 1u : 0u)
+              : "memory");
+          ok = all != 0;
+        }
+        if (!ok) break;
+        for (int sl0 = 0; sl0 < own; sl0 += 4) {
+          float v[16];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            float* r4 = v + 4 * k;
+            r4[0] = r4[1] = r4[2] = r4[3] = 0.f;
+            if (sl0 + k >= own) continue;
+#pragma unroll
+            for (int sp = 0; sp < kMaxSplit; ++sp)
+              if (sp < P.splits) {
+                const uint4 p = lds128(part0 + (uint32_t)((sl0 + k) * P.splits + sp) * (BM * 16) + mine16);
+                r4[0] += __uint_as_float(p.x); r4[1] += __uint_as_float(p.y); r4[2] += __uint_as_float(p.z); r4[3] += __uint_as_float(p.w);
+              }
+          }
+          emit(v, [&](int r) { return 4 * (split + (sl0 + (r >> 2)) * C) + (r & 3); });
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_acc_empty);
-      if (part != nullptr) {
-        // the CTA that stores a tile's last partial adds the partials in split order (a fixed order:
-        // the result does not depend on which CTA comes last) and writes the tile
-        __threadfence();
-        asm volatile("bar.sync 1, %0;" ::"n"(DQW * 32) : "memory");
-        if (dq == 0) s_last = atomicAdd(&P.arrivals[w.tile], 1) == P.splits - 1 ? 1 : 0;
-        asm volatile("bar.sync 1, %0;" ::"n"(DQW * 32) : "memory");
-        if (s_last) {
-          __threadfence();
-          const float4* base = reinterpret_cast<const float4*>(P.partial + (size_t)w.tile * P.splits * (size_t)(P.NT * P.BN) * BM);
-          const size_t stride4 = (size_t)(P.NT * P.BN) * BM / 4;
-          const int n4 = w.ntok * (BM / 4);
-          constexpr int kU = 4;  // float4 pieces per thread and round: their loads are in flight together
-          for (int i0 = dq; i0 < n4; i0 += kU * DQW * 32) {
-            float4 acc[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int sp = 0; sp < P.splits; ++sp) {
-              float4 v[kU];
-#pragma unroll
-              for (int u = 0; u < kU; ++u) {
-                const int i = i0 + u * DQW * 32;
-                v[u] = i < n4 ? __ldcg(base + sp * stride4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-              }
-#pragma unroll
-              for (int u = 0; u < kU; ++u) { acc[u].x += v[u].x; acc[u].y += v[u].y; acc[u].z += v[u].z; acc[u].w += v[u].w; }
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-              const int i = i0 + u * DQW * 32;
-              if (i >= n4) continue;
-              const int tok = i / (BM / 4), f = 4 * (i - tok * (BM / 4));
-              const int feat = w.ft * BM + f;
-              const size_t orow = (size_t)(w.tok0 + tok);
-              const float r4[4] = {acc[u].x, acc[u].y, acc[u].z, acc[u].w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e)
-                if (feat + e < J.O) {
-                  if (J.y_f32 != nullptr) J.y_f32[orow * J.ldy + feat + e] = r4[e];
-                  else J.y[orow * J.ldy + feat + e] = f2bf(r4[e]);
-                }
-            }
-          }
-          if (dq == 0) P.arrivals[w.tile] = 0;  // ready for the next launch
-        }
-      }
+      if (lane == 0) mbar_arrive(acc_free + 8 * ab);
+      if (++ab == (uint32_t)P.nacc) { ab = 0; aph ^= 1u; }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) {
+  if (warp == 3) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(P.tmem_cols) : "memory");
   }
 }
 
-// ---- grouped form: plan and row movement --------------------------------------------------------
+// ---- grouped form: sorting and row movement --------------------------------------------------------
 // counts[e] = rows routed to expert e (block-wide histogram), then seg[e] = exclusive scan
 __global__ void k_route_count(const uint32_t* rhs, int rows, int E, int* seg /*[E+1]*/, int* cursor /*[E]*/) {
   extern __shared__ int s_cnt[];
@@ -717,28 +964,6 @@ __global__ void k_gather_rows(const bf16_t* x, const uint32_t* lhs, const uint32
   uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)p * K);
   for (int i = threadIdx.x; i < K / 8; i += blockDim.x) dst[i] = src[i];
 }
-// work items of the grouped launch: expert e's rows in groups of `span`, every feature tile
-__global__ void k_plan_items(const int* seg, int E, int span, int f_tiles, int4* items, int* n_items, int max_items) {
-  __shared__ int s_off[1025];
-  const int e = threadIdx.x;
-  int mine = 0;
-  if (e < E) mine = ((seg[e + 1] - seg[e] + span - 1) / span) * f_tiles;
-  s_off[e + 1] = mine;
-  if (e == 0) s_off[0] = 0;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i <= (int)blockDim.x; ++i) s_off[i] += s_off[i - 1];
-    *n_items = min(s_off[blockDim.x], max_items);
-  }
-  __syncthreads();
-  if (e < E) {
-    int at = s_off[e];
-    const int first = seg[e], n = seg[e + 1] - seg[e];
-    for (int g = 0; g * span < n; ++g)
-      for (int ft = 0; ft < f_tiles; ++ft, ++at)
-        if (at < max_items) items[at] = make_int4(e, first + g * span, min(span, n - g * span), ft);
-  }
-}
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -757,23 +982,27 @@ EncodeTiledFn encode_tiled() {
 }
 
 std::mutex g_gemm_mu;
-std::set<std::pair<int, int>> g_gemm_granted;  // (device, format and warp count): shared-memory limit raised
 
-template <int KIND, int DQW>
+template <int KIND>
 int launch_qgemm(orn_ctx* ctx, cudaStream_t s, const GemmMaps& maps, const GemmParams& P, int grid, size_t smem) {
-  {
-    std::lock_guard<std::mutex> lock(g_gemm_mu);
-    if (!g_gemm_granted.count({ctx->device, KIND * 16 + DQW})) {
-      ORN_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_qgemm<KIND, DQW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));  // + static barriers
-      g_gemm_granted.insert({ctx->device, KIND * 16 + DQW});
-    }
-  }
-  k_qgemm<KIND, DQW><<<grid, gemm_threads(DQW), smem, s>>>(maps, P);
+  int rc = orn_grant_smem(ctx, reinterpret_cast<const void*>(k_qgemm<KIND>), kGemmSmem);
+  if (rc != ORN_OK) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(gemm_threads(KIND == ORN_BF16));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = P.splits / P.seq; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = P.splits > P.seq ? 1 : 0;
+  ORN_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_qgemm<KIND>, maps, P));
   if (ctx->kt == nullptr) return orn_launch_check(ctx, "k_qgemm");
   // per-kernel timing: one label per shape
   static std::set<std::string> pool;
   char buf[96];
-  snprintf(buf, sizeof buf, "k_qgemm kind=%d O=%d%s K=%d rows=%d %s", KIND, P.job[0].O, P.njobs > 1 ? "+" : "", P.K, P.rows, P.items ? "grouped" : "dense");
+  snprintf(buf, sizeof buf, "k_qgemm kind=%d O=%d%s K=%d rows=%d %s", KIND, P.job[0].O, P.njobs > 1 ? "+" : "", P.K, P.rows, P.seg ? "grouped" : "dense");
   std::lock_guard<std::mutex> lock(g_gemm_mu);
   return orn_launch_check(ctx, pool.insert(buf).first->c_str());
 }
@@ -784,33 +1013,24 @@ uint32_t raw_bytes(int kind) {
     case ORN_Q6K: return Fmt<ORN_Q6K>::kRawBytes;
     case ORN_A8: return Fmt<ORN_A8>::kRawBytes;
     case ORN_A4: return Fmt<ORN_A4>::kRawBytes;
-    default: return 0;
+    default: return Fmt<ORN_BF16>::kRawBytes;
   }
 }
 
 }  // namespace
 
-// device scratch of the grouped form: the item count, then the work items (an expert contributes
-// one item per feature tile and started group of rows; groups hold at least 128 rows)
-size_t qgemm_scratch_bytes(int rows, int E, int O) {
-  const int f_tiles = (O + BM - 1) / BM;
-  const size_t max_items = (size_t)f_tiles * ((size_t)E + rows / 128 + 1);
-  return 256 + max_items * sizeof(int4);
-}
-
 // y[rows, O] (row stride ldy) = x[rows, K] W^T.  grp != null: rows are sorted by expert, expert e
 // owns rows seg[e] .. seg[e+1]-1 (device array of E + 1 ints) and multiplies by W[e]; row p of the
-// result goes to output row row_map[p] when row_map is given.  scratch: qgemm_scratch_bytes() of
-// device memory for the grouped form.
+// result goes to output row row_map[p] when row_map is given.
 int f_qgemm(orn_ctx* ctx, cudaStream_t s, const orn_linear* L, const bf16_t* x, int rows, void* y, int ldy,
-            const QGemmGroup* grp, void* scratch, int out_f32, int bn_force) {
-  return f_qgemm_multi(ctx, s, &L, &y, &ldy, 1, x, rows, grp, scratch, out_f32, bn_force);
+            const QGemmGroup* grp, int out_f32) {
+  return f_qgemm_multi(ctx, s, &L, &y, &ldy, 1, x, rows, grp, out_f32);
 }
 
 // Up to four matrices of one format and row length over the same rows in ONE launch (the projections
 // of a layer that share their input): their feature tiles form one tile space.  n == 1 is f_qgemm.
 int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, void* const* ys, const int* ldys, int n,
-                  const bf16_t* x, int rows, const QGemmGroup* grp, void* scratch, int out_f32, int bn_force) {
+                  const bf16_t* x, int rows, const QGemmGroup* grp, int out_f32) {
   if (rows < 1) return ORN_OK;
   if (n < 1 || n > kMaxJobs) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: 1..4 matrices per launch");
   const orn_linear* L = Ls[0];
@@ -820,119 +1040,100 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
   if (L->K % BK) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: K must be a multiple of 64");
   if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: x must be 16-byte aligned");
   if (grp == nullptr && L->E != 1) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: a routed weight goes through the grouped form");
+  if (grp != nullptr && L->E > kMaxE) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: more than 1024 experts");
   EncodeTiledFn enc = encode_tiled();
   if (enc == nullptr) ORN_FAIL(ctx, ORN_ERR_CUDA, "gemm: the driver has no cuTensorMapEncodeTiled");
   GemmParams P;
+  memset(&P, 0, sizeof P);
   P.njobs = n;
-  P.f_tiles = 0;
   for (int j = 0; j < n; ++j) {
     GemmJob& J = P.job[j];
     J.O = Ls[j]->O; J.tile0 = P.f_tiles; J.ldy = ldys[j];
     J.y = out_f32 ? nullptr : reinterpret_cast<bf16_t*>(ys[j]);
     J.y_f32 = out_f32 ? reinterpret_cast<float*>(ys[j]) : nullptr;
+    J.vec8 = !out_f32 && (ldys[j] & 7) == 0 && (Ls[j]->O & 7) == 0 && (reinterpret_cast<uintptr_t>(ys[j]) & 15) == 0;
     P.f_tiles += (Ls[j]->O + BM - 1) / BM;
   }
-  P.K = L->K; P.rows = rows; P.err = ctx->dev_err;
-  P.row_map = grp ? grp->row_map : nullptr;
-  // token-tile width: wide tiles when there are many tokens per weight tile, narrow ones otherwise
-  int per = grp ? (rows + L->E - 1) / L->E : rows;  // expected tokens per weight tile
-  if (grp && grp->bn_hint > 0) per = grp->bn_hint;
-  int BN = per >= 128 ? 128 : ((per + 15) / 16) * 16;
-  if (BN < 16) BN = 16;
-  if (bn_force > 0) BN = bn_force;  // a caller that wants one tile shape whatever the row count
-  P.BN = BN;
-  // tokens per item: 256 for dense products over many rows (a weight tile is dequantised once for
-  // all of them; more would leave the IN ring too shallow to cover the TMA latency), a few tiles for
-  // routed rows (an expert with more rows than that takes several items)
-  P.NT = (int)kAccColsMax / BN;
-  if (grp == nullptr) P.NT = std::min(std::min(P.NT, (rows + BN - 1) / BN), BN >= 128 ? 2 : 8);
-  else P.NT = std::min(P.NT, BN >= 64 ? 4 : 2);
-  if (P.NT > 8) P.NT = 8;
-  // shared memory: as many IN slots as fit (TMA latency wants depth); tensor memory: the accumulators, then the W ring
-  const uint32_t in_raw = L->kind == ORN_BF16 ? kWTileBytes : raw_bytes(L->kind);
-  P.stage_bytes = in_raw + (uint32_t)P.NT * BN * 128u;
-  P.acc_cols = ((uint32_t)(P.NT * BN) + 31u) & ~31u;
   const bool direct = L->kind == ORN_BF16;
-  auto tmem_need = [&](int ws) {  // power of two that holds the accumulators and ws weight tiles
-    uint32_t c = 32;
-    while (c < P.acc_cols + (direct ? 0u : (uint32_t)ws * kWCols)) c <<= 1;
-    return c;
-  };
-  P.tmem_cols = tmem_need(2);
-  // Dense products over few rows are one token group: the K loop of an item is a chain of short
-  // latency-bound steps (about 0.65 us per K block), so the blocks of a tile are split over several
-  // CTAs whose f32 partials the last of them adds in split order.  The number of splits depends on
-  // (O, K) only, never on the row count, so that a row's bits do not depend on how many rows share
-  // the launch.
-  P.splits = 1; P.partial = nullptr; P.arrivals = nullptr;
-  if (grp == nullptr && rows <= kSplitMaxRows && L->K / BK >= 8) {
-    const int tiles = P.f_tiles * ((rows + P.NT * BN - 1) / (P.NT * BN));
-    // one round of items over the SMs, two CTAs on each where the tiles alone would leave SMs idle
-    // (97 tiles of an input projection: three splits instead of none)
+  const int KB = L->K / BK;
+  P.K = L->K; P.rows = rows; P.err = ctx->dev_err;
+  P.seg = grp ? grp->seg : nullptr;
+  P.row_map = grp ? grp->row_map : nullptr;
+  P.E = L->E;
+  // Dense products over few rows: the K blocks of a tile go to the CTAs of a cluster, which add their
+  // f32 partials in split order through distributed shared memory.  The number of splits depends on the
+  // matrices (and on rows only in steps of 256), so that a row's bits do not depend on the rows beside it:
+  // one round of items over the SMs, two where the tiles alone would leave half of the SMs idle, at
+  // least 4 K blocks per item, no split empty.
+  P.splits = 1; P.seq = 1;
+  if (grp == nullptr && rows <= kSplitMaxRows && KB >= 8) {
+    const int tiles = P.f_tiles * ((rows + 255) / 256);
     int sp = std::max(1, (tiles > ctx->sm_count / 2 ? 2 * ctx->sm_count : ctx->sm_count) / tiles);
-    sp = std::min(sp, std::min(8, L->K / BK / 4));               // at least 4 K blocks per item
-    if (sp > 1) {                                                 // no split may be empty
-      const int KBn = L->K / BK, per = (KBn + sp - 1) / sp;
-      sp = (KBn + per - 1) / per;
+    sp = std::min(sp, std::min(kMaxSplit, KB / 4));
+    if (sp > 1) {
+      const int per = (KB + sp - 1) / sp;
+      sp = (KB + per - 1) / per;
     }
-    const int groups = (rows + P.NT * BN - 1) / (P.NT * BN);
-    const size_t need = (size_t)P.f_tiles * groups * sp * (size_t)(P.NT * BN) * BM * sizeof(float);
-    if (sp > 1 && need <= kSplitPartialBytes && (size_t)P.f_tiles * groups <= kSplitTiles) {
-      // products on the side stream run beside products on the main one: a scratch of their own
-      const bool on_side = ctx->side != nullptr && s == ctx->side;
-      float*& partial = on_side ? ctx->split_partial_side : ctx->split_partial;
-      int*& arrivals = on_side ? ctx->split_arrivals_side : ctx->split_arrivals;
-      if (partial == nullptr) {
-        ORN_CHECK_CUDA(ctx, cudaMalloc((void**)&partial, kSplitPartialBytes));
-        ORN_CHECK_CUDA(ctx, cudaMalloc((void**)&arrivals, kSplitTiles * sizeof(int)));
-        ORN_CHECK_CUDA(ctx, cudaMemset(arrivals, 0, kSplitTiles * sizeof(int)));
-      }
-      P.splits = sp; P.partial = partial; P.arrivals = arrivals;
-    }
+    P.splits = sp;
   }
-  // A launch of narrow items with more items than SMs runs two CTAs per SM (each with half the
-  // shared memory and its own accumulator columns): an item's K loop is a chain of short,
-  // latency-bound steps, and two chains per SM overlap.
-  const int est_items = P.splits * P.f_tiles * (grp ? std::max(L->E, (rows + P.NT * BN - 1) / (P.NT * BN)) : (rows + P.NT * BN - 1) / (P.NT * BN));
-  int ctas = 1, dqw = 8;
-  size_t smem = 0;
-  // Launches of many narrow items (routed experts with a few rows each): small CTAs of 4 dequantising
-  // warps, two-slot rings, up to four per SM: an item's K loop is a latency chain, four chains overlap.
-  if (tmem_need(2) <= 128 && est_items > 2 * ctx->sm_count && P.splits == 1) {
-    // four CTAs share the SM's 512 tensor-memory columns and its shared memory: up to four IN slots each
-    int st = (int)(((226 * 1024) / 4 - 2048) / P.stage_bytes);
-    st = std::min(st, 4);
-    if (st < 2) st = 2;
-    const size_t need = 1024 + (size_t)st * P.stage_bytes;
-    const int fit = (int)((226 * 1024) / (need + 1024));  // + static shared memory and the allocation granule
-    if (fit >= 3) {
-      // the weight ring takes what the accumulators leave of the CTA's 128 columns: hand-offs between the
-      // dequantising warps and the MMA thread are a round trip of several hundred cycles per slot
-      ctas = std::min(4, fit); dqw = 4; P.w_stages = direct ? 1 : std::min<int>(kMaxW, (128 - (int)P.acc_cols) / (int)kWCols); P.stages = st;
-      P.tmem_cols = tmem_need(P.w_stages);
-      smem = need;
+  P.per = (KB + P.splits - 1) / P.splits;
+  // Token-tile width.  Few rows: one tile that holds them.  Many rows: the width (at most 128, so that two
+  // accumulators and the weight ring fit tensor memory) that finishes in the fewest MMA cycles over whole
+  // rounds of the SMs.  Routed rows: wide enough for an expert's rows in nearly every case (mean plus three
+  // standard deviations), since every further item of an expert dequantises its weights again, while
+  // columns up to about 96 hide behind the dequantisation.
+  auto up16 = [](int v) { return (v + 15) / 16 * 16; };
+  if (grp) {
+    const double per = grp->bn_hint > 0 ? grp->bn_hint : std::max(1, (rows + L->E - 1) / L->E);
+    const int want = (int)std::ceil(per + 3.0 * std::sqrt(per));
+    const int groups = (want + 127) / 128;
+    P.BN = std::max(16, up16((want + groups - 1) / groups));
+  } else if (rows <= 128 || P.splits > 1) {
+    P.BN = std::min(128, up16(rows));
+  } else {
+    int64_t best = -1;
+    for (int bn = 128; bn >= 80; bn -= 16) {
+      const int64_t items = (int64_t)P.f_tiles * ((rows + bn - 1) / bn);
+      const int64_t cost = (items + ctx->sm_count - 1) / ctx->sm_count * std::max(2 * bn, 200);
+      if (best < 0 || cost < best) { best = cost; P.BN = bn; }
     }
   }
-  if (ctas == 1 && tmem_need(2) <= 256 && est_items > ctx->sm_count) {
-    const size_t budget2 = 108 * 1024;
-    const int ws = direct ? 1 : std::min<int>(kMaxW, (256 - (int)P.acc_cols) / (int)kWCols);
-    const int st = (int)std::min<size_t>(kMaxIn, budget2 / P.stage_bytes);
-    if (st >= 3) {
-      ctas = 2; P.w_stages = ws; P.stages = st;
-      P.tmem_cols = tmem_need(ws);
-      smem = 1024 + (size_t)st * P.stage_bytes;
-    }
+  P.acc_cols = ((uint32_t)P.BN + 31u) & ~31u;
+  // Two or three ranges: one CTA takes them one after the other (no exchange; the tiles fill at least a third of
+  // the SMs).  More: clusters of at most four CTAs where the count and the memory allow (a GPC holds two clusters
+  // of eight at most, so eight do not place on every SM), each taking its ranges one after the other.
+  const size_t unit_b = (size_t)U * ((size_t)P.BN * 128 + (direct ? kWTileBytes : 0)), room = kGemmSmem - 1024;
+  const size_t raw_b = direct ? 0 : raw_bytes(L->kind);
+  auto part_bytes = [&](int c) { return c > 1 ? (size_t)((P.BN / 4 + c - 1) / c * P.splits) * (BM * 16) : 0; };
+  if (P.splits > 1) {
+    const int most = (512 - 2 * U * (int)kWCols) / (int)P.acc_cols;
+    int c = P.splits <= std::min(3, most) ? 1 : P.splits;
+    for (int t = std::min(4, P.splits); c > 1 && t >= 2; --t)
+      if (P.splits % t == 0 && P.splits / t <= most && part_bytes(t) + 2 * unit_b + 2 * raw_b <= room) { c = t; break; }
+    P.seq = P.splits / c;
   }
-  if (ctas == 1) {
-    P.w_stages = direct ? 1 : std::min<int>(kMaxW, (512 - (int)P.acc_cols) / (int)kWCols);
-    P.tmem_cols = tmem_need(P.w_stages);
-    const size_t budget = 200 * 1024;
-    P.stages = (int)std::min<size_t>(kMaxIn, budget / P.stage_bytes);
-    if (P.stages < 2) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: stage does not fit twice into shared memory");
-    // one CTA per SM (it may take all of tensor memory): pad the launch's shared memory above half of the SM's
-    smem = 1024 + (size_t)P.stages * P.stage_bytes;
-    if (smem < 120 * 1024) smem = 120 * 1024;
+  const int C = P.splits / P.seq;
+  // Tensor memory: the accumulators (two sets where an item has one) and an even number of units of weight
+  // tiles.  Shared memory: the units' token tiles, the partial sums that arrive from a cluster, raw slots.
+  P.raw_bytes = raw_bytes(L->kind);
+  P.nacc = P.seq == 1 ? 2 : 1;
+  const uint32_t accs = P.nacc * P.seq * P.acc_cols;
+  const size_t part = part_bytes(C);
+  if (direct) {
+    P.units = (int)std::min<size_t>(kMaxUnits, (room - part) / unit_b) & ~1;
+    P.raw_slots = P.units * U;
+    P.raw_bytes = kWTileBytes;
+  } else {
+    for (P.units = 6; P.units > 2; P.units -= 2)
+      if (accs + P.units * U * kWCols <= 512 && P.units * unit_b + 3 * P.raw_bytes + part <= room) break;
+    P.raw_slots = (int)std::min<size_t>(kMaxRaw, (room - part - P.units * unit_b) / P.raw_bytes);
   }
+  if (P.units < 2 || P.raw_slots < 1) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: the rings do not fit into shared memory");
+  const size_t rings = P.units * unit_b + (direct ? 0 : (size_t)P.raw_slots * P.raw_bytes) + part;
+  P.tmem_cols = 32;
+  while (P.tmem_cols < accs + (direct ? 0u : P.units * U * kWCols)) P.tmem_cols <<= 1;
+  // one CTA per SM (it may take all of tensor memory): never less than half of the SM's shared memory
+  const size_t smem = std::max<size_t>(120 * 1024, 1024 + rings);
   GemmMaps maps;
   memset(&maps, 0, sizeof maps);
   auto encode = [&](CUtensorMap* m, CUtensorMapDataType dt, void* base, uint64_t inner, uint64_t outer, uint64_t stride_bytes,
@@ -945,56 +1146,35 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
   bool ok = encode(&maps.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, const_cast<bf16_t*>(x), (uint64_t)L->K, (uint64_t)rows,
-                   (uint64_t)L->K * 2, BK, (uint32_t)BN, CU_TENSOR_MAP_SWIZZLE_128B);
+                   (uint64_t)L->K * 2, BK, (uint32_t)P.BN, CU_TENSOR_MAP_SWIZZLE_128B);
   for (int j = 0; j < n; ++j) {
     const orn_linear* Lj = Ls[j];
     WeightMaps& wm = maps.w[j];
     const uint64_t wrows = (uint64_t)Lj->E * Lj->O;
-    if (Lj->kind == ORN_BF16) {
-      ok = ok && encode(&wm.wsw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, Lj->w, (uint64_t)Lj->K, wrows, (uint64_t)Lj->rec, BK, BM,
+    auto box = [&](CUtensorMap* m, uint32_t bytes, CUtensorMapSwizzle sw) {
+      ok = ok && encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, Lj->w, (uint64_t)Lj->rec, wrows, (uint64_t)Lj->rec, bytes, BM, sw);
+    };
+    if (direct) {
+      ok = ok && encode(&wm.wide, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, Lj->w, (uint64_t)Lj->K, wrows, (uint64_t)Lj->rec, BK, BM,
                         CU_TENSOR_MAP_SWIZZLE_128B);
-    } else {
-      ok = ok && encode(&wm.w64, CU_TENSOR_MAP_DATA_TYPE_UINT8, Lj->w, (uint64_t)Lj->rec, wrows, (uint64_t)Lj->rec, 64, BM, CU_TENSOR_MAP_SWIZZLE_NONE);
-      ok = ok && encode(&wm.w32, CU_TENSOR_MAP_DATA_TYPE_UINT8, Lj->w, (uint64_t)Lj->rec, wrows, (uint64_t)Lj->rec, 32, BM, CU_TENSOR_MAP_SWIZZLE_NONE);
-      ok = ok && encode(&wm.w16, CU_TENSOR_MAP_DATA_TYPE_UINT8, Lj->w, (uint64_t)Lj->rec, wrows, (uint64_t)Lj->rec, 16, BM, CU_TENSOR_MAP_SWIZZLE_NONE);
+      continue;
     }
+    box(&wm.wide, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (L->kind == ORN_Q6K) box(&wm.mid, 64, CU_TENSOR_MAP_SWIZZLE_64B);
+    box(&wm.scale, L->kind == ORN_A4 ? 32 : 16, CU_TENSOR_MAP_SWIZZLE_NONE);
   }
   if (!ok) ORN_FAIL(ctx, ORN_ERR_CUDA, "gemm: cuTensorMapEncodeTiled failed");
-  int grid;
+  int grid = ctx->sm_count;
   if (grp == nullptr) {
-    P.items = nullptr; P.n_items = nullptr;
-    const int groups = (rows + P.NT * BN - 1) / (P.NT * BN);
-    P.dense_items = P.f_tiles * groups * P.splits;
-    grid = std::min(P.dense_items, ctas * ctx->sm_count);
-  } else {
-    if (L->E > 1024) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: more than 1024 experts");
-    if (scratch == nullptr) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: the grouped form needs scratch");
-    int* n_items = reinterpret_cast<int*>(scratch);
-    int4* items = reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(scratch) + 256);
-    const int max_items = (int)((qgemm_scratch_bytes(rows, L->E, P.f_tiles * BM) - 256) / sizeof(int4));
-    int threads = 32;
-    while (threads < L->E) threads <<= 1;
-    k_plan_items<<<1, threads, 0, s>>>(grp->seg, L->E, P.NT * BN, P.f_tiles, items, n_items, max_items);
-    int rc = orn_launch_check(ctx, "k_plan_items");
-    if (rc != ORN_OK) return rc;
-    P.items = items; P.n_items = n_items; P.dense_items = 0;
-    grid = ctas * ctx->sm_count;
-  }
-  if (dqw == 4) {
-    switch (L->kind) {
-      case ORN_Q4K: return launch_qgemm<ORN_Q4K, 4>(ctx, s, maps, P, grid, smem);
-      case ORN_Q6K: return launch_qgemm<ORN_Q6K, 4>(ctx, s, maps, P, grid, smem);
-      case ORN_A8: return launch_qgemm<ORN_A8, 4>(ctx, s, maps, P, grid, smem);
-      case ORN_BF16: return launch_qgemm<ORN_BF16, 4>(ctx, s, maps, P, grid, smem);
-      case ORN_A4: return launch_qgemm<ORN_A4, 4>(ctx, s, maps, P, grid, smem);
-    }
+    P.dense_tiles = P.f_tiles * ((rows + P.BN - 1) / P.BN);
+    grid = C > 1 ? P.dense_tiles * C : std::min(P.dense_tiles, ctx->sm_count);  // a cluster has one tile
   }
   switch (L->kind) {
-    case ORN_Q4K: return launch_qgemm<ORN_Q4K, 8>(ctx, s, maps, P, grid, smem);
-    case ORN_Q6K: return launch_qgemm<ORN_Q6K, 8>(ctx, s, maps, P, grid, smem);
-    case ORN_A8: return launch_qgemm<ORN_A8, 8>(ctx, s, maps, P, grid, smem);
-    case ORN_BF16: return launch_qgemm<ORN_BF16, 8>(ctx, s, maps, P, grid, smem);
-    case ORN_A4: return launch_qgemm<ORN_A4, 8>(ctx, s, maps, P, grid, smem);
+    case ORN_Q4K: return launch_qgemm<ORN_Q4K>(ctx, s, maps, P, grid, smem);
+    case ORN_Q6K: return launch_qgemm<ORN_Q6K>(ctx, s, maps, P, grid, smem);
+    case ORN_A8: return launch_qgemm<ORN_A8>(ctx, s, maps, P, grid, smem);
+    case ORN_BF16: return launch_qgemm<ORN_BF16>(ctx, s, maps, P, grid, smem);
+    case ORN_A4: return launch_qgemm<ORN_A4>(ctx, s, maps, P, grid, smem);
   }
   ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: unknown weight format");
 }

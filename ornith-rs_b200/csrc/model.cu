@@ -723,7 +723,7 @@ bool wide_exact() {
 // y[T, O] = x[T, K] W^T for a prompt chunk
 int wide_mm(orn_model* m, const orn_linear* L, const bf16_t* x, int T, bf16_t* y) {
   orn_ctx* ctx = m->ctx;
-  if (!wide_exact()) return f_qgemm(ctx, ctx->stream, L, x, T, y, L->O, nullptr, nullptr);
+  if (!wide_exact()) return f_qgemm(ctx, ctx->stream, L, x, T, y, L->O, nullptr);
   for (int r = 0; r < T; r += kMaxRows) {
     const int n = std::min(kMaxRows, T - r);
     CK(k_gemv(ctx, ctx->stream, L, x + (size_t)r * L->K, n, y + (size_t)r * L->O, 0));
@@ -764,10 +764,7 @@ int wide_reserve(orn_model* m, int rows) {
   A(&w.sy, R * H); A(&w.gs, R);
   A(&w.xs, R * k * H); A(&w.eg, R * k * I); A(&w.eu, R * k * I); A(&w.eact, R * k * I); A(&w.ey, R * k * H);
   if (rc == ORN_OK) {
-    const size_t big = std::max(qgemm_scratch_bytes((int)(R * k), (int)E, (int)H), qgemm_scratch_bytes((int)(R * k), (int)E, (int)I));
-    rc = orn_alloc(m->ctx, big, &w.gemm_scratch);
-    if (rc == ORN_OK) w.allocs.push_back(w.gemm_scratch);
-    if (rc == ORN_OK) rc = orn_alloc(m->ctx, gdn_chunk_scratch_bytes(rows, c.gdn_v_heads), &w.gdn_scratch);
+    rc = orn_alloc(m->ctx, gdn_chunk_scratch_bytes(rows, c.gdn_v_heads), &w.gdn_scratch);
     if (rc == ORN_OK) w.allocs.push_back(w.gdn_scratch);
   }
   if (rc != ORN_OK) {
@@ -826,10 +823,10 @@ int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, bf16_t*
     CK(k_gather_gemv(ctx, s, moe.sw_down, w.eact, w.perm_inv, w.inds, rows, w.ey));
   } else {
     QGemmGroup sorted{w.seg, nullptr, 0}, back{w.seg, w.perm, 0};
-    CK(f_qgemm(ctx, s, moe.sw_gate, w.xs, rows, w.eg, I, &sorted, w.gemm_scratch));
-    CK(f_qgemm(ctx, s, moe.sw_up, w.xs, rows, w.eu, I, &sorted, w.gemm_scratch));
+    CK(f_qgemm(ctx, s, moe.sw_gate, w.xs, rows, w.eg, I, &sorted));
+    CK(f_qgemm(ctx, s, moe.sw_up, w.xs, rows, w.eu, I, &sorted));
     CK(k_swiglu(ctx, s, w.eg, w.eu, rows * I, w.eact));
-    CK(f_qgemm(ctx, s, moe.sw_down, w.eact, rows, w.ey, H, &back, w.gemm_scratch));  // rows back in (token, slot) order
+    CK(f_qgemm(ctx, s, moe.sw_down, w.eact, rows, w.ey, H, &back));  // rows back in (token, slot) order
   }
   CK(k_moe_combine(ctx, s, w.scores, w.ey, w.gs, w.sy, T, c.top_k, H, c.norm_topk_prob, out));
   return ORN_OK;
