@@ -313,6 +313,10 @@ struct orn_batch {
   bf16_t *qg, *aq, *agate, *ak, *av, *att, *agated, *logits;
   float *greedy_scratch, *part;
   int part_chunks = 0;
+  // fewer rows than the tensor cores are used for: the fused decode kernels' scratch (kSmallRows rows)
+  bool small_ok = false;
+  bf16_t *sgates = nullptr, *sscores = nullptr, *seact = nullptr, *ssact = nullptr, *sgs = nullptr;
+  uint32_t* sinds = nullptr;
   // the MTP head's per-sequence state (depth 1): its own KV cache and positions, the hidden row its next draft reads
   bf16_t *mtp_kc = nullptr, *mtp_vc = nullptr, *hrow = nullptr, *hid0 = nullptr;
   bf16_t *memb = nullptr, *me = nullptr, *mh = nullptr, *mjoined = nullptr, *mx = nullptr, *dhid = nullptr;
@@ -505,6 +509,160 @@ __global__ void mtp_advance_kernel(int* mtp_pos, const int* keep, int B, int bas
   if (b < B) mtp_pos[b] += base + (keep ? keep[b] - 1 : 0);
 }
 
+// ---- fewer rows than the tensor cores are used for ----------------------------------------------
+// The single-sequence engine's fused kernels (fused.cu), four rows at a time where they take at most
+// four, all sequences at once where they are per sequence: the same bits as the one-kernel-per-op
+// path, a sixth of its launches, every weight read by the kernels built for few rows.  One sequence of
+// two rows: 9.9 -> 3.0 ms per cycle, bit for bit the same.
+constexpr int kSmallRows = 15;
+
+// the fused kernels serve every part of the model at these rows, on this GPU alone
+bool small_path(const orn_batch* bt, int rows, int world) {
+  return bt->small_ok && rows <= kSmallRows && world == 1 && !bt->split_attn && orn_use_fused(bt->m) &&
+         bt->B * std::max(bt->m->cfg.gdn_v_heads, 1) <= 960 && bt->B * bt->m->cfg.n_heads <= 256;
+}
+// jobs over `rows` rows of one prologue, at most four rows per launch
+int small_mm(orn_batch* bt, const FusedPrologue& fp, const FusedJob* jobs, int n, int rows) {
+  orn_ctx* ctx = bt->m->ctx;
+  for (int r = 0; r < rows; r += kMaxRows) {
+    FusedPrologue p = fp;
+    FusedJob j[4];
+    const size_t ka = fp.mode == PRO_MTPJOIN ? fp.K / 2 : fp.K;
+    p.a += r * ka;
+    if (p.b) p.b += (size_t)r * fp.K;
+    if (p.sum_out) p.sum_out += (size_t)r * fp.K;
+    if (p.norm_out) p.norm_out += (size_t)r * fp.K;
+    if (p.ids) p.ids += r;
+    for (int i = 0; i < n; ++i) { j[i] = jobs[i]; j[i].out += (size_t)r * jobs[i].lin->O; }
+    CK(f_norm_gemv(ctx, ctx->stream, std::min(kMaxRows, rows - r), p, j, n));
+  }
+  return ORN_OK;
+}
+// MoE block of the rows h = bf(a + b) -> bt->h, result -> bt->mo
+int small_moe(orn_batch* bt, const Moe& moe, const bf16_t* a, const bf16_t* b, const bf16_t* nw, int rows) {
+  orn_model* m = bt->m;
+  orn_ctx* ctx = m->ctx;
+  cudaStream_t s = ctx->stream;
+  const orn_config& c = m->cfg;
+  FusedPrologue fp;
+  fp.mode = PRO_ADDNORM; fp.K = c.hidden; fp.a = a; fp.b = b; fp.w = nw; fp.sum_out = bt->h; fp.norm_out = bt->n2; fp.eps = c.rms_eps;
+  FusedJob jobs[3];
+  jobs[0].lin = moe.gate; jobs[0].out = bt->sgates;
+  jobs[1].lin = moe.sh_gate; jobs[1].lin2 = moe.sh_up; jobs[1].out = bt->ssact; jobs[1].epi = EPI_SWIGLU;
+  jobs[2].lin = moe.sh_egate; jobs[2].out = bt->sgs;
+  CK(small_mm(bt, fp, jobs, 3, rows));
+  const size_t H = c.hidden, E = c.n_experts, k = c.top_k, I = c.expert_inter, SI = c.shared_inter;
+  for (int r = 0; r < rows; r += kMaxRows) {
+    const int n = std::min(kMaxRows, rows - r);
+    CK(f_moe_up(ctx, s, n, bt->sgates + r * E, bt->n2 + r * H, moe.sw_gate, moe.sw_up, c.top_k, bt->sinds + r * k, bt->sscores + r * k,
+                bt->seact + r * k * I));
+    CK(f_moe_down(ctx, s, n, bt->seact + r * k * I, bt->ssact + r * SI, bt->sinds + r * k, bt->sscores + r * k, bt->sgs + r, moe.sw_down,
+                  moe.sh_down, c.top_k, c.norm_topk_prob, bt->mo + r * H));
+  }
+  return ORN_OK;
+}
+// attention sub-block of B sequences of T rows -> bt->r; kv_only: stop once the KV rows are in the cache
+int small_attention(orn_batch* bt, const FusedPrologue& fp, const orn_linear* q_proj, const orn_linear* k_proj, const orn_linear* v_proj,
+                    const orn_linear* o_proj, const bf16_t* q_norm, const bf16_t* k_norm, int T, const int* pos, bf16_t* kc, bf16_t* vc,
+                    int keys, bool kv_only) {
+  orn_model* m = bt->m;
+  orn_ctx* ctx = m->ctx;
+  const orn_config& c = m->cfg;
+  const int R = bt->B * T;
+  FusedJob jobs[3];
+  jobs[0].lin = q_proj; jobs[0].out = bt->qg;
+  jobs[1].lin = k_proj; jobs[1].out = bt->ak;
+  jobs[2].lin = v_proj; jobs[2].out = bt->av;
+  CK(small_mm(bt, fp, jobs, 3, R));
+  CK(f_attn(ctx, ctx->stream, bt->qg, bt->ak, bt->av, q_norm, k_norm, kc, vc, pos, T, c.n_heads, c.n_kv_heads, c.head_dim, bt->cap,
+            c.rope_dims, m->lnb, c.rms_eps, bt->agated, orn_long_context(keys), bt->B));
+  if (kv_only) return ORN_OK;
+  FusedPrologue gp;
+  gp.mode = PRO_PLAIN; gp.K = c.n_heads * c.head_dim; gp.a = bt->agated;
+  FusedJob oj;
+  oj.lin = o_proj; oj.out = bt->r;
+  return small_mm(bt, gp, &oj, 1, R);
+}
+int small_body(orn_batch* bt, int T, int keys) {
+  orn_model* m = bt->m;
+  orn_ctx* ctx = m->ctx;
+  cudaStream_t s = ctx->stream;
+  const orn_config& c = m->cfg;
+  const int B = bt->B, R = B * T, H = c.hidden, S = c.gdn_conv_kernel - 1, D = orn_conv_dim(c), VD = c.gdn_v_heads * c.gdn_head_dim;
+  ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(bt->ids, bt->ids_h, sizeof(uint32_t) * (size_t)R, cudaMemcpyHostToDevice, s));
+  if (B > 1) {
+    conv_map_kernel<<<(R + 127) / 128, 128, 0, s>>>(bt->conv_map, B, T, bt->conv_rows, S);
+    CK(orn_launch_check(ctx, "conv_map"));
+  }
+  CK(k_embedding(ctx, s, m->embed, bt->ids, R, bt->h));
+  const bf16_t *pa = bt->h, *pb = nullptr;
+  bf16_t* const res = bt->x;
+  for (int i = 0; i < c.n_layers; ++i) {
+    const Layer& ly = m->layers[i];
+    FusedPrologue fp;
+    fp.mode = PRO_ADDNORM; fp.K = H; fp.a = pa; fp.b = pb; fp.w = ly.input_ln; fp.sum_out = res; fp.eps = c.rms_eps;
+    if (ly.linear) {
+      // one sequence: its rows go straight into the conv window; several: scattered
+      bf16_t* qkv = B == 1 ? bt->conv[i] + (size_t)S * D : bt->qkv;
+      FusedJob jobs[4];
+      jobs[0].lin = ly.in_qkv; jobs[0].out = qkv;
+      jobs[1].lin = ly.in_z; jobs[1].out = bt->z;
+      jobs[2].lin = ly.in_b; jobs[2].out = bt->b;
+      jobs[3].lin = ly.in_a; jobs[3].out = bt->a;
+      CK(small_mm(bt, fp, jobs, 4, R));
+      if (B > 1) {
+        scatter_rows_kernel<<<R, 128, 0, s>>>(bt->qkv, bt->conv_map, D, bt->conv[i]);
+        CK(orn_launch_check(ctx, "scatter_rows"));
+      }
+      CK(f_gdn(ctx, s, bt->conv[i], ly.conv_w, bt->a, bt->b, ly.a_log, ly.dt_bias, bt->ring[i], bt->nring, bt->cur, 0, T, c.gdn_k_heads,
+               c.gdn_v_heads, c.gdn_conv_kernel, 1e-6f, bt->gy, bt->z, ly.gdn_norm, c.rms_eps, bt->gated, B, (int64_t)bt->conv_rows * D));
+      FusedPrologue gp;
+      gp.mode = PRO_PLAIN; gp.K = VD; gp.a = bt->gated;
+      FusedJob oj;
+      oj.lin = ly.out_proj; oj.out = bt->r;
+      CK(small_mm(bt, gp, &oj, 1, R));
+    } else {
+      CK(small_attention(bt, fp, ly.q_proj, ly.k_proj, ly.v_proj, ly.o_proj, ly.q_norm, ly.k_norm, T, bt->pos, bt->kc[i], bt->vc[i], keys, false));
+    }
+    CK(small_moe(bt, ly.moe, res, bt->r, ly.post_ln, R));
+    pa = bt->h;
+    pb = bt->mo;
+  }
+  FusedPrologue hp;
+  hp.mode = PRO_ADDNORM; hp.K = H; hp.a = bt->h; hp.b = bt->mo; hp.w = m->norm; hp.norm_out = bt->normed; hp.eps = c.rms_eps;
+  FusedJob hj;
+  hj.lin = m->lm_head; hj.out = bt->logits;
+  CK(small_mm(bt, hp, &hj, 1, R));
+  CK(k_greedy(ctx, s, bt->logits, R, c.vocab, 1, bt->targets, bt->greedy_scratch));
+  ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(bt->targets_h, bt->targets, sizeof(uint32_t) * (size_t)R, cudaMemcpyDeviceToHost, s));
+  return ORN_OK;
+}
+// the MTP head for B sequences of one row: draft tokens -> bt->drafts, or (kv_only) just the KV rows
+int small_mtp(orn_batch* bt, const uint32_t* dev_ids, const bf16_t* hidden, int keys, bool kv_only) {
+  orn_model* m = bt->m;
+  orn_ctx* ctx = m->ctx;
+  const orn_config& c = m->cfg;
+  const Mtp& h = m->mtp;
+  const int B = bt->B, H = c.hidden;
+  FusedPrologue jp;
+  jp.mode = PRO_MTPJOIN; jp.K = 2 * H; jp.a = hidden; jp.w = h.pre_fc_norm_embedding; jp.w2 = h.pre_fc_norm_hidden; jp.emb = m->embed;
+  jp.ids = dev_ids; jp.eps = c.rms_eps;
+  FusedJob fj;
+  fj.lin = h.fc; fj.out = bt->mx;
+  CK(small_mm(bt, jp, &fj, 1, B));
+  FusedPrologue fp;
+  fp.mode = PRO_ADDNORM; fp.K = H; fp.a = bt->mx; fp.w = h.input_ln; fp.eps = c.rms_eps;
+  CK(small_attention(bt, fp, h.q_proj, h.k_proj, h.v_proj, h.o_proj, h.q_norm, h.k_norm, 1, bt->mtp_pos, bt->mtp_kc, bt->mtp_vc, keys, kv_only));
+  if (kv_only) return ORN_OK;
+  CK(small_moe(bt, h.moe, bt->mx, bt->r, h.post_ln, B));
+  FusedPrologue hp;
+  hp.mode = PRO_ADDNORM; hp.K = H; hp.a = bt->h; hp.b = bt->mo; hp.w = h.norm; hp.norm_out = bt->dhid; hp.eps = c.rms_eps;
+  FusedJob hj;
+  hj.lin = m->lm_head; hj.out = bt->logits;
+  CK(small_mm(bt, hp, &hj, 1, B));
+  return k_greedy(ctx, ctx->stream, bt->logits, B, c.vocab, 0, bt->drafts, bt->greedy_scratch);
+}
+
 // the device work of one step: everything between the upload of the ids and the download of the
 // targets, with fixed addresses and launch shapes (so that it can be captured once and replayed)
 int batch_body(orn_batch* bt, orn_ep* group, int T, int chunk, int nchunks) {
@@ -632,6 +790,14 @@ int32_t orn_batch_create(orn_model* m, int32_t B, int32_t T_max, int32_t cap, in
     A(&bt->mx, (size_t)B * H); A(&bt->dhid, (size_t)B * H); A(&bt->prim, (size_t)B); A(&bt->tok1, (size_t)B); A(&bt->drafts, (size_t)B);
     A(&bt->mtp_pos, (size_t)B);
   }
+  {
+    const size_t n = kSmallRows, E = c.n_experts, k = c.top_k;
+    A(&bt->sgates, n * E); A(&bt->sinds, n * k); A(&bt->sscores, n * k); A(&bt->seact, n * k * c.expert_inter);
+    A(&bt->ssact, n * c.shared_inter); A(&bt->sgs, n);
+    bt->small_ok = H <= 2048 && c.head_dim == 256 && c.n_experts <= 512 && k <= 8 && c.expert_inter <= 2048 && c.shared_inter <= 2048;
+    for (const Layer& ly : m->layers) bt->small_ok = bt->small_ok && orn_moe_fusable(ly.moe);
+    if (m->mtp.present) bt->small_ok = bt->small_ok && orn_moe_fusable(m->mtp.moe);
+  }
   A(&bt->greedy_scratch, greedy_scratch_floats((int)R, c.vocab));
   bt->part_chunks = (cap + kMinChunk - 1) / kMinChunk;
   A(&bt->part, (size_t)B * c.n_kv_heads * bt->part_chunks * 16 * kPartStride);
@@ -738,13 +904,16 @@ int32_t orn_batch_forward(orn_batch* bt, orn_ep* ep, const uint32_t* host_ids, i
   for (int b = 0; b < B; ++b) max_pos = std::max(max_pos, bt->h_pos[b]);
   int chunk, nchunks;
   split_shape(bt, max_pos + T, &chunk, &nchunks);
+  const bool small = exact && small_path(bt, R, world);
+  auto body = [&]() { return small ? small_body(bt, T, max_pos + T) : batch_body(bt, group, T, chunk, nchunks); };
   // the previous step's targets have been read (its download synchronised) before ids_h is rewritten
   ORN_CHECK_CUDA(ctx, cudaStreamSynchronize(s));
   memcpy(bt->ids_h, host_ids, sizeof(uint32_t) * (size_t)R);
   static int no_graph = -1;
   if (no_graph < 0) { const char* e = getenv("ORN_NO_GRAPH"); no_graph = (e && e[0] == '1') ? 1 : 0; }
   const bool eager = no_graph || ctx->kt != nullptr;
-  const uint64_t key = (uint64_t)T | ((uint64_t)nchunks << 8) | ((uint64_t)chunk << 28) | ((uint64_t)(exact ? 1 : 0) << 40);
+  const uint64_t key = (uint64_t)T | ((uint64_t)nchunks << 8) | ((uint64_t)chunk << 28) | ((uint64_t)(exact ? 1 : 0) << 40) |
+                       ((uint64_t)(small ? 1 : 0) << 41) | ((uint64_t)(small ? orn_long_context(max_pos + T) : 0) << 42);
   orn_batch::StepGraph& g = bt->graphs[key];
   if (g.exec != nullptr && g.group != group) {  // captured for another group: its collectives belong to that one
     cudaGraphExecDestroy(g.exec);
@@ -756,11 +925,11 @@ int32_t orn_batch_forward(orn_batch* bt, orn_ep* ep, const uint32_t* host_ids, i
     ctx->launches += g.launches;
   } else if (g.seen == 0 || eager) {
     g.seen += 1;  // the first step of a shape runs eagerly (scratch is allocated on first use); the second is captured
-    rc = batch_body(bt, group, T, chunk, nchunks);
+    rc = body();
   } else {
     const int64_t l0 = ctx->launches;
     ORN_CHECK_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    rc = batch_body(bt, group, T, chunk, nchunks);
+    rc = body();
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(s, &graph);
     if (rc != ORN_OK) { if (graph) cudaGraphDestroy(graph); return rc; }
@@ -813,9 +982,15 @@ int32_t orn_batch_commit(orn_batch* bt, const int32_t* host_keep) {
     if (bt->drafted && T == 2) {
       const Mtp& h = m->mtp;
       const bool exact = bt->exact || bt->B < 16;
-      CK(mtp_join(bt, bt->tok1, bt->hid0));
-      CK(batch_attention(bt, h.q_proj, h.k_proj, h.v_proj, h.o_proj, h.q_norm, h.k_norm, 1, bt->mtp_pos, bt->mtp_kc, bt->mtp_vc, exact,
+      int max_pos = 0;
+      for (int b = 0; b < bt->B; ++b) max_pos = std::max(max_pos, bt->h_mtp_pos[b]);
+      if (exact && small_path(bt, bt->B, bt->shard_world > 1 ? bt->shard_world : 1)) {
+        CK(small_mtp(bt, bt->tok1, bt->hid0, max_pos + 1, true));
+      } else {
+        CK(mtp_join(bt, bt->tok1, bt->hid0));
+        CK(batch_attention(bt, h.q_proj, h.k_proj, h.v_proj, h.o_proj, h.q_norm, h.k_norm, 1, bt->mtp_pos, bt->mtp_kc, bt->mtp_vc, exact,
                          0, 0, true));
+      }
       mtp_advance_kernel<<<(bt->B + 127) / 128, 128, 0, s>>>(bt->mtp_pos, bt->keep, bt->B, 0);
       CK(orn_launch_check(ctx, "mtp_advance"));
       for (int b = 0; b < bt->B; ++b) bt->h_mtp_pos[b] += host_keep[b] - 1;
@@ -855,18 +1030,22 @@ int32_t orn_batch_mtp_draft(orn_batch* bt, orn_ep* ep, const uint32_t* host_prim
   int chunk, nchunks;
   split_shape(bt, max_pos + 1, &chunk, &nchunks);
   CK(orn_upload(ctx, bt->prim, host_primary, sizeof(uint32_t) * (size_t)B));
-  CK(mtp_join(bt, bt->prim, bt->hrow));
-  CK(batch_attention(bt, h.q_proj, h.k_proj, h.v_proj, h.o_proj, h.q_norm, h.k_norm, 1, bt->mtp_pos, bt->mtp_kc, bt->mtp_vc, exact, chunk,
-                     nchunks, false));
-  CK(k_add_rms_norm(ctx, s, bt->mx, bt->r, h.post_ln, B, H, c.rms_eps, bt->h, bt->n2));
-  const orn_linear* sg = world > 1 ? bt->mtp_views[0] : h.moe.sw_gate;
-  const orn_linear* su = world > 1 ? bt->mtp_views[1] : h.moe.sw_up;
-  const orn_linear* sd = world > 1 ? bt->mtp_views[2] : h.moe.sw_down;
-  CK(orn_ep_moe_block(group, h.moe.gate, sg, su, sd, h.moe.sh_gate, h.moe.sh_up, h.moe.sh_down, h.moe.sh_egate, bt->n2, B, c.top_k,
-                      c.norm_topk_prob, bt->mo, nullptr));
-  CK(k_add_rms_norm(ctx, s, bt->h, bt->mo, h.norm, B, H, c.rms_eps, bt->x, bt->dhid));
-  CK(batch_mm(bt, m->lm_head, bt->dhid, B, bt->logits));
-  CK(k_greedy(ctx, s, bt->logits, B, c.vocab, 0, bt->drafts, bt->greedy_scratch));
+  if (exact && small_path(bt, B, world)) {
+    CK(small_mtp(bt, bt->prim, bt->hrow, max_pos + 1, false));
+  } else {
+    CK(mtp_join(bt, bt->prim, bt->hrow));
+    CK(batch_attention(bt, h.q_proj, h.k_proj, h.v_proj, h.o_proj, h.q_norm, h.k_norm, 1, bt->mtp_pos, bt->mtp_kc, bt->mtp_vc, exact, chunk,
+                       nchunks, false));
+    CK(k_add_rms_norm(ctx, s, bt->mx, bt->r, h.post_ln, B, H, c.rms_eps, bt->h, bt->n2));
+    const orn_linear* sg = world > 1 ? bt->mtp_views[0] : h.moe.sw_gate;
+    const orn_linear* su = world > 1 ? bt->mtp_views[1] : h.moe.sw_up;
+    const orn_linear* sd = world > 1 ? bt->mtp_views[2] : h.moe.sw_down;
+    CK(orn_ep_moe_block(group, h.moe.gate, sg, su, sd, h.moe.sh_gate, h.moe.sh_up, h.moe.sh_down, h.moe.sh_egate, bt->n2, B, c.top_k,
+                        c.norm_topk_prob, bt->mo, nullptr));
+    CK(k_add_rms_norm(ctx, s, bt->h, bt->mo, h.norm, B, H, c.rms_eps, bt->x, bt->dhid));
+    CK(batch_mm(bt, m->lm_head, bt->dhid, B, bt->logits));
+    CK(k_greedy(ctx, s, bt->logits, B, c.vocab, 0, bt->drafts, bt->greedy_scratch));
+  }
   mtp_advance_kernel<<<(B + 127) / 128, 128, 0, s>>>(bt->mtp_pos, nullptr, B, 1);
   CK(orn_launch_check(ctx, "mtp_advance"));
   for (int b = 0; b < B; ++b) bt->h_mtp_pos[b] += 1;

@@ -1451,30 +1451,32 @@ __global__ void __launch_bounds__(kDownThreads, 1) k_moe_down(MoeDownParams P, u
 // kernel 4: gated-delta front end + recurrence in one launch
 // ---------------------------------------------------------------------------
 struct GdnParams {
-  const bf16_t* conv;   // [S + T][D]: cached window rows then this call's qkv rows
+  const bf16_t* conv;   // per sequence (conv_stride elements apart): [S + T][D], cached window rows then this call's qkv rows
+  int64_t conv_stride;
   const bf16_t* cw;     // [D][Kc]
-  const bf16_t* a_in;   // [T][Hv]
-  const bf16_t* b_in;   // [T][Hv]
+  const bf16_t* a_in;   // [B][T][Hv]
+  const bf16_t* b_in;   // [B][T][Hv]
   const bf16_t* a_log;  // [Hv]
   const bf16_t* dt_bias;
-  float* ring;          // [nring][Hv][128][128]
-  const int* cur;
-  bf16_t* y;            // [T][Hv][128]
+  float* ring;          // [B][nring][Hv][128][128]
+  const int* cur;       // [B]
+  bf16_t* y;            // [B][T][Hv][128]
   int T, S, Kc, D, Hk, Hv, nring, final_only;
   float q_scale, k_scale, eps;
   // optional epilogue: rms_norm_gated of the outputs (kernels/ornith_norm.metal:119-185) by the
   // last CTA of each head to finish; null `gated_out` leaves y as the only output
-  const bf16_t* z;          // [T][Hv*128] gate rows
+  const bf16_t* z;          // [B][T][Hv*128] gate rows
   const bf16_t* norm_w;     // [128]
-  bf16_t* gated_out;        // [T][Hv*128]
-  unsigned int* arrivals;   // [Hv], zero between launches
+  bf16_t* gated_out;        // [B][T][Hv*128]
+  unsigned int* arrivals;   // [B][Hv], zero between launches
   float norm_eps;
 };
 
 constexpr int kGdnRows = 16;
 constexpr int kGdnMaxT = 4;
+constexpr int kGdnMaxHeads = 960;  // arrival counters of a launch: value heads over all its sequences
 
-// CTA = (head hv, block of kGdnRows state rows).  Threads 0 .. 4*kGdnRows-1 own the state (a row's
+// CTA = (head hv, block of kGdnRows state rows) of sequence blockIdx.z.  Threads 0 .. 4*kGdnRows-1 own the state (a row's
 // 128 floats over 4 lanes) and run the recurrence; the front end is spread over one warp per
 // (q or k, window token), one warp for the block's value rows and one for the gates, so that its
 // out-of-line calls run side by side: 2 T + 2 warps in all.
@@ -1497,8 +1499,11 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
   const int lir = threadIdx.x & 3;
   const size_t ssz = (size_t)p.Hv * 128 * 128;
   const size_t off = ((size_t)hv * 128 + row) * 128 + lir * 32;
-  const int cur = *p.cur;
-  const float* sin = p.ring + (size_t)(cur % p.nring) * ssz + off;
+  const int seq = blockIdx.z, row0 = seq * p.T;  // this sequence's first window row
+  const int cur = p.cur[seq];
+  float* const ring = p.ring + (size_t)seq * p.nring * ssz;
+  const bf16_t* const conv = p.conv + seq * p.conv_stride;
+  const float* sin = ring + (size_t)(cur % p.nring) * ssz + off;
   float S[32];
   if (owner) {  // a thread's 32 state floats are one 128-byte line: four requests of a whole sector each
 #pragma unroll
@@ -1522,7 +1527,7 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
       const int c0 = (isk ? key_dim + hk * 128 : hk * 128) + 4 * lane;
       uint2 xr[4], wr[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) xr[i] = *reinterpret_cast<const uint2*>(p.conv + (size_t)(t + i) * p.D + c0);
+      for (int i = 0; i < 4; ++i) xr[i] = *reinterpret_cast<const uint2*>(conv + (size_t)(t + i) * p.D + c0);
 #pragma unroll
       for (int r = 0; r < 4; ++r) wr[r] = *reinterpret_cast<const uint2*>(p.cw + (size_t)(c0 + r) * 4);
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1553,7 +1558,7 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
         const int cv = 2 * key_dim + hv * 128 + blockIdx.x * kGdnRows + r;
         bf16_t vr[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) vr[i] = p.conv[(size_t)(t + i) * p.D + cv];
+        for (int i = 0; i < 4; ++i) vr[i] = conv[(size_t)(t + i) * p.D + cv];
         const uint2 vw = *reinterpret_cast<const uint2*>(p.cw + (size_t)cv * 4);
         const float vtap[4] = {bf_lo(vw.x), bf_hi(vw.x), bf_lo(vw.y), bf_hi(vw.y)};
         float av = 0.f;
@@ -1563,7 +1568,7 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
       }
     } else if (lane < p.T) {
       // the head's gates of window token `lane`
-      const size_t i = (size_t)lane * p.Hv + hv;
+      const size_t i = (size_t)(row0 + lane) * p.Hv + hv;
       const float ga = bf2f(p.a_in[i]), gb = bf2f(p.b_in[i]), gdt = bf2f(p.dt_bias[hv]), gal = bf2f(p.a_log[hv]);
       const float sp = softplus_bf_call(bfr(ga + gdt));
       const float decay = expf_call(gal);
@@ -1575,7 +1580,7 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
     const int c0 = (warp == 0 ? hk * 128 : key_dim + hk * 128) + 4 * lane;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     for (int i = 0; i < p.Kc; ++i) {
-      const uint2 xv = *reinterpret_cast<const uint2*>(p.conv + (size_t)(t + i) * p.D + c0);
+      const uint2 xv = *reinterpret_cast<const uint2*>(conv + (size_t)(t + i) * p.D + c0);
       const float xs[4] = {bf_lo(xv.x), bf_hi(xv.x), bf_lo(xv.y), bf_hi(xv.y)};
 #pragma unroll
       for (int r = 0; r < 4; ++r) acc[r] = fmaf(xs[r], bf2f(p.cw[(size_t)(c0 + r) * p.Kc + i]), acc[r]);
@@ -1597,13 +1602,13 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
     for (int t = 0; t < p.T; ++t) {
       float acc = 0.f;
       for (int i = 0; i < p.Kc; ++i)
-        acc = fmaf(bf2f(p.conv[(size_t)(t + i) * p.D + c]), bf2f(p.cw[(size_t)c * p.Kc + i]), acc);
+        acc = fmaf(bf2f(conv[(size_t)(t + i) * p.D + c]), bf2f(p.cw[(size_t)c * p.Kc + i]), acc);
       s_v[t][threadIdx.x >> 2] = silu_bf_call(bfr(acc));
     }
   }
   if (threadIdx.x < p.T) {
     const int t = threadIdx.x;
-    const size_t i = (size_t)t * p.Hv + hv;
+    const size_t i = (size_t)(row0 + t) * p.Hv + hv;
     const float sp = softplus_bf_call(bfr(bf2f(p.a_in[i]) + bf2f(p.dt_bias[hv])));
     const float decay = expf_call(bf2f(p.a_log[hv]));
     s_g[t] = expf_call((-decay) * sp);
@@ -1647,10 +1652,10 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
     float o = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
     o = o + __shfl_xor_sync(0xffffffffu, o, 1);
     o = o + __shfl_xor_sync(0xffffffffu, o, 2);
-    if (lir == 0) p.y[((size_t)t * p.Hv + hv) * 128 + row] = f2bf(o);
+    if (lir == 0) p.y[((size_t)(row0 + t) * p.Hv + hv) * 128 + row] = f2bf(o);
     float* sout = nullptr;
-    if (!p.final_only) sout = p.ring + (size_t)((cur + 1 + t) % p.nring) * ssz + off;
-    else if (t + 1 == p.T) sout = p.ring + (size_t)((cur + 1) % p.nring) * ssz + off;
+    if (!p.final_only) sout = ring + (size_t)((cur + 1 + t) % p.nring) * ssz + off;
+    else if (t + 1 == p.T) sout = ring + (size_t)((cur + 1) % p.nring) * ssz + off;
     if (sout != nullptr) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -1668,9 +1673,9 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    const unsigned int prev = atomicAdd(p.arrivals + hv, 1u);
+    const unsigned int prev = atomicAdd(p.arrivals + seq * p.Hv + hv, 1u);
     s_last = (prev == gridDim.x - 1) ? 1u : 0u;
-    if (s_last) atomicExch(p.arrivals + hv, 0u);
+    if (s_last) atomicExch(p.arrivals + seq * p.Hv + hv, 0u);
   }
   __syncthreads();
   if (!s_last) return;
@@ -1678,7 +1683,7 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
   const uint2 wv = __ldg(reinterpret_cast<const uint2*>(p.norm_w + 4 * lane));
   const float wf[4] = {bf_lo(wv.x), bf_hi(wv.x), bf_lo(wv.y), bf_hi(wv.y)};
   for (int t = warp; t < p.T; t += (blockDim.x >> 5)) {
-    const size_t base = ((size_t)t * p.Hv + hv) * 128 + 4 * lane;
+    const size_t base = ((size_t)(row0 + t) * p.Hv + hv) * 128 + 4 * lane;
     const uint2 a2 = __ldcg(reinterpret_cast<const uint2*>(p.y + base));  // written by other CTAs: read through L2
     const uint2 z2 = __ldg(reinterpret_cast<const uint2*>(p.z + base));
     const float xv[4] = {bf_lo(a2.x), bf_hi(a2.x), bf_lo(a2.y), bf_hi(a2.y)};
@@ -1707,18 +1712,25 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
 // kernel 5: q/k norm + rotary + KV append + attention + output gate
 // ---------------------------------------------------------------------------
 struct AttnParams {
-  const bf16_t* qg;      // [T][Hq][2*256]: query | gate
-  const bf16_t* k;       // [T][Hkv][256]
-  const bf16_t* v;       // [T][Hkv][256]
+  const bf16_t* qg;      // [B][T][Hq][2*256]: query | gate
+  const bf16_t* k;       // [B][T][Hkv][256]
+  const bf16_t* v;       // [B][T][Hkv][256]
   const bf16_t* q_norm;  // [256]
   const bf16_t* k_norm;  // [256]
-  bf16_t* kc;            // [Hkv][cap][256]
+  bf16_t* kc;            // [B][Hkv][cap][256]
   bf16_t* vc;
-  const int* pos;
-  bf16_t* out;           // [T][Hq*256] gated attention output
+  const int* pos;        // [B]
+  bf16_t* out;           // [B][T][Hq*256] gated attention output
   int T, Hq, Hkv, cap, rope_dims;
   float lnb, scale, eps;
 };
+
+// the parameters as sequence `seq` sees them
+ORN_D void attn_sequence(AttnParams& p, int seq) {
+  const size_t row = (size_t)seq * p.T, cache = (size_t)seq * p.Hkv * p.cap * 256;
+  p.qg += row * p.Hq * 512; p.k += row * p.Hkv * 256; p.v += row * p.Hkv * 256; p.out += row * p.Hq * 256;
+  p.kc += cache; p.vc += cache; p.pos += seq;
+}
 
 // norm + rope of one 256-wide head row by one warp (8 dims per lane); the
 // result (bfloat16 values as floats) goes to dst[256]
@@ -1850,7 +1862,8 @@ __global__ void __launch_bounds__(1024) k_attn(AttnParams p) {
   __shared__ float s_max[32], s_sum[32], s_f[32];
   pdl_trigger();
   pdl_wait();
-  const int h = blockIdx.x, r = blockIdx.y;
+  const int h = blockIdx.x, seq = blockIdx.y / p.T, r = blockIdx.y - seq * p.T;
+  attn_sequence(p, seq);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int group = p.Hq / p.Hkv;
   const int kvh = h / group;
@@ -2154,11 +2167,11 @@ int f_moe_down(orn_ctx* ctx, cudaStream_t s, int M, const bf16_t* act, const bf1
 int f_gdn(orn_ctx* ctx, cudaStream_t s, const bf16_t* conv, const bf16_t* cw, const bf16_t* a, const bf16_t* b,
           const bf16_t* a_log, const bf16_t* dt_bias, float* ring, int nring, const int* cur, int final_only, int T,
           int Hk, int Hv, int Kc, float eps, bf16_t* y, const bf16_t* z, const bf16_t* norm_w, float norm_eps,
-          bf16_t* gated_out) {
+          bf16_t* gated_out, int B, int64_t conv_stride) {
   if (T > kGdnMaxT) ORN_FAIL(ctx, ORN_ERR_ARG, "fused gdn: at most 4 rows");
   if (!final_only && T + 1 > nring) ORN_FAIL(ctx, ORN_ERR_ARG, "fused gdn: window wider than the state ring");
   GdnParams p;
-  p.conv = conv; p.cw = cw; p.a_in = a; p.b_in = b; p.a_log = a_log; p.dt_bias = dt_bias; p.ring = ring;
+  p.conv = conv; p.conv_stride = conv_stride; p.cw = cw; p.a_in = a; p.b_in = b; p.a_log = a_log; p.dt_bias = dt_bias; p.ring = ring;
   p.cur = cur; p.y = y; p.T = T; p.S = Kc - 1; p.Kc = Kc; p.D = 2 * Hk * 128 + Hv * 128; p.Hk = Hk; p.Hv = Hv;
   p.nring = nring; p.final_only = final_only;
   const float inv_scale = 1.0f / sqrtf(128.0f);
@@ -2167,8 +2180,8 @@ int f_gdn(orn_ctx* ctx, cudaStream_t s, const bf16_t* conv, const bf16_t* cw, co
   p.eps = eps;
   p.z = z; p.norm_w = norm_w; p.gated_out = gated_out; p.norm_eps = norm_eps;
   p.arrivals = reinterpret_cast<unsigned int*>(ctx->dev_err) + 64;
-  if (gated_out != nullptr && Hv > 512) ORN_FAIL(ctx, ORN_ERR_ARG, "fused gdn: more than 512 value heads");
-  dim3 grid(128 / kGdnRows, Hv);
+  if (gated_out != nullptr && B * Hv > kGdnMaxHeads) ORN_FAIL(ctx, ORN_ERR_ARG, "fused gdn: too many value heads");
+  dim3 grid(128 / kGdnRows, Hv, B);
   const dim3 block(gdn_threads(T));
   // Unused dynamic shared memory caps the kernel at two CTAs per SM.  As a programmatic dependent
   // its CTAs become resident while the previous kernel drains, and without the cap the first SMs
@@ -2190,7 +2203,7 @@ int f_gdn(orn_ctx* ctx, cudaStream_t s, const bf16_t* conv, const bf16_t* cw, co
 // order), the partials (max, sum, out[256]) of all 32 groups go through global memory, and the CTA that
 // stores the last of them runs the same merge: the result has the bits of the one-CTA kernel.
 constexpr int kAttnSplit = 4;
-constexpr int kAttnMaxHeads = 128;
+constexpr int kAttnMaxHeads = 256;  // query heads over all sequences of a launch
 constexpr int kAttnPart = 260;  // floats per group partial: out[256], max, sum, pad
 __global__ void __launch_bounds__(256) k_attn_split(AttnParams p, float* part, int* arrivals) {
   constexpr int HD = 256;
@@ -2201,7 +2214,9 @@ __global__ void __launch_bounds__(256) k_attn_split(AttnParams p, float* part, i
   __shared__ int s_last;
   pdl_trigger();
   pdl_wait();
-  const int h = blockIdx.x, r = blockIdx.y, z = blockIdx.z;
+  const int h = blockIdx.x, seq = blockIdx.y / p.T, r = blockIdx.y - seq * p.T, z = blockIdx.z;
+  attn_sequence(p, seq);
+  const int slot = (seq * p.Hq + h) * kGdnMaxT + r;  // of the partials and the arrival counters
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = 8 * z + warp;  // this warp's key group
   const int group = p.Hq / p.Hkv;
@@ -2230,23 +2245,23 @@ __global__ void __launch_bounds__(256) k_attn_split(AttnParams p, float* part, i
   float mx = -INFINITY, sm = 0.f;
   attn_walk<8>(p, s_knew, qs, grp, L, pos, kvh, lane, o, mx, sm);
   // this group's partial to global memory
-  float* mine = part + (((size_t)h * kGdnMaxT + r) * 32 + grp) * kAttnPart;
+  float* mine = part + ((size_t)slot * 32 + grp) * kAttnPart;
   *reinterpret_cast<float4*>(mine + 8 * lane) = make_float4(o[0], o[1], o[2], o[3]);
   *reinterpret_cast<float4*>(mine + 8 * lane + 4) = make_float4(o[4], o[5], o[6], o[7]);
   if (lane == 0) { mine[HD] = mx; mine[HD + 1] = sm; }
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&arrivals[h * kGdnMaxT + r], 1) == kAttnSplit - 1 ? 1 : 0;
+  if (threadIdx.x == 0) s_last = atomicAdd(&arrivals[slot], 1) == kAttnSplit - 1 ? 1 : 0;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  const float* all = part + ((size_t)h * kGdnMaxT + r) * 32 * kAttnPart;
+  const float* all = part + (size_t)slot * 32 * kAttnPart;
   for (int i = threadIdx.x; i < 32 * HD; i += blockDim.x) s_o[i / HD][i % HD] = __ldcg(all + (size_t)(i / HD) * kAttnPart + (i % HD));
   if (threadIdx.x < 32) {
     s_max[threadIdx.x] = __ldcg(all + (size_t)threadIdx.x * kAttnPart + HD);
     s_sum[threadIdx.x] = __ldcg(all + (size_t)threadIdx.x * kAttnPart + HD + 1);
   }
-  if (threadIdx.x == 0) arrivals[h * kGdnMaxT + r] = 0;  // ready for the next launch
+  if (threadIdx.x == 0) arrivals[slot] = 0;  // ready for the next launch
   __syncthreads();
   if (warp == 0) {
     const float M = warp_max(s_max[lane]);
@@ -2273,7 +2288,7 @@ __global__ void __launch_bounds__(256) k_attn_split(AttnParams p, float* part, i
 
 int f_attn(orn_ctx* ctx, cudaStream_t s, const bf16_t* qg, const bf16_t* k, const bf16_t* v, const bf16_t* q_norm,
            const bf16_t* k_norm, bf16_t* kc, bf16_t* vc, const int* pos, int T, int Hq, int Hkv, int hd, int cap,
-           int rope_dims, float lnb, float eps, bf16_t* out, int long_context) {
+           int rope_dims, float lnb, float eps, bf16_t* out, int long_context, int B) {
   if (hd != 256) ORN_FAIL(ctx, ORN_ERR_ARG, "fused attention: head_dim must be 256");
   if (T > kGdnMaxT) ORN_FAIL(ctx, ORN_ERR_ARG, "fused attention: at most 4 rows");
   AttnParams p;
@@ -2287,12 +2302,12 @@ int f_attn(orn_ctx* ctx, cudaStream_t s, const bf16_t* qg, const bf16_t* k, cons
       ORN_CHECK_CUDA(ctx, cudaMalloc((void**)&ctx->attn_arrivals, sizeof(int) * kAttnMaxHeads * kGdnMaxT));
       ORN_CHECK_CUDA(ctx, cudaMemset(ctx->attn_arrivals, 0, sizeof(int) * kAttnMaxHeads * kGdnMaxT));
     }
-    if (Hq > kAttnMaxHeads) ORN_FAIL(ctx, ORN_ERR_ARG, "fused attention: more than 128 query heads");
-    dim3 sgrid(Hq, T, kAttnSplit);
+    if (B * Hq > kAttnMaxHeads) ORN_FAIL(ctx, ORN_ERR_ARG, "fused attention: more than 256 query heads");
+    dim3 sgrid(Hq, B * T, kAttnSplit);
     ORN_CHECK_CUDA(ctx, orn_launch_dependent(ctx, s, 4, k_attn_split, sgrid, dim3(256), 0, p, ctx->attn_partial, ctx->attn_arrivals));
     return orn_launch_check(ctx, "k_attn_split");
   }
-  dim3 grid(Hq, T);
+  dim3 grid(Hq, B * T);
   ORN_CHECK_CUDA(ctx, orn_launch_dependent(ctx, s, 4, k_attn, grid, dim3(1024), 0, p));
   return orn_launch_check(ctx, "k_attn");
 }

@@ -949,6 +949,9 @@ uint64_t splitmix64(uint64_t x) {
 
 int orn_model_finalize(orn_model* m) { return finalize(m); }
 bool orn_wide_exact() { return wide_exact(); }
+bool orn_use_fused(const orn_model* m) { return use_fused(m); }
+bool orn_moe_fusable(const Moe& moe) { return moe_fusable(moe); }
+int orn_long_context(int keys) { return long_context(keys); }
 int orn_conv_dim(const orn_config& c) { return conv_dim(c); }
 
 extern "C" {

@@ -125,4 +125,9 @@ struct orn_cache {
 int orn_model_finalize(orn_model* m);
 // ORN_WIDE_EXACT=1: wide paths compute their products with the row-invariant mat-vec kernels
 bool orn_wide_exact();
+// the fused decode kernels serve this model / this MoE block (ORN_UNFUSED=1: never)
+bool orn_use_fused(const orn_model* m);
+bool orn_moe_fusable(const Moe& moe);
+// whether a cache of this many keys takes the split form of the fused attention
+int orn_long_context(int keys);
 int orn_conv_dim(const orn_config& c);
