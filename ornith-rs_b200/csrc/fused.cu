@@ -42,9 +42,8 @@ struct SmallDiv {
   ORN_D int operator()(int n) const { return d > 1 ? (int)__umulhi((uint32_t)n, mg) : n; }
 };
 // four at once: the evaluations interleave in the pipelines instead of running one after another
-__device__ __noinline__ void expf4_call(float* v) {
-  const float a = orn_expf(v[0]), b = orn_expf(v[1]), c = orn_expf(v[2]), d = orn_expf(v[3]);
-  v[0] = a; v[1] = b; v[2] = c; v[3] = d;
+__device__ __noinline__ float4 expf4_call(float4 v) {
+  return make_float4(orn_expf(v.x), orn_expf(v.y), orn_expf(v.z), orn_expf(v.w));
 }
 __device__ __noinline__ float silu_bf_call(float x) { return orn_silu_bf(x); }
 __device__ __noinline__ float sigmoid_bf_call(float x) { return orn_sigmoid_bf(x); }
@@ -141,9 +140,10 @@ ORN_D void stage_zero_tail(const XStage& X) {
 // the CTA may stage while other warps do something else); no sync inside.  A thread owns whole
 // units of any row (rows x unit slots are one flat index space, so short rows keep every thread
 // busy): it moves the unit's P pieces to their permuted places and, for the formats that need it,
-// adds the unit's elements in ascending order into the staged sum.
+// adds the unit's elements in ascending order into the staged sum.  (The stage goes by value: a reference
+// taken by an out-of-line function would keep every kernel's stages in local memory.)
 template <int KIND>
-__device__ __noinline__ void stage_fill_part(const float* lin, int stride, const XStage& X, int tid, int nthreads) {
+__device__ __noinline__ void stage_fill_part(const float* lin, int stride, XStage X, int tid, int nthreads) {
   constexpr int P = Lay<KIND>::P, NS = Lay<KIND>::NS;
   const int padded = X.S * 32;  // unit slots per row, including the empty tail
   const int total = X.rows * padded;
@@ -171,7 +171,7 @@ __device__ __noinline__ void stage_fill_part(const float* lin, int stride, const
 
 // the same by every thread of the CTA
 template <int KIND>
-__device__ __noinline__ void stage_fill(const float* lin, int stride, const XStage& X) {
+__device__ __noinline__ void stage_fill(const float* lin, int stride, XStage X) {
   stage_fill_part<KIND>(lin, stride, X, threadIdx.x, blockDim.x);
 }
 ORN_D void stage_fill_kind(int kind, const float* lin, int stride, const XStage& X) {
@@ -804,7 +804,7 @@ ORN_D void run_prologue(const Prologue& P, const AddNormIn<M>& in, float* lin, f
         const int c = base + j * step;
         if (c < M * K) {
           const float4 f = make_float4(bf_lo(av[j].x), bf_hi(av[j].x), bf_lo(av[j].y), bf_hi(av[j].y));
-          const int m = c / K, k = c - m * K;
+          const int m = (M > 1 && c >= K) + (M > 2 && c >= 2 * K) + (M > 3 && c >= 3 * K), k = c - m * K;
           if (MASK & (1 << ORN_Q4K)) stage_piece<ORN_Q4K>(X[ORN_Q4K], m, k, f);
           if (MASK & (1 << ORN_Q6K)) stage_piece<ORN_Q6K>(X[ORN_Q6K], m, k, f);
           if (MASK & (1 << ORN_A8)) stage_piece<ORN_A8>(X[ORN_A8], m, k, f);
@@ -932,7 +932,7 @@ struct Cursor {
 constexpr int kMaxAcc = 32;  // R * pad(M) never exceeds this
 
 template <int M, int MASK, int KC>
-__global__ void __launch_bounds__(kFusedThreads, 1) k_norm_gemv(Prologue P, RowJobs J, uint32_t slot_bytes, int depth,
+__global__ void __launch_bounds__(kFusedThreads, 1) k_norm_gemv(const __grid_constant__ Prologue P, const __grid_constant__ RowJobs J, uint32_t slot_bytes, int depth,
                                                                 uint32_t ring_off, int late, int* err) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   float* smem = reinterpret_cast<float*>(smem_raw);
@@ -1093,7 +1093,8 @@ __device__ __noinline__ void warp_softmax_topk_n(const bf16_t* logits, int n, in
       float ev[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) ev[i] = xv[vw][i] - mx;  // absent entries are -inf - mx: their exp is not used
-      expf4_call(ev);
+      const float4 e4 = expf4_call(make_float4(ev[0], ev[1], ev[2], ev[3]));
+      ev[0] = e4.x; ev[1] = e4.y; ev[2] = e4.z; ev[3] = e4.w;
       float acc = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -1152,7 +1153,7 @@ ORN_D void warp_softmax_topk(const bf16_t* logits, int n, int k, float* probs, f
 }
 
 template <int KIND, int KC>
-__global__ void __launch_bounds__(kMoeThreads, 1) k_moe_up(MoeUpParams P, uint32_t slot_bytes, int depth,
+__global__ void __launch_bounds__(kMoeThreads, 1) k_moe_up(const __grid_constant__ MoeUpParams P, uint32_t slot_bytes, int depth,
                                                              uint32_t ring_off, int* err) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   float* smem = reinterpret_cast<float*>(smem_raw);
@@ -1287,7 +1288,7 @@ struct MoeDownParams {
 constexpr int kDownThreads = 512;
 
 template <int KIND, int KC>
-__global__ void __launch_bounds__(kDownThreads, 1) k_moe_down(MoeDownParams P, uint32_t slot_bytes, int depth,
+__global__ void __launch_bounds__(kDownThreads, 1) k_moe_down(const __grid_constant__ MoeDownParams P, uint32_t slot_bytes, int depth,
                                                                 uint32_t ring_off, int* err) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   float* smem = reinterpret_cast<float*>(smem_raw);
@@ -1484,7 +1485,7 @@ constexpr int kGdnStateThreads = kGdnRows * 4;
 __host__ __device__ constexpr int gdn_threads(int T) { return 32 * (2 * T + 2); }
 
 template <bool TAPS4>  // TAPS4: the convolution has 4 taps (every Qwen3.5 artifact); else any width
-__global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(GdnParams p) {
+__global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(const __grid_constant__ GdnParams p) {
   __shared__ float s_q[kGdnMaxT][128], s_k[kGdnMaxT][128], s_v[kGdnMaxT][kGdnRows];
   __shared__ float s_g[kGdnMaxT], s_beta[kGdnMaxT];
   pdl_trigger();
