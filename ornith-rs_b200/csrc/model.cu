@@ -33,23 +33,36 @@ __global__ void iota_div_kernel(uint32_t* lhs, uint32_t* ident, int n, int k) {
 __global__ void set_u32_kernel(uint32_t* p, uint32_t v) { *p = v; }
 __global__ void set_int_kernel(int* p, int v) { *p = v; }
 // mailbox = {primary, force flag[3], force token[3]} written by the host before each cycle;
-// slot < 0 places the primary at the head of the window, slot i applies draft i's override
-__global__ void mailbox_apply_kernel(const uint32_t* mb, uint32_t* window, int slot) {
-  if (slot < 0) window[0] = mb[0];
-  else if (mb[1 + slot] != 0) window[slot + 1] = mb[4 + slot];
+// slot < 0 places the primary at the head of the window (and empties the draft head's cache where each
+// cycle starts with a fresh one), slot i applies draft i's override
+__global__ void mailbox_apply_kernel(const uint32_t* mb, uint32_t* window, int slot, int* fresh_pos /*nullable*/) {
+  if (slot < 0) {
+    window[0] = mb[0];
+    if (fresh_pos != nullptr) *fresh_pos = 0;
+  } else if (mb[1 + slot] != 0) window[slot + 1] = mb[4 + slot];
 }
 __global__ void add_int_kernel(int* p, int v) { *p += v; }
 // FrSpec::map_id (src/frspec.rs:137-148, kernels/moe.metal:68-74 gather_u32)
 __global__ void gather_u32_kernel(const uint32_t* table, const uint32_t* idx, uint32_t* out) {
   *out = table[*idx];
 }
-// rows keep..keep+S-1 of every layer's conv window move to rows 0..S-1
-// (TrunkCapture::rewind, qwen3_5.rs:324-348: conv = slice of conv_input)
-__global__ void conv_shift_kernel(bf16_t* const* bufs, int S, int D, int keep) {
-  bf16_t* b = bufs[blockIdx.y];
-  int c = blockIdx.x * blockDim.x + threadIdx.x;  // over D/8 16-byte pieces
-  if (c >= D / 8) return;
-  uint4* p = reinterpret_cast<uint4*>(b);
+// The bookkeeping of a window in one launch: positions, state cursors and conv windows move by the kept
+// rows (rows keep .. keep+S-1 of a conv window become its rows 0 .. S-1: TrunkCapture::rewind, qwen3_5.rs:324-348), the draft head's position by mtp_step (mtp_pos nullable), the hidden row the
+// next draft reads is copied (hrow nullable).  grid: (pieces of a conv row, layers)
+__global__ void commit_window_kernel(int* pos, int keep, int* cur, int ring_step, int* mtp_pos, int mtp_step, bf16_t* const* bufs, int n_bufs,
+                                     int S, int D, const bf16_t* hsrc, bf16_t* hrow, int H) {
+  if (blockIdx.y == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      *pos += keep;
+      *cur += ring_step;
+      if (mtp_pos != nullptr) *mtp_pos += mtp_step;
+    }
+    if (hrow != nullptr)
+      for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < H; i += gridDim.x * blockDim.x) hrow[i] = hsrc[i];
+  }
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;  // over D/8 16-byte pieces
+  if (blockIdx.y >= n_bufs || c >= D / 8) return;
+  uint4* p = reinterpret_cast<uint4*>(bufs[blockIdx.y]);
   for (int j = 0; j < S; ++j) p[(size_t)j * (D / 8) + c] = p[(size_t)(j + keep) * (D / 8) + c];
 }
 __global__ void copy_bf16_kernel(const bf16_t* src, bf16_t* dst, int n) {
@@ -109,8 +122,9 @@ int build_workspace(orn_model* m) {
   CK(ws_alloc(m, &w.inds, R * k)); CK(ws_alloc(m, &w.lhs, R * k)); CK(ws_alloc(m, &w.ident, R * k));
   CK(ws_alloc(m, &w.logits, R * (size_t)c.vocab)); CK(ws_alloc(m, &w.dlogits, (size_t)c.vocab));
   CK(ws_alloc(m, &w.greedy_scratch, greedy_scratch_floats(kMaxRows, c.vocab)));
-  CK(ws_alloc(m, &w.ids, (size_t)8)); CK(ws_alloc(m, &w.window, (size_t)8));
-  CK(ws_alloc(m, &w.targets, (size_t)8)); CK(ws_alloc(m, &w.local, (size_t)1)); CK(ws_alloc(m, &w.mailbox, (size_t)16));
+  CK(ws_alloc(m, &w.ids, (size_t)8)); CK(ws_alloc(m, &w.window, (size_t)16));
+  w.targets = w.window + 8;  // one copy brings both to the host
+  CK(ws_alloc(m, &w.local, (size_t)1)); CK(ws_alloc(m, &w.mailbox, (size_t)16));
   CK(ws_alloc(m, &w.vh, R * H)); CK(ws_alloc(m, &w.hrow, H)); CK(ws_alloc(m, &w.dh, R * H));
   CK(ws_alloc(m, &w.memb, R * H)); CK(ws_alloc(m, &w.me, R * H)); CK(ws_alloc(m, &w.mh, R * H));
   CK(ws_alloc(m, &w.mjoined, R * 2 * H)); CK(ws_alloc(m, &w.mx, R * H));
@@ -312,23 +326,19 @@ int gdn_layer(orn_model* m, const Layer& ly, const bf16_t* x, int T, bf16_t* con
 
 // commit `keep` of the window's tokens: KV offset, conv windows, and the state
 // ring, which moves by one slot per kept snapshot (`ring_step` = keep after a
-// capture window, 1 after a call that kept only its final state)
-int commit(orn_cache* c, int keep, int ring_step) {
+// capture window, 1 after a call that kept only its final state); mtp_step moves the draft head's position,
+// hsrc is the hidden row that the next draft reads
+int commit(orn_cache* c, int keep, int ring_step, int mtp_step = 0, const bf16_t* hsrc = nullptr) {
   orn_model* m = c->m;
   orn_ctx* ctx = m->ctx;
-  cudaStream_t s = ctx->stream;
-  add_int_kernel<<<1, 1, 0, s>>>(c->pos, keep);
-  CK(orn_launch_check(ctx, "add_int"));
-  add_int_kernel<<<1, 1, 0, s>>>(c->cur, ring_step);
-  CK(orn_launch_check(ctx, "add_int"));
-  if (c->n_gdn > 0) {
-    const int S = m->cfg.gdn_conv_kernel - 1, D = conv_dim(m->cfg);
-    dim3 grid((D / 8 + 127) / 128, c->n_gdn);
-    conv_shift_kernel<<<grid, 128, 0, s>>>(c->conv_table, S, D, keep);
-    CK(orn_launch_check(ctx, "conv_shift"));
-  }
+  const int S = m->cfg.gdn_conv_kernel - 1, D = conv_dim(m->cfg);
+  dim3 grid((D / 8 + 127) / 128, std::max(1, c->n_gdn));
+  commit_window_kernel<<<grid, 128, 0, ctx->stream>>>(c->pos, keep, c->cur, ring_step, mtp_step != 0 ? c->mtp_pos : nullptr, mtp_step, c->conv_table,
+                                                      c->n_gdn, S, D, hsrc, hsrc ? m->ws.hrow : nullptr, m->cfg.hidden);
+  CK(orn_launch_check(ctx, "commit_window"));
   c->h_pos += keep;
   c->h_cur += ring_step;
+  c->h_mtp_pos += mtp_step;
   return ORN_OK;
 }
 
@@ -608,13 +618,15 @@ int head_greedy_dev(orn_model* m, const orn_linear* head, const bf16_t* hidden, 
 // One speculative cycle on the device: window[0] = primary, `want` draft levels
 // (mtp_generate.rs:99-135) with the harness's forced-draft overrides read from the
 // mailbox, then the verify forward with every row's greedy target.
-int cycle_body(orn_model* m, orn_cache* c, int want, bool use_frspec) {
+int cycle_body(orn_model* m, orn_cache* c, int want, bool use_frspec, bool fresh) {
   orn_ctx* ctx = m->ctx;
   cudaStream_t s = ctx->stream;
   Workspace& w = m->ws;
   const int H = m->cfg.hidden;
   const orn_linear* dlm = use_frspec ? m->fr_head : m->lm_head;
-  mailbox_apply_kernel<<<1, 1, 0, s>>>(w.mailbox, w.window, -1);
+  ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(w.mailbox, c->mailbox_h, 16 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+  mailbox_apply_kernel<<<1, 1, 0, s>>>(w.mailbox, w.window, -1, fresh ? c->mtp_pos : nullptr);
+  if (fresh) c->h_mtp_pos = 0;
   CK(orn_launch_check(ctx, "mailbox_apply"));
   const bf16_t* dh_in = w.hrow;
   for (int i = 0; i < want; ++i) {
@@ -627,33 +639,51 @@ int cycle_body(orn_model* m, orn_cache* c, int want, bool use_frspec) {
     } else {
       CK(k_greedy(ctx, s, w.dlogits, 1, dlm->O, 0, w.window + i + 1, w.greedy_scratch));
     }
-    mailbox_apply_kernel<<<1, 1, 0, s>>>(w.mailbox, w.window, i);
+    mailbox_apply_kernel<<<1, 1, 0, s>>>(w.mailbox, w.window, i, nullptr);
     CK(orn_launch_check(ctx, "mailbox_apply"));
     dh_in = dh_out;
   }
-  return forward_greedy_dev(m, c, w.window, want + 1, true, w.vh, w.targets);
+  CK(forward_greedy_dev(m, c, w.window, want + 1, true, w.vh, w.targets));
+  // window and targets in one copy to pinned memory: the one host round trip of the cycle (mtp_generate.rs:250-254)
+  ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(c->mailbox_h + 16, w.window, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  return ORN_OK;
+}
+
+// What follows the acceptance of k of `want` drafts: the window's commit and, under the Committed policy, the
+// re-encode of the accepted drafts into the draft head's cache (mtp_generate.rs:292-301)
+int accept_body(orn_model* m, orn_cache* c, int want, int k, bool committed) {
+  Workspace& w = m->ws;
+  // the head's cache stood at `off` when the cycle began and at off + want now: it keeps one row, then the accepted
+  CK(commit(c, k + 1, k + 1, committed ? 1 - want : 0, w.vh + (size_t)k * m->cfg.hidden));
+  if (committed && k > 0) return mtp_step(m, c, w.vh, w.window + 1, k, nullptr, w.dh, nullptr, true);
+  return ORN_OK;
 }
 
 // one autoregressive step: the token in targets[0] goes in, its successor comes out
 int ar_body(orn_model* m, orn_cache* c) {
   Workspace& w = m->ws;
-  return forward_greedy_dev(m, c, w.targets, 1, false, w.vh, w.targets);
+  CK(forward_greedy_dev(m, c, w.targets, 1, false, w.vh, w.targets));
+  ORN_CHECK_CUDA(m->ctx, cudaMemcpyAsync(c->mailbox_h + 24, w.targets, sizeof(uint32_t), cudaMemcpyDeviceToHost, m->ctx->stream));
+  return ORN_OK;
 }
 
 // Run a step body eagerly the first time a shape is seen, capture it into a CUDA
 // graph the second time and replay it afterwards.  The host-side bookkeeping the
 // body does (positions, counters) is repeated by hand on a replay.
-int run_step(orn_model* m, orn_cache* c, int kind /*0 cycle, 1 ar, 2 prefill rows*/, int want, bool use_frspec) {
+int run_step(orn_model* m, orn_cache* c, int kind /*0 cycle, 1 ar, 2 prefill rows, 3 acceptance*/, int want, bool use_frspec, bool committed = false,
+             int accepted = 0) {
   orn_ctx* ctx = m->ctx;
   cudaStream_t s = ctx->stream;
   const int n_rows = want + 1;
   // the launch shape of the fused attention changes once a cache passes kLongContext keys (the key
   // groups of a head spread over four CTAs): such steps are graphs of their own
-  const int key = kind * 64 + want * 2 + (use_frspec ? 1 : 0) + 4096 * long_context(c->h_pos + n_rows) +
-                  8192 * (kind == 0 ? long_context(c->h_mtp_pos + want) : 0);
+  const bool fresh = kind == 0 && !committed;  // the Cycle policy: an empty draft cache each cycle
+  const int mtp_end = kind == 0 ? (fresh ? 0 : c->h_mtp_pos) + want : kind == 3 ? c->h_mtp_pos - want + 1 + accepted : 0;
+  const int key = kind * 64 + want * 2 + (use_frspec ? 1 : 0) + (committed ? 256 : 0) + accepted * 512 +
+                  4096 * (kind == 3 ? 0 : long_context(c->h_pos + n_rows)) + 8192 * long_context(mtp_end);
   orn_cache::StepGraph& g = c->graphs[key];
-  if (c->h_pos + n_rows > m->cfg.max_ctx) ORN_FAIL(ctx, ORN_ERR_STATE, "forward: context exceeds max_ctx");
-  if (kind == 0 && c->h_mtp_pos + want > m->cfg.max_ctx) ORN_FAIL(ctx, ORN_ERR_STATE, "mtp: context exceeds max_ctx");
+  if (kind != 3 && c->h_pos + n_rows > m->cfg.max_ctx) ORN_FAIL(ctx, ORN_ERR_STATE, "forward: context exceeds max_ctx");
+  if (mtp_end > m->cfg.max_ctx) ORN_FAIL(ctx, ORN_ERR_STATE, "mtp: context exceeds max_ctx");
   static int no_graph = -1;
   if (no_graph < 0) { const char* e = getenv("ORN_NO_GRAPH"); no_graph = (e && e[0] == '1') ? 1 : 0; }
   const bool eager = no_graph || ctx->kt != nullptr;  // per-kernel times need eager launches
@@ -667,13 +697,17 @@ int run_step(orn_model* m, orn_cache* c, int kind /*0 cycle, 1 ar, 2 prefill row
   if (g.exec != nullptr && !eager) {
     ORN_CHECK_CUDA(ctx, cudaGraphLaunch(g.exec, s));
     ctx->launches += g.launches;
-    if (kind == 0) { c->h_mtp_pos += want; c->cap_T = n_rows; }
-    else if (kind == 1) { c->h_pos += 1; c->h_cur += 1; }
+    if (kind == 0) { c->h_mtp_pos = mtp_end; c->cap_T = n_rows; }
+    else if (kind == 3) {
+      c->h_pos += accepted + 1; c->h_cur += accepted + 1;
+      if (committed) c->h_mtp_pos = mtp_end;
+    } else if (kind == 1) { c->h_pos += 1; c->h_cur += 1; }
     else { c->h_pos += n_rows; c->h_cur += 1; }
     return ORN_OK;
   }
   auto body = [&]() {
-    if (kind == 0) return cycle_body(m, c, want, use_frspec);
+    if (kind == 0) return cycle_body(m, c, want, use_frspec, fresh);
+    if (kind == 3) return accept_body(m, c, want, accepted, committed);
     if (kind == 1) return ar_body(m, c);
     return forward_dev(m, c, m->ws.ids, n_rows, false, nullptr, nullptr);  // a window of prompt rows
   };
@@ -1199,7 +1233,7 @@ int32_t orn_cache_create(orn_model* m, orn_cache** out) {
     if (rc == ORN_OK) rc = orn_upload(m->ctx, k->conv_table, table.data(), sizeof(bf16_t*) * table.size());
   }
   if (rc != ORN_OK) { orn_cache_destroy(k); return rc; }
-  if (cudaMallocHost((void**)&k->mailbox_h, 16 * sizeof(uint32_t)) != cudaSuccess) {
+  if (cudaMallocHost((void**)&k->mailbox_h, 32 * sizeof(uint32_t)) != cudaSuccess) {
     orn_cache_destroy(k);
     ORN_FAIL(m->ctx, ORN_ERR_ALLOC, "cache_create: pinned mailbox");
   }
@@ -1302,11 +1336,11 @@ int32_t orn_generate_step(orn_model* m, orn_cache* c, const uint32_t* prompt, in
   int done = 0;
   CK(prefill(m, c, prompt, n_prompt, prefill_step, &done));
   cudaEventRecord(m->ev[3], ctx->stream);
-  uint32_t y = 0;
-  // step (generate.rs:139-150) on the last prompt token
-  CK(upload_ids(m, prompt + done, 1));
-  CK(forward_greedy_dev(m, c, w.ids, 1, false, w.vh, w.targets));
-  CK(orn_download(ctx, &y, w.targets, 4));
+  // step (generate.rs:139-150) on the last prompt token, as one more autoregressive step
+  ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(w.targets, prompt + done, sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->stream));
+  CK(run_step(m, c, 1, 0, false));
+  ORN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  uint32_t y = c->mailbox_h[24];
   {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, m->ev[2], m->ev[3]);
@@ -1318,12 +1352,12 @@ int32_t orn_generate_step(orn_model* m, orn_cache* c, const uint32_t* prompt, in
     // the next step is taken before the token is handed out (generate.rs:195-205);
     // the sampled token stays on the device and feeds the next forward directly
     CK(run_step(m, c, 1, 0, false));
-    uint32_t next = 0;
-    CK(orn_download(ctx, &next, w.targets, 4));
     m->prof.ar_steps += 1;
     n += 1;
-    if (!on_token(y, user)) break;
-    y = next;
+    const bool more = on_token(y, user) != 0;  // while the step runs
+    ORN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (!more) break;
+    y = c->mailbox_h[24];
   }
   cudaEventRecord(m->ev[3], ctx->stream);
   CK(orn_sync(ctx));
@@ -1360,25 +1394,24 @@ int32_t orn_generate_step_mtp(orn_model* m, orn_cache* c, const uint32_t* prompt
   int done = 0;
   CK(prefill(m, c, prompt, n_prompt, prefill_step, &done));
   cudaEventRecord(m->ev[3], s);
-  CK(upload_ids(m, prompt + done, 1));
-  CK(forward_greedy_dev(m, c, w.ids, 1, false, w.hrow, w.targets));
-  uint32_t primary = 0;
-  CK(orn_download(ctx, &primary, w.targets, 4));
+  ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(w.targets, prompt + done, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+  CK(run_step(m, c, 1, 0, false));
+  copy_bf16_kernel<<<(H + 255) / 256, 256, 0, s>>>(w.vh, w.hrow, H);
+  CK(orn_launch_check(ctx, "copy_bf16"));
+  ORN_CHECK_CUDA(ctx, cudaStreamSynchronize(s));
+  uint32_t primary = c->mailbox_h[24];
   {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, m->ev[2], m->ev[3]);
     m->prof.prefill_ms = ms;
   }
   cudaEventRecord(m->ev[2], s);
-  const orn_linear* dlm = use_frspec ? m->fr_head : m->lm_head;
+  const bool committed = policy == ORN_POLICY_COMMITTED;
   int emitted = 0;
   uint64_t cycle_idx = 0;
   CK(set_mtp_pos(c, 0));
-  uint32_t hbuf[16];
   bool stop = false;
   while (!stop) {
-    if (policy == ORN_POLICY_CYCLE) CK(set_mtp_pos(c, 0));  // a fresh cache each cycle
-    const int cycle_off = c->h_mtp_pos;
     int want = max_tokens - (emitted + 1);
     if (want < 0) want = 0;
     if (want > depth) want = depth;
@@ -1393,19 +1426,15 @@ int32_t orn_generate_step_mtp(orn_model* m, orn_cache* c, const uint32_t* prompt
         if (uni < force->p) { mb[1 + i] = 1; mb[4 + i] = force->stream[emitted + 1 + i]; }
       }
     }
-    ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(w.mailbox, mb, 16 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-    CK(run_step(m, c, 0, want, use_frspec != 0));
+    CK(run_step(m, c, 0, want, use_frspec != 0, committed));
     m->prof.draft_steps += want;
     if (want > 0) { stats->cycles += 1; stats->drafted += want; }
     cycle_idx += 1;
-    const int n_rows = want + 1;
     m->prof.verify_steps += 1;
-    // the one host round trip of the cycle (mtp_generate.rs:250-254)
-    ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(hbuf, w.targets, 4 * (size_t)n_rows, cudaMemcpyDeviceToHost, s));
-    ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(hbuf + 8, w.window, 4 * (size_t)n_rows, cudaMemcpyDeviceToHost, s));
     ORN_CHECK_CUDA(ctx, cudaStreamSynchronize(s));
-    const uint32_t* targets = hbuf;
-    const uint32_t* window = hbuf + 8;
+    uint32_t window[8];  // (the next cycle's copy may land in the pinned words while tokens are handed out)
+    memcpy(window, c->mailbox_h + 16, sizeof window);
+    const uint32_t* targets = c->mailbox_h + 24;
     int k = 0;
     while (k < want) {
       stats->reached_by_depth[k] += 1;
@@ -1415,13 +1444,8 @@ int32_t orn_generate_step_mtp(orn_model* m, orn_cache* c, const uint32_t* prompt
       k += 1;
     }
     const uint32_t next_primary = targets[k];
-    CK(orn_cache_rewind(c, k + 1));
-    if (policy == ORN_POLICY_COMMITTED) {
-      CK(set_mtp_pos(c, cycle_off + 1));
-      if (k > 0) CK(mtp_step(m, c, w.vh, w.window + 1, k, nullptr, w.dh, nullptr, true));
-    }
-    copy_bf16_kernel<<<(H + 255) / 256, 256, 0, s>>>(w.vh + (size_t)k * H, w.hrow, H);
-    CK(orn_launch_check(ctx, "copy_bf16"));
+    c->cap_T = 0;
+    CK(run_step(m, c, 3, want, false, committed, k));
     for (int i = 0; i <= k; ++i) {
       emitted += 1;
       if (!on_token(window[i], user)) { stop = true; break; }

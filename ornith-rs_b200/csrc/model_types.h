@@ -118,7 +118,7 @@ struct orn_cache {
     int fr_gen = 0;  // orn_model::fr_gen at capture time (FR-Spec graphs hold the pruned head's addresses)
   };
   std::map<int, StepGraph> graphs;
-  uint32_t* mailbox_h = nullptr;  // pinned
+  uint32_t* mailbox_h = nullptr;  // pinned: [0..16) to the device, [16..24) window and [24..32) targets back
 };
 
 // resolves every weight name the forward pass needs and builds the scratch (idempotent)
