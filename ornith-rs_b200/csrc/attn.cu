@@ -64,6 +64,85 @@ __global__ void kv_append_kernel(const bf16_t* k, const bf16_t* v, int T, int Hk
   reinterpret_cast<uint4*>(vc)[dst] = reinterpret_cast<const uint4*>(v)[src];
 }
 
+// The attention front of rows [rows] in one launch: query heads out of the projection's [row, head, query |
+// gate] layout, per-head norm, RoPE; key heads the same and into the cache with their value rows
+// (split_qgate, rms_norm, rope, kv_append: the same values).  A warp owns one (row, head): lane l holds
+// elements 4l .. 4l+3 and 128 + 4l .. 128 + 4l+3, the two virtual warps of the norm's sum.  head_dim 256,
+// rope_dims a multiple of 8 and at most 128 (a rotated pair lies in two lanes' first halves).
+// 2048 rows x 18 heads: six launches, 82 us -> one, 22 us; 128 rows: 5 us.
+struct FrontRows {
+  const bf16_t *qg, *k, *v;   // [rows][Hq][512], [rows][Hkv][256], [rows][Hkv][256]
+  const bf16_t *q_norm, *k_norm;
+  bf16_t *q, *kc, *vc;        // q [rows][Hq][256]; caches [seq][Hkv][cap][256]
+  const int* pos;             // position of each sequence's first row
+  int rows, Tb, Hq, Hkv, cap, dims;
+  float lnb, eps;
+};
+__global__ void __launch_bounds__(256) attn_front_kernel(const __grid_constant__ FrontRows p) {
+  constexpr int HD = 256;
+  const int lane = threadIdx.x & 31, heads = p.Hq + p.Hkv;
+  const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (item >= p.rows * heads) return;
+  const int row = item / heads, hh = item - row * heads;
+  const bool isq = hh < p.Hq;
+  const int h = isq ? hh : hh - p.Hq;
+  const int seq = p.Tb > 0 ? row / p.Tb : 0, tl = p.Tb > 0 ? row - seq * p.Tb : row;
+  const int position = p.pos[seq] + tl;
+  const bf16_t* src = isq ? p.qg + ((int64_t)row * p.Hq + h) * 2 * HD : p.k + ((int64_t)row * p.Hkv + h) * HD;
+  const bf16_t* w = isq ? p.q_norm : p.k_norm;
+  float x[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2*>(src + 128 * j + 4 * lane));
+    x[j][0] = __uint_as_float(u.x << 16); x[j][1] = __uint_as_float(u.x & 0xffff0000u);
+    x[j][2] = __uint_as_float(u.y << 16); x[j][3] = __uint_as_float(u.y & 0xffff0000u);
+  }
+  float ss[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    ss[j] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ss[j] = fmaf(x[j][i], x[j][i], ss[j]);
+    ss[j] = warp_sum(ss[j]);
+  }
+  const float inv = orn_rsqrtf((ss[0] + ss[1]) / (float)HD + p.eps);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2*>(w + 128 * j + 4 * lane));
+    const float wv[4] = {__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u)};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[j][i] = bfr(wv[i] * bfr(x[j][i] * inv));
+  }
+  // rotated pairs (i, i + half): the lower element in lane i / 4, the upper in lane (i + half) / 4
+  const int half = p.dims / 2, lanes = half / 4;
+  const bool low = lane < lanes, high = lane >= lanes && lane < 2 * lanes;
+  float other[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) other[i] = __shfl_sync(0xffffffffu, x[0][i], low ? lane + lanes : lane - lanes);
+  if (low || high) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int idx = 4 * (low ? lane : lane - lanes) + i;
+      const float ang = (float)position * orn_expf(-(float)idx * p.lnb);
+      float sn, cs;
+      orn_sincosf(ang, &sn, &cs);
+      const float x1 = low ? x[0][i] : other[i], x2 = low ? other[i] : x[0][i];
+      x[0][i] = low ? fmaf(x1, cs, -(x2 * sn)) : fmaf(x1, sn, x2 * cs);
+    }
+  }
+  bf16_t* dst = p.q + ((int64_t)row * p.Hq + h) * HD;
+  if (!isq) {
+    if (position >= p.cap) return;
+    const int64_t at = (((int64_t)seq * p.Hkv + h) * p.cap + position) * HD;
+    dst = p.kc + at;
+    reinterpret_cast<uint4*>(p.vc + at)[lane] = __ldg(reinterpret_cast<const uint4*>(p.v + ((int64_t)row * p.Hkv + h) * HD) + lane);
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    *reinterpret_cast<uint2*>(dst + 128 * j + 4 * lane) =
+        make_uint2((uint32_t)f2bf(x[j][0]) | ((uint32_t)f2bf(x[j][1]) << 16), (uint32_t)f2bf(x[j][2]) | ((uint32_t)f2bf(x[j][3]) << 16));
+}
+
 // hd == 256: 8 dims per lane
 __global__ void __launch_bounds__(1024)
 sdpa_decode_kernel(const bf16_t* __restrict__ q, const bf16_t* __restrict__ kc,
@@ -137,6 +216,17 @@ int k_rope(orn_ctx* ctx, cudaStream_t s, bf16_t* x, int T, int H, int hd, int di
   int n = T * H * (dims / 2);
   rope_kernel<<<(n + 127) / 128, 128, 0, s>>>(x, T, H, hd, dims, lnb, dev_offset, offset_add, 0);
   return orn_launch_check(ctx, "rope");
+}
+
+bool k_attn_front_ok(int hd, int dims) { return hd == 256 && dims % 8 == 0 && dims >= 8 && dims <= 128; }
+int k_attn_front(orn_ctx* ctx, cudaStream_t s, const bf16_t* qg, const bf16_t* k, const bf16_t* v, const bf16_t* q_norm, const bf16_t* k_norm,
+                 int rows, int Tb, int Hq, int Hkv, int cap, int dims, float lnb, float eps, const int* pos, bf16_t* q, bf16_t* kc, bf16_t* vc) {
+  FrontRows p;
+  p.qg = qg; p.k = k; p.v = v; p.q_norm = q_norm; p.k_norm = k_norm; p.q = q; p.kc = kc; p.vc = vc; p.pos = pos;
+  p.rows = rows; p.Tb = Tb; p.Hq = Hq; p.Hkv = Hkv; p.cap = cap; p.dims = dims; p.lnb = lnb; p.eps = eps;
+  const int warps = rows * (Hq + Hkv);
+  attn_front_kernel<<<(warps + 7) / 8, 256, 0, s>>>(p);
+  return orn_launch_check(ctx, "attn_front");
 }
 
 int k_kv_append(orn_ctx* ctx, cudaStream_t s, const bf16_t* k, const bf16_t* v, int T, int Hkv,

@@ -445,17 +445,23 @@ int batch_attention(orn_batch* bt, const orn_linear* q_proj, const orn_linear* k
     bf16_t* py[3] = {bt->ak, bt->av, bt->qg};
     CK(batch_mm_multi(bt, pl, py, kv_only ? 2 : 3, bt->n, R));
   }
-  CK(k_rms_norm(ctx, s, bt->ak, k_norm, R * Hkv, hd, c.rms_eps, bt->ak));
-  CK(k_rope_batched(ctx, s, bt->ak, B, T, Hkv, hd, c.rope_dims, m->lnb, pos));
-  CK(k_kv_append_batched(ctx, s, bt->ak, bt->av, B, T, Hkv, hd, bt->cap, pos, kc, vc));
-  if (kv_only) return ORN_OK;
-  CK(k_split_qgate(ctx, s, bt->qg, R, Hq, hd, bt->aq, bt->agate));
-  CK(k_rms_norm(ctx, s, bt->aq, q_norm, R * Hq, hd, c.rms_eps, bt->aq));
-  CK(k_rope_batched(ctx, s, bt->aq, B, T, Hq, hd, c.rope_dims, m->lnb, pos));
+  if (k_attn_front_ok(hd, c.rope_dims)) {
+    CK(k_attn_front(ctx, s, bt->qg, bt->ak, bt->av, q_norm, k_norm, R, T, kv_only ? 0 : Hq, Hkv, bt->cap, c.rope_dims, m->lnb, c.rms_eps, pos,
+                    bt->aq, kc, vc));
+    if (kv_only) return ORN_OK;
+  } else {
+    CK(k_rms_norm(ctx, s, bt->ak, k_norm, R * Hkv, hd, c.rms_eps, bt->ak));
+    CK(k_rope_batched(ctx, s, bt->ak, B, T, Hkv, hd, c.rope_dims, m->lnb, pos));
+    CK(k_kv_append_batched(ctx, s, bt->ak, bt->av, B, T, Hkv, hd, bt->cap, pos, kc, vc));
+    if (kv_only) return ORN_OK;
+    CK(k_split_qgate(ctx, s, bt->qg, R, Hq, hd, bt->aq, bt->agate));
+    CK(k_rms_norm(ctx, s, bt->aq, q_norm, R * Hq, hd, c.rms_eps, bt->aq));
+    CK(k_rope_batched(ctx, s, bt->aq, B, T, Hq, hd, c.rope_dims, m->lnb, pos));
+  }
   const float scale = 1.0f / sqrtf((float)hd);
   if ((exact && !bt->split_attn) || hd != 256 || NQ > 16) {
     CK(k_sdpa_decode_batched(ctx, s, bt->aq, kc, vc, B, T, Hq, Hkv, hd, bt->cap, pos, scale, bt->att));
-    CK(k_sigmoid_gate(ctx, s, bt->agate, bt->att, R * Hq * hd, 1, bt->agated));
+    CK(k_gate_rows(ctx, s, bt->qg, bt->att, R * Hq, bt->agated));
   } else {
     CK(launch_battn(ctx, s, bt->aq, kc, vc, pos, B, T, Hq, Hkv, bt->cap, scale, bt->part, nchunks, chunk, NQ));
     dim3 grid(NQ, Hkv, B);
@@ -702,10 +708,9 @@ int batch_body(orn_batch* bt, orn_ep* group, int T, int chunk, int nchunks) {
     const orn_linear* sg = world > 1 ? bt->views[3 * i] : ly.moe.sw_gate;
     const orn_linear* su = world > 1 ? bt->views[3 * i + 1] : ly.moe.sw_up;
     const orn_linear* sd = world > 1 ? bt->views[3 * i + 2] : ly.moe.sw_down;
-    CK(orn_ep_moe_block(group, ly.moe.gate, sg, su, sd, ly.moe.sh_gate, ly.moe.sh_up, ly.moe.sh_down, ly.moe.sh_egate, bt->n2, R,
-                        c.top_k, c.norm_topk_prob, bt->mo, nullptr));
-    const bf16_t* nw = i + 1 < c.n_layers ? m->layers[i + 1].input_ln : m->norm;
-    CK(k_add_rms_norm(ctx, s, bt->h, bt->mo, nw, R, H, c.rms_eps, bt->x, bt->n));
+    const MoeNextNorm next{bt->h, i + 1 < c.n_layers ? m->layers[i + 1].input_ln : m->norm, c.rms_eps, bt->x, bt->n};
+    CK(orn_ep_moe_block_norm(group, ly.moe.gate, sg, su, sd, ly.moe.sh_gate, ly.moe.sh_up, ly.moe.sh_down, ly.moe.sh_egate, bt->n2, R,
+                             c.top_k, c.norm_topk_prob, bt->mo, nullptr, &next));
   }
   ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(bt->normed, bt->n, sizeof(bf16_t) * (size_t)R * H, cudaMemcpyDeviceToDevice, s));  // the head's input survives it
   CK(batch_mm(bt, m->lm_head, bt->n, R, bt->logits));

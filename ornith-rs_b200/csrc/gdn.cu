@@ -114,6 +114,88 @@ __global__ void gdn_front_kernel(FrontParams p) {
   }
 }
 
+// The same front end for 4 taps and many rows: a warp owns a 128-channel slot for kFrontRun consecutive
+// rows of one sequence, so the taps are read once (32 bytes a lane) and a row of qkv once instead of four
+// times.  2048 rows: 92 -> 77 us, 128 rows as 64 pairs: 13 -> 11 us; bound by the arithmetic of SiLU.
+constexpr int kFrontRun = 8;
+__global__ void __launch_bounds__(128) gdn_front_run_kernel(const __grid_constant__ FrontParams p) {
+  const int lane = threadIdx.x & 31;
+  const int slot = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (slot >= p.D / 128) return;
+  const int rows = p.Tb > 0 ? p.Tb : p.T, runs = (rows + kFrontRun - 1) / kFrontRun;  // rows and runs of a sequence
+  const int seq = blockIdx.y / runs, t0 = (blockIdx.y - seq * runs) * kFrontRun, n = min(kFrontRun, rows - t0);
+  const int c0 = slot * 128 + lane * 4;
+  const bf16_t* cs = p.conv_state + seq * p.seq_stride;
+  const bf16_t* qk = p.qkv + seq * p.seq_stride;
+  auto window = [&](int j) {  // row j of the window [S cached rows | this call's rows]
+    return *reinterpret_cast<const uint2*>((j < 3 ? cs + (int64_t)j * p.D : qk + (int64_t)(j - 3) * p.D) + c0);
+  };
+  float tap[4][4];  // [channel][tap]
+  {
+    const uint4 wa = ldg128(p.cw + (int64_t)c0 * 4), wb = ldg128(p.cw + (int64_t)c0 * 4 + 8);
+    const uint32_t u[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      tap[r][0] = bf_lo(u[2 * r]); tap[r][1] = bf_hi(u[2 * r]); tap[r][2] = bf_lo(u[2 * r + 1]); tap[r][3] = bf_hi(u[2 * r + 1]);
+    }
+  }
+  uint2 x[kFrontRun + 3];
+#pragma unroll
+  for (int j = 0; j < kFrontRun + 3; ++j) x[j] = j < n + 3 ? window(t0 + j) : make_uint2(0, 0);
+  const int key_dim = p.Hk * 128;
+#pragma unroll
+  for (int i = 0; i < kFrontRun; ++i) {
+    if (i >= n) break;
+    const int64_t t = (int64_t)seq * rows + t0 + i;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float xs[4] = {bf_lo(x[i + j].x), bf_hi(x[i + j].x), bf_lo(x[i + j].y), bf_hi(x[i + j].y)};
+#pragma unroll
+      for (int r = 0; r < 4; ++r) acc[r] = fmaf(xs[r], tap[r][j], acc[r]);
+    }
+    float y[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) y[r] = orn_silu_bf(bfr(acc[r]));
+    bf16_t* dst;
+    if (slot < 2 * p.Hk) {
+      float sum = 0.f;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) sum = fmaf(y[r], y[r], sum);
+      sum = warp_sum(sum);
+      const float inv = orn_rsqrtf(sum / 128.0f + p.eps);
+      const bool is_q = slot < p.Hk;
+      dst = (is_q ? p.q : p.k) + t * key_dim + (is_q ? c0 : c0 - key_dim);
+      const float sc = is_q ? p.q_scale : p.k_scale;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) y[r] = sc * bfr(y[r] * inv);
+    } else {
+      dst = p.v + t * (p.D - 2 * key_dim) + (c0 - 2 * key_dim);
+    }
+    *reinterpret_cast<uint2*>(dst) = make_uint2((uint32_t)f2bf(y[0]) | ((uint32_t)f2bf(y[1]) << 16), (uint32_t)f2bf(y[2]) | ((uint32_t)f2bf(y[3]) << 16));
+    if (slot == 0)
+      for (int h = lane; h < p.Hv; h += 32) {
+        const int64_t at = t * p.Hv + h;
+        const float sp = orn_softplus_bf(bfr(bf2f(p.a_in[at]) + bf2f(p.dt_bias[h])));
+        const float decay = orn_expf(bf2f(p.a_log[h]));
+        p.g[at] = orn_expf((-decay) * sp);
+        p.beta[at] = f2bf(orn_sigmoid_bf(bf2f(p.b_in[at])));
+      }
+  }
+  if (p.conv_next != nullptr && p.Tb == 0 && t0 + n == rows)  // the next call's cached rows: the window's last three
+    for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(p.conv_next + (int64_t)j * p.D + c0) = window(rows + j);
+}
+// Runs pay off as soon as they fill the SMs (four warps each); below that one warp per row has the shorter
+// chain.  The run form wants 4 taps and 16-byte rows, and keeps no copy of the conv input.
+bool front_runs(const orn_ctx* ctx, const FrontParams& p, dim3* grid) {
+  const int rows = p.Tb > 0 ? p.Tb : p.T, seqs = p.Tb > 0 ? p.T / p.Tb : 1, slots = p.D / 128;
+  const int64_t runs = (int64_t)seqs * ((rows + kFrontRun - 1) / kFrontRun);
+  *grid = dim3((slots + 3) / 4, (unsigned)runs);
+  return p.Kc == 4 && p.conv_input == nullptr && p.D % 128 == 0 && rows > 1 &&
+         ((reinterpret_cast<uintptr_t>(p.cw) | reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0 &&
+         runs < 65536 && runs * slots >= 4 * ctx->sm_count;
+}
+
 struct DeltaParams {
   const bf16_t* q;     // [T, Hk, 128]
   const bf16_t* k;     // [T, Hk, 128]
@@ -274,7 +356,12 @@ int k_gdn_front(orn_ctx* ctx, cudaStream_t s, const bf16_t* conv_state, const bf
   p.k_scale = bfr(inv_scale);
   p.eps = eps;
   int slots = p.D / Dh;
-  dim3 grid((slots + 3) / 4, T);
+  dim3 grid;
+  if (front_runs(ctx, p, &grid)) {
+    gdn_front_run_kernel<<<grid, 128, 0, s>>>(p);
+    return orn_launch_check(ctx, "gdn_front");
+  }
+  grid = dim3((slots + 3) / 4, T);
   gdn_front_kernel<<<grid, 128, 0, s>>>(p);
   return orn_launch_check(ctx, "gdn_front");
 }
@@ -329,7 +416,12 @@ int k_gdn_front_batched(orn_ctx* ctx, cudaStream_t s, const bf16_t* conv, int64_
   p.k_scale = bfr(inv_scale);
   p.eps = eps;
   const int slots = p.D / Dh;
-  dim3 grid((slots + 3) / 4, B * Tb);
+  dim3 grid;
+  if (front_runs(ctx, p, &grid)) {
+    gdn_front_run_kernel<<<grid, 128, 0, s>>>(p);
+    return orn_launch_check(ctx, "gdn_front");
+  }
+  grid = dim3((slots + 3) / 4, B * Tb);
   gdn_front_kernel<<<grid, 128, 0, s>>>(p);
   return orn_launch_check(ctx, "gdn_front");
 }

