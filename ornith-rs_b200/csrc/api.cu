@@ -93,6 +93,12 @@ int32_t orn_ctx_create(int32_t device, orn_ctx** out) {
     delete c;
     return ORN_ERR_ALLOC;
   }
+  if (cudaMallocHost((void**)&c->err_h, sizeof(int)) != cudaSuccess) {
+    cudaFree(c->dev_err);
+    cudaStreamDestroy(c->stream);
+    delete c;
+    return ORN_ERR_ALLOC;
+  }
   const char* np = getenv("ORN_NO_PDL");
   const char* pg = getenv("ORN_PDL_MASK");
   if (pg) c->pdl_mask = atoi(pg);
@@ -113,6 +119,8 @@ int32_t orn_ctx_destroy(orn_ctx* ctx) {
   cudaFree(ctx->dev_err);
   cudaFree(ctx->attn_partial);
   cudaFree(ctx->attn_arrivals);
+  cudaFree(ctx->scratch);
+  cudaFreeHost(ctx->err_h);
   if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
@@ -122,6 +130,30 @@ int32_t orn_ctx_destroy(orn_ctx* ctx) {
 }
 
 }  // extern "C"
+
+int orn_scratch_take(orn_ctx* ctx, size_t bytes, void** p, size_t* got) {
+  {
+    std::lock_guard<std::mutex> hold(ctx->scratch_mutex);
+    if (ctx->scratch != nullptr && ctx->scratch_bytes >= bytes) {
+      *p = ctx->scratch; *got = ctx->scratch_bytes;
+      ctx->scratch = nullptr; ctx->scratch_bytes = 0;
+      return ORN_OK;
+    }
+  }
+  *got = bytes;
+  return orn_alloc(ctx, bytes, p);
+}
+void orn_scratch_give(orn_ctx* ctx, void* p, size_t got) {
+  void* drop = p;
+  if (got <= kScratchKeep) {
+    std::lock_guard<std::mutex> hold(ctx->scratch_mutex);
+    if (got > ctx->scratch_bytes) {  // keep the larger of the two
+      drop = ctx->scratch;
+      ctx->scratch = p; ctx->scratch_bytes = got;
+    }
+  }
+  if (drop) cudaFree(drop);
+}
 
 bool orn_side_stream(orn_ctx* ctx) {
   static const bool one = [] { const char* e = getenv("ORN_NO_SIDE_STREAM"); return e && e[0] == '1'; }();  // set once, thread-safe
@@ -147,10 +179,9 @@ extern "C" {
 
 int32_t orn_sync(orn_ctx* ctx) {
   if (!ctx) return ORN_ERR_ARG;
-  int flag = 0;
-  ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(&flag, ctx->dev_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  ORN_CHECK_CUDA(ctx, cudaMemcpyAsync(ctx->err_h, ctx->dev_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   ORN_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (flag != 0) {
+  if (*static_cast<volatile int*>(ctx->err_h) != 0) {
     cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), ctx->stream);
     ORN_FAIL(ctx, ORN_ERR_TIMEOUT, "a kernel gave up waiting (for its own asynchronous copies, or for a peer of an expert-parallel group)");
   }

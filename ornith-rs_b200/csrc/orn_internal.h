@@ -36,7 +36,18 @@ struct orn_ctx {
   // group partials and arrival counters of the fused attention's long-context form (fused.cu)
   float* attn_partial = nullptr;
   int* attn_arrivals = nullptr;
+  int* err_h = nullptr;  // pinned landing word of orn_sync's copy of *dev_err
+  // One device buffer kept for calls that need scratch and end with a synchronisation (orn_scratch_take):
+  // a call takes it out, so that two threads never share it, and gives it back; ctx_destroy frees it.
+  std::mutex scratch_mutex;
+  void* scratch = nullptr;
+  size_t scratch_bytes = 0;
 };
+// scratch of at least `bytes` for one call (the kept buffer where it is free and large enough); give it back
+// only when nothing in flight uses it.  Buffers above kScratchKeep are not kept.
+constexpr size_t kScratchKeep = (size_t)16 << 20;
+int orn_scratch_take(orn_ctx* ctx, size_t bytes, void** p, size_t* got);
+void orn_scratch_give(orn_ctx* ctx, void* p, size_t got);
 
 // Records an event after the launch just made and attributes the device time
 // since the previous mark to `what` (api.cu).
