@@ -215,17 +215,34 @@ struct DeltaParams {
 
 constexpr int kRowsPerCta = 16;
 
-// 32 bytes per request: a thread's 32 state floats are one 128-byte line, which four requests of a whole
-// sector each move instead of eight half sectors
-ORN_D void ld256(const float* p, float* v) {
-  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-               : "l"(p));
+// A warp's 8 state rows are 4 KB in one piece of memory, a lane's 32 floats one 128-byte line of it.  They
+// go through shared memory so that each request of the warp is 512 bytes in a row: a lane's own line, taken
+// a sector per request, costs 32 lines per request.  The 16-byte piece c of row r lies at c ^ (line of c,
+// parity of r) in its group of eight, so both sides touch all banks.
+constexpr int kStateWarp = 256;  // 16-byte pieces of a warp's rows
+ORN_D int state_piece(int r, int c) { return r * 32 + ((c & 24) | ((c ^ (c >> 3) ^ ((r & 1) << 2)) & 7)); }
+ORN_D void load_state(const float* rows, float4* stage, int lane, float* S) {
+  float4 v[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = __ldcs(reinterpret_cast<const float4*>(rows) + j * 32 + lane);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) stage[state_piece(j, lane)] = v[j];
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float4 x = stage[state_piece(lane >> 2, (lane & 3) * 8 + j)];
+    S[4 * j] = x.x; S[4 * j + 1] = x.y; S[4 * j + 2] = x.z; S[4 * j + 3] = x.w;
+  }
+  __syncwarp();
 }
-ORN_D void st256(float* p, const float* v) {
-  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]),
-               "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-               : "memory");
+ORN_D void store_state(float* rows, float4* stage, int lane, const float* S) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    stage[state_piece(lane >> 2, (lane & 3) * 8 + j)] = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) __stcs(reinterpret_cast<float4*>(rows) + j * 32 + lane, stage[state_piece(j, lane)]);
+  __syncwarp();
 }
 
 __global__ void __launch_bounds__(kRowsPerCta * 4) gated_delta_kernel(DeltaParams p) {
@@ -234,7 +251,10 @@ __global__ void __launch_bounds__(kRowsPerCta * 4) gated_delta_kernel(DeltaParam
   const int row = blockIdx.x * kRowsPerCta + (threadIdx.x >> 2);
   const int lir = threadIdx.x & 3;  // lane in row
   const size_t ssz = (size_t)p.Hv * 128 * 128;
-  const size_t off = ((size_t)hv * 128 + row) * 128 + lir * 32;
+  const int lane = threadIdx.x & 31;
+  __shared__ float4 s_stage[kRowsPerCta / 8][kStateWarp];
+  float4* stage = s_stage[threadIdx.x >> 5];
+  const size_t off = ((size_t)hv * 128 + blockIdx.x * kRowsPerCta + (threadIdx.x >> 5) * 8) * 128;  // this warp's rows
   const float* sin;
   int cur = 0;
   if (p.batched) {  // this sequence's rows, ring and cursor
@@ -250,8 +270,7 @@ __global__ void __launch_bounds__(kRowsPerCta * 4) gated_delta_kernel(DeltaParam
     sin = p.state + off;
   }
   float S[32];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) ld256(sin + 8 * i, S + 8 * i);
+  load_state(sin, stage, lane, S);
   // the inputs of step t + 1 are requested before step t's arithmetic: a long window (a prompt
   // chunk) otherwise pays one memory round trip per token on top of the recurrence's own chain
   struct StepIn {
@@ -324,15 +343,8 @@ __global__ void __launch_bounds__(kRowsPerCta * 4) gated_delta_kernel(DeltaParam
     }
     else if (p.snaps != nullptr) sout = p.snaps + (size_t)t * ssz + off;
     else if (t + 1 == p.T) sout = p.state + off;
-    if (sout != nullptr) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) st256(sout + 8 * i, S + 8 * i);
-    }
-    if (p.ring == nullptr && p.snaps != nullptr && t + 1 == p.T) {
-      float* so = p.state + off;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) st256(so + 8 * i, S + 8 * i);
-    }
+    if (sout != nullptr) store_state(sout, stage, lane, S);
+    if (p.ring == nullptr && p.snaps != nullptr && t + 1 == p.T) store_state(p.state + off, stage, lane, S);
   }
 }
 }  // namespace
