@@ -245,7 +245,12 @@ ORN_D void store_state(float* rows, float4* stage, int lane, const float* S) {
   __syncwarp();
 }
 
-__global__ void __launch_bounds__(kRowsPerCta * 4) gated_delta_kernel(DeltaParams p) {
+// AHEAD: the inputs of step t + 1 are requested before step t's arithmetic.  A long window otherwise pays a
+// memory round trip per token on top of the recurrence's own chain; a window of a few rows is bound by the
+// states' traffic and wants the registers for more warps (181 -> 127 registers, 10 -> 16 warps per
+// SM; 64 windows of two rows: 110 -> 86 us).
+template <bool AHEAD>
+__global__ void __launch_bounds__(kRowsPerCta * 4, AHEAD ? 1 : 8) gated_delta_kernel(const __grid_constant__ DeltaParams p) {
   const int hv = blockIdx.y;
   const int hk = hv / (p.Hv / p.Hk);
   const int row = blockIdx.x * kRowsPerCta + (threadIdx.x >> 2);
@@ -257,53 +262,45 @@ __global__ void __launch_bounds__(kRowsPerCta * 4) gated_delta_kernel(DeltaParam
   const size_t off = ((size_t)hv * 128 + blockIdx.x * kRowsPerCta + (threadIdx.x >> 5) * 8) * 128;  // this warp's rows
   const float* sin;
   int cur = 0;
-  if (p.batched) {  // this sequence's rows, ring and cursor
-    const size_t z = blockIdx.z;
-    p.q += z * p.T * p.Hk * 128; p.k += z * p.T * p.Hk * 128; p.v += z * p.T * p.Hv * 128;
-    p.g += z * p.T * p.Hv; p.beta += z * p.T * p.Hv; p.y += z * p.T * p.Hv * 128;
-    p.ring += z * p.nring * ssz; p.cur += z;
-  }
-  if (p.ring != nullptr) {
-    cur = *p.cur;
-    sin = p.ring + (size_t)(cur % p.nring) * ssz + off;
+  // batched: this sequence's rows, ring and cursor
+  const size_t z = p.batched ? blockIdx.z : 0, row0 = z * p.T;
+  float* ring = p.ring != nullptr ? p.ring + z * p.nring * ssz : nullptr;
+  if (ring != nullptr) {
+    cur = p.cur[z];
+    sin = ring + (size_t)(cur % p.nring) * ssz + off;
   } else {
     sin = p.state + off;
   }
   float S[32];
-  load_state(sin, stage, lane, S);
-  // the inputs of step t + 1 are requested before step t's arithmetic: a long window (a prompt
-  // chunk) otherwise pays one memory round trip per token on top of the recurrence's own chain
   struct StepIn {
     uint4 kv[4], qv[4];
     float g;
     bf16_t beta, v;
   };
   auto fetch = [&](int t, StepIn& in) {
-    const bf16_t* kp = p.k + ((size_t)t * p.Hk + hk) * 128 + lir * 32;
-    const bf16_t* qp = p.q + ((size_t)t * p.Hk + hk) * 128 + lir * 32;
+    const bf16_t* kp = p.k + ((row0 + t) * p.Hk + hk) * 128 + lir * 32;
+    const bf16_t* qp = p.q + ((row0 + t) * p.Hk + hk) * 128 + lir * 32;
 #pragma unroll
     for (int i = 0; i < 4; ++i) { in.kv[i] = ldg128(kp + 8 * i); in.qv[i] = ldg128(qp + 8 * i); }
-    in.g = p.g[(size_t)t * p.Hv + hv];
-    in.beta = p.beta[(size_t)t * p.Hv + hv];
-    in.v = p.v[((size_t)t * p.Hv + hv) * 128 + row];
+    in.g = p.g[(row0 + t) * p.Hv + hv];
+    in.beta = p.beta[(row0 + t) * p.Hv + hv];
+    in.v = p.v[((row0 + t) * p.Hv + hv) * 128 + row];
   };
   StepIn now, nxt;
   fetch(0, now);
+  load_state(sin, stage, lane, S);
   for (int t = 0; t < p.T; ++t) {
-    if (t + 1 < p.T) fetch(t + 1, nxt);
-    float kf[32], qf[32];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint4 kv = now.kv[i], qv = now.qv[i];
-      kf[8 * i] = bf_lo(kv.x); kf[8 * i + 1] = bf_hi(kv.x); kf[8 * i + 2] = bf_lo(kv.y); kf[8 * i + 3] = bf_hi(kv.y);
-      kf[8 * i + 4] = bf_lo(kv.z); kf[8 * i + 5] = bf_hi(kv.z); kf[8 * i + 6] = bf_lo(kv.w); kf[8 * i + 7] = bf_hi(kv.w);
-      qf[8 * i] = bf_lo(qv.x); qf[8 * i + 1] = bf_hi(qv.x); qf[8 * i + 2] = bf_lo(qv.y); qf[8 * i + 3] = bf_hi(qv.y);
-      qf[8 * i + 4] = bf_lo(qv.z); qf[8 * i + 5] = bf_hi(qv.z); qf[8 * i + 6] = bf_lo(qv.w); qf[8 * i + 7] = bf_hi(qv.w);
-    }
+    if (AHEAD && t + 1 < p.T) fetch(t + 1, nxt);
+    if (!AHEAD && t > 0) fetch(t, now);
+    // element e of the packed keys and queries, unpacked where it is used
+    auto at = [](const uint4 (&w)[4], int e) {
+      const uint4 u = w[e >> 3];
+      const uint32_t x = (e & 4) ? ((e & 2) ? u.w : u.z) : ((e & 2) ? u.y : u.x);
+      return (e & 1) ? bf_hi(x) : bf_lo(x);
+    };
     const float gt = now.g;
     const float bt = bf2f(now.beta);
     const float vt = bf2f(now.v);
-    now = nxt;
     float part[8];
 #pragma unroll
     for (int pb = 0; pb < 8; ++pb) {
@@ -312,7 +309,7 @@ __global__ void __launch_bounds__(kRowsPerCta * 4) gated_delta_kernel(DeltaParam
       for (int i = 0; i < 4; ++i) {
         const int e = pb * 4 + i;
         S[e] = S[e] * gt;
-        acc = fmaf(S[e], kf[e], acc);
+        acc = fmaf(S[e], at(now.kv, e), acc);
       }
       part[pb] = acc;
     }
@@ -326,25 +323,26 @@ __global__ void __launch_bounds__(kRowsPerCta * 4) gated_delta_kernel(DeltaParam
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int e = pb * 4 + i;
-        S[e] = fmaf(kf[e], delta, S[e]);
-        acc = fmaf(S[e], qf[e], acc);
+        S[e] = fmaf(at(now.kv, e), delta, S[e]);
+        acc = fmaf(S[e], at(now.qv, e), acc);
       }
       part[pb] = acc;
     }
     float o = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
     o = o + __shfl_xor_sync(0xffffffffu, o, 1);
     o = o + __shfl_xor_sync(0xffffffffu, o, 2);
-    if (lir == 0) p.y[((size_t)t * p.Hv + hv) * 128 + row] = f2bf(o);
+    if (lir == 0) p.y[((row0 + t) * p.Hv + hv) * 128 + row] = f2bf(o);
 
     float* sout = nullptr;
-    if (p.ring != nullptr) {
-      if (!p.ring_final) sout = p.ring + (size_t)((cur + 1 + t) % p.nring) * ssz + off;
-      else if (t + 1 == p.T) sout = p.ring + (size_t)((cur + 1) % p.nring) * ssz + off;
+    if (ring != nullptr) {
+      if (!p.ring_final) sout = ring + (size_t)((cur + 1 + t) % p.nring) * ssz + off;
+      else if (t + 1 == p.T) sout = ring + (size_t)((cur + 1) % p.nring) * ssz + off;
     }
     else if (p.snaps != nullptr) sout = p.snaps + (size_t)t * ssz + off;
     else if (t + 1 == p.T) sout = p.state + off;
     if (sout != nullptr) store_state(sout, stage, lane, S);
-    if (p.ring == nullptr && p.snaps != nullptr && t + 1 == p.T) store_state(p.state + off, stage, lane, S);
+    if (ring == nullptr && p.snaps != nullptr && t + 1 == p.T) store_state(p.state + off, stage, lane, S);
+    if (AHEAD) now = nxt;
   }
 }
 }  // namespace
@@ -381,7 +379,8 @@ int k_gdn_front(orn_ctx* ctx, cudaStream_t s, const bf16_t* conv_state, const bf
 static int launch_delta(orn_ctx* ctx, cudaStream_t s, DeltaParams& p, int B = 1) {
   if (p.Hv % p.Hk != 0) ORN_FAIL(ctx, ORN_ERR_ARG, "gated_delta: Hv % Hk != 0");
   dim3 grid(128 / kRowsPerCta, p.Hv, B);
-  gated_delta_kernel<<<grid, kRowsPerCta * 4, 0, s>>>(p);
+  if (p.T > 8) gated_delta_kernel<true><<<grid, kRowsPerCta * 4, 0, s>>>(p);
+  else gated_delta_kernel<false><<<grid, kRowsPerCta * 4, 0, s>>>(p);
   return orn_launch_check(ctx, "gated_delta");
 }
 
