@@ -247,3 +247,26 @@ def test_batched_mtp_cycles_equal_the_single_sequence_engine(pkg, ctx):
         assert out[b] == mtp[b][:len(out[b])], b
     bt.free()
     gm.free()
+
+
+@pytest.mark.parametrize("B,T", [(1, 1), (1, 2), (2, 2), (5, 1), (7, 2), (15, 1)])
+def test_few_rows_take_the_fused_kernels(pkg, ctx, B, T):
+    """Up to 15 rows, in groups of four per launch (1, 2, 4, 5, 14 and 15 rows): the bits of the
+    single-sequence engine, at different depths of the sequences' caches."""
+    cfg = hp.tiny_config(pkg.Config)
+    gm = hp.upload_model(pkg, ctx, cfg, hp.tiny_model_weights(cfg, seed=15))
+    rng = np.random.default_rng(B)
+    windows = [rng.integers(0, cfg.vocab, (B, T)).astype(np.uint32) for _ in range(4)]
+    keeps = [rng.integers(1, T + 1, B).astype(np.int32) for _ in range(4)]
+    bt = pkg.Batch(gm, B, t_max=T, cap=32)
+    got = []
+    for w, k in zip(windows, keeps):
+        tg, hid = bt.forward(w, want_hidden=True)
+        got.append((hid.numpy().reshape(B, T, cfg.hidden).copy(), tg.reshape(B, T).copy()))
+        bt.commit(k)
+    for b in range(B):
+        for i, ((wh, wt), (gh, gt)) in enumerate(zip(run_single(pkg, gm, windows, keeps, b), got)):
+            assert np.array_equal(wh.reshape(-1, cfg.hidden), gh[b]), (b, i)
+            assert np.array_equal(wt, gt[b]), (b, i)
+    bt.free()
+    gm.free()

@@ -146,3 +146,19 @@ def test_gemm_rejects_bad_shapes(pkg, ctx):
     assert ctx._lib.orn_gemm(ctx.h, L.h, x.ptr, 16, y.ptr, 0) != 0
     L.free()
     ctx.sync()
+
+
+@pytest.mark.parametrize("kind", [orc.Q4K, orc.Q6K, orc.A8, orc.BF16, orc.A4])
+@pytest.mark.parametrize("M,O,K", [(1, 33, 256), (17, 129, 1536), (129, 128, 4096), (512, 130, 768), (513, 127, 256), (257, 8, 1024)])
+def test_gemm_edges_of_its_tiles_and_splits(pkg, ctx, kind, M, O, K):
+    """One past and one short of the 128-feature tile, the 128- and 256-row steps and the 512-row end of
+    the split-K rule; one super-block of K up to sixteen, so ranges of K in one CTA, in tensor memory one
+    after the other, and over a cluster; O not a multiple of 8 (no 16-byte stores)."""
+    rng = np.random.default_rng(31 * kind + M + O)
+    W = hp.make_weights(rng, kind, 1, O, K)
+    x = hp.f32_to_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    L = lin_of(pkg, ctx, W)
+    got = L.matmul_wide(ctx.upload(x), M, out_f32=True).numpy()
+    want = orc.gemv(W, x, M, f32=True)
+    assert max_rel(got, want) <= TOL, max_rel(got, want)
+    L.free()

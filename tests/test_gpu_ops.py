@@ -426,3 +426,51 @@ def test_errors_are_reported_not_fatal(pkg, ctx):
     x = ctx.zeros((16,), np.uint16)
     assert lib.orn_sdpa_decode(ctx.h, x.ptr, x.ptr, x.ptr, 1, 16, 2, 128, 64, 0, 1.0, x.ptr) == -1
     ctx.sync()  # the context is still usable
+
+
+@pytest.mark.parametrize("rows,n", [(1, 64), (9, 128), (17, 124), (8, 130), (3, 4096), (2, 2049)])
+def test_norm_forms(pkg, ctx, rows, n):
+    """Several short rows per CTA (n <= 128) with a ragged last CTA, rows narrower than their warps, and
+    lengths that the 8-byte form cannot take; in place, as the attention front end uses it."""
+    rng = np.random.default_rng(rows + 3 * n)
+    a, b, z = bf(rng, (rows, n), 3.0), bf(rng, (rows, n)), bf(rng, (rows, n))
+    w = hp.f32_to_bf16(1.0 + 0.1 * rng.standard_normal(n).astype(np.float32))
+    d, h, o, dw = ctx.upload(a), ctx.empty((rows, n), np.uint16), ctx.empty((rows, n), np.uint16), ctx.upload(w)
+    ctx.check(ctx._lib.orn_add_rms_norm(ctx.h, d.ptr, ctx.upload(b).ptr, dw.ptr, rows, n, 1e-6, h.ptr, o.ptr), "add_rms")
+    rh, ro = orc.add_rms_norm(a, b, w, rows, n, 1e-6)
+    assert np.array_equal(h.numpy(), rh) and np.array_equal(o.numpy(), ro)
+    ctx.check(ctx._lib.orn_rms_norm_gated(ctx.h, d.ptr, dw.ptr, ctx.upload(z).ptr, rows, n, 1e-6, o.ptr), "gated")
+    assert np.array_equal(o.numpy(), orc.rms_norm_gated(a, w, z, rows, n, 1e-6))
+    ctx.check(ctx._lib.orn_rms_norm(ctx.h, d.ptr, dw.ptr, rows, n, 1e-6, d.ptr), "rms")
+    assert np.array_equal(d.numpy(), orc.rms_norm(a, w, rows, n, 1e-6))
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 1001, 4096])
+def test_swiglu_lengths(pkg, ctx, n):
+    """Lengths that the eight-element form takes and lengths that it does not."""
+    rng = np.random.default_rng(n)
+    g, u = bf(rng, (n,), 3.0), bf(rng, (n,))
+    o = ctx.empty((n,), np.uint16)
+    ctx.check(ctx._lib.orn_swiglu(ctx.h, ctx.upload(g).ptr, ctx.upload(u).ptr, n, o.ptr), "swiglu")
+    assert np.array_equal(o.numpy(), orc.swiglu(g, u))
+
+
+@pytest.mark.parametrize("T", [8, 9, 104, 157])
+def test_gated_delta_window_lengths(pkg, ctx, T):
+    """Both sides of the two dispatches: up to 8 rows the recurrence does not fetch ahead; from about a
+    hundred rows the front end takes runs of eight (104: whole runs, 157: a ragged last one)."""
+    rng = np.random.default_rng(70 + T)
+    Hk, Hv, Dh, Kc = 16, 32, 128, 4
+    i = gdn_inputs(rng, T)
+    ref = orc.gdn_front(i["conv_state"], i["qkv"], i["cw"], i["a"], i["b"], i["a_log"], i["dt_bias"], T, Hk, Hv, Dh, Kc)
+    o = run_front(ctx, i, T, Hk, Hv, Dh, Kc)
+    for name, r in zip(["conv_next", "q", "k", "v", "beta"], ref[:5]):
+        assert np.array_equal(o[name].numpy(), r), name
+    assert np.array_equal(o["g"].numpy().view(np.uint32), ref[5].view(np.uint32))
+    st_ref = (0.1 * rng.standard_normal((Hv, 128, 128))).astype(np.float32)
+    st, y = ctx.upload(st_ref), ctx.empty((T, Hv, 128), np.uint16)
+    y_ref = orc.gated_delta(ref[1], ref[2], ref[3], ref[5], ref[4], st_ref, T, Hk, Hv)
+    ctx.check(ctx._lib.orn_gated_delta(ctx.h, o["q"].ptr, o["k"].ptr, o["v"].ptr, o["g"].ptr, o["beta"].ptr, st.ptr, T, Hk, Hv, y.ptr,
+                                       None), "gated_delta")
+    assert np.array_equal(y.numpy(), y_ref)
+    assert np.array_equal(st.numpy().view(np.uint32), st_ref.view(np.uint32))
