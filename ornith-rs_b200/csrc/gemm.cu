@@ -1029,6 +1029,24 @@ int f_qgemm(orn_ctx* ctx, cudaStream_t s, const orn_linear* L, const bf16_t* x, 
 
 // Up to four matrices of one format and row length over the same rows in ONE launch (the projections
 // of a layer that share their input): their feature tiles form one tile space.  n == 1 is f_qgemm.
+// Dense products over few rows: the K blocks of a tile go to the CTAs of a cluster, which add their
+// f32 partials in split order through distributed shared memory.  The number of splits depends on the
+// matrices (and on rows only in steps of 256), so that a row's bits do not depend on the rows beside it:
+// one round of items over the SMs, two where the tiles alone would leave half of the SMs idle, at
+// least 4 K blocks per item, no split empty.
+int f_qgemm_splits(const orn_ctx* ctx, int f_tiles, int rows, int K) {
+  const int KB = K / BK;
+  if (rows > kSplitMaxRows || KB < 8) return 1;
+  const int tiles = f_tiles * ((rows + 255) / 256);
+  int sp = std::max(1, (tiles > ctx->sm_count / 2 ? 2 * ctx->sm_count : ctx->sm_count) / tiles);
+  sp = std::min(sp, std::min(kMaxSplit, KB / 4));
+  if (sp > 1) {
+    const int per = (KB + sp - 1) / sp;
+    sp = (KB + per - 1) / per;
+  }
+  return sp;
+}
+
 int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, void* const* ys, const int* ldys, int n,
                   const bf16_t* x, int rows, const QGemmGroup* grp, int out_f32) {
   if (rows < 1) return ORN_OK;
@@ -1060,22 +1078,8 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
   P.seg = grp ? grp->seg : nullptr;
   P.row_map = grp ? grp->row_map : nullptr;
   P.E = L->E;
-  // Dense products over few rows: the K blocks of a tile go to the CTAs of a cluster, which add their
-  // f32 partials in split order through distributed shared memory.  The number of splits depends on the
-  // matrices (and on rows only in steps of 256), so that a row's bits do not depend on the rows beside it:
-  // one round of items over the SMs, two where the tiles alone would leave half of the SMs idle, at
-  // least 4 K blocks per item, no split empty.
-  P.splits = 1; P.seq = 1;
-  if (grp == nullptr && rows <= kSplitMaxRows && KB >= 8) {
-    const int tiles = P.f_tiles * ((rows + 255) / 256);
-    int sp = std::max(1, (tiles > ctx->sm_count / 2 ? 2 * ctx->sm_count : ctx->sm_count) / tiles);
-    sp = std::min(sp, std::min(kMaxSplit, KB / 4));
-    if (sp > 1) {
-      const int per = (KB + sp - 1) / sp;
-      sp = (KB + per - 1) / per;
-    }
-    P.splits = sp;
-  }
+  P.splits = grp == nullptr ? f_qgemm_splits(ctx, P.f_tiles, rows, L->K) : 1;
+  P.seq = 1;
   P.per = (KB + P.splits - 1) / P.splits;
   // Token-tile width.  Few rows: one tile that holds them.  Many rows: the width (at most 128, so that two
   // accumulators and the weight ring fit tensor memory) that finishes in the fewest MMA cycles over whole

@@ -30,7 +30,6 @@ __global__ void iota_div_kernel(uint32_t* lhs, uint32_t* ident, int n, int k) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) { lhs[i] = (uint32_t)(i / k); ident[i] = (uint32_t)i; }
 }
-__global__ void set_u32_kernel(uint32_t* p, uint32_t v) { *p = v; }
 __global__ void set_int_kernel(int* p, int v) { *p = v; }
 // mailbox = {primary, force flag[3], force token[3]} written by the host before each cycle;
 // slot < 0 places the primary at the head of the window (and empties the draft head's cache where each
@@ -765,7 +764,8 @@ int wide_mm(orn_model* m, const orn_linear* L, const bf16_t* x, int T, bf16_t* y
   return ORN_OK;
 }
 // several products of the same rows: neighbours of one format share a launch (more tiles per round of the
-// SMs, and a narrow matrix is no launch of its own)
+// SMs, and a narrow matrix is no launch of its own) while that leaves the ranges of K of each of them, and so
+// its bits, as they are alone
 int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear*, bf16_t*>> jobs, const bf16_t* x, int T) {
   const auto* j = jobs.begin();
   const int n = (int)jobs.size();
@@ -773,7 +773,11 @@ int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear
     const orn_linear* pl[4];
     void* py[4];
     int ld[4], k = 0;
-    for (; i + k < n && k < 4 && j[i + k].first->kind == j[i].first->kind && j[i + k].first->K == j[i].first->K; ++k) {
+    auto splits = [&](int tiles) { return f_qgemm_splits(m->ctx, tiles, T, j[i].first->K); };
+    for (int tiles = 0; i + k < n && k < 4 && j[i + k].first->kind == j[i].first->kind && j[i + k].first->K == j[i].first->K; ++k) {
+      const int own = (j[i + k].first->O + 127) / 128;
+      if (k > 0 && (splits(tiles + own) != splits(own) || splits(tiles + own) != splits(tiles))) break;
+      tiles += own;
       pl[k] = j[i + k].first; py[k] = j[i + k].second; ld[k] = pl[k]->O;
     }
     if (wide_exact())
@@ -901,7 +905,6 @@ int prefill_wide(orn_model* m, orn_cache* cc, int T, bf16_t* normed_out /*nullab
   WideWs& w = m->wide;
   const orn_config& c = m->cfg;
   const int H = c.hidden, S = c.gdn_conv_kernel - 1, D = conv_dim(c);
-  const int VD = c.gdn_v_heads * c.gdn_head_dim, QD = c.n_heads * c.head_dim, KVD = c.n_kv_heads * c.head_dim;
   const int Hq = c.n_heads, Hkv = c.n_kv_heads, hd = c.head_dim;
   if (cc->h_pos + T > c.max_ctx) ORN_FAIL(ctx, ORN_ERR_STATE, "forward: context exceeds max_ctx");
   CK(k_embedding(ctx, s, m->embed, w.ids, T, w.x));
