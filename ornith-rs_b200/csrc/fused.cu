@@ -1484,10 +1484,15 @@ constexpr int kGdnMaxHeads = 960;  // arrival counters of a launch: value heads 
 constexpr int kGdnStateThreads = kGdnRows * 4;
 __host__ __device__ constexpr int gdn_threads(int T) { return 32 * (2 * T + 2); }
 
-template <bool TAPS4>  // TAPS4: the convolution has 4 taps (every Qwen3.5 artifact); else any width
-__global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(const __grid_constant__ GdnParams p) {
+// TAPS4: the convolution has 4 taps (every Qwen3.5 artifact); else any width.  LINES: the state moves in whole
+// lines through shared memory and two CTAs of ten warps fit an SM, which pays for windows of three and four
+// rows (one read and as many writes of the state: 60 tokens at verify width 4 112.8 -> 110.9 ms); with two rows
+// it changes nothing, with one the extra step of the chain costs more than it saves (64 tokens +0.4 %).
+template <bool TAPS4, bool LINES>
+__global__ void __launch_bounds__(gdn_threads(kGdnMaxT), LINES ? 2 : 1) k_gdn(const __grid_constant__ GdnParams p) {
   __shared__ float s_q[kGdnMaxT][128], s_k[kGdnMaxT][128], s_v[kGdnMaxT][kGdnRows];
   __shared__ float s_g[kGdnMaxT], s_beta[kGdnMaxT];
+  __shared__ float4 s_stage[LINES ? kGdnRows / 8 : 1][LINES ? kStateWarp : 1];
   pdl_trigger();
   const int hv = blockIdx.y;
   const int hk = hv / (p.Hv / p.Hk);
@@ -1499,20 +1504,26 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(const __grid_cons
   const int row = blockIdx.x * kGdnRows + ((threadIdx.x >> 2) & (kGdnRows - 1));
   const int lir = threadIdx.x & 3;
   const size_t ssz = (size_t)p.Hv * 128 * 128;
-  const size_t off = ((size_t)hv * 128 + row) * 128 + lir * 32;
+  // LINES: an owning warp's eight rows; else the lane's own line
+  const size_t off = LINES ? ((size_t)hv * 128 + blockIdx.x * kGdnRows + (warp & (kGdnRows / 8 - 1)) * 8) * 128
+                           : ((size_t)hv * 128 + row) * 128 + lir * 32;
   const int seq = blockIdx.z, row0 = seq * p.T;  // this sequence's first window row
   const int cur = p.cur[seq];
   float* const ring = p.ring + (size_t)seq * p.nring * ssz;
   const bf16_t* const conv = p.conv + seq * p.conv_stride;
   const float* sin = ring + (size_t)(cur % p.nring) * ssz + off;
   float S[32];
-  if (owner) {  // a thread's 32 state floats are one 128-byte line: four requests of a whole sector each
+  if (owner) {
+    if constexpr (LINES) {
+      request_state(sin, lane, S);
+    } else {  // four requests of a whole sector each
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                   : "=f"(S[8 * i]), "=f"(S[8 * i + 1]), "=f"(S[8 * i + 2]), "=f"(S[8 * i + 3]), "=f"(S[8 * i + 4]),
-                     "=f"(S[8 * i + 5]), "=f"(S[8 * i + 6]), "=f"(S[8 * i + 7])
-                   : "l"(sin + 8 * i));
+      for (int i = 0; i < 4; ++i)
+        asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(S[8 * i]), "=f"(S[8 * i + 1]), "=f"(S[8 * i + 2]), "=f"(S[8 * i + 3]), "=f"(S[8 * i + 4]),
+                       "=f"(S[8 * i + 5]), "=f"(S[8 * i + 6]), "=f"(S[8 * i + 7])
+                     : "l"(sin + 8 * i));
+    }
   }
   // The state and the ring position were written by an earlier step (a graph launch, a copy or a
   // host read lies in between), not by the kernel this one may overlap: only what follows reads
@@ -1618,6 +1629,8 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(const __grid_cons
     }
   __syncthreads();
   // ---- recurrence (kernels/gated_delta.metal:36-142), by the threads that own the state
+  float4* const stage = s_stage[LINES ? warp & (kGdnRows / 8 - 1) : 0];
+  if (LINES && owner) take_state(stage, lane, S);
   if (owner)
   for (int t = 0; t < p.T; ++t) {
     const float* kf = s_k[t] + lir * 32;
@@ -1657,7 +1670,8 @@ __global__ void __launch_bounds__(gdn_threads(kGdnMaxT)) k_gdn(const __grid_cons
     float* sout = nullptr;
     if (!p.final_only) sout = ring + (size_t)((cur + 1 + t) % p.nring) * ssz + off;
     else if (t + 1 == p.T) sout = ring + (size_t)((cur + 1) % p.nring) * ssz + off;
-    if (sout != nullptr) {
+    if (LINES && sout != nullptr) store_state(sout, stage, lane, S);
+    if (!LINES && sout != nullptr) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(sout + 8 * i), "f"(S[8 * i]),
@@ -2187,14 +2201,12 @@ int f_gdn(orn_ctx* ctx, cudaStream_t s, const bf16_t* conv, const bf16_t* cw, co
   // Unused dynamic shared memory caps the kernel at two CTAs per SM.  As a programmatic dependent
   // its CTAs become resident while the previous kernel drains, and without the cap the first SMs
   // to come free would take sixteen CTAs each instead of the grid spreading over the whole part.
-  const size_t pad = 100 * 1024;
+  const size_t pad = 96 * 1024;
   // the kernel also has static shared memory: ask for the pad, not for the maximum
-  {
-    int rc = Kc == 4 ? grant_smem(ctx, k_gdn<true>, pad) : grant_smem(ctx, k_gdn<false>, pad);
-    if (rc != ORN_OK) return rc;
-  }
-  if (Kc == 4) ORN_CHECK_CUDA(ctx, orn_launch_dependent(ctx, s, 3, k_gdn<true>, grid, block, pad, p));
-  else ORN_CHECK_CUDA(ctx, orn_launch_dependent(ctx, s, 3, k_gdn<false>, grid, block, pad, p));
+  void (*const kern)(GdnParams) = Kc == 4 ? (T > 2 ? k_gdn<true, true> : k_gdn<true, false>) : (T > 2 ? k_gdn<false, true> : k_gdn<false, false>);
+  const int rc = grant_smem(ctx, kern, pad);
+  if (rc != ORN_OK) return rc;
+  ORN_CHECK_CUDA(ctx, orn_launch_dependent(ctx, s, 3, kern, grid, block, pad, p));
   return orn_launch_check(ctx, "k_gdn");
 }
 

@@ -215,36 +215,6 @@ struct DeltaParams {
 
 constexpr int kRowsPerCta = 16;
 
-// A warp's 8 state rows are 4 KB in one piece of memory, a lane's 32 floats one 128-byte line of it.  They
-// go through shared memory so that each request of the warp is 512 bytes in a row: a lane's own line, taken
-// a sector per request, costs 32 lines per request.  The 16-byte piece c of row r lies at c ^ (line of c,
-// parity of r) in its group of eight, so both sides touch all banks.
-constexpr int kStateWarp = 256;  // 16-byte pieces of a warp's rows
-ORN_D int state_piece(int r, int c) { return r * 32 + ((c & 24) | ((c ^ (c >> 3) ^ ((r & 1) << 2)) & 7)); }
-ORN_D void load_state(const float* rows, float4* stage, int lane, float* S) {
-  float4 v[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = __ldcs(reinterpret_cast<const float4*>(rows) + j * 32 + lane);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) stage[state_piece(j, lane)] = v[j];
-  __syncwarp();
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float4 x = stage[state_piece(lane >> 2, (lane & 3) * 8 + j)];
-    S[4 * j] = x.x; S[4 * j + 1] = x.y; S[4 * j + 2] = x.z; S[4 * j + 3] = x.w;
-  }
-  __syncwarp();
-}
-ORN_D void store_state(float* rows, float4* stage, int lane, const float* S) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-    stage[state_piece(lane >> 2, (lane & 3) * 8 + j)] = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
-  __syncwarp();
-#pragma unroll
-  for (int j = 0; j < 8; ++j) __stcs(reinterpret_cast<float4*>(rows) + j * 32 + lane, stage[state_piece(j, lane)]);
-  __syncwarp();
-}
-
 // AHEAD: the inputs of step t + 1 are requested before step t's arithmetic.  A long window otherwise pays a
 // memory round trip per token on top of the recurrence's own chain; a window of a few rows is bound by the
 // states' traffic and wants the registers for more warps (181 -> 127 registers, 10 -> 16 warps per
@@ -288,7 +258,8 @@ __global__ void __launch_bounds__(kRowsPerCta * 4, AHEAD ? 1 : 8) gated_delta_ke
   };
   StepIn now, nxt;
   fetch(0, now);
-  load_state(sin, stage, lane, S);
+  request_state(sin, lane, S);
+  take_state(stage, lane, S);
   for (int t = 0; t < p.T; ++t) {
     if (AHEAD && t + 1 < p.T) fetch(t + 1, nxt);
     if (!AHEAD && t > 0) fetch(t, now);

@@ -262,4 +262,39 @@ ORN_D uint32_t ldg32_stream(const void* p) {
   asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
+
+// The 128 x 128 state of a gated-delta head, eight rows per warp: 4 KB in one piece of memory, of which a
+// lane computes on 32 floats, one 128-byte line (row lane / 4, columns 32 (lane % 4) ..).  The rows go
+// through shared memory so that each request of the warp is 512 bytes in a row: a lane's own line, taken a
+// sector per request, costs 32 lines per request.  The 16-byte piece c of row r lies at c ^ (line of c,
+// parity of r) in its group of eight, so both sides touch all banks.
+constexpr int kStateWarp = 256;  // 16-byte pieces of a warp's rows
+ORN_D int state_piece(int r, int c) { return r * 32 + ((c & 24) | ((c ^ (c >> 3) ^ ((r & 1) << 2)) & 7)); }
+ORN_D void request_state(const float* rows, int lane, float* S) {  // piece 32 j + lane into S[4 j ..]
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float4 v = __ldcs(reinterpret_cast<const float4*>(rows) + j * 32 + lane);
+    S[4 * j] = v.x; S[4 * j + 1] = v.y; S[4 * j + 2] = v.z; S[4 * j + 3] = v.w;
+  }
+}
+ORN_D void take_state(float4* stage, int lane, float* S) {  // what request_state brought -> the lane's own columns
+#pragma unroll
+  for (int j = 0; j < 8; ++j) stage[state_piece(j, lane)] = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float4 x = stage[state_piece(lane >> 2, (lane & 3) * 8 + j)];
+    S[4 * j] = x.x; S[4 * j + 1] = x.y; S[4 * j + 2] = x.z; S[4 * j + 3] = x.w;
+  }
+  __syncwarp();
+}
+ORN_D void store_state(float* rows, float4* stage, int lane, const float* S) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    stage[state_piece(lane >> 2, (lane & 3) * 8 + j)] = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) __stcs(reinterpret_cast<float4*>(rows) + j * 32 + lane, stage[state_piece(j, lane)]);
+  __syncwarp();
+}
 #endif  // __CUDACC__
