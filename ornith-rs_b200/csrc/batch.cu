@@ -545,7 +545,7 @@ int small_mm(orn_batch* bt, const FusedPrologue& fp, const FusedJob* jobs, int n
   return ORN_OK;
 }
 // MoE block of the rows h = bf(a + b) -> bt->h, result -> bt->mo
-int small_moe(orn_batch* bt, const Moe& moe, const bf16_t* a, const bf16_t* b, const bf16_t* nw, int rows) {
+int small_moe(orn_batch* bt, const Moe& moe, const bf16_t* a, const bf16_t* b, const bf16_t* nw, int rows, const L2Hint& hint = {}) {
   orn_model* m = bt->m;
   orn_ctx* ctx = m->ctx;
   cudaStream_t s = ctx->stream;
@@ -561,7 +561,7 @@ int small_moe(orn_batch* bt, const Moe& moe, const bf16_t* a, const bf16_t* b, c
   for (int r = 0; r < rows; r += kMaxRows) {
     const int n = std::min(kMaxRows, rows - r);
     CK(f_moe_up(ctx, s, n, bt->sgates + r * E, bt->n2 + r * H, moe.sw_gate, moe.sw_up, c.top_k, bt->sinds + r * k, bt->sscores + r * k,
-                bt->seact + r * k * I));
+                bt->seact + r * k * I, r + kMaxRows < rows ? L2Hint() : hint));
     CK(f_moe_down(ctx, s, n, bt->seact + r * k * I, bt->ssact + r * SI, bt->sinds + r * k, bt->sscores + r * k, bt->sgs + r, moe.sw_down,
                   moe.sh_down, c.top_k, c.norm_topk_prob, bt->mo + r * H));
   }
@@ -630,7 +630,7 @@ int small_body(orn_batch* bt, int T, int keys) {
     } else {
       CK(small_attention(bt, fp, ly.q_proj, ly.k_proj, ly.v_proj, ly.o_proj, ly.q_norm, ly.k_norm, T, bt->pos, bt->kc[i], bt->vc[i], keys, false));
     }
-    CK(small_moe(bt, ly.moe, res, bt->r, ly.post_ln, R));
+    CK(small_moe(bt, ly.moe, res, bt->r, ly.post_ln, R, hint_next(i + 1 < c.n_layers ? &m->layers[i + 1] : nullptr, m->lm_head)));
     pa = bt->h;
     pb = bt->mo;
   }

@@ -1036,6 +1036,17 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_norm_gemv(const __grid_con
   }
 }
 
+// Requests the hinted ranges, 4 KB per request (16 and 64 KB: a third of the gain), as caller `who` of `n`.
+// One warp per CTA, before the wait for the routing, while the expert weights cannot be requested yet: behind
+// them the same requests cost 2 %.
+ORN_D void request_l2(const L2Hint& h, int who, int n) {
+  constexpr uint32_t kPiece = 4096;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    for (uint32_t o = (uint32_t)who * kPiece; o < h.bytes[r]; o += (uint32_t)n * kPiece)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(h.at[r] + o), "r"(min(kPiece, h.bytes[r] - o)) : "memory");
+}
+
 // ---------------------------------------------------------------------------
 // kernel 2: router top-k in the prologue, routed expert gate/up + SwiGLU
 // ---------------------------------------------------------------------------
@@ -1154,7 +1165,7 @@ ORN_D void warp_softmax_topk(const bf16_t* logits, int n, int k, float* probs, f
 
 template <int KIND, int KC>
 __global__ void __launch_bounds__(kMoeThreads, 1) k_moe_up(const __grid_constant__ MoeUpParams P, uint32_t slot_bytes, int depth,
-                                                             uint32_t ring_off, int* err) {
+                                                             uint32_t ring_off, int* err, const __grid_constant__ L2Hint hint) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   float* smem = reinterpret_cast<float*>(smem_raw);
   constexpr int RT = up_rows(KIND, KC);
@@ -1171,6 +1182,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) k_moe_up(const __grid_constant
   pdl_trigger();
   Ring R;
   ring_setup(R, smem_raw + ring_off, slot_bytes, depth, err);
+  if (warp == kMoeThreads / 32 - 1) request_l2(hint, lane * gridDim.x + blockIdx.x, gridDim.x * 32);
   pdl_wait();  // the routing (and so the first weight tile) depends on the previous kernel's logits
   // the first M warps route their token while the other warps stage x: one barrier for both
   if (warp < M)
@@ -2055,7 +2067,7 @@ int launch_norm_gemv(orn_ctx* ctx, cudaStream_t s, const Prologue& P, RowJobs& J
 }
 
 template <int KIND, int KC>
-int launch_moe_up_k(orn_ctx* ctx, cudaStream_t s, const MoeUpParams& P) {
+int launch_moe_up_k(orn_ctx* ctx, cudaStream_t s, const MoeUpParams& P, const L2Hint& hint) {
   const int M = P.M;
   size_t fixed = stage_floats(KIND, M, P.H) * sizeof(float) + (size_t)M * P.k * 4;
   fixed = (fixed + 127) & ~(size_t)127;
@@ -2069,7 +2081,7 @@ int launch_moe_up_k(orn_ctx* ctx, cudaStream_t s, const MoeUpParams& P) {
   rc = set_smem(ctx, k_moe_up<KIND, KC>, bytes);
   if (rc != ORN_OK) return rc;
   ORN_CHECK_CUDA(ctx, orn_launch_dependent(ctx, s, 1, k_moe_up<KIND, KC>, dim3(ctx->sm_count), dim3(kMoeThreads), bytes,
-                                           P, slot, depth, ring_off, ctx->dev_err));
+                                           P, slot, depth, ring_off, ctx->dev_err, hint));
   return orn_launch_check(ctx, launch_label(ctx, "k_moe_up", M, KIND, P.I, P.H));
 }
 
@@ -2134,7 +2146,7 @@ int f_norm_gemv(orn_ctx* ctx, cudaStream_t s, int M, const FusedPrologue& fp, co
 }
 
 int f_moe_up(orn_ctx* ctx, cudaStream_t s, int M, const bf16_t* logits, const bf16_t* x, const orn_linear* gate,
-             const orn_linear* up, int k, uint32_t* inds, bf16_t* scores, bf16_t* act) {
+             const orn_linear* up, int k, uint32_t* inds, bf16_t* scores, bf16_t* act, const L2Hint& hint) {
   if (gate->kind != up->kind || gate->K != up->K || gate->O != up->O)
     ORN_FAIL(ctx, ORN_ERR_ARG, "moe: gate and up experts must share format and shape");
   if (M < 1 || M > 4) ORN_FAIL(ctx, ORN_ERR_ARG, "moe_up: 1..4 rows");
@@ -2145,7 +2157,7 @@ int f_moe_up(orn_ctx* ctx, cudaStream_t s, int M, const bf16_t* logits, const bf
   if (P.H % 256) ORN_FAIL(ctx, ORN_ERR_ARG, "moe_up: hidden must be a multiple of 256");
   if (P.H > 4096) ORN_FAIL(ctx, ORN_ERR_ARG, "moe_up: hidden above 4096");
 #define ORN_UP(KIND) \
-  return P.H > 2048 ? launch_moe_up_k<KIND, 2>(ctx, s, P) : launch_moe_up_k<KIND, 1>(ctx, s, P)
+  return P.H > 2048 ? launch_moe_up_k<KIND, 2>(ctx, s, P, hint) : launch_moe_up_k<KIND, 1>(ctx, s, P, hint)
   switch (gate->kind) {
     case ORN_Q4K: ORN_UP(ORN_Q4K);
     case ORN_Q6K: ORN_UP(ORN_Q6K);

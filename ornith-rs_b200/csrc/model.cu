@@ -361,7 +361,7 @@ bool moe_fusable(const Moe& e) {
 
 // MoE block from the pre-norm pair (a, b): h = bf(a+b) -> w.h, norm with `nw`,
 // router + shared expert + routed experts + combine -> w.mo   (three kernels)
-int moe_fused(orn_model* m, const Moe& moe, const bf16_t* a, const bf16_t* b, const bf16_t* nw, int T) {
+int moe_fused(orn_model* m, const Moe& moe, const bf16_t* a, const bf16_t* b, const bf16_t* nw, int T, const L2Hint& hint = {}) {
   orn_ctx* ctx = m->ctx;
   cudaStream_t s = ctx->stream;
   Workspace& w = m->ws;
@@ -384,7 +384,7 @@ int moe_fused(orn_model* m, const Moe& moe, const bf16_t* a, const bf16_t* b, co
   jobs[1].lin = moe.sh_gate; jobs[1].lin2 = moe.sh_up; jobs[1].out = w.sact; jobs[1].epi = EPI_SWIGLU;
   jobs[2].lin = moe.sh_egate; jobs[2].out = w.gs;
   CK(f_norm_gemv(ctx, s, T, fp, jobs, 3));
-  CK(f_moe_up(ctx, s, T, w.gates, w.normed2, moe.sw_gate, moe.sw_up, c.top_k, w.inds, w.scores, w.eact));
+  CK(f_moe_up(ctx, s, T, w.gates, w.normed2, moe.sw_gate, moe.sw_up, c.top_k, w.inds, w.scores, w.eact, hint));
   CK(f_moe_down(ctx, s, T, w.eact, w.sact, w.inds, w.scores, w.gs, moe.sw_down, moe.sh_down, c.top_k,
                 c.norm_topk_prob, w.mo));
   return ORN_OK;
@@ -470,7 +470,7 @@ int trunk_layers(orn_model* m, orn_cache* cc, const uint32_t* dev_ids, int T, bo
       oj.lin = ly.o_proj; oj.out = w.r;
       CK(f_norm_gemv(ctx, s, T, gp, &oj, 1));
     }
-    CK(moe_fused(m, ly.moe, w.x, w.r, ly.post_ln, T));
+    CK(moe_fused(m, ly.moe, w.x, w.r, ly.post_ln, T, hint_next(i + 1 < c.n_layers ? &m->layers[i + 1] : nullptr, m->lm_head)));
     pa = w.h;
     pb = w.mo;
   }

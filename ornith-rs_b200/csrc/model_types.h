@@ -75,6 +75,14 @@ struct WideWs {
 
 using namespace ornm;
 
+// what the step reads behind a layer's experts: the next layer's input projections, or the head's first rows
+inline L2Hint hint_next(const Layer* next, const orn_linear* head) {
+  L2Hint h;
+  if (next == nullptr) h.add(head);
+  else if (next->linear) for (const orn_linear* l : {next->in_qkv, next->in_z, next->in_b, next->in_a}) h.add(l);
+  else for (const orn_linear* l : {next->q_proj, next->k_proj, next->v_proj}) h.add(l);
+  return h;
+}
 struct orn_model {
   orn_ctx* ctx = nullptr;
   orn_config cfg{};
