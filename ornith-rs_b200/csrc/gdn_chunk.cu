@@ -107,14 +107,22 @@ __global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(PrepParams p) {
         Po[s * kC + r] = f2bf(dec * qk[nt][e]);
       }
   }
-  for (int i = threadIdx.x; i < kC * 128; i += blockDim.x) {
-    const int s = i >> 7, d = i & 127;
-    const float kv = bf2f(*reinterpret_cast<const bf16_t*>(Kb + s * kPitchK + 2 * d));
-    const float qv = bf2f(*reinterpret_cast<const bf16_t*>(Qb + s * kPitchK + 2 * d));
-    const float e = expf(L[s]);
-    Kg[i] = f2bf(e * kv);
-    Qg[i] = f2bf(e * qv);
-    Kd[i] = f2bf(expf(L[kC - 1] - L[s]) * kv);
+  for (int i = threadIdx.x; i < kC * 16; i += blockDim.x) {  // eight elements of a row at a time
+    const int s = i >> 4, pc = i & 15;
+    const float e = expf(L[s]), f = expf(L[kC - 1] - L[s]);
+    const uint4 kv = *reinterpret_cast<const uint4*>(Kb + s * kPitchK + 16 * pc), qv = *reinterpret_cast<const uint4*>(Qb + s * kPitchK + 16 * pc);
+    const uint32_t kw[4] = {kv.x, kv.y, kv.z, kv.w}, qw[4] = {qv.x, qv.y, qv.z, qv.w};
+    uint32_t kg[4], qg[4], kd[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float k0 = __uint_as_float(kw[j] << 16), k1 = __uint_as_float(kw[j] & 0xffff0000u);
+      kg[j] = pack_bf16x2(e * k0, e * k1);
+      qg[j] = pack_bf16x2(e * __uint_as_float(qw[j] << 16), e * __uint_as_float(qw[j] & 0xffff0000u));
+      kd[j] = pack_bf16x2(f * k0, f * k1);
+    }
+    reinterpret_cast<uint4*>(Kg)[i] = make_uint4(kg[0], kg[1], kg[2], kg[3]);
+    reinterpret_cast<uint4*>(Qg)[i] = make_uint4(qg[0], qg[1], qg[2], qg[3]);
+    reinterpret_cast<uint4*>(Kd)[i] = make_uint4(kd[0], kd[1], kd[2], kd[3]);
   }
   if (threadIdx.x == 0) p.gc[(size_t)hv * p.nchunks + c] = expf(L[kC - 1]);
   __syncthreads();
