@@ -22,8 +22,8 @@
 //   warps 8..15   dequantise: two groups of four warps, a group owns every second unit of two K blocks
 //                 (128 weights a thread: one feature row), stores them with tcgen05.st into TENSOR MEMORY,
 //                 where the MMA takes its A operand from, and hands the unit over with one arrival per
-//                 warp.  Fewer, longer steps won over sixteen warps of one K block each (154 -> 118 us for
-//                 1024 routed Q4_K rows): a hand-over costs a warp several hundred cycles of waiting
+//                 warp.  Fewer, longer steps won over sixteen warps of one K block each (with the
+//                 rest of this layout 146 -> 137 us for 1024 routed Q4_K rows): a hand-over costs a warp several hundred cycles of waiting
 //                 whatever it carries, and with 128 registers the conversions of a step interleave
 //   warp 1        issues 4 tcgen05.mma (128 x BN x 16, bf16 in, f32 accumulate) per K block and one
 //                 commit per unit: a commit occupies the issuing thread for about 160 cycles, twice
@@ -252,8 +252,8 @@ ORN_D uint32_t lds16(uint32_t addr) {
 //   0x6400 | q           is the half 1024 + q   (q in bits 0..3 or a whole byte)
 //   0x5400 | (q << 4)    is the half   64 + q   (q in bits 4..7)
 // The scale then needs one packed fma per two weights and one conversion packs the bfloat16 pair: 1.1
-// ALU instructions per 4-bit weight instead of 2, 1.0 instead of 1.5 per 8-bit weight (the grouped
-// Q4_K product of 1024 routed rows: 140 -> 112 us).
+// ALU instructions per 4-bit weight instead of 2, 1.0 instead of 1.5 per 8-bit weight (with the rest
+// of this layout the grouped Q6_K product of 1024 routed rows: 110 -> 74 us).
 ORN_D float add_lo(uint32_t h2, float c) {  // low half of h2 + c
   float d;
   asm("{\n.reg .b16 l, h;\nmov.b32 {l, h}, %1;\nadd.rn.f32.f16 %0, l, %2;\n}\n" : "=f"(d) : "r"(h2), "f"(c));
