@@ -362,7 +362,7 @@ int batch_mm_multi(orn_batch* bt, const orn_linear* const* Ls, bf16_t* const* ys
   }
   // the first group of matrices on the main stream, the others beside it on the side stream (a small
   // projection of another format next to the big one is a launch of a few CTAs that would otherwise wait
-  // its turn); the side stream's products have their own split-K scratch
+  // its turn)
   bool forked = false;
   int i = 0;
   while (i < n) {

@@ -818,7 +818,7 @@ int wide_reserve(orn_model* m, int rows) {
   A(&w.gy, R * VD); A(&w.gated, R * VD);
   A(&w.qg, R * 2 * QD); A(&w.aq, R * QD); A(&w.agate, R * QD); A(&w.ak, R * KVD); A(&w.av, R * KVD);
   A(&w.att, R * QD); A(&w.agated, R * QD);
-  A(&w.gates, R * E); A(&w.probs, R * E); A(&w.scores, R * k); A(&w.sg, R * SI); A(&w.su, R * SI); A(&w.sact, R * SI);
+  A(&w.gates, R * E); A(&w.scores, R * k); A(&w.sg, R * SI); A(&w.su, R * SI); A(&w.sact, R * SI);
   A(&w.sy, R * H); A(&w.gs, R);
   A(&w.xs, R * k * H); A(&w.eg, R * k * I); A(&w.eu, R * k * I); A(&w.eact, R * k * I); A(&w.ey, R * k * H);
   if (rc == ORN_OK) {

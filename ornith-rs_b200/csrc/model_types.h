@@ -67,7 +67,7 @@ struct WideWs {
   bf16_t *cb, *z, *a, *b, *gq, *gk, *gv, *beta, *gy, *gated;
   float* gg;
   bf16_t *qg, *aq, *agate, *ak, *av, *att, *agated;
-  bf16_t *gates, *probs, *scores, *sg, *su, *sact, *sy, *gs;
+  bf16_t *gates, *scores, *sg, *su, *sact, *sy, *gs;
   bf16_t *xs, *eg, *eu, *eact, *ey;
 };
 
