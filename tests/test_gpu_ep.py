@@ -142,6 +142,35 @@ def test_library_block_world_of_one_equals_the_oracle(pkg, ctx, ep):
         l.free()
 
 
+@pytest.mark.parametrize("R", [5, 15, 16, 17])
+def test_library_block_few_rows_one_call_after_the_other(pkg, ctx, ep, R):
+    """Default arithmetic below and at 16 rows, where the shared expert changes from mat-vecs to the tensor
+    cores: its launches run beside the routed experts, in order among themselves.  Three calls on other rows
+    each, none waited for in between, so a launch that reads what its predecessor has not written yet would
+    find the rows of the call before.  Bound, per row in the 2-norm: the oracle rounds to bfloat16 at the same
+    six places (gate, up, their product, down, weighted, sum) and each may come out one step, 2^-8, apart:
+    sqrt(6) 2^-8 = 0.0096 where they are independent, 2^-6 with room for rows whose terms cancel."""
+    import orn_oracle as orc
+    import helpers as hp
+    H, E, I, k = (SHAPE[n] for n in "HEIk")
+    ws = eh.layer_weights(31, H, E, I)
+    L = {n: pkg.Linear.from_numpy(ctx, w.kind, w.w, w.s, w.b, E=w.E, O=w.O, K=w.K) for n, w in ws.items()}
+    group = ep.LibEp(ctx)
+    xs = [eh.rows_of(40 + i, 0, R, H) for i in range(3)]
+    dx, di = [ctx.upload(x) for x in xs], [ctx.empty((R, k), np.uint32) for _ in xs]
+    ys = [group.moe_block(L, x, R, k, 1, inds=i) for x, i in zip(dx, di)]
+    ctx.sync()
+    for x, y, i in zip(xs, ys, di):
+        want, want_inds = orc.moe_block(ws, x, R, k, 1)
+        assert np.array_equal(i.numpy(), want_inds)
+        g, w = hp.bf16_to_f32(y.numpy()).astype(np.float64), hp.bf16_to_f32(want).astype(np.float64)
+        off = np.linalg.norm(g - w, axis=1) / np.linalg.norm(w, axis=1)
+        assert off.max() <= 2.0 ** -6, off
+    group.close()
+    for l in L.values():
+        l.free()
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
 def test_library_block_two_gpus_equal_the_single_device_block(tmp_path):
     H, E, I, k = (SHAPE[n] for n in "HEIk")
