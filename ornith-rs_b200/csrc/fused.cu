@@ -2323,9 +2323,14 @@ int f_attn(orn_ctx* ctx, cudaStream_t s, const bf16_t* qg, const bf16_t* k, cons
   p.eps = eps;
   if (long_context) {
     if (ctx->attn_partial == nullptr) {  // first use: never inside a capture (a shape runs eagerly once before it is captured)
-      ORN_CHECK_CUDA(ctx, cudaMalloc((void**)&ctx->attn_partial, sizeof(float) * (size_t)kAttnMaxHeads * kGdnMaxT * 32 * kAttnPart));
-      ORN_CHECK_CUDA(ctx, cudaMalloc((void**)&ctx->attn_arrivals, sizeof(int) * kAttnMaxHeads * kGdnMaxT));
-      ORN_CHECK_CUDA(ctx, cudaMemset(ctx->attn_arrivals, 0, sizeof(int) * kAttnMaxHeads * kGdnMaxT));
+      void *partial = nullptr, *arrivals = nullptr;
+      int rc = orn_alloc(ctx, sizeof(float) * (size_t)kAttnMaxHeads * kGdnMaxT * 32 * kAttnPart, &partial);
+      if (rc == ORN_OK) rc = orn_alloc(ctx, sizeof(int) * kAttnMaxHeads * kGdnMaxT, &arrivals);
+      // in the stream's order: it does not wait for the legacy stream
+      if (rc == ORN_OK) rc = orn_memset(ctx, arrivals, 0, sizeof(int) * kAttnMaxHeads * kGdnMaxT);
+      if (rc != ORN_OK) { cudaFree(partial); cudaFree(arrivals); return rc; }
+      ctx->attn_partial = static_cast<float*>(partial);
+      ctx->attn_arrivals = static_cast<int*>(arrivals);
     }
     if (B * Hq > kAttnMaxHeads) ORN_FAIL(ctx, ORN_ERR_ARG, "fused attention: more than 256 query heads");
     dim3 sgrid(Hq, B * T, kAttnSplit);
