@@ -332,7 +332,7 @@ struct orn_batch {
     cudaGraphExec_t exec = nullptr;
     int seen = 0;
     int64_t launches = 0;
-    orn_ep* group = nullptr;
+    uint64_t group = 0;  // orn_ep_serial of the group it was captured with
   };
   std::map<uint64_t, StepGraph> graphs;  // keyed by (rows per window, split-KV launch shape, arithmetic)
   // this rank's slices of the routed experts when the group has several ranks (views, not copies)
@@ -920,7 +920,7 @@ int32_t orn_batch_forward(orn_batch* bt, orn_ep* ep, const uint32_t* host_ids, i
   const uint64_t key = (uint64_t)T | ((uint64_t)nchunks << 8) | ((uint64_t)chunk << 28) | ((uint64_t)(exact ? 1 : 0) << 40) |
                        ((uint64_t)(small ? 1 : 0) << 41) | ((uint64_t)(small ? orn_long_context(max_pos + T) : 0) << 42);
   orn_batch::StepGraph& g = bt->graphs[key];
-  if (g.exec != nullptr && g.group != group) {  // captured for another group: its collectives belong to that one
+  if (g.exec != nullptr && g.group != orn_ep_serial(group)) {  // captured for another group: its collectives belong to that one
     cudaGraphExecDestroy(g.exec);
     g = orn_batch::StepGraph();
   }
@@ -943,7 +943,7 @@ int32_t orn_batch_forward(orn_batch* bt, orn_ep* ep, const uint32_t* host_ids, i
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) { g.exec = nullptr; ORN_FAIL(ctx, ORN_ERR_CUDA, std::string("batch_forward: cudaGraphInstantiate: ") + cudaGetErrorString(e)); }
     g.launches = ctx->launches - l0;
-    g.group = group;
+    g.group = orn_ep_serial(group);
     ORN_CHECK_CUDA(ctx, cudaGraphLaunch(g.exec, s));
   }
   if (rc != ORN_OK) return rc;

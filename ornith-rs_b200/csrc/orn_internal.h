@@ -228,6 +228,8 @@ struct MoeNextNorm {
   float eps;
   bf16_t *sum, *out;
 };
+// a number no other group of this process ever has (a new group may get the address of a destroyed one)
+uint64_t orn_ep_serial(const orn_ep* ep);
 // orn_ep_moe_block; with `next`, that add and norm as well (dev_out is then scratch)
 int orn_ep_moe_block_norm(orn_ep* ep, const orn_linear* gate, const orn_linear* sw_gate, const orn_linear* sw_up,
                           const orn_linear* sw_down, const orn_linear* sh_gate, const orn_linear* sh_up,

@@ -249,6 +249,32 @@ def test_batched_mtp_cycles_equal_the_single_sequence_engine(pkg, ctx):
     gm.free()
 
 
+def test_a_captured_step_belongs_to_the_group_it_was_captured_with(pkg, ctx):
+    """A step captured with one expert-parallel group is not replayed for the next group, which may sit at the
+    first one's address: default arithmetic first, then a group of exact arithmetic, against a batch that has
+    only known the second."""
+    from ornith_rs_b200 import ep
+    cfg = hp.tiny_config(pkg.Config)
+    gm = hp.upload_model(pkg, ctx, cfg, hp.tiny_model_weights(cfg, seed=16))
+    B = 8
+    ids = np.random.default_rng(4).integers(0, cfg.vocab, (B, 2)).astype(np.uint32)
+    outs = []
+    for first in (True, False):
+        bt = pkg.Batch(gm, B, t_max=2, cap=64)
+        if first:
+            group = ep.LibEp(ctx)
+            for _ in range(3):      # eager, captured, replayed
+                bt.forward(ids, ep=group)
+            group.close()
+            bt.reset()
+        group = ep.LibEp(ctx, exact=True)
+        outs.append(bt.forward(ids, ep=group, want_hidden=True)[1].numpy().copy())
+        bt.free()
+        group.close()
+    assert np.array_equal(outs[0], outs[1])
+    gm.free()
+
+
 @pytest.mark.parametrize("B,T", [(1, 1), (1, 2), (2, 2), (5, 1), (7, 2), (15, 1)])
 def test_few_rows_take_the_fused_kernels(pkg, ctx, B, T):
     """Up to 15 rows, in groups of four per launch (1, 2, 4, 5, 14 and 15 rows): the bits of the
