@@ -1,5 +1,5 @@
-"""What the tensor-core product (csrc/gemm.cu: k_qgemm) does when a bounded wait runs out, checked as a state
-machine over every interleaving.
+"""What the tensor-core product (csrc/gemm.cu: k_qgemm) and the streaming kernels (csrc/fused.cu) do when a bounded
+wait runs out, checked as a state machine over every interleaving.
 
 One CTA: two of the epilogue's warps stand for the four.  A warp waits for its accumulators with a limit of its own (the
 wait may run out at any moment, also just before the accumulators arrive), goes on to a named barrier that all
@@ -153,6 +153,16 @@ def test_a_cta_stays_while_anything_can_land_in_it(C):
 def test_the_model_finds_what_lands_too_late(meet, drain, what):
     with pytest.raises(AssertionError, match=what):
         explore_cluster(2, meet, drain)
+
+
+def test_a_streaming_warp_stays_while_its_copies_are_in_flight():
+    """The rings of the streaming kernels: a warp waits as a whole, and one that gives up waits for what it has
+    requested.  As above with one CTA: the warp is the CTA, a tile is the box."""
+    src = open(os.path.join(CSRC, "fused.cu")).read()
+    wait = src[src.index("// lane 0: two bulk copies"):src.index("// carve the rings of all warps")]
+    assert len(re.findall(r"__all_sync\(0xffffffffu, mbar_try_wait\(", wait)) == len(re.findall(r"\bmbar_try_wait\(", wait)) > 0
+    assert len(re.findall(r"\bmbar_try_wait\(", src)) == 1 + len(re.findall(r"\bmbar_try_wait\(", wait))   # no wait elsewhere
+    explore_cluster(1, meet=True, drain=bool(re.search(r"for \(int i = 0; i < depth && ring_poll\(", wait)))
 
 
 def test_only_single_lanes_wait_for_themselves():
