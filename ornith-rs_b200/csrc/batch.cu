@@ -429,6 +429,20 @@ int ensure_shards(orn_batch* bt, int rank, int world) {
   return ORN_OK;
 }
 
+// key rows bt->ak (norm and RoPE to come) and value rows bt->av of B windows of T rows -> the caches, and nothing else
+int kv_rows(orn_batch* bt, const bf16_t* k_norm, int T, const int* pos, bf16_t* kc, bf16_t* vc) {
+  orn_model* m = bt->m;
+  orn_ctx* ctx = m->ctx;
+  cudaStream_t s = ctx->stream;
+  const orn_config& c = m->cfg;
+  const int B = bt->B, R = B * T, Hkv = c.n_kv_heads, hd = c.head_dim;
+  if (k_attn_front_ok(hd, c.rope_dims))
+    return k_attn_front(ctx, s, nullptr, bt->ak, bt->av, nullptr, k_norm, R, T, 0, Hkv, bt->cap, c.rope_dims, m->lnb, c.rms_eps, pos, nullptr, kc, vc);
+  CK(k_rms_norm(ctx, s, bt->ak, k_norm, R * Hkv, hd, c.rms_eps, bt->ak));
+  CK(k_rope_batched(ctx, s, bt->ak, B, T, Hkv, hd, c.rope_dims, m->lnb, pos));
+  return k_kv_append_batched(ctx, s, bt->ak, bt->av, B, T, Hkv, hd, bt->cap, pos, kc, vc);
+}
+
 // the attention sub-block over bt->n for B * T rows (T rows per sequence at positions pos[b] ...):
 // projections, per-head norms, RoPE, KV append, attention, output gate, output projection -> bt->r.
 // kv_only: stop after the KV rows are in the cache (the MTP head's re-encode of accepted tokens)
@@ -445,15 +459,12 @@ int batch_attention(orn_batch* bt, const orn_linear* q_proj, const orn_linear* k
     bf16_t* py[3] = {bt->ak, bt->av, bt->qg};
     CK(batch_mm_multi(bt, pl, py, kv_only ? 2 : 3, bt->n, R));
   }
+  if (kv_only) return kv_rows(bt, k_norm, T, pos, kc, vc);
   if (k_attn_front_ok(hd, c.rope_dims)) {
-    CK(k_attn_front(ctx, s, bt->qg, bt->ak, bt->av, q_norm, k_norm, R, T, kv_only ? 0 : Hq, Hkv, bt->cap, c.rope_dims, m->lnb, c.rms_eps, pos,
+    CK(k_attn_front(ctx, s, bt->qg, bt->ak, bt->av, q_norm, k_norm, R, T, Hq, Hkv, bt->cap, c.rope_dims, m->lnb, c.rms_eps, pos,
                     bt->aq, kc, vc));
-    if (kv_only) return ORN_OK;
   } else {
-    CK(k_rms_norm(ctx, s, bt->ak, k_norm, R * Hkv, hd, c.rms_eps, bt->ak));
-    CK(k_rope_batched(ctx, s, bt->ak, B, T, Hkv, hd, c.rope_dims, m->lnb, pos));
-    CK(k_kv_append_batched(ctx, s, bt->ak, bt->av, B, T, Hkv, hd, bt->cap, pos, kc, vc));
-    if (kv_only) return ORN_OK;
+    CK(kv_rows(bt, k_norm, T, pos, kc, vc));
     CK(k_split_qgate(ctx, s, bt->qg, R, Hq, hd, bt->aq, bt->agate));
     CK(k_rms_norm(ctx, s, bt->aq, q_norm, R * Hq, hd, c.rms_eps, bt->aq));
     CK(k_rope_batched(ctx, s, bt->aq, B, T, Hq, hd, c.rope_dims, m->lnb, pos));
@@ -521,6 +532,10 @@ __global__ void mtp_advance_kernel(int* mtp_pos, const int* keep, int B, int bas
 // path, a sixth of its launches, every weight read by the kernels built for few rows.  One sequence of
 // two rows: 9.9 -> 3.0 ms per cycle, bit for bit the same.
 constexpr int kSmallRows = 15;
+// The re-encode (one row per sequence, keys and values only) has little to read per launch, and every CTA of the
+// fused kernels rebuilds the norms of both of its inputs: up to this many sequences.  A commit, fused / one kernel
+// per op: one sequence 70 / 80 us, two 79 / 86, four 98 / 90, seven 138 / 112, fifteen 230 / 166.
+constexpr int kSmallEncode = 2;
 
 // the fused kernels serve every part of the model at these rows, on this GPU alone
 bool small_path(const orn_batch* bt, int rows, int world) {
@@ -567,7 +582,8 @@ int small_moe(orn_batch* bt, const Moe& moe, const bf16_t* a, const bf16_t* b, c
   }
   return ORN_OK;
 }
-// attention sub-block of B sequences of T rows -> bt->r; kv_only: stop once the KV rows are in the cache
+// attention sub-block of B sequences of T rows -> bt->r; kv_only: keys and values are projected and appended, no
+// query and no walk over the cache
 int small_attention(orn_batch* bt, const FusedPrologue& fp, const orn_linear* q_proj, const orn_linear* k_proj, const orn_linear* v_proj,
                     const orn_linear* o_proj, const bf16_t* q_norm, const bf16_t* k_norm, int T, const int* pos, bf16_t* kc, bf16_t* vc,
                     int keys, bool kv_only) {
@@ -579,10 +595,10 @@ int small_attention(orn_batch* bt, const FusedPrologue& fp, const orn_linear* q_
   jobs[0].lin = q_proj; jobs[0].out = bt->qg;
   jobs[1].lin = k_proj; jobs[1].out = bt->ak;
   jobs[2].lin = v_proj; jobs[2].out = bt->av;
-  CK(small_mm(bt, fp, jobs, 3, R));
+  CK(small_mm(bt, fp, kv_only ? jobs + 1 : jobs, kv_only ? 2 : 3, R));
+  if (kv_only) return kv_rows(bt, k_norm, T, pos, kc, vc);
   CK(f_attn(ctx, ctx->stream, bt->qg, bt->ak, bt->av, q_norm, k_norm, kc, vc, pos, T, c.n_heads, c.n_kv_heads, c.head_dim, bt->cap,
             c.rope_dims, m->lnb, c.rms_eps, bt->agated, orn_long_context(keys), bt->B));
-  if (kv_only) return ORN_OK;
   FusedPrologue gp;
   gp.mode = PRO_PLAIN; gp.K = c.n_heads * c.head_dim; gp.a = bt->agated;
   FusedJob oj;
@@ -989,7 +1005,7 @@ int32_t orn_batch_commit(orn_batch* bt, const int32_t* host_keep) {
       const bool exact = bt->exact || bt->B < 16;
       int max_pos = 0;
       for (int b = 0; b < bt->B; ++b) max_pos = std::max(max_pos, bt->h_mtp_pos[b]);
-      if (exact && small_path(bt, bt->B, bt->shard_world > 1 ? bt->shard_world : 1)) {
+      if (exact && bt->B <= kSmallEncode && small_path(bt, bt->B, bt->shard_world > 1 ? bt->shard_world : 1)) {
         CK(small_mtp(bt, bt->tok1, bt->hid0, max_pos + 1, true));
       } else {
         CK(mtp_join(bt, bt->tok1, bt->hid0));

@@ -275,6 +275,28 @@ def test_a_captured_step_belongs_to_the_group_it_was_captured_with(pkg, ctx):
     gm.free()
 
 
+@pytest.mark.parametrize("B", [1, 5])
+def test_re_encode_writes_keys_and_values_only(pkg, ctx, B):
+    """Below 16 sequences too: the commit of an accepted draft projects keys and values and appends them; no
+    query, no walk over the cache.  (That the rows have the single-sequence engine's bits is the test above.)"""
+    cfg = hp.tiny_config(pkg.Config)
+    gm = hp.upload_model(pkg, ctx, cfg, hp.tiny_model_weights(cfg, seed=17))
+    bt = pkg.Batch(gm, B, t_max=2, cap=64)
+    bt.fill_random(20, seed=1)
+    prim = np.arange(B, dtype=np.uint32)
+    drafts = bt.mtp_draft(prim)
+    bt.forward(np.stack([prim, drafts], 1))
+    ctx.ktime_begin()
+    bt.commit(np.full(B, 2, np.int32))
+    names = ctx.ktime_end()
+    assert not [n for n in names if n.startswith(("k_attn", "sdpa", "battn"))], names
+    assert names["attn_front"][0] == 1
+    wide = "%dx%d" % (2 * cfg.n_heads * cfg.head_dim, cfg.hidden)
+    assert not [n for n in names if wide in n], names      # the label of a launch names its first matrix
+    bt.free()
+    gm.free()
+
+
 @pytest.mark.parametrize("B,T", [(1, 1), (1, 2), (2, 2), (5, 1), (7, 2), (15, 1)])
 def test_few_rows_take_the_fused_kernels(pkg, ctx, B, T):
     """Up to 15 rows, in groups of four per launch (1, 2, 4, 5, 14 and 15 rows): the bits of the
