@@ -529,8 +529,11 @@ __global__ void mtp_advance_kernel(int* mtp_pos, const int* keep, int B, int bas
 // ---- fewer rows than the tensor cores are used for ----------------------------------------------
 // The single-sequence engine's fused kernels (fused.cu), four rows at a time where they take at most
 // four, all sequences at once where they are per sequence: the same bits as the one-kernel-per-op
-// path, a sixth of its launches, every weight read by the kernels built for few rows.  One sequence of
-// two rows: 9.9 -> 3.0 ms per cycle, bit for bit the same.
+// path, a sixth of its launches, every weight read by the kernels built for few rows, bit for bit the same.
+// Both sides at 700 cached positions, one kernel per op -> fused, ms per window: 1 row 7.0 -> 2.0, 2 rows 8.5 -> 2.5,
+// 4 rows 11.4 -> 3.9, 5 rows 13.0 -> 5.9, 8 rows 16.4 -> 7.3, 12 rows 21.4 -> 10.8, 14 rows 23.7 -> 13.0, 15 rows
+// 25.1 -> 14.3 (a group of four rows costs about 3.4); 16 rows take 7.8 on the tensor cores, whose products are not
+// row-invariant.  Drafts: 1 row 423 -> 237 us, 4 rows 659 -> 373, 7 rows 971 -> 654.
 constexpr int kSmallRows = 15;
 // The re-encode (one row per sequence, keys and values only) has little to read per launch, and every CTA of the
 // fused kernels rebuilds the norms of both of its inputs: up to this many sequences.  A commit, fused / one kernel
@@ -540,7 +543,7 @@ constexpr int kSmallEncode = 2;
 // the fused kernels serve every part of the model at these rows, on this GPU alone
 bool small_path(const orn_batch* bt, int rows, int world) {
   return bt->small_ok && rows <= kSmallRows && world == 1 && !bt->split_attn && orn_use_fused(bt->m) &&
-         bt->B * std::max(bt->m->cfg.gdn_v_heads, 1) <= 960 && bt->B * bt->m->cfg.n_heads <= 256;
+         bt->B * std::max(bt->m->cfg.gdn_v_heads, 1) <= kGdnMaxHeads && bt->B * bt->m->cfg.n_heads <= kAttnMaxHeads;
 }
 // jobs over `rows` rows of one prologue, at most four rows per launch
 int small_mm(orn_batch* bt, const FusedPrologue& fp, const FusedJob* jobs, int n, int rows) {

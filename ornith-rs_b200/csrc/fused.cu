@@ -1502,7 +1502,6 @@ struct GdnParams {
 
 constexpr int kGdnRows = 16;
 constexpr int kGdnMaxT = 4;
-constexpr int kGdnMaxHeads = 960;  // arrival counters of a launch: value heads over all its sequences
 
 // CTA = (head hv, block of kGdnRows state rows) of sequence blockIdx.z.  Threads 0 .. 4*kGdnRows-1 own the state (a row's
 // 128 floats over 4 lanes) and run the recurrence; the front end is spread over one warp per
@@ -2221,7 +2220,7 @@ int f_gdn(orn_ctx* ctx, cudaStream_t s, const bf16_t* conv, const bf16_t* cw, co
   p.k_scale = bfr(inv_scale);
   p.eps = eps;
   p.z = z; p.norm_w = norm_w; p.gated_out = gated_out; p.norm_eps = norm_eps;
-  p.arrivals = reinterpret_cast<unsigned int*>(ctx->dev_err) + 64;
+  p.arrivals = reinterpret_cast<unsigned int*>(ctx->dev_err) + kArrivalsAt;
   if (gated_out != nullptr && B * Hv > kGdnMaxHeads) ORN_FAIL(ctx, ORN_ERR_ARG, "fused gdn: too many value heads");
   dim3 grid(128 / kGdnRows, Hv, B);
   const dim3 block(gdn_threads(T));
@@ -2243,7 +2242,6 @@ int f_gdn(orn_ctx* ctx, cudaStream_t s, const bf16_t* conv, const bf16_t* cw, co
 // order), the partials (max, sum, out[256]) of all 32 groups go through global memory, and the CTA that
 // stores the last of them runs the same merge: the result has the bits of the one-CTA kernel.
 constexpr int kAttnSplit = 4;
-constexpr int kAttnMaxHeads = 256;  // query heads over all sequences of a launch
 constexpr int kAttnPart = 260;  // floats per group partial: out[256], max, sum, pad
 __global__ void __launch_bounds__(256) k_attn_split(AttnParams p, float* part, int* arrivals) {
   constexpr int HD = 256;

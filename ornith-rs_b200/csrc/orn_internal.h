@@ -14,6 +14,12 @@
 #include "../../include/ornith_cuda.h"
 #include "orn_common.cuh"
 
+// Words of a context's dev_err: [0] the error flag of bounded waits, [32] the wait probe's answer, from
+// kArrivalsAt on the arrival counters of the gated-delta kernel's heads
+constexpr int kDevWords = 1024, kArrivalsAt = 64;
+constexpr int kGdnMaxHeads = kDevWords - kArrivalsAt;  // value heads over all sequences of a launch
+constexpr int kAttnMaxHeads = 256;                     // query heads over all sequences of a split attention launch
+
 struct orn_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
