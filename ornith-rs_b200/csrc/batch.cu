@@ -310,7 +310,7 @@ struct orn_batch {
   uint32_t *ids, *targets, *conv_map;
   bf16_t *x, *n, *r, *h, *n2, *mo, *qkv, *z, *a, *b, *gq, *gk, *gv, *beta, *gy, *gated;
   float* gg;
-  bf16_t *qg, *aq, *agate, *ak, *av, *att, *agated, *logits;
+  bf16_t *qg, *aq, *ak, *av, *att, *agated, *logits;
   float *greedy_scratch, *part;
   int part_chunks = 0;
   // fewer rows than the tensor cores are used for: the fused decode kernels' scratch (kSmallRows rows)
@@ -465,7 +465,7 @@ int batch_attention(orn_batch* bt, const orn_linear* q_proj, const orn_linear* k
                     bt->aq, kc, vc));
   } else {
     CK(kv_rows(bt, k_norm, T, pos, kc, vc));
-    CK(k_split_qgate(ctx, s, bt->qg, R, Hq, hd, bt->aq, bt->agate));
+    CK(k_split_qgate(ctx, s, bt->qg, R, Hq, hd, bt->aq, nullptr));
     CK(k_rms_norm(ctx, s, bt->aq, q_norm, R * Hq, hd, c.rms_eps, bt->aq));
     CK(k_rope_batched(ctx, s, bt->aq, B, T, Hq, hd, c.rope_dims, m->lnb, pos));
   }
@@ -804,7 +804,7 @@ int32_t orn_batch_create(orn_model* m, int32_t B, int32_t T_max, int32_t cap, in
   A(&bt->qkv, R * D); A(&bt->z, R * VD); A(&bt->a, R * c.gdn_v_heads); A(&bt->b, R * c.gdn_v_heads);
   A(&bt->gq, R * KD); A(&bt->gk, R * KD); A(&bt->gv, R * VD); A(&bt->beta, R * c.gdn_v_heads); A(&bt->gg, R * c.gdn_v_heads);
   A(&bt->gy, R * VD); A(&bt->gated, R * VD);
-  A(&bt->qg, R * 2 * QD); A(&bt->aq, R * QD); A(&bt->agate, R * QD); A(&bt->ak, R * KVD); A(&bt->av, R * KVD);
+  A(&bt->qg, R * 2 * QD); A(&bt->aq, R * QD); A(&bt->ak, R * KVD); A(&bt->av, R * KVD);
   A(&bt->att, R * QD); A(&bt->agated, R * QD);
   A(&bt->logits, R * (size_t)c.vocab);
   A(&bt->normed, R * H);

@@ -816,7 +816,7 @@ int wide_reserve(orn_model* m, int rows) {
   A(&w.cb, (S + R) * D); A(&w.z, R * VD); A(&w.a, R * c.gdn_v_heads); A(&w.b, R * c.gdn_v_heads);
   A(&w.gq, R * KD); A(&w.gk, R * KD); A(&w.gv, R * VD); A(&w.beta, R * c.gdn_v_heads); A(&w.gg, R * c.gdn_v_heads);
   A(&w.gy, R * VD); A(&w.gated, R * VD);
-  A(&w.qg, R * 2 * QD); A(&w.aq, R * QD); A(&w.agate, R * QD); A(&w.ak, R * KVD); A(&w.av, R * KVD);
+  A(&w.qg, R * 2 * QD); A(&w.aq, R * QD); A(&w.ak, R * KVD); A(&w.av, R * KVD);
   A(&w.att, R * QD); A(&w.agated, R * QD);
   A(&w.gates, R * E); A(&w.scores, R * k); A(&w.sg, R * SI); A(&w.su, R * SI); A(&w.sact, R * SI);
   A(&w.sy, R * H); A(&w.gs, R);
@@ -935,7 +935,7 @@ int prefill_wide(orn_model* m, orn_cache* cc, int T, bf16_t* normed_out /*nullab
         CK(k_attn_front(ctx, s, w.qg, w.ak, w.av, ly.q_norm, ly.k_norm, T, 0, Hq, Hkv, c.max_ctx, c.rope_dims, m->lnb, c.rms_eps, cc->pos,
                         w.aq, cc->kc[i], cc->vc[i]));
       } else {
-        CK(k_split_qgate(ctx, s, w.qg, T, Hq, hd, w.aq, w.agate));
+        CK(k_split_qgate(ctx, s, w.qg, T, Hq, hd, w.aq, nullptr));
         CK(k_rms_norm(ctx, s, w.aq, ly.q_norm, T * Hq, hd, c.rms_eps, w.aq));
         CK(k_rms_norm(ctx, s, w.ak, ly.k_norm, T * Hkv, hd, c.rms_eps, w.ak));
         CK(k_rope(ctx, s, w.aq, T, Hq, hd, c.rope_dims, m->lnb, cc->pos, 0));

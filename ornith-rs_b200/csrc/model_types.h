@@ -66,7 +66,7 @@ struct WideWs {
   bf16_t *x, *n, *r, *h, *n2, *mo;
   bf16_t *cb, *z, *a, *b, *gq, *gk, *gv, *beta, *gy, *gated;
   float* gg;
-  bf16_t *qg, *aq, *agate, *ak, *av, *att, *agated;
+  bf16_t *qg, *aq, *ak, *av, *att, *agated;
   bf16_t *gates, *scores, *sg, *su, *sact, *sy, *gs;
   bf16_t *xs, *eg, *eu, *eact, *ey;
 };

@@ -429,14 +429,14 @@ __global__ void moe_combine_norm_kernel(const bf16_t* __restrict__ scores, const
   *reinterpret_cast<uint2*>(out + (int64_t)t * dim + c) = pack4(xv);
 }
 
-// q_proj output [T, Hq, 2*hd] -> queries [T,Hq,hd], gate [T,Hq,hd]
+// q_proj output [T, Hq, 2*hd] -> queries [T,Hq,hd], gate [T,Hq,hd] (nullable)
 // (qwen3_5.rs:441-443 slice_inner x2)
 __global__ void split_qgate_kernel(const bf16_t* qg, int n /*T*Hq*/, int hd, bf16_t* q, bf16_t* gate) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n * hd) return;
   int r = i / hd, d = i - r * hd;
   q[i] = qg[(int64_t)r * 2 * hd + d];
-  gate[i] = qg[(int64_t)r * 2 * hd + hd + d];
+  if (gate != nullptr) gate[i] = qg[(int64_t)r * 2 * hd + hd + d];
 }
 // concat_inner (mtp.rs:186): out[t] = [a[t], b[t]]
 __global__ void concat2_kernel(const bf16_t* a, const bf16_t* b, int T, int n, bf16_t* out) {
