@@ -521,13 +521,14 @@ int launch_grouped(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf1
   int z = L->E == 1 ? (max_rows + kGroupBatch - 1) / kGroupBatch : 4;
   if (z < 1) z = 1;
   if (z > 64) z = 64;
-  // one small dense matrix (a router): narrower blocks, so that the launch fills the part; one step of rows
-  // per warp while that leaves less than one block per SM (24 rows of a 256-row router: 18.3 -> 11.6 us)
+  // one small dense matrix (a router): narrower blocks, so that the launch fills the part; 16 rows, one step of
+  // two per warp, while blocks of 32 are fewer than the SMs (24 rows of a 256-row router: 18.3 -> 11.6 us).  Rows
+  // of up to 32 units go four to a warp, which are 32 rows a step already.
+  const int units = L->K / Fmt<KIND>::kWeightsPerUnit;
   const int wide_blocks = (L->O + 31) / 32 * z;
-  const int rpb = L->E != 1 || L->O > 1024 ? kGroupRows : wide_blocks < ctx->sm_count ? 16 : 32;
+  const int rpb = L->E != 1 || L->O > 1024 ? kGroupRows : units > 32 && wide_blocks < ctx->sm_count ? 16 : 32;
   const int blocks1 = (L->O + rpb - 1) / rpb, blocks2 = L2 ? (L2->O + rpb - 1) / rpb : 0;
   dim3 grid(blocks1 + blocks2, L->E, z);
-  const int units = L->K / Fmt<KIND>::kWeightsPerUnit;
   const LinDev d1 = lin_dev(L), d2 = L2 ? lin_dev(L2) : d1;
   if (units > 32) grouped_gemv_kernel<KIND, 2, 2><<<grid, kGroupThreads, smem, st>>>(d1, xs, seg, y, row_map, rpb, d2, y2, blocks1);
   else grouped_gemv_kernel<KIND, 4, 1><<<grid, kGroupThreads, smem, st>>>(d1, xs, seg, y, row_map, rpb, d2, y2, blocks1);
