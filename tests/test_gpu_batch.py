@@ -318,3 +318,66 @@ def test_few_rows_take_the_fused_kernels(pkg, ctx, B, T):
             assert np.array_equal(wt, gt[b]), (b, i)
     bt.free()
     gm.free()
+
+
+def cycles_equal(pkg, ctx, gm, B, cap, exact, n, keep_of):
+    """n cycles (draft, window [primary, draft], commit of keep_of(cycle, b) rows) of B sequences against the
+    single-sequence engine's op-level cycle, sequence by sequence: drafts, targets and hidden rows bit for bit."""
+    cfg = gm.cfg
+    bt = pkg.Batch(gm, B, t_max=2, cap=cap, exact=exact)
+    primary = np.arange(7, 7 + B).astype(np.uint32)
+    got = []
+    for cyc in range(n):
+        drafts = bt.mtp_draft(primary)
+        tg, hid = bt.forward(np.stack([primary, drafts], 1), want_hidden=True)
+        keep = np.array([keep_of(cyc, b) for b in range(B)], np.int32)
+        bt.commit(keep)
+        got.append((drafts.copy(), tg.copy(), hid.numpy().reshape(B, 2, cfg.hidden).copy()))
+        primary = tg[np.arange(B), keep - 1].copy()
+    positions = list(bt.positions())
+    bt.free()
+    cache = gm.make_cache()
+    for b in range(B):
+        cache.reset()
+        ctx.check(ctx._lib.orn_cache_set_mtp_offset(cache.h, 0), "mtp offset")
+        hrow, prim = ctx.upload(np.zeros((1, cfg.hidden), np.uint16)), 7 + b
+        for cyc, (drafts, tg, hid) in enumerate(got):
+            off = ctx._lib.orn_cache_mtp_offset(cache.h)
+            draft = gm.mtp_forward(cache, hrow, [prim])
+            vh = gm.forward(cache, np.array([prim, draft], np.uint32), capture=True)
+            want = gm.head_greedy(vh, 2)
+            rows = vh.numpy()
+            assert int(drafts[b]) == draft and np.array_equal(tg[b], want), (b, cyc)
+            assert np.array_equal(hid[b], rows.reshape(2, cfg.hidden)), (b, cyc)
+            keep = keep_of(cyc, b)
+            cache.rewind(keep)
+            ctx.check(ctx._lib.orn_cache_set_mtp_offset(cache.h, off + 1), "mtp offset")
+            if keep == 2:
+                gm.mtp_forward(cache, vh, [draft], kv_only=True)
+            hrow, prim = ctx.upload(rows.reshape(2, cfg.hidden)[keep - 1:keep].copy()), int(want[keep - 1])
+    cache.free()
+    return positions
+
+
+def test_split_attention_of_several_sequences_has_the_single_engines_bits(pkg, ctx):
+    """Three sequences whose trunk and draft caches pass 512 keys, where the attention of a head spreads over four
+    CTAs with partials and arrival counters per sequence, each at its own cycle, so that captured steps of both
+    forms replay."""
+    cfg = hp.tiny_config(pkg.Config, max_ctx=640)
+    gm = hp.upload_model(pkg, ctx, cfg, hp.tiny_model_weights(cfg, seed=18))
+    pos = cycles_equal(pkg, ctx, gm, 3, 640, False, 350, lambda cyc, b: 1 if cyc % (b + 2) == 0 else 2)
+    assert min(pos) > 520 and max(pos) < 640 and len(set(pos)) == 3
+    gm.free()
+
+
+@pytest.mark.parametrize("B,over", [(8, dict(rope_dims=8)), (8, dict(rope_dims=36)), (8, dict(rope_dims=128)),
+                                    (8, dict(rope_dims=256)), (2, dict(rope_dims=36)), (2, dict(rope_dims=128)),
+                                    (8, dict(hidden=256, top_k=1)), (8, dict(hidden=768, top_k=8))])
+def test_passes_between_the_products_at_their_edges(pkg, ctx, B, over):
+    """The attention front (rotated dims from one lane pair to the whole first half of a head, and outside its
+    rule: 36 and 256), the output gate, and combine + add + norm (one expert and the most a model may
+    have, eight; rows of 64 and of 192 threads) in a batch of exact products, against the single-sequence engine's bits."""
+    cfg = hp.tiny_config(pkg.Config, **over)
+    gm = hp.upload_model(pkg, ctx, cfg, hp.tiny_model_weights(cfg, seed=19))
+    cycles_equal(pkg, ctx, gm, B, 32, True, 4, lambda cyc, b: 1 + (cyc + b) % 2)
+    gm.free()
