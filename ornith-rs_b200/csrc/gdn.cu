@@ -217,8 +217,8 @@ constexpr int kRowsPerCta = 16;
 
 // AHEAD: the inputs of step t + 1 are requested before step t's arithmetic.  A long window otherwise pays a
 // memory round trip per token on top of the recurrence's own chain; a window of a few rows is bound by the
-// states' traffic and wants the registers for more warps (181 -> 127 registers, 10 -> 16 warps per
-// SM; 64 windows of two rows: 110 -> 86 us).
+// states' traffic and wants the registers for more warps (AHEAD 181 registers and 10 warps per SM, the other form
+// 127 and 16; 64 windows of two rows: 110 us ahead, 86 us not).
 template <bool AHEAD>
 __global__ void __launch_bounds__(kRowsPerCta * 4, AHEAD ? 1 : 8) gated_delta_kernel(const __grid_constant__ DeltaParams p) {
   const int hv = blockIdx.y;

@@ -11,7 +11,7 @@
 //
 // Shape of the kernel.  The contraction runs with the WEIGHTS as the A operand and the TOKENS as
 // the B operand, D[feature, token] = sum_k W[feature, k] x[token, k]: the tensor core's M is always
-// a full 128 features, its N is the token-tile width BN (16..256), so a launch with few tokens per
+// a full 128 features, its N is the token-tile width BN (16..128), so a launch with few tokens per
 // expert (a routed prompt chunk, a batched decode step) wastes no tensor-core work on padding.
 // One persistent CTA per SM walks work items (feature tile of 128, up to BN tokens, a range of K);
 // its warps have fixed roles and meet only at mbarriers:

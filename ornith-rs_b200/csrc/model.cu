@@ -1461,7 +1461,7 @@ int32_t orn_generate_step_mtp(orn_model* m, orn_cache* c, const uint32_t* prompt
     cycle_idx += 1;
     m->prof.verify_steps += 1;
     ORN_CHECK_CUDA(ctx, cudaStreamSynchronize(s));
-    uint32_t window[8];  // (the next cycle's copy may land in the pinned words while tokens are handed out)
+    uint32_t window[8];  // a copy of its own: on_token runs the caller's code
     memcpy(window, c->mailbox_h + 16, sizeof window);
     const uint32_t* targets = c->mailbox_h + 24;
     int k = 0;
