@@ -381,3 +381,9 @@ def test_passes_between_the_products_at_their_edges(pkg, ctx, B, over):
     gm = hp.upload_model(pkg, ctx, cfg, hp.tiny_model_weights(cfg, seed=19))
     cycles_equal(pkg, ctx, gm, B, 32, True, 4, lambda cyc, b: 1 + (cyc + b) % 2)
     gm.free()
+
+
+@pytest.mark.parametrize("B,T", [(1, 4), (3, 4), (5, 3)])
+def test_few_rows_in_windows_of_three_and_four(pkg, ctx, B, T):
+    """As above: windows above two rows move the recurrent states in whole lines, several sequences side by side."""
+    test_few_rows_take_the_fused_kernels(pkg, ctx, B, T)
