@@ -19,8 +19,8 @@
 //                 per slot: the scales of a super-block are fetched once, rows arrive as 128-byte
 //                 swizzled boxes that the dequantising threads read without bank conflicts
 //   warp 2        TMA of the token tiles [BN, 64] (and of bf16 weights)
-//   warps 8..15   dequantise: two groups of four warps, a group owns every second unit of two K blocks
-//                 (128 weights a thread: one feature row), stores them with tcgen05.st into TENSOR MEMORY,
+//   warps 8..     dequantise: two or three groups of four warps, a group owns every second (third) unit of two K
+//                 blocks (128 weights a thread: one feature row), stores them with tcgen05.st into TENSOR MEMORY,
 //                 where the MMA takes its A operand from, and hands the unit over with one arrival per
 //                 warp.  Fewer, longer steps won over sixteen warps of one K block each (with the
 //                 rest of this layout 146 -> 137 us for 1024 routed Q4_K rows): a hand-over costs a warp several hundred cycles of waiting
@@ -55,10 +55,10 @@ namespace {
 
 constexpr int BM = 128;            // features per tile: the tensor core's M
 constexpr int BK = 64;             // weights per K block: one 128-byte swizzle row of bf16
-constexpr int kDqGroups = 2, kDqWarps = 8;
+constexpr int kDqWarps = 4;     // dequantising warps of a group: one per quadrant of the 128 features
 constexpr int kSB = 4;          // K blocks of a super-block (256 weights), the step of the raw ring
 constexpr int U = 2;            // K blocks of a unit, the step of the ring the MMA reads
-constexpr int gemm_threads(bool direct) { return direct ? 256 : 256 + 32 * kDqWarps; }
+constexpr int gemm_threads(int groups) { return 256 + 32 * kDqWarps * groups; }
 constexpr uint32_t kWCols = BK / 2;     // tensor-memory columns of one dequantised 128 x 64 tile (two bf16 per column)
 constexpr int kSplitMaxRows = 512;      // dense products up to this many rows may split K
 constexpr int kMaxSplit = 8;            // = the portable cluster size: the splits of a tile are one cluster
@@ -641,8 +641,8 @@ __device__ __forceinline__ void leave_late(uint32_t b0, int raw_slots, int units
   __syncthreads();
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(gemm_threads(KIND == ORN_BF16), 1) k_qgemm(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmParams P) {
+template <int KIND, int G /*groups of dequantising warps*/>
+__global__ void __launch_bounds__(gemm_threads(G), 1) k_qgemm(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmParams P) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t s_bar[2 * kMaxRaw + 2 * kMaxUnits + 6];
   __shared__ int4 s_items[kItemCache];
@@ -667,10 +667,10 @@ __global__ void __launch_bounds__(gemm_threads(KIND == ORN_BF16), 1) k_qgemm(con
   if (threadIdx.x == 0) {
     for (int i = 0; i < (kDirect ? 0 : RS); ++i) {
       mbar_init(raw_full + 8 * i, 1);
-      mbar_init(raw_free + 8 * i, kDqWarps);
+      mbar_init(raw_free + 8 * i, G * kDqWarps);
     }
     for (int i = 0; i < NU; ++i) {
-      mbar_init(full + 8 * i, kDirect ? 1 : 1 + kDqWarps / kDqGroups);
+      mbar_init(full + 8 * i, kDirect ? 1 : 1 + kDqWarps);
       mbar_init(free_ + 8 * i, 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -816,8 +816,9 @@ __global__ void __launch_bounds__(gemm_threads(KIND == ORN_BF16), 1) k_qgemm(con
   } else if (warp >= 8) {
     // ---- dequantising warps
     const int g = (warp - 8) >> 2, q = warp & 3, r = 32 * q + lane;
+    int c = g, half = 0;  // this group's unit of the next super-block: 0, 1, or 2 for none
     const uint32_t wcol = tmem_w + ((uint32_t)(q * 32) << 16);
-    int us = g, rs = 0, i = 0, sb = 0, sb1 = -1;  // the group owns every second unit of the ring (NU is even)
+    int us = g, rs = 0, i = 0, sb = 0, sb1 = -1;  // the group owns every G-th unit of the ring (at least G long)
     uint32_t uph = 1, rph = 0;
     bool ok = true;
     typename F::Raw R;
@@ -826,15 +827,24 @@ __global__ void __launch_bounds__(gemm_threads(KIND == ORN_BF16), 1) k_qgemm(con
     // moves on to the next unit of the CTA's items and reads this thread's part of it into R; false when none is left.
     // Every unit is converted whole: blocks outside the item's K range are never multiplied.
     auto next = [&]() {
-      if (sb > sb1) {
-        if (i >= mine) return false;
-        const Item w = item(i++);
-        sb = w.kb0 / kSB; sb1 = (w.kb1 - 1) / kSB;
+      for (;;) {
+        if (sb > sb1) {
+          if (i >= mine) return false;
+          const Item w = item(i++);
+          sb = w.kb0 / kSB; sb1 = (w.kb1 - 1) / kSB;
+        }
+        ok = mbar_wait_warp(raw_full + 8 * rs, rph, P.err);
+        if (!ok) return false;
+        half = c;
+        c = G == 2 ? c : c == 2 ? 0 : c + 1;
+        if (G == 2 || half < kSB / U) {
+          F::load(R, raw0 + (uint32_t)rs * P.raw_bytes, r, half, sb++);
+          return true;
+        }
+        ++sb;  // the other groups have both of its units
+        if (lane == 0) mbar_arrive(raw_free + 8 * rs);
+        if (++rs == RS) { rs = 0; rph ^= 1u; }
       }
-      ok = mbar_wait_warp(raw_full + 8 * rs, rph, P.err);
-      if (!ok) return false;
-      F::load(R, raw0 + (uint32_t)rs * P.raw_bytes, r, g, sb++);
-      return true;
     };
     bool more = next();
     while (more) {
@@ -842,8 +852,8 @@ __global__ void __launch_bounds__(gemm_threads(KIND == ORN_BF16), 1) k_qgemm(con
       if (!ok) break;
       tc_fence_after();
       const uint32_t dst = wcol + (uint32_t)us * (U * kWCols), done = full + 8 * us, rfree = raw_free + 8 * rs;
-      F::convert(R, g, M, [&](int h, const uint32_t* v) { tmem_st16(dst + 16 * h, v); });
-      if ((us += kDqGroups) >= NU) { us = g; uph ^= 1u; }
+      F::convert(R, half, M, [&](int h, const uint32_t* v) { tmem_st16(dst + 16 * h, v); });
+      if ((us += G) >= NU) { us -= NU; uph ^= 1u; }
       if (++rs == RS) { rs = 0; rph ^= 1u; }
       tmem_st_wait();
       tc_fence_before();  // ordered before the MMA warp's reads through the barrier below
@@ -1061,13 +1071,13 @@ EncodeTiledFn encode_tiled() {
 
 std::mutex g_gemm_mu;
 
-template <int KIND>
+template <int KIND, int G>
 int launch_qgemm(orn_ctx* ctx, cudaStream_t s, const GemmMaps& maps, const GemmParams& P, int grid, size_t smem) {
-  int rc = orn_grant_smem(ctx, reinterpret_cast<const void*>(k_qgemm<KIND>), kGemmSmem);
+  int rc = orn_grant_smem(ctx, reinterpret_cast<const void*>(k_qgemm<KIND, G>), kGemmSmem);
   if (rc != ORN_OK) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(gemm_threads(KIND == ORN_BF16));
+  cfg.blockDim = dim3(gemm_threads(G));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
@@ -1075,7 +1085,7 @@ int launch_qgemm(orn_ctx* ctx, cudaStream_t s, const GemmMaps& maps, const GemmP
   at[0].val.clusterDim.x = P.splits / P.seq; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = P.splits > P.seq ? 1 : 0;
-  ORN_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_qgemm<KIND>, maps, P));
+  ORN_CHECK_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_qgemm<KIND, G>, maps, P));
   if (ctx->kt == nullptr) return orn_launch_check(ctx, "k_qgemm");
   // per-kernel timing: one label per shape
   static std::set<std::string> pool;
@@ -1151,6 +1161,12 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
     P.f_tiles += (Ls[j]->O + BM - 1) / BM;
   }
   const bool direct = L->kind == ORN_BF16;
+  // Groups of dequantising warps.  Dense products that do not split K are tiles of 80 to 128 tokens, whose weight ring is
+  // two to four units: a third group keeps a unit more under way (1001 x 2048 -> 8192 affine-8 55.3 -> 48.8 us, a
+  // prompt of 6621 rows 14.01 -> 13.67 ms).  Routed rows and split products have long rings and are bound by the
+  // instructions of all roles, where four more warps with fewer registers cost (1024 routed Q4_K rows 126 -> 130 us,
+  // Q6_K 78 -> 89 us; 64 sequences with split products on three groups 17.8 -> 18.7 ms).
+  const int G = grp == nullptr && rows > kSplitMaxRows ? 3 : 2;
   const int KB = L->K / BK;
   P.K = L->K; P.rows = rows; P.err = ctx->dev_err;
   P.seg = grp ? grp->seg : nullptr;
@@ -1188,10 +1204,10 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
   const size_t raw_b = direct ? 0 : raw_bytes(L->kind);
   auto part_bytes = [&](int c) { return c > 1 ? (size_t)((P.BN / 4 + c - 1) / c * P.splits) * (BM * 16) : 0; };
   if (P.splits > 1) {
-    const int most = (512 - 2 * U * (int)kWCols) / (int)P.acc_cols;
+    const int most = (512 - G * U * (int)kWCols) / (int)P.acc_cols;
     int c = P.splits <= std::min(3, most) ? 1 : P.splits;
     for (int t = std::min(4, P.splits); c > 1 && t >= 2; --t)
-      if (P.splits % t == 0 && P.splits / t <= most && part_bytes(t) + 2 * unit_b + 2 * raw_b <= room) { c = t; break; }
+      if (P.splits % t == 0 && P.splits / t <= most && part_bytes(t) + G * unit_b + 2 * raw_b <= room) { c = t; break; }
     P.seq = P.splits / c;
   }
   const int C = P.splits / P.seq;
@@ -1206,11 +1222,12 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
     P.raw_slots = P.units * U;
     P.raw_bytes = kWTileBytes;
   } else {
-    for (P.units = 6; P.units > 2; P.units -= 2)
-      if (accs + P.units * U * kWCols <= 512 && P.units * unit_b + 3 * P.raw_bytes + part <= room) break;
+    // (two groups own even and odd units, so their ring has an even number; three take a raw slot less for a unit more)
+    for (P.units = 6; P.units > G; P.units -= G == 2 ? 2 : 1)
+      if (accs + P.units * U * kWCols <= 512 && P.units * unit_b + (G == 2 || P.units > 4 ? 3 : 2) * P.raw_bytes + part <= room) break;
     P.raw_slots = (int)std::min<size_t>(kMaxRaw, (room - part - P.units * unit_b) / P.raw_bytes);
   }
-  if (P.units < 2 || P.raw_slots < 1) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: the rings do not fit into shared memory");
+  if (P.units < (direct ? 2 : G) || accs + (direct ? 0 : P.units * U * kWCols) > 512 || P.raw_slots < 1) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: the rings do not fit into shared memory");
   const size_t rings = P.units * unit_b + (direct ? 0 : (size_t)P.raw_slots * P.raw_bytes) + part;
   P.tmem_cols = 32;
   while (P.tmem_cols < accs + (direct ? 0u : P.units * U * kWCols)) P.tmem_cols <<= 1;
@@ -1251,13 +1268,15 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
     P.dense_tiles = P.f_tiles * ((rows + P.BN - 1) / P.BN);
     grid = C > 1 ? P.dense_tiles * C : std::min(P.dense_tiles, ctx->sm_count);  // a cluster has one tile
   }
+#define QGEMM(kind) return G == 2 ? launch_qgemm<kind, 2>(ctx, s, maps, P, grid, smem) : launch_qgemm<kind, 3>(ctx, s, maps, P, grid, smem)
   switch (L->kind) {
-    case ORN_Q4K: return launch_qgemm<ORN_Q4K>(ctx, s, maps, P, grid, smem);
-    case ORN_Q6K: return launch_qgemm<ORN_Q6K>(ctx, s, maps, P, grid, smem);
-    case ORN_A8: return launch_qgemm<ORN_A8>(ctx, s, maps, P, grid, smem);
-    case ORN_BF16: return launch_qgemm<ORN_BF16>(ctx, s, maps, P, grid, smem);
-    case ORN_A4: return launch_qgemm<ORN_A4>(ctx, s, maps, P, grid, smem);
+    case ORN_Q4K: QGEMM(ORN_Q4K);
+    case ORN_Q6K: QGEMM(ORN_Q6K);
+    case ORN_A8: QGEMM(ORN_A8);
+    case ORN_BF16: return launch_qgemm<ORN_BF16, 0>(ctx, s, maps, P, grid, smem);
+    case ORN_A4: QGEMM(ORN_A4);
   }
+#undef QGEMM
   ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: unknown weight format");
 }
 
