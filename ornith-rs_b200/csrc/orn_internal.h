@@ -234,6 +234,8 @@ struct MoeNextNorm {
   float eps;
   bf16_t *sum, *out;
 };
+// counting sort of a routing table in one launch where it is short enough (E <= 256, 8192 routes), as orn_ep_moe_block sorts its own
+bool orn_route_small(orn_ctx* ctx, cudaStream_t s, const uint32_t* inds, int routes, int E, int* seg, uint32_t* perm, int* rc);
 // a number no other group of this process ever has (a new group may get the address of a destroyed one)
 uint64_t orn_ep_serial(const orn_ep* ep);
 // orn_ep_moe_block; with `next`, that add and norm as well (dev_out is then scratch)
