@@ -345,11 +345,7 @@ namespace {
 int batch_mm(orn_batch* bt, const orn_linear* L, const bf16_t* x, int R, bf16_t* y) {
   orn_ctx* ctx = bt->m->ctx;
   if (R >= 16 && !bt->exact && L->K % 64 == 0) return f_qgemm(ctx, ctx->stream, L, x, R, y, L->O, nullptr);
-  for (int r = 0; r < R; r += kMaxRows) {
-    const int n = std::min(kMaxRows, R - r);
-    CK(k_gemv(ctx, ctx->stream, L, x + (size_t)r * L->K, n, y + (size_t)r * L->O, 0));
-  }
-  return ORN_OK;
+  return k_gemv(ctx, ctx->stream, L, x, R, y, 0);
 }
 
 // several projections of the same rows: consecutive matrices that share format and row length go

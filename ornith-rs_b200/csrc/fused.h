@@ -82,3 +82,8 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
 int f_route_sort(orn_ctx* ctx, cudaStream_t s, const uint32_t* rhs, int rows, int E, int* seg, int* cursor, uint32_t* perm);
 int f_gather_rows(orn_ctx* ctx, cudaStream_t s, const bf16_t* x, const uint32_t* lhs /*nullable*/, const uint32_t* perm,
                   int rows, int K, bf16_t* xs);
+
+// ---- rows.cu: the row-invariant mat-vec over many rows
+bool f_rows_ok(const orn_linear* L);
+int f_rows(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, bf16_t* const* ys, int n, const bf16_t* xs, int rows,
+           const int* seg = nullptr /*rows sorted by expert: device [E + 1]*/, const uint32_t* row_map = nullptr);

@@ -25,6 +25,7 @@
 // cores: the work per weight is one byte-permute, one add and M fmas.
 #include <cuda_fp16.h>
 
+#include "fused.h"
 #include "orn_internal.h"
 #include "orn_quant.cuh"
 
@@ -375,10 +376,18 @@ int dispatch_m(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16_t*
 
 }  // namespace
 
+namespace {
+// the product of many rows (rows.cu) takes this matrix and these rows
+bool rows_path(const orn_linear* L, const bf16_t* xs) { return f_rows_ok(L) && (reinterpret_cast<uintptr_t>(xs) & 15) == 0; }
+}  // namespace
+
 int k_gemv(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16_t* x, int M, void* y,
            int out_f32) {
-  // more than four rows: groups of four, each group re-reading the weights
-  // (the decode path never has more; prefill chunks do)
+  if (M > 4 && !out_f32 && rows_path(L, x)) {
+    bf16_t* yb = static_cast<bf16_t*>(y);
+    return f_rows(ctx, st, &L, &yb, 1, x, M);
+  }
+  // what rows.cu does not take (affine 4-bit, float32 results): groups of four rows, each re-reading the weights
   for (int m0 = 0; m0 < M; m0 += 4) {
     int mm = M - m0 < 4 ? M - m0 : 4;
     const bf16_t* xs = x + (int64_t)m0 * L->K;
@@ -540,6 +549,7 @@ int launch_grouped(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf1
 int k_grouped_gemv(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16_t* xs, const int* seg, bf16_t* y,
                    const uint32_t* row_map, int max_rows) {
   if (L->E > 65535) ORN_FAIL(ctx, ORN_ERR_ARG, "grouped gemv: more than 65535 experts");
+  if (rows_path(L, xs)) return f_rows(ctx, st, &L, &y, 1, xs, max_rows, seg, row_map);
   switch (L->kind) {
     case ORN_Q4K: return launch_grouped<ORN_Q4K>(ctx, st, L, xs, seg, y, row_map, max_rows);
     case ORN_Q6K: return launch_grouped<ORN_Q6K>(ctx, st, L, xs, seg, y, row_map, max_rows);
@@ -556,6 +566,11 @@ int k_grouped_gemv2(orn_ctx* ctx, cudaStream_t st, const orn_linear* L1, bf16_t*
   if (L1->kind != L2->kind || L1->K != L2->K || L1->E != 1 || L2->E != 1) {
     int rc = k_grouped_gemv(ctx, st, L1, xs, seg, y1, nullptr, max_rows);
     return rc != ORN_OK ? rc : k_grouped_gemv(ctx, st, L2, xs, seg, y2, nullptr, max_rows);
+  }
+  if (rows_path(L1, xs)) {
+    const orn_linear* Ls[2] = {L1, L2};
+    bf16_t* ys[2] = {y1, y2};
+    return f_rows(ctx, st, Ls, ys, 2, xs, max_rows, seg);
   }
   switch (L1->kind) {
     case ORN_Q4K: return launch_grouped<ORN_Q4K>(ctx, st, L1, xs, seg, y1, nullptr, max_rows, L2, y2);

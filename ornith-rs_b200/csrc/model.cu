@@ -26,9 +26,12 @@
 
 namespace {
 
-__global__ void iota_div_kernel(uint32_t* lhs, uint32_t* ident, int n, int k) {
+__global__ void iota_div_kernel(uint32_t* lhs, uint32_t* ident /*nullable*/, int n, int k) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) { lhs[i] = (uint32_t)(i / k); ident[i] = (uint32_t)i; }
+  if (i < n) {
+    lhs[i] = (uint32_t)(i / k);
+    if (ident != nullptr) ident[i] = (uint32_t)i;
+  }
 }
 __global__ void set_int_kernel(int* p, int v) { *p = v; }
 // mailbox = {primary, force flag[3], force token[3]} written by the host before each cycle;
@@ -756,12 +759,8 @@ bool wide_exact() {
 // y[T, O] = x[T, K] W^T for a prompt chunk
 int wide_mm(orn_model* m, const orn_linear* L, const bf16_t* x, int T, bf16_t* y) {
   orn_ctx* ctx = m->ctx;
-  if (!wide_exact()) return f_qgemm(ctx, ctx->stream, L, x, T, y, L->O, nullptr);
-  for (int r = 0; r < T; r += kMaxRows) {
-    const int n = std::min(kMaxRows, T - r);
-    CK(k_gemv(ctx, ctx->stream, L, x + (size_t)r * L->K, n, y + (size_t)r * L->O, 0));
-  }
-  return ORN_OK;
+  if (!m->wide.exact) return f_qgemm(ctx, ctx->stream, L, x, T, y, L->O, nullptr);
+  return k_gemv(ctx, ctx->stream, L, x, T, y, 0);
 }
 // several products of the same rows: neighbours of one format share a launch (more tiles per round of the
 // SMs, and a narrow matrix is no launch of its own) while that leaves the ranges of K of each of them, and so
@@ -776,11 +775,15 @@ int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear
     auto splits = [&](int tiles) { return f_qgemm_splits(m->ctx, tiles, T, j[i].first->K); };
     for (int tiles = 0; i + k < n && k < 4 && j[i + k].first->kind == j[i].first->kind && j[i + k].first->K == j[i].first->K; ++k) {
       const int own = (j[i + k].first->O + 127) / 128;
-      if (k > 0 && (splits(tiles + own) != splits(own) || splits(tiles + own) != splits(tiles))) break;
+      if (!m->wide.exact && k > 0 && (splits(tiles + own) != splits(own) || splits(tiles + own) != splits(tiles))) break;
       tiles += own;
       pl[k] = j[i + k].first; py[k] = j[i + k].second; ld[k] = pl[k]->O;
     }
-    if (wide_exact())
+    if (m->wide.exact && f_rows_ok(pl[0])) {
+      bf16_t* yb[4];
+      for (int q = 0; q < k; ++q) yb[q] = static_cast<bf16_t*>(py[q]);
+      CK(f_rows(m->ctx, m->ctx->stream, pl, yb, k, x, T));
+    } else if (m->wide.exact)
       for (int q = 0; q < k; ++q) CK(wide_mm(m, pl[q], x, T, static_cast<bf16_t*>(py[q])));
     else
       CK(f_qgemm_multi(m->ctx, m->ctx->stream, pl, py, ld, k, x, T));
@@ -790,6 +793,13 @@ int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear
 }
 constexpr int kWideMinRows = 64;    // measured: below about 60 rows the 4-row mat-vec windows are faster (the
                                     // reference's own crossover, kquant.rs MM_ROW_LIMIT, is 16 on its hardware)
+// Shorter chunks have the bits of the four-row windows whatever way they go.  From 13 rows on all of them go through the
+// wide path's launches with row-invariant products (rows.cu), which read a layer's weights once, an expert's for all its
+// rows.  Windows / one piece, ms for the whole model: 8 rows 6.3 / 8.0, 12 rows 9.4 / 9.3, 16 rows 12.5 / 10.6, 24 rows
+// 18.7 / 12.7, 48 rows 37.5 / 19.6, 63 rows 49.6 / 23.5.  Its attention walks a row's keys in one CTA, where the
+// windows spread long caches, so behind many cached positions the windows stay.
+constexpr int kRowsMin = 13;
+constexpr int kRowsMaxKeys = 1024;
 constexpr int kWideMaxRows = 8192;  // widest chunk of the wide path (the reference's default chunk is 2048, generate.rs:25)
 
 int wide_reserve(orn_model* m, int rows) {
@@ -811,7 +821,6 @@ int wide_reserve(orn_model* m, int rows) {
     if (rc == ORN_OK) { w.allocs.push_back(d); *p = (std::remove_reference_t<decltype(**p)>*)d; }
   };
   A(&w.ids, R); A(&w.lhs, R * k); A(&w.perm, R * k); A(&w.inds, R * k); A(&w.seg, 2 * E + 4);
-  A(&w.ident, R * k); A(&w.sorted_e, R * k); A(&w.perm_inv, R * k);
   A(&w.x, R * H); A(&w.n, R * H); A(&w.r, R * H); A(&w.h, R * H); A(&w.n2, R * H); A(&w.mo, R * H);
   A(&w.cb, (S + R) * D); A(&w.z, R * VD); A(&w.a, R * c.gdn_v_heads); A(&w.b, R * c.gdn_v_heads);
   A(&w.gq, R * KD); A(&w.gk, R * KD); A(&w.gv, R * VD); A(&w.beta, R * c.gdn_v_heads); A(&w.gg, R * c.gdn_v_heads);
@@ -831,21 +840,12 @@ int wide_reserve(orn_model* m, int rows) {
     return rc;
   }
   const int n = rows * c.top_k;
-  iota_div_kernel<<<(n + 255) / 256, 256, 0, m->ctx->stream>>>(w.lhs, w.ident, n, c.top_k);
+  iota_div_kernel<<<(n + 255) / 256, 256, 0, m->ctx->stream>>>(w.lhs, nullptr, n, c.top_k);
   CK(orn_launch_check(m->ctx, "iota_div"));
   w.cap = rows;
   return ORN_OK;
 }
 
-// sorted_e[p] = expert of sorted row p; perm_inv[original row] = its sorted position
-__global__ void perm_tables_kernel(const uint32_t* perm, const uint32_t* inds, int rows, uint32_t* sorted_e, uint32_t* perm_inv) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < rows) {
-    const uint32_t o = perm[p];
-    sorted_e[p] = inds[o];
-    perm_inv[o] = (uint32_t)p;
-  }
-}
 __global__ void copy_u4_kernel(const uint4* src, uint4* dst, size_t n) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = src[i];
@@ -864,12 +864,9 @@ int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, const M
   CK(k_softmax_topk(ctx, s, w.gates, T, E, c.top_k, w.inds, w.scores));
   CK(f_route_sort(ctx, s, w.inds, rows, E, w.seg, w.seg + E + 1, w.perm));
   CK(f_gather_rows(ctx, s, x, w.lhs, w.perm, rows, H, w.xs));
-  if (wide_exact()) {
-    // the routed rows through the row-invariant gather mat-vec, in sorted order like the products below
-    perm_tables_kernel<<<(rows + 255) / 256, 256, 0, s>>>(w.perm, w.inds, rows, w.sorted_e, w.perm_inv);
-    CK(orn_launch_check(ctx, "perm_tables"));
-    CK(k_gather_gemv(ctx, s, moe.sw_gate, w.xs, w.ident, w.sorted_e, rows, w.eg));
-    CK(k_gather_gemv(ctx, s, moe.sw_up, w.xs, w.ident, w.sorted_e, rows, w.eu));
+  if (w.exact) {
+    CK(k_grouped_gemv(ctx, s, moe.sw_gate, w.xs, w.seg, w.eg, nullptr, rows));
+    CK(k_grouped_gemv(ctx, s, moe.sw_up, w.xs, w.seg, w.eu, nullptr, rows));
   } else {
     QGemmGroup sorted{w.seg, nullptr, 0};
     if (moe.sw_gate->kind == moe.sw_up->kind) {  // gate and up of every expert in one launch
@@ -884,8 +881,8 @@ int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, const M
   }
   CK(k_swiglu2(ctx, s, w.sg, w.su, (size_t)T * SI, w.sact, w.eg, w.eu, w.seg + E, I, w.eact));  // shared and routed rows
   CK(wide_mm(m, moe.sh_down, w.sact, T, w.sy));
-  if (wide_exact()) {
-    CK(k_gather_gemv(ctx, s, moe.sw_down, w.eact, w.perm_inv, w.inds, rows, w.ey));
+  if (w.exact) {
+    CK(k_grouped_gemv(ctx, s, moe.sw_down, w.eact, w.seg, w.ey, w.perm, rows));
   } else {
     QGemmGroup back{w.seg, w.perm, 0};
     CK(f_qgemm(ctx, s, moe.sw_down, w.eact, rows, w.ey, H, &back));  // rows back in (token, slot) order
@@ -899,10 +896,11 @@ int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, const M
 // One prompt chunk of T rows (ids on the device in wide.ids) through the trunk: the layer
 // sequence of TextModel::forward_hidden (qwen3_5.rs:578-695) with every projection as one wide
 // product.  Only the caches matter (generate::prefill discards the hidden rows, generate.rs:90-136).
-int prefill_wide(orn_model* m, orn_cache* cc, int T, bf16_t* normed_out /*nullable: [T, H] rows after the final norm*/) {
+int prefill_wide(orn_model* m, orn_cache* cc, int T, bool exact, bf16_t* normed_out /*nullable: [T, H] rows after the final norm*/) {
   orn_ctx* ctx = m->ctx;
   cudaStream_t s = ctx->stream;
   WideWs& w = m->wide;
+  w.exact = exact;
   const orn_config& c = m->cfg;
   const int H = c.hidden, S = c.gdn_conv_kernel - 1, D = conv_dim(c);
   const int Hq = c.n_heads, Hkv = c.n_kv_heads, hd = c.head_dim;
@@ -921,7 +919,7 @@ int prefill_wide(orn_model* m, orn_cache* cc, int T, bf16_t* normed_out /*nullab
       CK(wide_mm_multi(m, {{ly.in_qkv, qkv}, {ly.in_z, w.z}, {ly.in_b, w.b}, {ly.in_a, w.a}}, w.n, T));
       CK(k_gdn_front(ctx, s, w.cb, qkv, ly.conv_w, w.a, w.b, ly.a_log, ly.dt_bias, T, c.gdn_k_heads, c.gdn_v_heads,
                      c.gdn_head_dim, c.gdn_conv_kernel, 1e-6f, cc->conv[i], w.gq, w.gk, w.gv, w.beta, w.gg, nullptr));
-      if (wide_exact())  // token by token, the decode path's arithmetic
+      if (exact)  // token by token, the decode path's arithmetic
         CK(k_gated_delta_ring(ctx, s, w.gq, w.gk, w.gv, w.gg, w.beta, cc->ring[i], kRing, cc->cur, 1, T, c.gdn_k_heads,
                               c.gdn_v_heads, w.gy));
       else  // chunkwise on the tensor cores; the state after the chunk's last token goes to ring slot cur + 1
@@ -942,7 +940,7 @@ int prefill_wide(orn_model* m, orn_cache* cc, int T, bf16_t* normed_out /*nullab
         CK(k_rope(ctx, s, w.ak, T, Hkv, hd, c.rope_dims, m->lnb, cc->pos, 0));
         CK(k_kv_append(ctx, s, w.ak, w.av, T, Hkv, hd, c.max_ctx, cc->pos, 0, cc->kc[i], cc->vc[i]));
       }
-      if (wide_exact() || hd != 256)  // the row-invariant kernel: one pass over the cache per (head, row)
+      if (exact || hd != 256)  // the row-invariant kernel: one pass over the cache per (head, row)
         CK(k_sdpa_decode(ctx, s, w.aq, cc->kc[i], cc->vc[i], T, Hq, Hkv, hd, c.max_ctx, cc->pos, 0, 1.0f / sqrtf((float)hd),
                          w.att));
       else
@@ -976,13 +974,15 @@ int prefill(orn_model* m, orn_cache* cc, const uint32_t* prompt, int n, int pref
   while (n - done > keep_last) {
     int chunk = std::min(step, n - done - keep_last);
     int off = 0;
-    if (chunk >= kWideMinRows && use_wide_prefill() && use_fused_env()) {
-      // a chunk wide enough for the tensor cores (the reference's tile path, kquant.rs:783-812)
+    const bool wide = chunk >= kWideMinRows;
+    if ((wide || (chunk >= kRowsMin && cc->h_pos + chunk <= kRowsMaxKeys)) && use_wide_prefill() && use_fused_env()) {
+      // a chunk wide enough for the tensor cores (the reference's tile path, kquant.rs:783-812), or a short one
+      // through the same launches with row-invariant products
       chunk = std::min(chunk, kWideMaxRows);
-      CK(wide_reserve(m, chunk));
+      CK(wide_reserve(m, std::max(chunk, kWideMinRows)));
       ORN_CHECK_CUDA(m->ctx, cudaMemcpyAsync(m->wide.ids, prompt + done, sizeof(uint32_t) * (size_t)chunk,
                                              cudaMemcpyHostToDevice, m->ctx->stream));
-      CK(prefill_wide(m, cc, chunk, normed_out ? normed_out + (size_t)done * m->cfg.hidden : nullptr));
+      CK(prefill_wide(m, cc, chunk, !wide || wide_exact(), normed_out ? normed_out + (size_t)done * m->cfg.hidden : nullptr));
       off = chunk;
     }
     while (off < chunk) {

@@ -58,9 +58,9 @@ struct Workspace {
 // activation scratch of the prompt path: one chunk of up to `cap` rows through the layers
 struct WideWs {
   int cap = 0;
+  bool exact = false;  // of the chunk under way: products row by row alike, to the bit
   std::vector<void*> allocs;
   uint32_t *ids = nullptr, *lhs = nullptr, *perm = nullptr, *inds = nullptr;
-  uint32_t *ident = nullptr, *sorted_e = nullptr, *perm_inv = nullptr;  // ORN_WIDE_EXACT only
   int* seg = nullptr;
   void* gdn_scratch = nullptr;  // per-chunk operands of the chunkwise gated-delta recurrence
   bf16_t *x, *n, *r, *h, *n2, *mo;

@@ -44,6 +44,26 @@ def test_one_layer_hidden_rows_within_rounding(pkg, ctx, interval, what):
     gm.free()
 
 
+@pytest.mark.parametrize("n,step", [(13, 2048), (17, 2048), (50, 2048), (63, 2048), (100, 30), (45, 32)])
+def test_short_chunks_have_the_bits_of_the_four_row_windows(pkg, ctx, n, step):
+    """Chunks of 13 to 63 rows in one piece (the smallest, the largest, several behind one another with a shorter
+    last one) against windows of four rows, at the model's layer shapes: hidden rows, and the tokens that follow."""
+    m = pkg.TextModel(ctx, pkg.qwen35_config(max_ctx=256, n_layers=4))
+    m.init_random(9)
+    ids = np.random.default_rng(n).integers(0, m.cfg.vocab, n).astype(np.uint32)
+    c = m.make_cache()
+    want = m.prefill(c, ids, prefill_step=4, want_hidden=True).numpy()
+    c.reset()
+    got = m.prefill(c, ids, prefill_step=step, want_hidden=True).numpy()
+    assert np.array_equal(got, want)
+    c.reset()
+    a = pkg.generate_step(m, c, ids, 4, prefill_step=4)
+    c.reset()
+    assert pkg.generate_step(m, c, ids, 4, prefill_step=step) == a
+    c.free()
+    m.free()
+
+
 def test_wide_prefill_and_generation_on_the_tiny_model(pkg, ctx):
     cfg = hp.tiny_config(pkg.Config, max_ctx=160)
     W = hp.tiny_model_weights(cfg, seed=5)
