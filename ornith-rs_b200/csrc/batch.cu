@@ -92,9 +92,11 @@ __global__ void set_ints_kernel(int* p, int n, int v) {
 // grid (chunks, Hkv, B), 4 warps.  The G * Tb <= 16 queries that share a KV head (query j is head
 // kvh * G + j / Tb, window row j % Tb) form the 16-row A operand of mma.sync.m16n8k16 (bf16 in, f32
 // out); a CTA owns `chunk` consecutive keys of one (sequence, KV head), its warps take 16-key tiles
-// round robin.  Per warp a private 3-stage cp.async pipeline brings a tile's K and V rows (16 x 512 B
+// round robin.  Per warp a private cp.async ring of three places brings a tile's K rows, then its V rows (16 x 512 B
 // each, rows padded to 528 B so that ldmatrix reads without bank conflicts) into shared memory;
-// rows at or beyond the sequence's length arrive as zeros.  Per tile: S = Q K^T (32 MMAs), online
+// rows at or beyond the sequence's length arrive as zeros.  110 KB a CTA, so that two share an SM: with places for
+// K and V together (three tiles, 210 KB) nothing moved while a CTA began or merged (a cycle of 64 sequences at 4096
+// positions, eleven launches of this kernel: 17.60 -> 17.17 ms).  Per tile: S = Q K^T (32 MMAs), online
 // softmax in the base-2 domain on the accumulator fragments, P (bf16) V (32 MMAs, V fragments through
 // ldmatrix.trans).  The warps' partials merge through shared memory and the CTA writes one
 // (max, sum, out[256]) per query; battn_merge_kernel folds the chunks.
@@ -102,7 +104,7 @@ constexpr int kAttWarps = 4;
 constexpr int kAttRowB = 528;                        // bytes per staged row: 256 bf16 + 16 B pad
 constexpr int kAttTile = 16 * kAttRowB;              // one 16-key tile of K or of V
 constexpr int kAttStages = 3;
-constexpr int kAttWarpBytes = kAttStages * 2 * kAttTile;                   // 50688
+constexpr int kAttWarpBytes = kAttStages * kAttTile;                       // 25344
 constexpr int kAttSmem = 16 * kAttRowB + kAttWarps * kAttWarpBytes;        // Q + the warps' pipelines
 static_assert(kAttWarpBytes >= 16 * 256 * 4 + 2 * 16 * 4, "a warp's partial must fit its pipeline memory");
 
@@ -141,21 +143,18 @@ __global__ void __launch_bounds__(kAttWarps * 32) battn_partial_kernel(const bf1
   const size_t base = (((size_t)b * Hkv + kvh) * cap) * HD;
   const int ntiles = (k1 - k0 + 15) / 16;
   const int my_tiles = ntiles > warp ? (ntiles - warp + kAttWarps - 1) / kAttWarps : 0;
-  auto issue = [&](int i) {  // this warp's i-th tile into stage i % kAttStages
+  uint32_t put = mine_s;  // the ring's next place: K of a tile, V of it, K of the next
+  auto issue = [&](const bf16_t* cache, int i) {  // K or V rows of this warp's i-th tile
     if (i < my_tiles) {
       const int n0 = k0 + 16 * (warp + kAttWarps * i);
-      const uint32_t dst = mine_s + (i % kAttStages) * 2 * kAttTile;
 #pragma unroll
-      for (int it = 0; it < 16; ++it) {
-        const int p = it * 32 + lane, row = p >> 5, piece = p & 31;
+      for (int row = 0; row < 16; ++row) {
         const int n = n0 + row;
-        const int ok = n < Lmax ? 16 : 0;
-        const size_t src = base + (size_t)min(n, cap - 1) * HD + 8 * piece;
-        cp_async16(dst + row * kAttRowB + 16 * piece, kc + src, ok);
-        cp_async16(dst + kAttTile + row * kAttRowB + 16 * piece, vc + src, ok);
+        cp_async16(put + row * kAttRowB + 16 * lane, cache + base + (size_t)min(n, cap - 1) * HD + 8 * lane, n < Lmax ? 16 : 0);
       }
     }
     cp_async_commit();
+    put = put == mine_s + (kAttStages - 1) * kAttTile ? mine_s : put + kAttTile;
   };
   float o[32][4];
 #pragma unroll
@@ -167,13 +166,19 @@ __global__ void __launch_bounds__(kAttWarps * 32) battn_partial_kernel(const bf1
   const uint32_t a_off = ((lane & 7) + 8 * ((lane >> 3) & 1)) * kAttRowB + 16 * (lane >> 4);
   const uint32_t k_off = ((lane & 7) + 8 * (lane >> 4)) * kAttRowB + 16 * ((lane >> 3) & 1);
   const uint32_t v_off = ((lane & 7) + 8 * ((lane >> 3) & 1)) * kAttRowB + 16 * (lane >> 4);
-  issue(0);
-  issue(1);
+  issue(kc, 0);
+  issue(vc, 0);
+  uint32_t at = mine_s;
+  auto next_place = [&]() {
+    const uint32_t p = at;
+    at = at == mine_s + (kAttStages - 1) * kAttTile ? mine_s : at + kAttTile;
+    return p;
+  };
   for (int i = 0; i < my_tiles; ++i) {
-    issue(i + 2);
+    issue(kc, i + 1);
     cp_async_wait<2>();
     __syncwarp();
-    const uint32_t ks = mine_s + (i % kAttStages) * 2 * kAttTile, vs = ks + kAttTile;
+    const uint32_t ks = next_place();
     const int n0 = k0 + 16 * (warp + kAttWarps * i);
     float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
@@ -215,6 +220,10 @@ __global__ void __launch_bounds__(kAttWarps * 32) battn_partial_kernel(const bf1
     }
     uint32_t pa[4] = {pack_bf16x2(pr[0][0], pr[0][1]), pack_bf16x2(pr[0][2], pr[0][3]), pack_bf16x2(pr[1][0], pr[1][1]),
                       pack_bf16x2(pr[1][2], pr[1][3])};
+    issue(vc, i + 1);  // where the keys were: every lane has read them (the shuffles and the vote above)
+    cp_async_wait<2>();
+    __syncwarp();
+    const uint32_t vs = next_place();
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       uint32_t bv[4];
@@ -222,7 +231,7 @@ __global__ void __launch_bounds__(kAttWarps * 32) battn_partial_kernel(const bf1
       mma16816(o[2 * j], pa, bv[0], bv[1]);
       mma16816(o[2 * j + 1], pa, bv[2], bv[3]);
     }
-    __syncwarp();  // the stage is refilled by the next iteration's issue
+    __syncwarp();  // the next iteration's keys come where these values were
   }
   cp_async_wait<0>();
   __syncwarp();
