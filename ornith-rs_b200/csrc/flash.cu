@@ -78,20 +78,30 @@ __global__ void __launch_bounds__(kFaWarps * 32, 2) flash_prefill_kernel(const b
     }
     __syncthreads();
     const uint32_t kt = st_s + (i & 1) * kFaStage, vt = kt + kFaKeys * kFaRowB;
+    // the scores of both 16-key steps of the tile first: a query fragment is read once for 32 keys (shared memory is as
+    // busy as the tensor pipe here) and four chains of products run side by side instead of two
+    float sc[2][2][4];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) sc[c >> 3][(c >> 2) & 1][c & 3] = 0.f;
+    if (i * kFaKeys <= wlast) {
+#pragma unroll
+      for (int kk = 0; kk < 16; ++kk) {
+        uint32_t a[4], b0[4], b1[4];
+        ldsm4(q_s + a_off + 32 * kk, a);
+        ldsm4(kt + k_off + 32 * kk, b0);
+        ldsm4(kt + 16 * kFaRowB + k_off + 32 * kk, b1);
+        mma16816(sc[0][0], a, b0[0], b0[1]);
+        mma16816(sc[0][1], a, b0[2], b0[3]);
+        mma16816(sc[1][0], a, b1[0], b1[1]);
+        mma16816(sc[1][1], a, b1[2], b1[3]);
+      }
+    }
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int n0 = i * kFaKeys + 16 * half;
       if (n0 > wlast) continue;  // warp-uniform: every key of this step is in the future of every row
-      const uint32_t ks = kt + half * 16 * kFaRowB, vs = vt + half * 16 * kFaRowB;
-      float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-      for (int kk = 0; kk < 16; ++kk) {
-        uint32_t a[4], bk[4];
-        ldsm4(q_s + a_off + 32 * kk, a);
-        ldsm4(ks + k_off + 32 * kk, bk);
-        mma16816(s[0], a, bk[0], bk[1]);
-        mma16816(s[1], a, bk[2], bk[3]);
-      }
+      const uint32_t vs = vt + half * 16 * kFaRowB;
+      float (&s)[2][4] = sc[half];
       const bool all_visible = n0 + 16 <= p0 + wrow + 1;  // warp-uniform: the first row already sees the step's last key
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
