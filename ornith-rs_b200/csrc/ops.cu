@@ -142,8 +142,7 @@ ORN_D void swiglu8(const bf16_t* g, const bf16_t* u, bf16_t* out) {
   const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
   uint32_t o[4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e)
-    o[e] = (uint32_t)f2bf(orn_swiglu_bf(lo_of(gw[e]), lo_of(uw[e]))) | ((uint32_t)f2bf(orn_swiglu_bf(hi_of(gw[e]), hi_of(uw[e]))) << 16);
+  for (int e = 0; e < 4; ++e) o[e] = bf2_mul(orn_silu_bf2(gw[e]), uw[e]);
   *reinterpret_cast<uint4*>(out) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 // eight elements per thread where the length and the pointers allow it
@@ -164,8 +163,7 @@ __global__ void gate_rows_kernel(const bf16_t* __restrict__ qg, const bf16_t* __
   const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, aw[4] = {av.x, av.y, av.z, av.w};
   uint32_t o[4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e)
-    o[e] = (uint32_t)f2bf(orn_sigmoid_bf(lo_of(gw[e])) * lo_of(aw[e])) | ((uint32_t)f2bf(orn_sigmoid_bf(hi_of(gw[e])) * hi_of(aw[e])) << 16);
+  for (int e = 0; e < 4; ++e) o[e] = bf2_mul(orn_sigmoid_bf2(gw[e]), aw[e]);
   *reinterpret_cast<uint4*>(out + 8 * i) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 __global__ void add_kernel(const bf16_t* a, const bf16_t* b, int n, bf16_t* out) {
@@ -384,7 +382,8 @@ __global__ void __launch_bounds__(128) moe_combine_wide_kernel(const bf16_t* __r
 __global__ void moe_combine_norm_kernel(const bf16_t* __restrict__ scores, const bf16_t* __restrict__ y, const bf16_t* __restrict__ gate,
                                         const bf16_t* __restrict__ shared, int k, int dim, int normalize, const bf16_t* __restrict__ h,
                                         const bf16_t* __restrict__ w, float eps, bf16_t* __restrict__ sum, bf16_t* __restrict__ out) {
-  __shared__ float red[32], s_w[8], s_g;
+  __shared__ float red[32];
+  __shared__ uint32_t s_w[8], s_g;  // a weight in both halves of a word
   const int t = blockIdx.x, c = 4 * threadIdx.x;
   const bool in = c < dim;
   uint2 yr[8], sh = make_uint2(0, 0), hr = sh, wr = sh;
@@ -401,34 +400,25 @@ __global__ void moe_combine_norm_kernel(const bf16_t* __restrict__ scores, const
     float denom = 0.f;
     if (normalize)
       for (int j = 0; j < k; ++j) denom = bfr(bf2f(s[j]) + denom);
-    if ((int)threadIdx.x < k) s_w[threadIdx.x] = normalize ? bfr(bf2f(s[threadIdx.x]) / denom) : bf2f(s[threadIdx.x]);
-    if (threadIdx.x == 31) s_g = orn_sigmoid_bf(bf2f(gate[t]));
+    if ((int)threadIdx.x < k) s_w[threadIdx.x] = bf2_dup(normalize ? bf2f(s[threadIdx.x]) / denom : bf2f(s[threadIdx.x]));
+    if (threadIdx.x == 31) s_g = bf2_dup(orn_sigmoid_bf(bf2f(gate[t])));
   }
   __syncthreads();
-  float acc[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
+  uint2 acc = make_uint2(0, 0);
 #pragma unroll
   for (int j = 0; j < 8; ++j)
-    if (in && j < k) {
-      unpack4(yr[j], v);
+    if (in && j < k) acc = make_uint2(bf2_add(bf2_mul(yr[j].x, s_w[j]), acc.x), bf2_add(bf2_mul(yr[j].y, s_w[j]), acc.y));
+  acc = make_uint2(bf2_add(hr.x, bf2_add(acc.x, bf2_mul(sh.x, s_g))), bf2_add(hr.y, bf2_add(acc.y, bf2_mul(sh.y, s_g))));
+  float xv[4], ss = 0.f;
+  unpack4(in ? acc : make_uint2(0, 0), xv);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[i] = bfr(bfr(v[i] * s_w[j]) + acc[i]);
-    }
-  float xv[4], hv[4], ss = 0.f;
-  unpack4(sh, v);
-  unpack4(hr, hv);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    xv[i] = in ? bfr(hv[i] + bfr(acc[i] + bfr(s_g * v[i]))) : 0.f;
-    ss = fmaf(xv[i], xv[i], ss);
-  }
+  for (int i = 0; i < 4; ++i) ss = fmaf(xv[i], xv[i], ss);
   const float total = block_sum_ordered(ss, red);
   const float inv = orn_rsqrtf(total / (float)dim + eps);
   if (!in) return;
-  if (sum != nullptr) *reinterpret_cast<uint2*>(sum + (int64_t)t * dim + c) = pack4(xv);
-  unpack4(wr, v);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) xv[i] = bfr(v[i] * bfr(xv[i] * inv));
-  *reinterpret_cast<uint2*>(out + (int64_t)t * dim + c) = pack4(xv);
+  if (sum != nullptr) *reinterpret_cast<uint2*>(sum + (int64_t)t * dim + c) = acc;
+  *reinterpret_cast<uint2*>(out + (int64_t)t * dim + c) =
+      make_uint2(bf2_mul(wr.x, bf2_pack(xv[0] * inv, xv[1] * inv)), bf2_mul(wr.y, bf2_pack(xv[2] * inv, xv[3] * inv)));
 }
 
 // q_proj output [T, Hq, 2*hd] -> queries [T,Hq,hd], gate [T,Hq,hd] (nullable)

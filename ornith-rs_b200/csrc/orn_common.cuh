@@ -210,6 +210,52 @@ ORN_HD float orn_silu_bf(float x) { return bfr(x * orn_sigmoid_bf(x)); }
 // swiglu in bfloat16: bf( bf(g*sigmoid(g)) * u )   (ornith_elementwise.metal:94-105)
 ORN_HD float orn_swiglu_bf(float g, float u) { return bfr(orn_silu_bf(g) * u); }
 
+#ifdef __CUDACC__
+// Two bfloat16 values in a word.  A product or sum of two bfloat16 values rounded once to bfloat16 is what the float form
+// rounds to: the product is exact in float, and a sum that is not has an addend below 2^-16 of the other, far from a
+// tie.  One instruction for two elements instead of the operation, the conversion and the widening of each, which is what
+// bounds the passes between the products: 2048 prompt rows' SwiGLU 28.5 -> 16.3 us, conv front 71 -> 53, combine and
+// norm 38 -> 27, output gate 17.5 -> 12.
+ORN_D uint32_t bf2_mul(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+ORN_D uint32_t bf2_add(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+ORN_D uint32_t bf2_pack(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+ORN_D uint32_t bf2_dup(float v) { return bf2_pack(v, v); }
+// orn_sigmoid_bf of both
+ORN_D uint32_t orn_sigmoid_bf2(uint32_t x) {
+  const uint32_t a2 = x & 0x7fff7fffu;
+  float e[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float a = __uint_as_float(i ? a2 & 0xffff0000u : a2 << 16);
+    const float h = a * 1.44269504f, l = fmaf(a, 1.44269504f, -h) + a * 1.92596299e-8f;
+    asm("ex2.approx.f32 %0, %1;" : "=f"(e[i]) : "f"(h));
+    e[i] = fmaf(e[i], l * 0.693147181f, e[i]);
+    e[i] = a > 88.5f ? orn_u2f(0x7f800000u) : e[i];
+  }
+  const uint32_t d = bf2_add(bf2_pack(e[0], e[1]), 0x3f803f80u);
+  float y0, y1;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(y0) : "f"(__uint_as_float(d << 16)));
+  asm("rcp.approx.f32 %0, %1;" : "=f"(y1) : "f"(__uint_as_float(d & 0xffff0000u)));
+  const uint32_t y = bf2_pack(y0, y1), z = bf2_add(y ^ 0x80008000u, 0x3f803f80u);  // 1 - y
+  uint32_t neg;  // the sign of each half, over all of its bits (the intrinsic has no sign mode)
+  asm("prmt.b32 %0, %1, 0, 0xbb99;" : "=r"(neg) : "r"(x));
+  return (y & neg) | (z & ~neg);
+}
+ORN_D uint32_t orn_silu_bf2(uint32_t x) { return bf2_mul(x, orn_sigmoid_bf2(x)); }
+#endif
+
 // softplus evaluated in bfloat16 as logaddexp(x, 0) = max + log1p(exp(min-max))
 // (kernels/ornith_logaddexp.h:13-23)
 ORN_HD float orn_softplus_bf(float x /* bf16 value */) {
