@@ -351,15 +351,18 @@ struct orn_batch {
 
 namespace {
 
+// the tensor cores compute this product of R rows
+bool batch_wide(const orn_batch* bt, const orn_linear* L, int R) { return R >= 16 && !bt->exact && L->K % 64 == 0; }
 int batch_mm(orn_batch* bt, const orn_linear* L, const bf16_t* x, int R, bf16_t* y) {
   orn_ctx* ctx = bt->m->ctx;
-  if (R >= 16 && !bt->exact && L->K % 64 == 0) return f_qgemm(ctx, ctx->stream, L, x, R, y, L->O, nullptr);
+  if (batch_wide(bt, L, R)) return f_qgemm(ctx, ctx->stream, L, x, R, y, L->O, nullptr);
   return k_gemv(ctx, ctx->stream, L, x, R, y, 0);
 }
 
 // several projections of the same rows: consecutive matrices that share format and row length go
-// out as one tensor-core launch (their feature tiles form one tile space)
-int batch_mm_multi(orn_batch* bt, const orn_linear* const* Ls, bf16_t* const* ys, int n, const bf16_t* x, int R) {
+// out as one tensor-core launch (their feature tiles form one tile space); map0: output rows of the first (tensor
+// cores only)
+int batch_mm_multi(orn_batch* bt, const orn_linear* const* Ls, bf16_t* const* ys, int n, const bf16_t* x, int R, const uint32_t* map0 = nullptr) {
   orn_ctx* ctx = bt->m->ctx;
   if (!(R >= 16 && !bt->exact)) {
     for (int i = 0; i < n; ++i) CK(batch_mm(bt, Ls[i], x, R, ys[i]));
@@ -385,7 +388,7 @@ int batch_mm_multi(orn_batch* bt, const orn_linear* const* Ls, bf16_t* const* ys
     void* yv[4];
     int ld[4];
     for (int k = i; k < j; ++k) { yv[k - i] = ys[k]; ld[k - i] = Ls[k]->O; }
-    if (Ls[i]->K % 64 == 0) CK(f_qgemm_multi(ctx, st, Ls + i, yv, ld, j - i, x, R));
+    if (Ls[i]->K % 64 == 0) CK(f_qgemm_multi(ctx, st, Ls + i, yv, ld, j - i, x, R, nullptr, 0, i == 0 ? map0 : nullptr));
     else for (int k = i; k < j; ++k) CK(batch_mm(bt, Ls[k], x, R, ys[k]));
     i = j;
   }
@@ -713,10 +716,15 @@ int batch_body(orn_batch* bt, orn_ep* group, int T, int chunk, int nchunks) {
     const Layer& ly = m->layers[i];
     if (ly.linear) {
       const orn_linear* pl[4] = {ly.in_qkv, ly.in_z, ly.in_b, ly.in_a};
-      bf16_t* py[4] = {bt->qkv, bt->z, bt->b, bt->a};
-      CK(batch_mm_multi(bt, pl, py, 4, bt->n, R));
-      scatter_rows_kernel<<<R, 128, 0, s>>>(bt->qkv, bt->conv_map, D, bt->conv[i]);  // row (b, t) -> window row S + t of sequence b
-      CK(orn_launch_check(ctx, "scatter_rows"));
+      // row (b, t) of the qkv projection belongs in window row S + t of sequence b: the tensor-core product stores it
+      // there (a copy of its own took 6.5 us a layer)
+      const bool direct = batch_wide(bt, ly.in_qkv, R);
+      bf16_t* py[4] = {direct ? bt->conv[i] : bt->qkv, bt->z, bt->b, bt->a};
+      CK(batch_mm_multi(bt, pl, py, 4, bt->n, R, direct ? bt->conv_map : nullptr));
+      if (!direct) {
+        scatter_rows_kernel<<<R, 128, 0, s>>>(bt->qkv, bt->conv_map, D, bt->conv[i]);
+        CK(orn_launch_check(ctx, "scatter_rows"));
+      }
       CK(k_gdn_front_batched(ctx, s, bt->conv[i], (int64_t)bt->conv_rows * D, ly.conv_w, bt->a, bt->b, ly.a_log, ly.dt_bias, B, T,
                              c.gdn_k_heads, c.gdn_v_heads, c.gdn_head_dim, c.gdn_conv_kernel, 1e-6f, bt->gq, bt->gk, bt->gv,
                              bt->beta, bt->gg));

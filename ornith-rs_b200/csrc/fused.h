@@ -78,7 +78,8 @@ int f_qgemm(orn_ctx* ctx, cudaStream_t s, const orn_linear* L, const bf16_t* x, 
 // up to four matrices of one format and row length over the same rows in one launch
 int f_qgemm_splits(const orn_ctx* ctx, int f_tiles, int rows, int K);  // ranges of K of a dense launch with that many 128-feature tiles
 int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, void* const* ys, const int* ldys, int n,
-                  const bf16_t* x, int rows, const QGemmGroup* grp = nullptr, int out_f32 = 0);
+                  const bf16_t* x, int rows, const QGemmGroup* grp = nullptr, int out_f32 = 0,
+                  const uint32_t* map0 = nullptr /*dense: output rows of the first matrix*/);
 int f_route_sort(orn_ctx* ctx, cudaStream_t s, const uint32_t* rhs, int rows, int E, int* seg, int* cursor, uint32_t* perm);
 int f_gather_rows(orn_ctx* ctx, cudaStream_t s, const bf16_t* x, const uint32_t* lhs /*nullable*/, const uint32_t* perm,
                   int rows, int K, bf16_t* xs);

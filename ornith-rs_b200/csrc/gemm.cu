@@ -79,6 +79,7 @@ struct GemmJob {
   bf16_t* y;
   float* y_f32;        // non-null: float32 output instead of bfloat16
   int vec8;            // y may be stored eight bfloat16 at a time
+  const uint32_t* row_map;  // nullable: output row of (sorted) row p
 };
 struct GemmParams {
   int njobs;
@@ -88,7 +89,6 @@ struct GemmParams {
   int dense_tiles;     // dense: feature tiles x token groups
   int rows;            // rows of x (dense) / of the sorted row space (grouped)
   int K;
-  const uint32_t* row_map;   // nullable: output row of sorted row p
   int BN, f_tiles;
   int raw_slots, units;      // slots of the raw ring, units of the MMA's ring
   uint32_t raw_bytes;        // bytes of one raw slot
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(gemm_threads(G), 1) k_qgemm(const __grid_const
         if (J.vec8) {
           const int row = (int)(threadIdx.x & 127) >> 3, piece = threadIdx.x & 7, t = tok(row);
           size_t orow = 0;
-          if (t < w.ntok) orow = P.row_map != nullptr ? P.row_map[w.tok0 + t] : (size_t)(w.tok0 + t);
+          if (t < w.ntok) orow = J.row_map != nullptr ? J.row_map[w.tok0 + t] : (size_t)(w.tok0 + t);
           bf16_t* st = &s_stage[sbuf][0][q * 32 + lane];
 #pragma unroll
           for (int r = 0; r < 16; ++r) st[r * kStageLd] = f2bf(v[r]);
@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(gemm_threads(G), 1) k_qgemm(const __grid_const
         for (int r = 0; r < 16; ++r) {
           const int t = tok(r);
           if (t < w.ntok && fo < J.O) {
-            const size_t orow = P.row_map != nullptr ? P.row_map[w.tok0 + t] : (size_t)(w.tok0 + t);
+            const size_t orow = J.row_map != nullptr ? J.row_map[w.tok0 + t] : (size_t)(w.tok0 + t);
             const size_t at = orow * J.ldy + fo;
             if (J.y_f32 != nullptr) J.y_f32[at] = v[r];
             else J.y[at] = f2bf(v[r]);
@@ -1110,6 +1110,7 @@ uint32_t raw_bytes(int kind) {
 // y[rows, O] (row stride ldy) = x[rows, K] W^T.  grp != null: rows are sorted by expert, expert e
 // owns rows seg[e] .. seg[e+1]-1 (device array of E + 1 ints) and multiplies by W[e]; row p of the
 // result goes to output row row_map[p] when row_map is given.
+// (map0 of f_qgemm_multi: the same for the first matrix of a dense launch.)
 int f_qgemm(orn_ctx* ctx, cudaStream_t s, const orn_linear* L, const bf16_t* x, int rows, void* y, int ldy,
             const QGemmGroup* grp, int out_f32) {
   return f_qgemm_multi(ctx, s, &L, &y, &ldy, 1, x, rows, grp, out_f32);
@@ -1136,7 +1137,7 @@ int f_qgemm_splits(const orn_ctx* ctx, int f_tiles, int rows, int K) {
 }
 
 int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, void* const* ys, const int* ldys, int n,
-                  const bf16_t* x, int rows, const QGemmGroup* grp, int out_f32) {
+                  const bf16_t* x, int rows, const QGemmGroup* grp, int out_f32, const uint32_t* map0) {
   if (rows < 1) return ORN_OK;
   if (n < 1 || n > kMaxJobs) ORN_FAIL(ctx, ORN_ERR_ARG, "gemm: 1..4 matrices per launch");
   const orn_linear* L = Ls[0];
@@ -1155,6 +1156,7 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
   for (int j = 0; j < n; ++j) {
     GemmJob& J = P.job[j];
     J.O = Ls[j]->O; J.tile0 = P.f_tiles; J.ldy = ldys[j];
+    J.row_map = grp ? grp->row_map : j == 0 ? map0 : nullptr;
     J.y = out_f32 ? nullptr : reinterpret_cast<bf16_t*>(ys[j]);
     J.y_f32 = out_f32 ? reinterpret_cast<float*>(ys[j]) : nullptr;
     J.vec8 = !out_f32 && (ldys[j] & 7) == 0 && (Ls[j]->O & 7) == 0 && (reinterpret_cast<uintptr_t>(ys[j]) & 15) == 0;
@@ -1170,7 +1172,6 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
   const int KB = L->K / BK;
   P.K = L->K; P.rows = rows; P.err = ctx->dev_err;
   P.seg = grp ? grp->seg : nullptr;
-  P.row_map = grp ? grp->row_map : nullptr;
   P.E = L->E;
   P.splits = grp == nullptr ? f_qgemm_splits(ctx, P.f_tiles, rows, L->K) : 1;
   P.seq = 1;
