@@ -757,37 +757,53 @@ bool wide_exact() {
   return v == 1;
 }
 // y[T, O] = x[T, K] W^T for a prompt chunk
-int wide_mm(orn_model* m, const orn_linear* L, const bf16_t* x, int T, bf16_t* y) {
-  orn_ctx* ctx = m->ctx;
-  if (!m->wide.exact) return f_qgemm(ctx, ctx->stream, L, x, T, y, L->O, nullptr);
-  return k_gemv(ctx, ctx->stream, L, x, T, y, 0);
+int wide_mm(orn_model* m, const orn_linear* L, const bf16_t* x, int T, bf16_t* y, cudaStream_t st) {
+  if (!m->wide.exact) return f_qgemm(m->ctx, st, L, x, T, y, L->O, nullptr);
+  return k_gemv(m->ctx, st, L, x, T, y, 0);
 }
 // several products of the same rows: neighbours of one format share a launch (more tiles per round of the
 // SMs, and a narrow matrix is no launch of its own) while that leaves the ranges of K of each of them, and so
-// its bits, as they are alone
-int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear*, bf16_t*>> jobs, const bf16_t* x, int T) {
+// its bits, as they are alone.  fork: what follows the first launch and is narrow (the gates of a recurrent layer, a
+// few tiles that leave most SMs idle for 11 us) runs on the side stream beside it.
+int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear*, bf16_t*>> jobs, const bf16_t* x, int T, cudaStream_t st,
+                  bool fork = false) {
+  orn_ctx* ctx = m->ctx;
+  bool forked = false;
+  if (fork && (fork = orn_side_stream(ctx))) ORN_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev_fork, st));
   const auto* j = jobs.begin();
   const int n = (int)jobs.size();
   for (int i = 0; i < n;) {
     const orn_linear* pl[4];
     void* py[4];
     int ld[4], k = 0;
+    int features = 0;
     auto splits = [&](int tiles) { return f_qgemm_splits(m->ctx, tiles, T, j[i].first->K); };
     for (int tiles = 0; i + k < n && k < 4 && j[i + k].first->kind == j[i].first->kind && j[i + k].first->K == j[i].first->K; ++k) {
       const int own = (j[i + k].first->O + 127) / 128;
       if (!m->wide.exact && k > 0 && (splits(tiles + own) != splits(own) || splits(tiles + own) != splits(tiles))) break;
       tiles += own;
+      features += j[i + k].first->O;
       pl[k] = j[i + k].first; py[k] = j[i + k].second; ld[k] = pl[k]->O;
     }
+    const bool beside = fork && i > 0 && features <= 256;
+    if (beside && !forked) {
+      ORN_CHECK_CUDA(ctx, cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
+      forked = true;
+    }
+    const cudaStream_t on = beside ? ctx->side : st;
     if (m->wide.exact && f_rows_ok(pl[0])) {
       bf16_t* yb[4];
       for (int q = 0; q < k; ++q) yb[q] = static_cast<bf16_t*>(py[q]);
-      CK(f_rows(m->ctx, m->ctx->stream, pl, yb, k, x, T));
+      CK(f_rows(ctx, on, pl, yb, k, x, T));
     } else if (m->wide.exact)
-      for (int q = 0; q < k; ++q) CK(wide_mm(m, pl[q], x, T, static_cast<bf16_t*>(py[q])));
+      for (int q = 0; q < k; ++q) CK(wide_mm(m, pl[q], x, T, static_cast<bf16_t*>(py[q]), on));
     else
-      CK(f_qgemm_multi(m->ctx, m->ctx->stream, pl, py, ld, k, x, T));
+      CK(f_qgemm_multi(ctx, on, pl, py, ld, k, x, T));
     i += k;
+  }
+  if (forked) {
+    ORN_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->side));
+    ORN_CHECK_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_join, 0));
   }
   return ORN_OK;
 }
@@ -860,8 +876,21 @@ int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, const M
   WideWs& w = m->wide;
   const orn_config& c = m->cfg;
   const int rows = T * c.top_k, H = c.hidden, I = c.expert_inter, SI = c.shared_inter, E = c.n_experts;
-  CK(wide_mm_multi(m, {{moe.gate, w.gates}, {moe.sh_egate, w.gs}, {moe.sh_gate, w.sg}, {moe.sh_up, w.su}}, x, T));
+  CK(wide_mm_multi(m, {{moe.gate, w.gates}, {moe.sh_egate, w.gs}}, x, T, s));
   CK(k_softmax_topk(ctx, s, w.gates, T, E, c.top_k, w.inds, w.scores));
+  // The shared expert depends on x only: its three launches run on the side stream beside the sort of the routes, whose
+  // kernels leave the SMs idle, and are joined before the combine (a prompt of 97 rows 1647 -> 1509 us, the gates of the
+  // recurrent layers on the side stream among it; forked before the router, whose product they then hold up: 1534).
+  const bool side = orn_side_stream(ctx);
+  const cudaStream_t ss = side ? ctx->side : s;
+  if (side) {
+    ORN_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev_fork, s));
+    ORN_CHECK_CUDA(ctx, cudaStreamWaitEvent(ss, ctx->ev_fork, 0));
+  }
+  CK(wide_mm_multi(m, {{moe.sh_gate, w.sg}, {moe.sh_up, w.su}}, x, T, ss));
+  CK(k_swiglu(ctx, ss, w.sg, w.su, T * SI, w.sact));
+  CK(wide_mm(m, moe.sh_down, w.sact, T, w.sy, ss));
+  if (side) ORN_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev_join, ss));
   CK(f_route_sort(ctx, s, w.inds, rows, E, w.seg, w.seg + E + 1, w.perm));
   CK(f_gather_rows(ctx, s, x, w.lhs, w.perm, rows, H, w.xs));
   if (w.exact) {
@@ -879,14 +908,14 @@ int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, const M
       CK(f_qgemm(ctx, s, moe.sw_up, w.xs, rows, w.eu, I, &sorted));
     }
   }
-  CK(k_swiglu2(ctx, s, w.sg, w.su, (size_t)T * SI, w.sact, w.eg, w.eu, w.seg + E, I, w.eact));  // shared and routed rows
-  CK(wide_mm(m, moe.sh_down, w.sact, T, w.sy));
+  CK(k_swiglu2(ctx, s, nullptr, nullptr, 0, nullptr, w.eg, w.eu, w.seg + E, I, w.eact));
   if (w.exact) {
     CK(k_grouped_gemv(ctx, s, moe.sw_down, w.eact, w.seg, w.ey, w.perm, rows));
   } else {
     QGemmGroup back{w.seg, w.perm, 0};
     CK(f_qgemm(ctx, s, moe.sw_down, w.eact, rows, w.ey, H, &back));  // rows back in (token, slot) order
   }
+  if (side) ORN_CHECK_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));
   if (k_moe_combine_norm_ok(c.top_k, H))
     return k_moe_combine_norm(ctx, s, w.scores, w.ey, w.gs, w.sy, T, c.top_k, H, c.norm_topk_prob, next.h, next.w, next.eps, next.sum, next.out);
   CK(k_moe_combine(ctx, s, w.scores, w.ey, w.gs, w.sy, T, c.top_k, H, c.norm_topk_prob, w.mo));
@@ -916,7 +945,7 @@ int prefill_wide(orn_model* m, orn_cache* cc, int T, bool exact, bf16_t* normed_
                                                                  reinterpret_cast<uint4*>(w.cb), n16);
       CK(orn_launch_check(ctx, "copy_u4"));
       bf16_t* qkv = w.cb + (size_t)S * D;
-      CK(wide_mm_multi(m, {{ly.in_qkv, qkv}, {ly.in_z, w.z}, {ly.in_b, w.b}, {ly.in_a, w.a}}, w.n, T));
+      CK(wide_mm_multi(m, {{ly.in_qkv, qkv}, {ly.in_z, w.z}, {ly.in_b, w.b}, {ly.in_a, w.a}}, w.n, T, s, true));
       CK(k_gdn_front(ctx, s, w.cb, qkv, ly.conv_w, w.a, w.b, ly.a_log, ly.dt_bias, T, c.gdn_k_heads, c.gdn_v_heads,
                      c.gdn_head_dim, c.gdn_conv_kernel, 1e-6f, cc->conv[i], w.gq, w.gk, w.gv, w.beta, w.gg, nullptr));
       if (exact)  // token by token, the decode path's arithmetic
@@ -926,9 +955,9 @@ int prefill_wide(orn_model* m, orn_cache* cc, int T, bool exact, bf16_t* normed_
         CK(k_gated_delta_chunked(ctx, s, w.gq, w.gk, w.gv, w.gg, w.beta, nullptr, cc->ring[i], kRing, cc->cur, T, c.gdn_k_heads,
                                  c.gdn_v_heads, w.gy, w.gdn_scratch));
       CK(k_rms_norm_gated(ctx, s, w.gy, ly.gdn_norm, w.z, T * c.gdn_v_heads, c.gdn_head_dim, c.rms_eps, w.gated));
-      CK(wide_mm(m, ly.out_proj, w.gated, T, w.r));
+      CK(wide_mm(m, ly.out_proj, w.gated, T, w.r, s));
     } else {
-      CK(wide_mm_multi(m, {{ly.q_proj, w.qg}, {ly.k_proj, w.ak}, {ly.v_proj, w.av}}, w.n, T));
+      CK(wide_mm_multi(m, {{ly.q_proj, w.qg}, {ly.k_proj, w.ak}, {ly.v_proj, w.av}}, w.n, T, s));
       if (k_attn_front_ok(hd, c.rope_dims)) {
         CK(k_attn_front(ctx, s, w.qg, w.ak, w.av, ly.q_norm, ly.k_norm, T, 0, Hq, Hkv, c.max_ctx, c.rope_dims, m->lnb, c.rms_eps, cc->pos,
                         w.aq, cc->kc[i], cc->vc[i]));
@@ -946,7 +975,7 @@ int prefill_wide(orn_model* m, orn_cache* cc, int T, bool exact, bf16_t* normed_
       else
         CK(k_flash_prefill(ctx, s, w.aq, cc->kc[i], cc->vc[i], T, Hq, Hkv, hd, c.max_ctx, cc->pos, 1.0f / sqrtf((float)hd), w.att));
       CK(k_gate_rows(ctx, s, w.qg, w.att, T * Hq, w.agated));
-      CK(wide_mm(m, ly.o_proj, w.agated, T, w.r));
+      CK(wide_mm(m, ly.o_proj, w.agated, T, w.r, s));
     }
     CK(k_add_rms_norm(ctx, s, w.x, w.r, ly.post_ln, T, H, c.rms_eps, w.h, w.n2));
     const bool last = i + 1 == c.n_layers;
