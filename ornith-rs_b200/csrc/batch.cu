@@ -537,12 +537,12 @@ __global__ void mtp_advance_kernel(int* mtp_pos, const int* keep, int B, int bas
 // ---- fewer rows than the tensor cores are used for ----------------------------------------------
 // The single-sequence engine's fused kernels (fused.cu), four rows at a time where they take at most
 // four, all sequences at once where they are per sequence: the same bits as the one-kernel-per-op
-// path, a sixth of its launches, every weight read by the kernels built for few rows, bit for bit the same.
-// Both sides at 700 cached positions, one kernel per op -> fused, ms per window: 1 row 7.0 -> 2.0, 2 rows 8.5 -> 2.5,
-// 4 rows 11.4 -> 3.9, 5 rows 13.0 -> 5.9, 8 rows 16.4 -> 7.3, 12 rows 21.4 -> 10.8, 14 rows 23.7 -> 13.0, 15 rows
-// 25.1 -> 14.3 (a group of four rows costs about 3.4); 16 rows take 7.8 on the tensor cores, whose products are not
-// row-invariant.  Drafts: 1 row 423 -> 237 us, 4 rows 659 -> 373, 7 rows 971 -> 654.
-constexpr int kSmallRows = 15;
+// path with its row-invariant products of many rows (rows.cu).  A group of four rows costs about 3.4 ms, every
+// further row of the other path little.  Fused / one kernel per op, ms per window at 700 cached positions: 6 rows
+// 6.3 / 6.7, 8 rows 7.2 / 7.5, 10 rows 9.6 / 8.5, 12 rows 10.7 / 9.0, 14 rows 12.9 / 9.9 (at 3500 positions 8 rows 8.3 /
+// 8.1, 14 rows 14.8 / 11.2); 16 rows take 7.0 on the tensor cores, whose products are not row-invariant.  Drafts, us:
+// 5 rows 556 / 653, 7 rows 648 / 689, 10 rows 907 / 823.
+constexpr int kSmallRows = 8;
 // The re-encode (one row per sequence, keys and values only) has little to read per launch, and every CTA of the
 // fused kernels rebuilds the norms of both of its inputs: up to this many sequences.  A commit, fused / one kernel
 // per op: one sequence 70 / 80 us, two 79 / 86, four 98 / 90, seven 138 / 112, fifteen 230 / 166.

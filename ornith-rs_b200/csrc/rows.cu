@@ -183,9 +183,10 @@ int launch_r(orn_ctx* ctx, cudaStream_t s, RowsParams& P, int E) {
 template <int KIND, int MAX>
 int launch_max(orn_ctx* ctx, cudaStream_t s, RowsParams& P, int E, int features) {
   if (E > 1) return launch_r<KIND, 2>(ctx, s, P, E);
-  // a narrow matrix: two rows a CTA, so that the launch reaches more SMs
-  if ((features + 31) / 32 * ((P.rows + MAX - 1) / MAX) < ctx->sm_count) return launch_r<KIND, 2>(ctx, s, P, E);
-  return launch_r<KIND, MAX>(ctx, s, P, E);
+  // a narrow matrix: four or two rows a CTA, so that the launch reaches more SMs
+  const int ctas = (features + 31) / 32;
+  if (ctas * ((P.rows + MAX - 1) / MAX) >= ctx->sm_count) return launch_r<KIND, MAX>(ctx, s, P, E);
+  return ctas * ((P.rows + 3) / 4) >= ctx->sm_count ? launch_r<KIND, 4>(ctx, s, P, E) : launch_r<KIND, 2>(ctx, s, P, E);
 }
 
 }  // namespace

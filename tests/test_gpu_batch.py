@@ -320,6 +320,12 @@ def test_few_rows_take_the_fused_kernels(pkg, ctx, B, T):
     gm.free()
 
 
+@pytest.mark.parametrize("B,T", [(4, 2), (9, 1), (3, 3), (12, 1)])
+def test_few_rows_on_either_side_of_the_fused_kernels_limit(pkg, ctx, B, T):
+    """Eight rows take the fused kernels, nine to fifteen one kernel per op: the same bits either way."""
+    test_few_rows_take_the_fused_kernels(pkg, ctx, B, T)
+
+
 def cycles_equal(pkg, ctx, gm, B, cap, exact, n, keep_of):
     """n cycles (draft, window [primary, draft], commit of keep_of(cycle, b) rows) of B sequences against the
     single-sequence engine's op-level cycle, sequence by sequence: drafts, targets and hidden rows bit for bit."""
