@@ -322,7 +322,7 @@ struct orn_batch {
   bf16_t *qg, *aq, *ak, *av, *att, *agated, *logits;
   float *greedy_scratch, *part;
   int part_chunks = 0;
-  // fewer rows than the tensor cores are used for: the fused decode kernels' scratch (kSmallRows rows)
+  // fewer rows than the tensor cores are used for: the fused decode kernels' scratch (kSmallDraft rows)
   bool small_ok = false;
   bf16_t *sgates = nullptr, *sscores = nullptr, *seact = nullptr, *ssact = nullptr, *sgs = nullptr;
   uint32_t* sinds = nullptr;
@@ -540,17 +540,18 @@ __global__ void mtp_advance_kernel(int* mtp_pos, const int* keep, int B, int bas
 // path with its row-invariant products of many rows (rows.cu).  A group of four rows costs about 3.4 ms, every
 // further row of the other path little.  Fused / one kernel per op, ms per window at 700 cached positions: 6 rows
 // 6.3 / 6.7, 8 rows 7.2 / 7.5, 10 rows 9.6 / 8.5, 12 rows 10.7 / 9.0, 14 rows 12.9 / 9.9 (at 3500 positions 8 rows 8.3 /
-// 8.1, 14 rows 14.8 / 11.2); 16 rows take 7.0 on the tensor cores, whose products are not row-invariant.  Drafts, us:
-// 5 rows 556 / 653, 7 rows 648 / 689, 10 rows 907 / 823.
-constexpr int kSmallRows = 8;
+// 8.1, 14 rows 14.8 / 11.2); 16 rows take 7.0 on the tensor cores, whose products are not row-invariant.  A draft is one
+// layer and the head, where the fused kernels stay ahead: 5 rows 556 / 653 us, 7 rows 648 / 689; from there on the two
+// are level, and a cycle of 12 sequences at 1500 positions takes 9.80 ms with fused drafts, 9.95 without.
+constexpr int kSmallRows = 8, kSmallDraft = 15;
 // The re-encode (one row per sequence, keys and values only) has little to read per launch, and every CTA of the
 // fused kernels rebuilds the norms of both of its inputs: up to this many sequences.  A commit, fused / one kernel
 // per op: one sequence 70 / 80 us, two 79 / 86, four 98 / 90, seven 138 / 112, fifteen 230 / 166.
 constexpr int kSmallEncode = 2;
 
 // the fused kernels serve every part of the model at these rows, on this GPU alone
-bool small_path(const orn_batch* bt, int rows, int world) {
-  return bt->small_ok && rows <= kSmallRows && world == 1 && !bt->split_attn && orn_use_fused(bt->m) &&
+bool small_path(const orn_batch* bt, int rows, int limit, int world) {
+  return bt->small_ok && rows <= limit && world == 1 && !bt->split_attn && orn_use_fused(bt->m) &&
          bt->B * std::max(bt->m->cfg.gdn_v_heads, 1) <= kGdnMaxHeads && bt->B * bt->m->cfg.n_heads <= kAttnMaxHeads;
 }
 // jobs over `rows` rows of one prologue, at most four rows per launch
@@ -828,7 +829,7 @@ int32_t orn_batch_create(orn_model* m, int32_t B, int32_t T_max, int32_t cap, in
     A(&bt->mtp_pos, (size_t)B);
   }
   {
-    const size_t n = kSmallRows, E = c.n_experts, k = c.top_k;
+    const size_t n = kSmallDraft, E = c.n_experts, k = c.top_k;
     A(&bt->sgates, n * E); A(&bt->sinds, n * k); A(&bt->sscores, n * k); A(&bt->seact, n * k * c.expert_inter);
     A(&bt->ssact, n * c.shared_inter); A(&bt->sgs, n);
     bt->small_ok = H <= 2048 && c.head_dim == 256 && c.n_experts <= 512 && k <= 8 && c.expert_inter <= 2048 && c.shared_inter <= 2048;
@@ -941,7 +942,7 @@ int32_t orn_batch_forward(orn_batch* bt, orn_ep* ep, const uint32_t* host_ids, i
   for (int b = 0; b < B; ++b) max_pos = std::max(max_pos, bt->h_pos[b]);
   int chunk, nchunks;
   split_shape(bt, max_pos + T, &chunk, &nchunks);
-  const bool small = exact && small_path(bt, R, world);
+  const bool small = exact && small_path(bt, R, kSmallRows, world);
   auto body = [&]() { return small ? small_body(bt, T, max_pos + T) : batch_body(bt, group, T, chunk, nchunks); };
   // the previous step's targets have been read (its download synchronised) before ids_h is rewritten
   ORN_CHECK_CUDA(ctx, cudaStreamSynchronize(s));
@@ -1021,7 +1022,7 @@ int32_t orn_batch_commit(orn_batch* bt, const int32_t* host_keep) {
       const bool exact = bt->exact || bt->B < 16;
       int max_pos = 0;
       for (int b = 0; b < bt->B; ++b) max_pos = std::max(max_pos, bt->h_mtp_pos[b]);
-      if (exact && bt->B <= kSmallEncode && small_path(bt, bt->B, bt->shard_world > 1 ? bt->shard_world : 1)) {
+      if (exact && bt->B <= kSmallEncode && small_path(bt, bt->B, kSmallEncode, bt->shard_world > 1 ? bt->shard_world : 1)) {
         CK(small_mtp(bt, bt->tok1, bt->hid0, max_pos + 1, true));
       } else {
         CK(mtp_join(bt, bt->tok1, bt->hid0));
@@ -1067,7 +1068,7 @@ int32_t orn_batch_mtp_draft(orn_batch* bt, orn_ep* ep, const uint32_t* host_prim
   int chunk, nchunks;
   split_shape(bt, max_pos + 1, &chunk, &nchunks);
   CK(orn_upload(ctx, bt->prim, host_primary, sizeof(uint32_t) * (size_t)B));
-  if (exact && small_path(bt, B, world)) {
+  if (exact && small_path(bt, B, kSmallDraft, world)) {
     CK(small_mtp(bt, bt->prim, bt->hrow, max_pos + 1, false));
   } else {
     CK(mtp_join(bt, bt->prim, bt->hrow));

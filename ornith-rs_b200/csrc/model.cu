@@ -816,6 +816,7 @@ constexpr int kWideMinRows = 64;    // measured: below about 60 rows the 4-row m
 // windows spread long caches, so behind many cached positions the windows stay.
 constexpr int kRowsMin = 13;
 constexpr int kRowsMaxKeys = 1024;
+constexpr int kRowsMaxK = 6144;  // longest row the grouped product takes in every format
 constexpr int kWideMaxRows = 8192;  // widest chunk of the wide path (the reference's default chunk is 2048, generate.rs:25)
 
 int wide_reserve(orn_model* m, int rows) {
@@ -1004,7 +1005,8 @@ int prefill(orn_model* m, orn_cache* cc, const uint32_t* prompt, int n, int pref
     int chunk = std::min(step, n - done - keep_last);
     int off = 0;
     const bool wide = chunk >= kWideMinRows;
-    if ((wide || (chunk >= kRowsMin && cc->h_pos + chunk <= kRowsMaxKeys)) && use_wide_prefill() && use_fused_env()) {
+    const bool rows = chunk >= kRowsMin && cc->h_pos + chunk <= kRowsMaxKeys && m->cfg.hidden <= kRowsMaxK && m->cfg.expert_inter <= kRowsMaxK;
+    if ((wide || rows) && use_wide_prefill() && use_fused_env()) {
       // a chunk wide enough for the tensor cores (the reference's tile path, kquant.rs:783-812), or a short one
       // through the same launches with row-invariant products
       chunk = std::min(chunk, kWideMaxRows);

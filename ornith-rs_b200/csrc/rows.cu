@@ -192,7 +192,7 @@ int launch_max(orn_ctx* ctx, cudaStream_t s, RowsParams& P, int E, int features)
 }  // namespace
 
 bool f_rows_ok(const orn_linear* L) {
-  return L->kind != ORN_A4 && L->K % 256 == 0 && L->E <= 65535 && (size_t)(L->E > 1 ? 8 : 4) * kRowWarps * L->rec <= kRowSmem;
+  return L->kind != ORN_A4 && L->K % 256 == 0 && L->E <= 65535 && L->O <= 1000000 /* tiles of 16 features in a grid's y */ && (size_t)(L->E > 1 ? 8 : 4) * kRowWarps * L->rec <= kRowSmem;
 }
 
 // Up to four matrices of one format and row length over the same rows, or (seg given) one matrix over rows sorted by

@@ -322,7 +322,7 @@ def test_few_rows_take_the_fused_kernels(pkg, ctx, B, T):
 
 @pytest.mark.parametrize("B,T", [(4, 2), (9, 1), (3, 3), (12, 1)])
 def test_few_rows_on_either_side_of_the_fused_kernels_limit(pkg, ctx, B, T):
-    """Eight rows take the fused kernels, nine to fifteen one kernel per op: the same bits either way."""
+    """Windows of eight rows take the fused kernels, of nine to fifteen one kernel per op: the same bits either way."""
     test_few_rows_take_the_fused_kernels(pkg, ctx, B, T)
 
 
