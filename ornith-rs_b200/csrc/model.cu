@@ -807,8 +807,8 @@ int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear
   }
   return ORN_OK;
 }
-constexpr int kWideMinRows = 64;    // measured: below about 60 rows the 4-row mat-vec windows are faster (the
-                                    // reference's own crossover, kquant.rs MM_ROW_LIMIT, is 16 on its hardware)
+constexpr int kWideMinRows = 64;    // from here on prompt rows come from the tensor cores (the reference's own
+                                    // crossover, kquant.rs MM_ROW_LIMIT, is 16 on its hardware)
 // Shorter chunks have the bits of the four-row windows whatever way they go.  From 13 rows on all of them go through the
 // wide path's launches with row-invariant products (rows.cu), which read a layer's weights once, an expert's for all its
 // rows.  Windows / one piece, ms for the whole model: 8 rows 6.3 / 8.0, 12 rows 9.4 / 9.3, 16 rows 12.5 / 10.6, 24 rows

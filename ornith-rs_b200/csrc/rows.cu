@@ -9,9 +9,10 @@
 //     widened once for all of those rows (1.5 instructions; the four-row windows do it for every four rows);
 //   * activations come as bfloat16 through L1 and are widened once per unit for R features;
 //   * a warp owns its R features: their records lie behind one another and come by cp.async into the warp's own piece
-//     of shared memory.  Warps never meet; two or three CTAs of four warps on an SM cover each other's copies.
+//     of shared memory.  Warps never meet; two to four CTAs of four warps on an SM cover each other's copies.
 // FMA work of a unit of 16 weights, 8 rows x 8 features: 512 packed multiply-adds of 1024 cycles in about 1500.
-// Prompt windows of the reply with 51 prompt tokens: see model.cu where the rule is.
+// 50 rows, 2048 -> 12288 affine-8: 110 us, half of that bound (255 registers leave two warps per scheduler).  What it
+// replaced there read the weights once per four rows, 13 launches of about 17 us.
 #include <algorithm>
 
 #include "fused.h"
@@ -196,8 +197,10 @@ bool f_rows_ok(const orn_linear* L) {
 }
 
 // Up to four matrices of one format and row length over the same rows, or (seg given) one matrix over rows sorted by
-// expert.  Dense rows go eight at a time (a unit of Q4_K is 32 weights: four), every group in CTAs of its own; an
-// expert's rows, one or two as a rule, four at a time in the CTA that holds its features.
+// expert.  Dense rows go eight at a time (a unit of Q4_K is 32 weights: four), two groups a CTA where there are many; an
+// expert's rows, one or two as a rule, two at a time in the CTA that holds its features, which leaves registers for twice
+// the warps (400 rows over 256 Q4_K experts 87 us four at a time, 76 two; two tiles a warp only where a row is one step
+// long: Q6_K of 512 weights 98 -> 95 us, Q4_K of 2048 76 -> 80).
 int f_rows(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, bf16_t* const* ys, int n, const bf16_t* xs, int rows, const int* seg,
            const uint32_t* row_map) {
   if (rows < 1) return ORN_OK;
