@@ -371,19 +371,16 @@ int batch_mm_multi(orn_batch* bt, const orn_linear* const* Ls, bf16_t* const* ys
   // the first group of matrices on the main stream, the others beside it on the side stream (a small
   // projection of another format next to the big one is a launch of a few CTAs that would otherwise wait
   // its turn)
-  bool forked = false;
+  SideWork side = orn_side_work(ctx, ctx->stream, n > 1);
   int i = 0;
   while (i < n) {
     int j = i + 1;
     while (j < n && j - i < 4 && Ls[j]->kind == Ls[i]->kind && Ls[j]->K == Ls[i]->K && Ls[i]->K % 64 == 0) ++j;
     cudaStream_t st = ctx->stream;
-    if (i > 0 && Ls[i]->K % 64 == 0 && orn_side_stream(ctx)) {
-      if (!forked) {
-        ORN_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream));
-        ORN_CHECK_CUDA(ctx, cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-        forked = true;
-      }
-      st = ctx->side;
+    if (i > 0 && Ls[i]->K % 64 == 0) {
+      if (!side.open()) ORN_CHECK_CUDA(ctx, side.mark());
+      ORN_CHECK_CUDA(ctx, side.start());
+      st = side.stream();
     }
     void* yv[4];
     int ld[4];
@@ -392,10 +389,8 @@ int batch_mm_multi(orn_batch* bt, const orn_linear* const* Ls, bf16_t* const* ys
     else for (int k = i; k < j; ++k) CK(batch_mm(bt, Ls[k], x, R, ys[k]));
     i = j;
   }
-  if (forked) {
-    ORN_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->side));
-    ORN_CHECK_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
-  }
+  ORN_CHECK_CUDA(ctx, side.done());
+  ORN_CHECK_CUDA(ctx, side.join());
   return ORN_OK;
 }
 

@@ -768,8 +768,8 @@ int wide_mm(orn_model* m, const orn_linear* L, const bf16_t* x, int T, bf16_t* y
 int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear*, bf16_t*>> jobs, const bf16_t* x, int T, cudaStream_t st,
                   bool fork = false) {
   orn_ctx* ctx = m->ctx;
-  bool forked = false;
-  if (fork && (fork = orn_side_stream(ctx))) ORN_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev_fork, st));
+  SideWork side = orn_side_work(ctx, st, fork);
+  ORN_CHECK_CUDA(ctx, side.mark());
   const auto* j = jobs.begin();
   const int n = (int)jobs.size();
   for (int i = 0; i < n;) {
@@ -785,12 +785,9 @@ int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear
       features += j[i + k].first->O;
       pl[k] = j[i + k].first; py[k] = j[i + k].second; ld[k] = pl[k]->O;
     }
-    const bool beside = fork && i > 0 && features <= 256;
-    if (beside && !forked) {
-      ORN_CHECK_CUDA(ctx, cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-      forked = true;
-    }
-    const cudaStream_t on = beside ? ctx->side : st;
+    const bool beside = i > 0 && features <= 256;
+    if (beside) ORN_CHECK_CUDA(ctx, side.start());
+    const cudaStream_t on = beside ? side.stream() : st;
     if (m->wide.exact && f_rows_ok(pl[0])) {
       bf16_t* yb[4];
       for (int q = 0; q < k; ++q) yb[q] = static_cast<bf16_t*>(py[q]);
@@ -801,10 +798,8 @@ int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear
       CK(f_qgemm_multi(ctx, on, pl, py, ld, k, x, T));
     i += k;
   }
-  if (forked) {
-    ORN_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->side));
-    ORN_CHECK_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_join, 0));
-  }
+  ORN_CHECK_CUDA(ctx, side.done());
+  ORN_CHECK_CUDA(ctx, side.join());
   return ORN_OK;
 }
 constexpr int kWideMinRows = 64;    // from here on prompt rows come from the tensor cores (the reference's own
@@ -882,16 +877,14 @@ int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, const M
   // The shared expert depends on x only: its three launches run on the side stream beside the sort of the routes, whose
   // kernels leave the SMs idle, and are joined before the combine (a prompt of 97 rows 1647 -> 1509 us, the gates of the
   // recurrent layers on the side stream among it; forked before the router, whose product they then hold up: 1534).
-  const bool side = orn_side_stream(ctx);
-  const cudaStream_t ss = side ? ctx->side : s;
-  if (side) {
-    ORN_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev_fork, s));
-    ORN_CHECK_CUDA(ctx, cudaStreamWaitEvent(ss, ctx->ev_fork, 0));
-  }
+  SideWork side = orn_side_work(ctx, s);
+  const cudaStream_t ss = side.stream();
+  ORN_CHECK_CUDA(ctx, side.mark());
+  ORN_CHECK_CUDA(ctx, side.start());
   CK(wide_mm_multi(m, {{moe.sh_gate, w.sg}, {moe.sh_up, w.su}}, x, T, ss));
   CK(k_swiglu(ctx, ss, w.sg, w.su, T * SI, w.sact));
   CK(wide_mm(m, moe.sh_down, w.sact, T, w.sy, ss));
-  if (side) ORN_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev_join, ss));
+  ORN_CHECK_CUDA(ctx, side.done());
   CK(f_route_sort(ctx, s, w.inds, rows, E, w.seg, w.seg + E + 1, w.perm));
   CK(f_gather_rows(ctx, s, x, w.lhs, w.perm, rows, H, w.xs));
   if (w.exact) {
@@ -916,7 +909,7 @@ int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, const M
     QGemmGroup back{w.seg, w.perm, 0};
     CK(f_qgemm(ctx, s, moe.sw_down, w.eact, rows, w.ey, H, &back));  // rows back in (token, slot) order
   }
-  if (side) ORN_CHECK_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_join, 0));
+  ORN_CHECK_CUDA(ctx, side.join());
   if (k_moe_combine_norm_ok(c.top_k, H))
     return k_moe_combine_norm(ctx, s, w.scores, w.ey, w.gs, w.sy, T, c.top_k, H, c.norm_topk_prob, next.h, next.w, next.eps, next.sum, next.out);
   CK(k_moe_combine(ctx, s, w.scores, w.ey, w.gs, w.sy, T, c.top_k, H, c.norm_topk_prob, w.mo));

@@ -13,6 +13,7 @@
 
 #include "../../include/ornith_cuda.h"
 #include "orn_common.cuh"
+#include "side.h"
 
 // Words of a context's dev_err: [0] the error flag of bounded waits, [32] the wait probe's answer, from
 // kArrivalsAt on the arrival counters of the gated-delta kernel's heads
@@ -128,6 +129,11 @@ static inline LinDev lin_dev(const orn_linear* l) {
 // when they cannot be had, inside a capture that began before they existed, with per-kernel timing on, or
 // when ORN_NO_SIDE_STREAM=1 asks for one stream
 bool orn_side_stream(orn_ctx* ctx);
+// work beside `main` on it; two: false where the caller wants one stream all the same
+inline SideWork orn_side_work(orn_ctx* ctx, cudaStream_t main, bool two = true) {
+  two = two && orn_side_stream(ctx);  // which makes the stream and its events on first use
+  return SideWork(main, two ? ctx->side : nullptr, ctx->ev_fork, ctx->ev_join);
+}
 
 static inline int orn_launch_check(orn_ctx* ctx, const char* what) {
   cudaError_t e = cudaGetLastError();
