@@ -220,7 +220,8 @@ __global__ void __launch_bounds__(kAttWarps * 32) battn_partial_kernel(const bf1
     }
     uint32_t pa[4] = {pack_bf16x2(pr[0][0], pr[0][1]), pack_bf16x2(pr[0][2], pr[0][3]), pack_bf16x2(pr[1][0], pr[1][1]),
                       pack_bf16x2(pr[1][2], pr[1][3])};
-    issue(vc, i + 1);  // where the keys were: every lane has read them (the shuffles and the vote above)
+    __syncwarp();  // every lane has read the keys (shuffles and votes order no memory accesses)
+    issue(vc, i + 1);  // where the keys were
     cp_async_wait<2>();
     __syncwarp();
     const uint32_t vs = next_place();
