@@ -106,6 +106,9 @@ int32_t orn_debug_wait_probe(orn_ctx* ctx, uint32_t rounds);
  * a few seconds for the peer's, gives up, and the following orn_sync returns ORN_ERR_TIMEOUT once.
  * One GPU, one process, no peer. */
 int32_t orn_debug_ep_wait_probe(orn_ctx* ctx);
+/* Test hook for what the library does without memory: the nth device allocation from here on (1 = the next one)
+ * fails with ORN_ERR_ALLOC, on the host, as if the device were full; 0 takes the request back. */
+int32_t orn_debug_fail_alloc(orn_ctx* ctx, int32_t nth);
 
 /* device-side stopwatch on the context's stream (CUDA events; the reference's
  * ORNITH_PROF GPUStart/GPUEnd sums, src/metal/mod.rs:197-284) */

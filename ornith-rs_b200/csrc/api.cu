@@ -220,6 +220,12 @@ int32_t orn_debug_wait_probe(orn_ctx* ctx, uint32_t rounds) {
   return f_wait_probe(ctx, ctx->stream, rounds, ctx->dev_err + 32);
 }
 
+int32_t orn_debug_fail_alloc(orn_ctx* ctx, int32_t nth) {
+  if (!ctx || nth < 0) return ORN_ERR_ARG;
+  ctx->fail_alloc = nth;
+  return ORN_OK;
+}
+
 int32_t orn_timer_start(orn_ctx* ctx) {
   if (!ctx) return ORN_ERR_ARG;
   if (!ctx->t0) {
@@ -243,6 +249,7 @@ const char* orn_last_error(orn_ctx* ctx) { return ctx ? ctx->err.c_str() : "null
 int32_t orn_alloc(orn_ctx* ctx, size_t nbytes, void** dev_out) {
   if (!ctx || !dev_out) return ORN_ERR_ARG;
   *dev_out = nullptr;
+  if (ctx->fail_alloc > 0 && --ctx->fail_alloc == 0) ORN_FAIL(ctx, ORN_ERR_ALLOC, "alloc: failed on request");
   cudaSetDevice(ctx->device);
   cudaError_t e = cudaMalloc(dev_out, nbytes ? nbytes : 16);
   if (e != cudaSuccess) {

@@ -999,11 +999,16 @@ int prefill(orn_model* m, orn_cache* cc, const uint32_t* prompt, int n, int pref
     int off = 0;
     const bool wide = chunk >= kWideMinRows;
     const bool rows = chunk >= kRowsMin && cc->h_pos + chunk <= kRowsMaxKeys && m->cfg.hidden <= kRowsMaxK && m->cfg.expert_inter <= kRowsMaxK;
-    if ((wide || rows) && use_wide_prefill() && use_fused_env()) {
+    bool one_piece = (wide || rows) && use_wide_prefill() && use_fused_env();
+    if (one_piece) {
+      chunk = std::min(chunk, kWideMaxRows);
+      const int rc = wide_reserve(m, std::max(chunk, kWideMinRows));
+      one_piece = wide || rc != ORN_ERR_ALLOC;  // a short chunk has the windows where there is no memory for its workspace
+      if (one_piece) CK(rc);
+    }
+    if (one_piece) {
       // a chunk wide enough for the tensor cores (the reference's tile path, kquant.rs:783-812), or a short one
       // through the same launches with row-invariant products
-      chunk = std::min(chunk, kWideMaxRows);
-      CK(wide_reserve(m, std::max(chunk, kWideMinRows)));
       ORN_CHECK_CUDA(m->ctx, cudaMemcpyAsync(m->wide.ids, prompt + done, sizeof(uint32_t) * (size_t)chunk,
                                              cudaMemcpyHostToDevice, m->ctx->stream));
       CK(prefill_wide(m, cc, chunk, !wide || wide_exact(), normed_out ? normed_out + (size_t)done * m->cfg.hidden : nullptr));

@@ -43,6 +43,7 @@ struct orn_ctx {
   // group partials and arrival counters of the fused attention's long-context form (fused.cu)
   float* attn_partial = nullptr;
   int* attn_arrivals = nullptr;
+  int fail_alloc = 0;    // orn_debug_fail_alloc: allocations until the one that fails (0: none does)
   int* err_h = nullptr;  // pinned landing word of orn_sync's copy of *dev_err
   // One device buffer kept for calls that need scratch and end with a synchronisation (orn_scratch_take):
   // a call takes it out, so that two threads never share it, and gives it back; ctx_destroy frees it.

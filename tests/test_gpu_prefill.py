@@ -64,6 +64,37 @@ def test_short_chunks_have_the_bits_of_the_four_row_windows(pkg, ctx, n, step):
     m.free()
 
 
+@pytest.mark.parametrize("nth", [1, 41])
+def test_a_short_chunk_needs_no_workspace(pkg, ctx, nth):
+    """The first or the last allocation of the one-piece path's workspace fails: a chunk of 13 to 63 rows goes in windows of
+    four rows, with the same bits; a chunk of 64 rows says what is missing, and both go on once there is memory."""
+    m = pkg.TextModel(ctx, pkg.qwen35_config(max_ctx=256, n_layers=1))
+    m.init_random(9)
+    ids = np.random.default_rng(nth).integers(0, m.cfg.vocab, 64).astype(np.uint32)
+    c, lib = m.make_cache(), ctx._lib
+    want = m.prefill(c, ids[:50], prefill_step=4, want_hidden=True).numpy()
+    out = ctx.empty((64, m.cfg.hidden), np.uint16)
+
+    def prefill(n, fail):
+        c.reset()
+        assert lib.orn_debug_fail_alloc(ctx.h, fail) == 0
+        l0 = ctx.launches()
+        rc = lib.orn_prefill(m.h, c.h, ids.ctypes.data, n, 2048, out.ptr)
+        assert lib.orn_debug_fail_alloc(ctx.h, 0) == 0
+        return rc, ctx.launches() - l0
+
+    rc, in_windows = prefill(50, nth)
+    assert rc == 0, lib.orn_last_error(ctx.h)
+    assert np.array_equal(out.numpy()[:50], want)
+    assert prefill(64, nth)[0] != 0 and c.offset == 0
+    rc, in_one = prefill(50, 0)
+    assert rc == 0 and np.array_equal(out.numpy()[:50], want)
+    assert in_one < in_windows
+    assert prefill(64, 0)[0] == 0 and c.offset == 64
+    c.free()
+    m.free()
+
+
 def test_wide_prefill_and_generation_on_the_tiny_model(pkg, ctx):
     cfg = hp.tiny_config(pkg.Config, max_ctx=160)
     W = hp.tiny_model_weights(cfg, seed=5)
