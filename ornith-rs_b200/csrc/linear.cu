@@ -377,13 +377,19 @@ int dispatch_m(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16_t*
 }  // namespace
 
 namespace {
-// the product of many rows (rows.cu) takes this matrix and these rows
-bool rows_path(const orn_linear* L, const bf16_t* xs) { return f_rows_ok(L) && (reinterpret_cast<uintptr_t>(xs) & 15) == 0; }
+// Activations are read 16 bytes at a time, by the mat-vec of Q6_K 8: rows that start elsewhere are refused here.
+int aligned_rows(orn_ctx* ctx, const bf16_t* x, int bytes) {
+  if (reinterpret_cast<uintptr_t>(x) % bytes != 0) ORN_FAIL(ctx, ORN_ERR_ARG, "gemv: rows must start on a multiple of " + std::to_string(bytes) + " bytes");
+  return ORN_OK;
+}
+int gemv_align(const orn_linear* L) { return L->kind == ORN_Q6K ? 8 : 16; }
 }  // namespace
 
 int k_gemv(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16_t* x, int M, void* y,
            int out_f32) {
-  if (M > 4 && !out_f32 && rows_path(L, x)) {
+  int rc = aligned_rows(ctx, x, gemv_align(L));
+  if (rc != ORN_OK) return rc;
+  if (M > 4 && !out_f32 && f_rows_ok(L) && reinterpret_cast<uintptr_t>(x) % 16 == 0) {
     bf16_t* yb = static_cast<bf16_t*>(y);
     return f_rows(ctx, st, &L, &yb, 1, x, M);
   }
@@ -393,7 +399,6 @@ int k_gemv(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16_t* x, 
     const bf16_t* xs = x + (int64_t)m0 * L->K;
     void* ys = out_f32 ? (void*)((float*)y + (int64_t)m0 * L->O)
                        : (void*)((bf16_t*)y + (int64_t)m0 * L->O);
-    int rc;
     switch (L->kind) {
       case ORN_Q4K: rc = dispatch_m<ORN_Q4K>(ctx, st, L, xs, mm, ys, out_f32); break;
       case ORN_Q6K: rc = dispatch_m<ORN_Q6K>(ctx, st, L, xs, mm, ys, out_f32); break;
@@ -409,6 +414,8 @@ int k_gemv(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16_t* x, 
 int k_gather_gemv(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16_t* x,
                   const uint32_t* lhs, const uint32_t* rhs, int rows, bf16_t* y) {
   if (rows <= 0) return ORN_OK;
+  const int rc = aligned_rows(ctx, x, gemv_align(L));
+  if (rc != ORN_OK) return rc;
   switch (L->kind) {
     case ORN_Q4K: return dispatch_gemv<ORN_Q4K, 1>(ctx, st, L, x, y, 0, lhs, rhs, rows);
     case ORN_Q6K: return dispatch_gemv<ORN_Q6K, 1>(ctx, st, L, x, y, 0, lhs, rhs, rows);
@@ -549,7 +556,9 @@ int launch_grouped(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf1
 int k_grouped_gemv(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16_t* xs, const int* seg, bf16_t* y,
                    const uint32_t* row_map, int max_rows) {
   if (L->E > 65535) ORN_FAIL(ctx, ORN_ERR_ARG, "grouped gemv: more than 65535 experts");
-  if (rows_path(L, xs)) return f_rows(ctx, st, &L, &y, 1, xs, max_rows, seg, row_map);
+  const int rc = aligned_rows(ctx, xs, 16);
+  if (rc != ORN_OK) return rc;
+  if (f_rows_ok(L)) return f_rows(ctx, st, &L, &y, 1, xs, max_rows, seg, row_map);
   switch (L->kind) {
     case ORN_Q4K: return launch_grouped<ORN_Q4K>(ctx, st, L, xs, seg, y, row_map, max_rows);
     case ORN_Q6K: return launch_grouped<ORN_Q6K>(ctx, st, L, xs, seg, y, row_map, max_rows);
@@ -567,7 +576,9 @@ int k_grouped_gemv2(orn_ctx* ctx, cudaStream_t st, const orn_linear* L1, bf16_t*
     int rc = k_grouped_gemv(ctx, st, L1, xs, seg, y1, nullptr, max_rows);
     return rc != ORN_OK ? rc : k_grouped_gemv(ctx, st, L2, xs, seg, y2, nullptr, max_rows);
   }
-  if (rows_path(L1, xs)) {
+  const int rc = aligned_rows(ctx, xs, 16);
+  if (rc != ORN_OK) return rc;
+  if (f_rows_ok(L1)) {
     const orn_linear* Ls[2] = {L1, L2};
     bf16_t* ys[2] = {y1, y2};
     return f_rows(ctx, st, Ls, ys, 2, xs, max_rows, seg);

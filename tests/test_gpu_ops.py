@@ -490,3 +490,37 @@ def test_gemv_of_many_rows_has_the_bits_of_the_one_row_kernel(pkg, ctx, kind, M,
     for m in range(M):
         assert np.array_equal(got[m], L.matmul(ctx.upload(x[m:m + 1]), 1).numpy()[0]), m
     L.free()
+
+
+@pytest.mark.parametrize("kind", [orc.Q4K, orc.Q6K, orc.A8, orc.BF16, orc.A4])
+def test_gemv_of_rows_that_start_anywhere(pkg, ctx, kind):
+    """Rows off the 16 bytes that the kernels read at a time are refused on the host; those of Q6_K, read 8 bytes at a
+    time by the mat-vec, have the bits of aligned ones, whatever their number (the product of many rows leaves them to
+    groups of four)."""
+    O, K, M = 33, 512, 9
+    L = pkg.Linear.random(ctx, kind, 1, O, K, 3)
+    x = hp.f32_to_bf16(np.random.default_rng(kind).standard_normal((M, K)).astype(np.float32))
+    dx = ctx.upload(np.concatenate([np.zeros(4, np.uint16), x.reshape(-1)]))
+    one = ctx.upload(np.zeros(M, np.uint32))
+    y, lib = ctx.empty((M, O), np.uint16), ctx._lib
+    for off in (2, 8):
+        for rows in (1, 4, 5, M):
+            served = kind == orc.Q6K and off == 8
+            assert (lib.orn_gemv(ctx.h, L.h, dx.at(off), rows, y.ptr, 0) == 0) == served, (off, rows)
+            if served:
+                assert np.array_equal(y.numpy()[:rows], L.matmul(ctx.upload(x[:rows]), rows).numpy()), rows
+        assert (lib.orn_gather_gemv(ctx.h, L.h, dx.at(off), one.ptr, one.ptr, M, y.ptr) == 0) == served
+    ctx.sync()
+    L.free()
+
+
+@pytest.mark.parametrize("kind,K", [(orc.A4, 512), (orc.A8, 320), (orc.BF16, 72)])
+def test_gemv_of_many_rows_that_rows_cu_does_not_take(pkg, ctx, kind, K):
+    """Affine 4-bit and row lengths off 256: groups of four rows, against the mat-vec of one row."""
+    M, O = 9, 40
+    L = pkg.Linear.random(ctx, kind, 1, O, K, 3)
+    x = hp.f32_to_bf16(np.random.default_rng(K).standard_normal((M, K)).astype(np.float32))
+    got = L.matmul(ctx.upload(x), M).numpy()
+    for m in range(M):
+        assert np.array_equal(got[m], L.matmul(ctx.upload(x[m:m + 1]), 1).numpy()[0]), m
+    L.free()
