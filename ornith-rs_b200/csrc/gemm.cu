@@ -1177,10 +1177,15 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
   P.seq = 1;
   P.per = (KB + P.splits - 1) / P.splits;
   // Token-tile width.  Few rows: one tile that holds them.  Many rows: the width (at most 128, so that two
-  // accumulators and the weight ring fit tensor memory) that finishes in the fewest MMA cycles over whole
-  // rounds of the SMs.  Routed rows: wide enough for an expert's rows in nearly every case (mean plus three
-  // standard deviations), since every further item of an expert dequantises its weights again, while
-  // columns up to about 96 hide behind the dequantisation.
+  // accumulators and the weight ring fit tensor memory) that finishes first over whole rounds of the SMs.  With two
+  // groups a tile of 96 tokens or less costs what 100 do, a wider one its columns.  With three its weights, converted
+  // once per tile, are nearly all of it: a round of 128 / 112 / 96 / 80 tokens takes 9.5 / 9.2 / 8.8 / 8.6 us at 6621
+  // rows 2048 -> 8192 affine-8 (2048 rows 2048 -> 4096: 48 us at the 128 of that rule, 56 at the 96 of the other).
+  // bfloat16 weights, which nothing converts, have a ring of two units beside 96 tokens or more and of four beside 80:
+  // 2048 rows 2048 -> 4096 take 61.5 / 63.5 / 69.7 / 51.2 us, 513 rows 4096 -> 2048 36.9 / 34.8 / 34.8 / 24.6.  Routed
+  // rows: wide enough for an expert's rows in nearly every case (mean plus three standard deviations), since every
+  // further item of an expert dequantises its weights again, while columns up to about 96 hide behind the
+  // dequantisation.
   auto up16 = [](int v) { return (v + 15) / 16 * 16; };
   if (grp) {
     const double per = grp->bn_hint > 0 ? grp->bn_hint : std::max(1, (rows + L->E - 1) / L->E);
@@ -1189,11 +1194,13 @@ int f_qgemm_multi(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, voi
     P.BN = std::max(16, up16((want + groups - 1) / groups));
   } else if (rows <= 128 || P.splits > 1) {
     P.BN = std::min(128, up16(rows));
+  } else if (direct && rows > kSplitMaxRows) {
+    P.BN = 80;
   } else {
     int64_t best = -1;
     for (int bn = 128; bn >= 80; bn -= 16) {
       const int64_t items = (int64_t)P.f_tiles * ((rows + bn - 1) / bn);
-      const int64_t cost = (items + ctx->sm_count - 1) / ctx->sm_count * std::max(2 * bn, 200);
+      const int64_t cost = (items + ctx->sm_count - 1) / ctx->sm_count * (G == 3 ? bn + 380 : std::max(2 * bn, 200));
       if (best < 0 || cost < best) { best = cost; P.BN = bn; }
     }
   }
