@@ -80,6 +80,21 @@ def main():
     long_ids = rng.integers(0, cfg.vocab, 70).astype(np.uint32)
     out["full_prefill_sha"] = sha(gm.prefill(c, long_ids, prefill_step=2048, want_hidden=True).numpy())
     out["full_after_prefill"] = sha(gm.forward(c, prompt[:3]).numpy())
+    c.reset()
+    out["full_short_sha"] = sha(gm.prefill(c, long_ids[:50], prefill_step=2048, want_hidden=True).numpy())
+    c.reset()
+    again = gm.prefill(c, long_ids, prefill_step=2048, want_hidden=True).numpy()   # nothing of the passes before shows
+    out["full_prefill_again_sha"] = sha(again)
+    # a batch on the tensor cores: eager, captured and replayed
+    bt = pkg.Batch(gm, 9, t_max=2, cap=64)
+    rows = []
+    for i in range(4):
+        ids = rng.integers(0, cfg.vocab, (9, 2)).astype(np.uint32)
+        tg, hid = bt.forward(ids, want_hidden=True)
+        rows += [hid.numpy().copy(), tg.astype(np.uint16)]
+        bt.commit(np.full(9, 1 + i % 2, np.int32))
+    out["full_batch_sha"] = sha(np.concatenate([r.reshape(-1) for r in rows]))
+    bt.free()
     c.free()
     gm.free()
     ctx.close()

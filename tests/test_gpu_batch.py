@@ -297,10 +297,9 @@ def test_re_encode_writes_keys_and_values_only(pkg, ctx, B):
     gm.free()
 
 
-@pytest.mark.parametrize("B,T", [(1, 1), (1, 2), (2, 2), (5, 1), (7, 2), (15, 1)])
-def test_few_rows_take_the_fused_kernels(pkg, ctx, B, T):
-    """Up to 15 rows, in groups of four per launch (1, 2, 4, 5, 14 and 15 rows): the bits of the
-    single-sequence engine, at different depths of the sequences' caches."""
+def windows_equal(pkg, ctx, B, T, fused):
+    """Four windows of B * T rows against the single-sequence engine, bit for bit, at different depths of the sequences'
+    caches; and which kernels they take."""
     cfg = hp.tiny_config(pkg.Config)
     gm = hp.upload_model(pkg, ctx, cfg, hp.tiny_model_weights(cfg, seed=15))
     rng = np.random.default_rng(B)
@@ -312,6 +311,10 @@ def test_few_rows_take_the_fused_kernels(pkg, ctx, B, T):
         tg, hid = bt.forward(w, want_hidden=True)
         got.append((hid.numpy().reshape(B, T, cfg.hidden).copy(), tg.reshape(B, T).copy()))
         bt.commit(k)
+    ctx.ktime_begin()
+    bt.forward(windows[0])
+    names = ctx.ktime_end()
+    assert ("k_gdn" in names, "gated_delta" in names) == (fused, not fused), names
     for b in range(B):
         for i, ((wh, wt), (gh, gt)) in enumerate(zip(run_single(pkg, gm, windows, keeps, b), got)):
             assert np.array_equal(wh.reshape(-1, cfg.hidden), gh[b]), (b, i)
@@ -320,10 +323,16 @@ def test_few_rows_take_the_fused_kernels(pkg, ctx, B, T):
     gm.free()
 
 
-@pytest.mark.parametrize("B,T", [(4, 2), (9, 1), (3, 3), (12, 1)])
-def test_few_rows_on_either_side_of_the_fused_kernels_limit(pkg, ctx, B, T):
-    """Windows of eight rows take the fused kernels, of nine to fifteen one kernel per op: the same bits either way."""
-    test_few_rows_take_the_fused_kernels(pkg, ctx, B, T)
+@pytest.mark.parametrize("B,T", [(1, 1), (1, 2), (2, 2), (5, 1), (4, 2), (8, 1)])
+def test_few_rows_take_the_fused_kernels(pkg, ctx, B, T):
+    """Up to eight rows, in groups of four per launch (1, 2, 4, 5 and 8 rows)."""
+    windows_equal(pkg, ctx, B, T, True)
+
+
+@pytest.mark.parametrize("B,T", [(9, 1), (3, 3), (12, 1), (7, 2), (15, 1), (3, 4), (5, 3)])
+def test_nine_to_fifteen_rows_take_one_kernel_per_op(pkg, ctx, B, T):
+    """The other side of that limit, up to the last row count without tensor cores: the same bits."""
+    windows_equal(pkg, ctx, B, T, False)
 
 
 def cycles_equal(pkg, ctx, gm, B, cap, exact, n, keep_of):
@@ -389,7 +398,7 @@ def test_passes_between_the_products_at_their_edges(pkg, ctx, B, over):
     gm.free()
 
 
-@pytest.mark.parametrize("B,T", [(1, 4), (3, 4), (5, 3)])
+@pytest.mark.parametrize("B,T", [(1, 4), (1, 3), (2, 3), (2, 4)])
 def test_few_rows_in_windows_of_three_and_four(pkg, ctx, B, T):
-    """As above: windows above two rows move the recurrent states in whole lines, several sequences side by side."""
-    test_few_rows_take_the_fused_kernels(pkg, ctx, B, T)
+    """As above: windows above two rows move the recurrent states in whole lines, one sequence and two side by side."""
+    windows_equal(pkg, ctx, B, T, True)

@@ -112,7 +112,7 @@ def test_config2_moe_layer_256_experts_fused(pkg, ctx, T):
 def _run_worker(env_over):
     env = dict(os.environ)
     for k in ("ORN_UNFUSED", "ORN_NO_GRAPH", "ORN_NO_PDL", "ORN_PDL_MASK", "ORN_KTIME", "ORN_WIDE_EXACT",
-              "ORN_NO_WIDE_PREFILL"):
+              "ORN_NO_WIDE_PREFILL", "ORN_NO_SIDE_STREAM"):
         env.pop(k, None)
     env.update(env_over)
     r = subprocess.run([sys.executable, os.path.join(ROOT, "tests", "env_worker.py")], env=env, capture_output=True,
@@ -150,6 +150,16 @@ def test_chunked_prompt_path_is_exact_with_exact_products():
         assert exact[key] == narrow[key], key
     tensor = _run_worker({})
     assert tensor["tiny_prefill_sha"] != narrow["tiny_prefill_sha"]   # really another arithmetic
+
+
+def test_one_stream_gives_the_bits_of_two():
+    """ORN_NO_SIDE_STREAM=1: a prompt on the tensor cores, one in a piece with row-invariant products, the window decoded
+    behind it and a batch (eager, captured, replayed), whose shared expert and narrow projections otherwise run beside
+    the main stream."""
+    two, one = _run_worker({}), _run_worker({"ORN_NO_SIDE_STREAM": "1"})
+    for key in ("tiny_prefill_sha", "tiny_after_prefill", "full_prefill_sha", "full_after_prefill", "full_short_sha", "full_batch_sha"):
+        assert one[key] == two[key], key
+    assert two["full_prefill_again_sha"] == two["full_prefill_sha"]
 
 
 def test_bounded_wait_gives_up_and_the_context_survives(pkg, ctx):

@@ -180,3 +180,42 @@ def test_three_groups_give_the_bits_of_two(pkg, ctx, kind, M, O, K):
         want = L.matmul_wide(ctx.upload(np.ascontiguousarray(x[r:r + n])), n).numpy()
         assert np.array_equal(got[r:r + n], want), r
     L.free()
+
+
+@pytest.mark.parametrize("kind", [orc.A8, orc.A4])
+@pytest.mark.parametrize("M,O,K", [(514, 2560, 320), (777, 19100, 832)])
+def test_three_groups_over_a_partial_super_block(pkg, ctx, kind, M, O, K):
+    """Affine formats take every K that is a multiple of 64: 3 and 7 units a tile, the last of them half a unit in a
+    partial super-block, which the groups that skip it step over."""
+    test_three_groups_give_the_bits_of_two(pkg, ctx, kind, M, O, K)
+
+
+@pytest.mark.parametrize("kind", [orc.A8, orc.A4])
+def test_partial_super_blocks_match_the_oracle(pkg, ctx, kind):
+    """What the test above compares with, and three groups themselves, at a K of five blocks."""
+    rng = np.random.default_rng(kind)
+    M, O, K = 530, 130, 320
+    W = hp.make_weights(rng, kind, 1, O, K)
+    x = hp.f32_to_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    want = orc.gemv(W, x, M, f32=True)
+    L = lin_of(pkg, ctx, W)
+    dx = ctx.upload(x)
+    assert max_rel(L.matmul_wide(dx, M, out_f32=True).numpy(), want) <= TOL
+    assert max_rel(L.matmul_wide(dx, 256, out_f32=True).numpy(), want[:256]) <= TOL
+    L.free()
+
+
+@pytest.mark.parametrize("kind,K", [(orc.Q4K, 768), (orc.Q6K, 768), (orc.A8, 832), (orc.A4, 320), (orc.BF16, 320)])
+def test_several_matrices_in_a_launch_of_many_rows(pkg, ctx, kind, K):
+    """More than 512 rows of three matrices in one launch, more tiles than SMs, so that a CTA goes from one matrix to the
+    next: the bits of each matrix on its own."""
+    import ctypes as C
+    M, Os = 600, (9000, 130, 1000)
+    x = ctx.upload(hp.f32_to_bf16(np.random.default_rng(kind).standard_normal((M, K)).astype(np.float32)))
+    Ls = [pkg.Linear.random(ctx, kind, 1, O, K, 7 + O) for O in Os]
+    ys = [ctx.empty((M, O), np.float32) for O in Os]
+    ctx.check(ctx._lib.orn_gemm_multi(ctx.h, (C.c_void_p * 3)(*[l.h for l in Ls]), 3, x.ptr, M, (C.c_void_p * 3)(*[y.ptr for y in ys]), 1),
+              "orn_gemm_multi")
+    for L, y in zip(Ls, ys):
+        assert np.array_equal(y.numpy().view(np.uint32), L.matmul_wide(x, M, out_f32=True).numpy().view(np.uint32)), L.O
+        L.free()
