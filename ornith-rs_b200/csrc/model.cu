@@ -745,7 +745,7 @@ bool use_wide_prefill() {
   return v == 1;
 }
 // ORN_WIDE_EXACT=1 keeps the chunked prompt path but computes every product with the row-invariant
-// mat-vec kernels (groups of four rows; routed rows one by one): the chunk plumbing (conv windows,
+// kernels (an expert's rows together; one by one where they are longer than that takes): the chunk plumbing (conv windows,
 // KV append, causal attention over the chunk, the T-step recurrence, the expert sort) then has to
 // reproduce the 4-row windows bit for bit, which is how the tests check it
 bool wide_exact() {
@@ -811,7 +811,8 @@ constexpr int kWideMinRows = 64;    // from here on prompt rows come from the te
 // windows spread long caches, so behind many cached positions the windows stay.
 constexpr int kRowsMin = 13;
 constexpr int kRowsMaxKeys = 1024;
-constexpr int kRowsMaxK = 6144;  // longest row the grouped product takes in every format
+constexpr int kRowsMaxK = 6144;  // longest row the grouped row-invariant product takes in every format
+bool rows_held(const orn_config& c) { return c.hidden <= kRowsMaxK && c.expert_inter <= kRowsMaxK; }
 constexpr int kWideMaxRows = 8192;  // widest chunk of the wide path (the reference's default chunk is 2048, generate.rs:25)
 
 int wide_reserve(orn_model* m, int rows) {
@@ -886,11 +887,18 @@ int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, const M
   CK(wide_mm(m, moe.sh_down, w.sact, T, w.sy, ss));
   ORN_CHECK_CUDA(ctx, side.done());
   CK(f_route_sort(ctx, s, w.inds, rows, E, w.seg, w.seg + E + 1, w.perm));
-  CK(f_gather_rows(ctx, s, x, w.lhs, w.perm, rows, H, w.xs));
-  if (w.exact) {
+  const bool by_row = w.exact && !rows_held(c);  // no sorted rows: every route on its own, in (token, slot) order
+  if (by_row) {
+    iota_div_kernel<<<(rows + 255) / 256, 256, 0, s>>>(w.perm, nullptr, rows, 1);
+    CK(orn_launch_check(ctx, "iota_div"));
+    CK(k_gather_gemv(ctx, s, moe.sw_gate, x, w.lhs, w.inds, rows, w.eg));
+    CK(k_gather_gemv(ctx, s, moe.sw_up, x, w.lhs, w.inds, rows, w.eu));
+  } else if (w.exact) {
+    CK(f_gather_rows(ctx, s, x, w.lhs, w.perm, rows, H, w.xs));
     CK(k_grouped_gemv(ctx, s, moe.sw_gate, w.xs, w.seg, w.eg, nullptr, rows));
     CK(k_grouped_gemv(ctx, s, moe.sw_up, w.xs, w.seg, w.eu, nullptr, rows));
   } else {
+    CK(f_gather_rows(ctx, s, x, w.lhs, w.perm, rows, H, w.xs));
     QGemmGroup sorted{w.seg, nullptr, 0};
     if (moe.sw_gate->kind == moe.sw_up->kind) {  // gate and up of every expert in one launch
       const orn_linear* pl[2] = {moe.sw_gate, moe.sw_up};
@@ -903,7 +911,9 @@ int moe_block_wide(orn_model* m, const Moe& moe, const bf16_t* x, int T, const M
     }
   }
   CK(k_swiglu2(ctx, s, nullptr, nullptr, 0, nullptr, w.eg, w.eu, w.seg + E, I, w.eact));
-  if (w.exact) {
+  if (by_row) {
+    CK(k_gather_gemv(ctx, s, moe.sw_down, w.eact, w.perm, w.inds, rows, w.ey));
+  } else if (w.exact) {
     CK(k_grouped_gemv(ctx, s, moe.sw_down, w.eact, w.seg, w.ey, w.perm, rows));
   } else {
     QGemmGroup back{w.seg, w.perm, 0};
@@ -998,7 +1008,7 @@ int prefill(orn_model* m, orn_cache* cc, const uint32_t* prompt, int n, int pref
     int chunk = std::min(step, n - done - keep_last);
     int off = 0;
     const bool wide = chunk >= kWideMinRows;
-    const bool rows = chunk >= kRowsMin && cc->h_pos + chunk <= kRowsMaxKeys && m->cfg.hidden <= kRowsMaxK && m->cfg.expert_inter <= kRowsMaxK;
+    const bool rows = chunk >= kRowsMin && cc->h_pos + chunk <= kRowsMaxKeys && rows_held(m->cfg);
     bool one_piece = (wide || rows) && use_wide_prefill() && use_fused_env();
     if (one_piece) {
       chunk = std::min(chunk, kWideMaxRows);

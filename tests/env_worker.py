@@ -50,6 +50,15 @@ def main():
     out["tiny_after_prefill"] = sha(gm.forward(c, prompt[:2]).numpy())   # the caches it left behind
     c.free()
     gm.free()
+    # experts whose rows are longer than the grouped row-invariant product takes; the fused kernels refuse them, so that
+    # there are two row-invariant ways for a prompt of 70 rows
+    if os.environ.get("ORN_WIDE_EXACT") or os.environ.get("ORN_UNFUSED"):
+        gm = pkg.TextModel(ctx, hp.tiny_config(pkg.Config, n_layers=4, n_experts=4, top_k=2, expert_inter=7936))
+        gm.init_random(3)
+        c = gm.make_cache()
+        out["long_rows_sha"] = sha(gm.prefill(c, long_ids, prefill_step=2048, want_hidden=True).numpy())
+        c.free()
+        gm.free()
     # full-width layers, random-init on the device
     cfg = pkg.qwen35_config(max_ctx=96, n_layers=4)
     gm = pkg.TextModel(ctx, cfg)
