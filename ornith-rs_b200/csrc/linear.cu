@@ -433,6 +433,8 @@ int k_gather_gemv(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16
 // records come from HBM once (later groups find them in L1/L2) and every row is
 // computed with exactly the one-row arithmetic of gemv_kernel: the result bits
 // do not depend on how the rows are grouped.
+// What rows.cu does not take: affine 4-bit, row lengths of affine 8-bit and bfloat16 that
+// are no multiple of 256 or too long for its shared memory, more than a million features.
 // ---------------------------------------------------------------------------
 namespace {
 constexpr int kGroupThreads = 256;  // 8 warps
@@ -578,7 +580,7 @@ int k_grouped_gemv2(orn_ctx* ctx, cudaStream_t st, const orn_linear* L1, bf16_t*
   }
   const int rc = aligned_rows(ctx, xs, 16);
   if (rc != ORN_OK) return rc;
-  if (f_rows_ok(L1)) {
+  if (f_rows_ok(L1) && f_rows_ok(L2)) {
     const orn_linear* Ls[2] = {L1, L2};
     bf16_t* ys[2] = {y1, y2};
     return f_rows(ctx, st, Ls, ys, 2, xs, max_rows, seg);

@@ -788,7 +788,7 @@ int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear
     const bool beside = i > 0 && features <= 256;
     if (beside) ORN_CHECK_CUDA(ctx, side.start());
     const cudaStream_t on = beside ? side.stream() : st;
-    if (m->wide.exact && f_rows_ok(pl[0])) {
+    if (m->wide.exact && std::all_of(pl, pl + k, f_rows_ok)) {
       bf16_t* yb[4];
       for (int q = 0; q < k; ++q) yb[q] = static_cast<bf16_t*>(py[q]);
       CK(f_rows(ctx, on, pl, yb, k, x, T));

@@ -24,6 +24,7 @@ namespace {
 
 constexpr int kRowWarps = 4;  // per CTA
 constexpr size_t kRowSmem = 200 * 1024;
+constexpr int kRowMaxO = 65535 * 4 * kRowWarps;  // features of a launch: a grid's y, four features a warp
 
 struct RowsTile {
   const uint8_t* w;
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_rows(const __grid_constant__
 
 template <int KIND, int R, int MAX>
 int launch_rows(orn_ctx* ctx, cudaStream_t s, RowsParams& P, int E) {
-  const int rows = P.rows;
+  const int64_t rows = P.rows;
   for (int j = 0; j < P.njobs; ++j) {
     P.job[j].tile0 = P.tiles;
     P.tiles += (P.job[j].O + R - 1) / R;
@@ -171,9 +172,9 @@ int launch_rows(orn_ctx* ctx, cudaStream_t s, RowsParams& P, int E) {
   P.slots = E > 1 && P.units <= 32 ? 2 : 1;  // short rows: two tiles a warp
   int rc = orn_grant_smem(ctx, reinterpret_cast<const void*>(k_rows<KIND, R, MAX>), kRowSmem);
   if (rc != ORN_OK) return rc;
-  const int g = (rows + MAX - 1) / MAX, gx = E > 1 ? 1 : g * P.tiles > 8 * kRowWarps * ctx->sm_count ? (g + 1) / 2 : g;
+  const int64_t g = (rows + MAX - 1) / MAX, gx = E > 1 ? 1 : g * P.tiles > 8 * kRowWarps * ctx->sm_count ? (g + 1) / 2 : g;
   const int per = kRowWarps * P.slots;
-  k_rows<KIND, R, MAX><<<dim3(gx, (P.tiles + per - 1) / per, E), 32 * kRowWarps, (size_t)kRowWarps * P.slots * P.tile_bytes, s>>>(P);
+  k_rows<KIND, R, MAX><<<dim3((unsigned)gx, (P.tiles + per - 1) / per, E), 32 * kRowWarps, (size_t)kRowWarps * P.slots * P.tile_bytes, s>>>(P);
   return orn_launch_check(ctx, "k_rows");
 }
 // eight features a warp while their records stay below 18 KB, so that three CTAs fit an SM
@@ -185,7 +186,7 @@ template <int KIND, int MAX>
 int launch_max(orn_ctx* ctx, cudaStream_t s, RowsParams& P, int E, int features) {
   if (E > 1) return launch_r<KIND, 2>(ctx, s, P, E);
   // a narrow matrix: four or two rows a CTA, so that the launch reaches more SMs
-  const int ctas = (features + 31) / 32;
+  const int64_t ctas = (features + 31) / 32;
   if (ctas * ((P.rows + MAX - 1) / MAX) >= ctx->sm_count) return launch_r<KIND, MAX>(ctx, s, P, E);
   return ctas * ((P.rows + 3) / 4) >= ctx->sm_count ? launch_r<KIND, 4>(ctx, s, P, E) : launch_r<KIND, 2>(ctx, s, P, E);
 }
@@ -193,7 +194,7 @@ int launch_max(orn_ctx* ctx, cudaStream_t s, RowsParams& P, int E, int features)
 }  // namespace
 
 bool f_rows_ok(const orn_linear* L) {
-  return L->kind != ORN_A4 && L->K % 256 == 0 && L->E <= 65535 && L->O <= 1000000 /* tiles of 16 features in a grid's y */ && (size_t)(L->E > 1 ? 8 : 4) * kRowWarps * L->rec <= kRowSmem;
+  return L->kind != ORN_A4 && L->K % 256 == 0 && L->E <= 65535 && L->O <= kRowMaxO && (size_t)(L->E > 1 ? 8 : 4) * kRowWarps * L->rec <= kRowSmem;
 }
 
 // Up to four matrices of one format and row length over the same rows, or (seg given) one matrix over rows sorted by
@@ -217,7 +218,17 @@ int f_rows(orn_ctx* ctx, cudaStream_t s, const orn_linear* const* Ls, bf16_t* co
   P.njobs = n; P.K = L->K; P.rec = g.rec; P.b0 = g.b0; P.b1 = g.b1;
   P.xs = xs; P.seg = seg; P.rows = rows; P.row_map = row_map;
   int features = 0;
-  for (int j = 0; j < n; ++j) features += Ls[j]->O;
+  for (int j = 0; j < n; ++j) {
+    if (Ls[j]->O > kRowMaxO) ORN_FAIL(ctx, ORN_ERR_ARG, "rows: more features than a launch holds");
+    features += Ls[j]->O;
+  }
+  if (features > kRowMaxO) {  // (n > 1) one matrix after the other
+    for (int j = 0; j < n; ++j) {
+      const int rc = f_rows(ctx, s, Ls + j, ys + j, 1, xs, rows, seg, row_map);
+      if (rc != ORN_OK) return rc;
+    }
+    return ORN_OK;
+  }
   switch (L->kind) {
     case ORN_Q4K: P.units = L->K / 32; return launch_max<ORN_Q4K, 4>(ctx, s, P, L->E, features);
     case ORN_Q6K: P.units = L->K / 16; return launch_max<ORN_Q6K, 8>(ctx, s, P, L->E, features);

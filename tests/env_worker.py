@@ -59,6 +59,15 @@ def main():
         out["long_rows_sha"] = sha(gm.prefill(c, long_ids, prefill_step=2048, want_hidden=True).numpy())
         c.free()
         gm.free()
+        # a shared expert whose gate and up rows are together more features than a launch of the product of many rows holds
+        gm = pkg.TextModel(ctx, hp.tiny_config(pkg.Config, n_layers=1, hidden=1280, shared_inter=525056))
+        gm.init_random(3)
+        for name, o, k in (("gate_proj", 525056, 1280), ("up_proj", 525056, 1280), ("down_proj", 1280, 525056)):
+            gm.set_linear("layers.0.mlp.shared_expert." + name, pkg.Linear.random(ctx, pkg.BF16, 1, o, k, len(name)))
+        c = gm.make_cache()
+        out["many_features_sha"] = sha(gm.prefill(c, long_ids[:17], prefill_step=2048, want_hidden=True).numpy())
+        c.free()
+        gm.free()
     # full-width layers, random-init on the device
     cfg = pkg.qwen35_config(max_ctx=96, n_layers=4)
     gm = pkg.TextModel(ctx, cfg)

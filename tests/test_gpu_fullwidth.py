@@ -144,12 +144,15 @@ def test_chunked_prompt_path_is_exact_with_exact_products():
     the 4-row windows (ORN_NO_WIDE_PREFILL=1) bit for bit: hidden rows of the prompt and the hidden
     rows of a window decoded on top of the caches it left.  With the tensor-core products the same
     path differs from it by rounding only (tests/test_gpu_prefill.py).  Experts whose rows are longer
-    than the grouped row-invariant product takes go one row at a time (long_rows, against one kernel per op)."""
+    than the grouped row-invariant product takes go one row at a time (long_rows), and matrices that are more features than
+    a launch holds one after the other (many_features), both against one kernel per op."""
     narrow = _run_worker({"ORN_NO_WIDE_PREFILL": "1"})
     exact = _run_worker({"ORN_WIDE_EXACT": "1"})
     for key in ("tiny_prefill_sha", "tiny_after_prefill", "full_prefill_sha", "full_after_prefill"):
         assert exact[key] == narrow[key], key
-    assert exact["long_rows_sha"] == _run_worker({"ORN_UNFUSED": "1"})["long_rows_sha"]
+    unfused = _run_worker({"ORN_UNFUSED": "1"})
+    for key in ("long_rows_sha", "many_features_sha"):
+        assert exact[key] == unfused[key], key
     tensor = _run_worker({})
     assert tensor["tiny_prefill_sha"] != narrow["tiny_prefill_sha"]   # really another arithmetic
 

@@ -514,6 +514,19 @@ def test_gemv_of_rows_that_start_anywhere(pkg, ctx, kind):
     L.free()
 
 
+@pytest.mark.parametrize("M", [5, 9])
+def test_gemv_of_more_features_than_a_grid_holds(pkg, ctx, M):
+    """2.2 million features, more than a launch of rows.cu holds, go in groups of four rows.  Against the mat-vec of one
+    row."""
+    O, K = 2200001, 256
+    L = pkg.Linear.random(ctx, orc.Q4K, 1, O, K, 3)
+    x = hp.f32_to_bf16(np.random.default_rng(M).standard_normal((M, K)).astype(np.float32))
+    got = L.matmul(ctx.upload(x), M).numpy()
+    for m in range(M):
+        assert np.array_equal(got[m], L.matmul(ctx.upload(x[m:m + 1]), 1).numpy()[0]), m
+    L.free()
+
+
 @pytest.mark.parametrize("kind,K", [(orc.A4, 512), (orc.A8, 320), (orc.BF16, 72)])
 def test_gemv_of_many_rows_that_rows_cu_does_not_take(pkg, ctx, kind, K):
     """Affine 4-bit and row lengths off 256: groups of four rows, against the mat-vec of one row."""
