@@ -389,6 +389,10 @@ int k_gemv(orn_ctx* ctx, cudaStream_t st, const orn_linear* L, const bf16_t* x, 
            int out_f32) {
   int rc = aligned_rows(ctx, x, gemv_align(L));
   if (rc != ORN_OK) return rc;
+  // Five rows on are rows.cu's in every format it takes (groups of four rows / rows.cu, us, matrices cold in L2; 5 rows, 8
+  // rows: affine-8 8192 x 2048 22.8 / 17.0, 28.8 / 17.1, 2048 x 6144 22.0 / 16.4, 26.7 / 16.4; Q4_K 512 x 2048 12.7 / 6.2,
+  // 17.2 / 6.2, 2048 x 6144 26.5 / 15.3, 34.9 / 18.5; Q6_K 8192 x 2048 28.6 / 18.5, 34.8 / 18.5; bfloat16 8192 x 2048
+  // 22.5 / 18.5, 26.4 / 20.4, 2048 x 4096 18.5 / 16.7, 19.7 / 18.5).
   if (M > 4 && !out_f32 && f_rows_ok(L) && reinterpret_cast<uintptr_t>(x) % 16 == 0) {
     bf16_t* yb = static_cast<bf16_t*>(y);
     return f_rows(ctx, st, &L, &yb, 1, x, M);

@@ -177,18 +177,23 @@ int launch_rows(orn_ctx* ctx, cudaStream_t s, RowsParams& P, int E) {
   k_rows<KIND, R, MAX><<<dim3((unsigned)gx, (P.tiles + per - 1) / per, E), 32 * kRowWarps, (size_t)kRowWarps * P.slots * P.tile_bytes, s>>>(P);
   return orn_launch_check(ctx, "k_rows");
 }
-// eight features a warp while their records stay below 18 KB, so that three CTAs fit an SM
-template <int KIND, int MAX>
-int launch_r(orn_ctx* ctx, cudaStream_t s, RowsParams& P, int E) {
-  return 8 * P.rec <= 18 * 1024 ? launch_rows<KIND, 8, MAX>(ctx, s, P, E) : launch_rows<KIND, 4, MAX>(ctx, s, P, E);
-}
+// Eight features a warp while their records stay below 18 KB, so that three CTAs fit an SM, four of longer rows.
 template <int KIND, int MAX>
 int launch_max(orn_ctx* ctx, cudaStream_t s, RowsParams& P, int E, int features) {
-  if (E > 1) return launch_r<KIND, 2>(ctx, s, P, E);
+  const bool eight = 8 * P.rec <= 18 * 1024;
+  if (E > 1) return eight ? launch_rows<KIND, 8, 2>(ctx, s, P, E) : launch_rows<KIND, 4, 2>(ctx, s, P, E);
   // a narrow matrix: four or two rows a CTA, so that the launch reaches more SMs
   const int64_t ctas = (features + 31) / 32;
-  if (ctas * ((P.rows + MAX - 1) / MAX) >= ctx->sm_count) return launch_r<KIND, MAX>(ctx, s, P, E);
-  return ctas * ((P.rows + 3) / 4) >= ctx->sm_count ? launch_r<KIND, 4>(ctx, s, P, E) : launch_r<KIND, 2>(ctx, s, P, E);
+  const bool full = ctas * ((P.rows + MAX - 1) / MAX) >= ctx->sm_count, half = ctas * ((P.rows + 3) / 4) >= ctx->sm_count;
+  if (eight) return full ? launch_rows<KIND, 8, MAX>(ctx, s, P, E) : half ? launch_rows<KIND, 8, 4>(ctx, s, P, E) : launch_rows<KIND, 8, 2>(ctx, s, P, E);
+  // Long rows are tiles of 9 to 50 KB a warp, which every further group of rows copies again while few CTAs share an SM.
+  // Of affine-8 and bfloat16, the most bytes a weight, two rows a CTA do not pay for that (two / four rows, us: affine-8
+  // 2048 x 4096 8 rows 18.7 / 12.3, 2048 x 6144 5 rows 23.3 / 16.4; bfloat16 2048 x 4096 6 rows 27.6 / 16.7, where the
+  // mat-vec of four rows at a time takes 18.5), of the k-quants they do (Q6_K 2048 x 4096 5 rows 12.6 / 14.4, Q4_K 2048 x 6144
+  // 15.4 / 19.5).  bfloat16 is never better off with eight (four / eight: 8192 x 2048 5 rows 18.5 / 24.7, 50 rows 78 / 88).
+  constexpr bool kQuant = KIND == ORN_Q4K || KIND == ORN_Q6K;
+  constexpr int kMost = KIND == ORN_BF16 ? 4 : MAX, kLeast = kQuant ? 2 : 4;
+  return full ? launch_rows<KIND, 4, kMost>(ctx, s, P, E) : half ? launch_rows<KIND, 4, 4>(ctx, s, P, E) : launch_rows<KIND, 4, kLeast>(ctx, s, P, E);
 }
 
 }  // namespace

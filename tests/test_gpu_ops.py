@@ -477,12 +477,12 @@ def test_gated_delta_window_lengths(pkg, ctx, T):
 
 
 @pytest.mark.parametrize("kind", [orc.Q4K, orc.Q6K, orc.A8, orc.BF16])
-@pytest.mark.parametrize("M,O,K", [(5, 33, 256), (8, 257, 768), (13, 1030, 2048), (50, 300, 2048), (63, 36, 4096)])
+@pytest.mark.parametrize("M,O,K", [(5, 33, 256), (8, 257, 768), (13, 1030, 2048), (50, 300, 2048), (63, 36, 4096), (7, 2563, 4096), (16, 2563, 4096)])
 def test_gemv_of_many_rows_has_the_bits_of_the_one_row_kernel(pkg, ctx, kind, M, O, K):
     """rows.cu against the mat-vec of one row (which the tests above hold to the oracle bit for bit): groups of eight,
     four and two rows with every remainder, fewer units than lanes (K = 256) and a last round that is not full (768),
-    features off the eight of a warp, narrow matrices (two rows a CTA) and wide ones, rows too long for eight
-    features."""
+    features off the eight of a warp, narrow matrices (two rows a CTA, four where rows are too long for eight
+    features a warp) and wide ones."""
     rng = np.random.default_rng(17 * kind + M + O)
     L = pkg.Linear.random(ctx, kind, 1, O, K, 3)
     x = hp.f32_to_bf16(rng.standard_normal((M, K)).astype(np.float32))
