@@ -165,12 +165,14 @@ def test_gemm_edges_of_its_tiles_and_splits(pkg, ctx, kind, M, O, K):
 
 
 @pytest.mark.parametrize("kind", [orc.Q4K, orc.Q6K, orc.A8, orc.A4])
-@pytest.mark.parametrize("M,O,K", [(514, 2560, 256), (777, 19100, 768), (1100, 19072, 1280)])
+@pytest.mark.parametrize("M,O,K", [(514, 2560, 256), (514, 19100, 256), (600, 19072, 512), (777, 19100, 768), (1100, 19072, 1280)])
 def test_three_groups_give_the_bits_of_two(pkg, ctx, kind, M, O, K):
-    """More than 512 rows: three groups take the units of K in turn, on and on over the tiles of a CTA (more tiles
-    than SMs), with 2, 6 and 10 units a tile: every group starts tiles on either half of a super-block and skips
-    super-blocks in between.  Against the same rows 256 at a time, which two groups compute without a split of K here
-    (fewer than eight K blocks, or more feature tiles than SMs) and the tests above hold to the oracle."""
+    """More than 512 rows: three groups take the units of K in turn, on and on over the tiles of a CTA.  Feature counts
+    of 19072 and more are more tiles than SMs, with 2, 4, 6 and 10 units a tile: with 2, a group has no unit at all in
+    every third tile; with 2, 4 and 10 its first unit moves from tile to tile, with 6 every tile starts alike.  (The first
+    size is one tile a CTA, whose third group has nothing.)  Against the same rows 256 at a time, which two groups
+    compute without a split of K here (fewer than eight K blocks, or more feature tiles than SMs) and the tests above hold to the
+    oracle."""
     rng = np.random.default_rng(91 * kind + M + O)
     L = pkg.Linear.random(ctx, kind, 1, O, K, 5)
     x = hp.f32_to_bf16(rng.standard_normal((M, K)).astype(np.float32))

@@ -64,6 +64,32 @@ def test_short_chunks_have_the_bits_of_the_four_row_windows(pkg, ctx, n, step):
     m.free()
 
 
+@pytest.mark.parametrize("prefix,n", [(449, 63), (470, 60), (512, 13), (974, 50), (962, 63)])
+def test_short_chunks_behind_cached_positions(pkg, ctx, prefix, n):
+    """A chunk of 13 to 63 rows behind a chunk of the tensor cores, against windows of four rows behind the same: up to 512
+    keys, across them (where the windows' attention spreads over more CTAs) and past them, up to 1024 keys in one piece and
+    from 1025 on in windows.  Hidden rows, and a window decoded behind them."""
+    m = pkg.TextModel(ctx, pkg.qwen35_config(max_ctx=1088, n_layers=4))
+    m.init_random(9)
+    ids = np.random.default_rng(prefix).integers(0, m.cfg.vocab, prefix + n + 3).astype(np.uint32)
+    c = m.make_cache()
+    got = []
+    for step in (4, 2048):
+        c.reset()
+        m.prefill(c, ids[:prefix], prefill_step=2048)
+        l0 = ctx.launches()
+        rows = m.prefill(c, ids[prefix:prefix + n], prefill_step=step, want_hidden=True).numpy()
+        launches = ctx.launches() - l0
+        assert c.offset == prefix + n
+        got.append((rows, m.forward(c, ids[prefix + n:]).numpy(), launches))
+    (want, behind, in_windows), (rows, after, in_one) = got
+    assert np.array_equal(rows, want)
+    assert np.array_equal(after, behind)
+    assert (in_one < in_windows) == (prefix + n <= 1024)
+    c.free()
+    m.free()
+
+
 @pytest.mark.parametrize("nth", [1, 41])
 def test_a_short_chunk_needs_no_workspace(pkg, ctx, nth):
     """The first or the last allocation of the one-piece path's workspace fails: a chunk of 13 to 63 rows goes in windows of
