@@ -537,12 +537,15 @@ __global__ void mtp_advance_kernel(int* mtp_pos, const int* keep, int B, int bas
 // further row of the other path little.  Fused / one kernel per op, ms per window at 700 cached positions: 6 rows
 // 6.3 / 6.7, 8 rows 7.2 / 7.5, 10 rows 9.6 / 8.5, 12 rows 10.7 / 9.0, 14 rows 12.9 / 9.9 (at 3500 positions 8 rows 8.3 /
 // 8.1, 14 rows 14.8 / 11.2); 16 rows take 7.0 on the tensor cores, whose products are not row-invariant.  A draft is one
-// layer and the head, where the fused kernels stay ahead: 5 rows 556 / 653 us, 7 rows 648 / 689; from there on the two
-// are level, and a cycle of 12 sequences at 1500 positions takes 9.80 ms with fused drafts, 9.95 without.
+// layer and the head.  The fused kernels are ahead up to 7 rows (5 rows 542 / 612 us, 7 rows 633 / 644) and level at 8.  Above,
+// the draft of a model of four layers takes less with one kernel per op (10 rows 890 / 802, 15 rows 1230 / 1052), but the whole cycle
+// of the forty-layer model, drafts fused / one kernel per op, is the shorter with fused ones: 9, 10, 12, 15 sequences 8.60 /
+// 8.77, 8.97 / 9.14, 9.60 / 9.77, 10.66 / 10.71 ms at 700 positions, 9.02 / 9.13, 9.51 / 9.69, 10.22 / 10.36, 11.28 / 11.27
+// at 4000 (medians of 60, quartiles within 0.03).
 constexpr int kSmallRows = 8, kSmallDraft = 15;
 // The re-encode (one row per sequence, keys and values only) has little to read per launch, and every CTA of the
-// fused kernels rebuilds the norms of both of its inputs: up to this many sequences.  A commit, fused / one kernel
-// per op: one sequence 70 / 80 us, two 79 / 86, four 98 / 90, seven 138 / 112, fifteen 230 / 166.
+// fused kernels rebuilds the norms of both of its inputs: up to this many sequences.  A commit at 700 positions, fused /
+// one kernel per op: one sequence 54 / 69 us, two 66 / 70, three 75 / 75, four 87 / 73, seven 122 / 86, fifteen 213 / 102.
 constexpr int kSmallEncode = 2;
 
 // the fused kernels serve every part of the model at these rows, on this GPU alone

@@ -805,8 +805,8 @@ int wide_mm_multi(orn_model* m, std::initializer_list<std::pair<const orn_linear
 constexpr int kWideMinRows = 64;    // from here on prompt rows come from the tensor cores (the reference's own
                                     // crossover, kquant.rs MM_ROW_LIMIT, is 16 on its hardware)
 // Shorter chunks have the bits of the four-row windows whatever way they go.  From 13 rows on all of them go through the
-// wide path's launches with row-invariant products (rows.cu), which read a layer's weights once, an expert's for all its
-// rows.  Windows / one piece, ms for the whole model: 8 rows 6.3 / 8.0, 12 rows 9.4 / 9.3, 16 rows 12.5 / 10.6, 24 rows
+// wide path's launches with row-invariant products (rows.cu), for which a layer's weights come from HBM once (each group of
+// rows copies them again out of L2), an expert's for all its rows.  Windows / one piece, ms for the whole model: 8 rows 6.3 / 8.0, 12 rows 9.4 / 9.3, 16 rows 12.5 / 10.6, 24 rows
 // 18.7 / 12.7, 48 rows 37.5 / 19.6, 63 rows 49.6 / 23.5.  Its attention walks a row's keys in one CTA, where the
 // windows spread long caches, so behind many cached positions the windows stay.
 constexpr int kRowsMin = 13;

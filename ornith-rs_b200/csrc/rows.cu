@@ -11,8 +11,10 @@
 //   * a warp owns its R features: their records lie behind one another and come by cp.async into the warp's own piece
 //     of shared memory.  Warps never meet; two to four CTAs of four warps on an SM cover each other's copies.
 // FMA work of a unit of 16 weights, 8 rows x 8 features: 512 packed multiply-adds of 1024 cycles in about 1500.
-// 50 rows, 2048 -> 12288 affine-8: 110 us, half of that bound (255 registers leave two warps per scheduler).  What it
-// replaced there read the weights once per four rows, 13 launches of about 17 us.
+// 50 rows, 2048 -> 12288 affine-8: 110 us.  Its multiply-adds are 31 % of what the float32 pipe could do in that time (34 %
+// with the rows padded to 56), the pipe is active 55 % of the cycles, issue slots are 53 % busy: 255 registers leave two
+// warps a scheduler, whose chains of dependent packed multiply-adds leave the rest empty.  What it replaced there
+// read the weights once per four rows, 13 launches of about 17 us.
 #include <algorithm>
 
 #include "fused.h"
